@@ -47,7 +47,7 @@ def build(ref: bool | None = None, fast: bool = False) -> None:
     if fast:
         subprocess.run(["make", "-s", "-C", HERE, "fast"], check=True)
     if ref is None:
-        ref = os.path.isdir(REF_SRC)
+        ref = os.path.isdir(os.path.join(REF_SRC, "00_CommonFiles"))   # an empty mount point holds no sources
     if ref:
         subprocess.run(["make", "-s", "-C", HERE, "ref", "ref_fast", f"REF={REF_SRC}"], check=True)
         tt = os.path.isdir(os.path.join(REF_SRC, "02_Transport_Equation"))
