@@ -294,20 +294,19 @@ long long fg_launch_count(void);
  * record events or order their own work around it. */
 void *fg_system_stream(const fg_system *s);
 
-/* Time the batched EBE matvec of these systems alone: reps back-to-back
- * matvecs (all colours) of V[0] into the Arnoldi work vector, in FP64
+/* Time the batched Krylov matvec of these systems alone: reps back-to-back
+ * matvecs (the assembled operator) of V[0] into a work vector, in FP64
  * (precision 64) or FP32 (32), timed with CUDA events on the first
  * system's stream.  *ms_per_matvec receives the mean; *bytes the
- * algorithmic bytes of one matvec: nel*(S*S*w + S*4) + 2*n*w summed over
- * the systems.  Requires a previous solve (workspace) on every system. */
+ * algorithmic bytes of one matvec: slots*(ndof*ndof*w + 4) + 2*n*w summed
+ * over the systems (slots: coupled node pairs, one column each).  Requires a previous solve (workspace) on every system. */
 int fg_bench_matvec(fg_system *const *systems, int count, int precision, int reps,
                     double *ms_per_matvec, double *bytes);
 
 /* Autotuner: times candidate launch shapes of a batch on the batch itself
  * (one restart cycle each, CUDA events on the first system's stream) --
  * the dof-part size of the Krylov kernels (256 ... 16384 dofs) and, for
- * 3x3 blocks in FP32, the matvec kernel (bulk-copy pipeline or register
- * kernel) -- and keeps the fastest for the process, keyed by (block size,
+ * 3x3 blocks in FP32, the rows per thread of the matvec -- and keeps the fastest for the process, keyed by (block size,
  * precision, batch-size class floor(log2(batch dofs))).  Every later batch
  * of that key (fg_solve_batch, fg_solve_resident, the request server) uses
  * it.  The systems need resident right-hand sides (fg_transport_prepare or
@@ -317,8 +316,8 @@ int fg_bench_matvec(fg_system *const *systems, int count, int precision, int rep
  * launch shapes are fixed). */
 typedef struct {
     int part_dofs;        /* dofs per part of the Krylov kernels            */
-    int mv3_pipeline;     /* 3x3 FP32 matvec: 1 bulk-copy pipeline, 0 the
-                             register kernel (other blocks: 1)              */
+    int mv3_pipeline;     /* matvec: 1 four rows per thread in batches of
+                             more than a wave of rows, 0 always one         */
     double ms_per_cycle;  /* one restart cycle of the batch with it         */
     int from_cache;       /* taken from the cache, not measured now         */
     int candidates;       /* launch shapes timed                            */

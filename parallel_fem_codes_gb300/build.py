@@ -27,6 +27,7 @@ UNITS = [
     ("meshio.cpp", []),
     ("system.cu", []),
     ("krylov.cu", []),
+    ("rows.cu", []),
     ("setup.cu", ["-fmad=false"]),
     ("noalloc.cu", []),
     ("server.cu", []),

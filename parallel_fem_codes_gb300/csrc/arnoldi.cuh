@@ -252,7 +252,7 @@ __device__ __forceinline__ double part_update(const SysDev &D, const DChunk &k, 
     return nrm;
 }
 
-// pass 1: w = M^-1 t (t cleared), h1_j = <v_j, w>, j = 0..i
+// pass 1: h1_j = <v_j, w>, j = 0..i (w = M^-1 A v_i from the matvec)
 template <typename T>
 __global__ void __launch_bounds__(kThreads)
 k_dots1(const SysDev *__restrict__ sys, const DChunk *__restrict__ ch, const int *__restrict__ nch, int i)
@@ -264,24 +264,7 @@ k_dots1(const SysDev *__restrict__ sys, const DChunk *__restrict__ ch, const int
         const DChunk k = ch[c];
         const SysDev &D = sys[k.sys];
         if (!D.st->in_cycle) continue;
-        T *w = (T *)D.w, *t = (T *)D.t;
-        const T *invd = sizeof(T) == 8 ? (const T *)D.invd64 : (const T *)D.invd32;
-        constexpr int N = Pk<T>::N;
-        typename Pk<T>::type zero;
-#pragma unroll
-        for (int c = 0; c < N; ++c) zero.v[c] = (T)0;
-        for (int q = k.d0 + threadIdx.x * N; q < k.d1; q += blockDim.x * N) {
-            if (!precond_separate(D.precond)) {
-                auto tv = ld_pk(t + q);
-                if (D.precond == FG_PRECOND_DIAG) {
-                    auto iv = ld_pk(invd + q);
-#pragma unroll
-                    for (int c = 0; c < N; ++c) tv.v[c] *= iv.v[c];
-                }
-                st_pk(w + q, tv);
-            }
-            st_pk(t + q, zero);
-        }
+        const T *w = (const T *)D.w;
         __syncthreads();
         part_dots<T>(D, k, i, w, red);
         __syncthreads();
@@ -294,7 +277,7 @@ k_dots1(const SysDev *__restrict__ sys, const DChunk *__restrict__ ch, const int
 }
 
 // Mixed-precision pass 1 (classical Gram-Schmidt with a Gram correction):
-// w = M^-1 t (t cleared), s = V^T w and the new column g = V^T v_i of the
+// s = V^T w (w = M^-1 A v_i) and the new column g = V^T v_i of the
 // basis' Gram matrix G = V^T V in one sweep.  The last part forms
 // c = s + (s - G s): the coefficients of the two classical passes of CGS2
 // (h1 = s, h2 = V^T (w - V s) = s - G s) with the second one taken from G
@@ -311,24 +294,7 @@ k_dots1g(const SysDev *__restrict__ sys, const DChunk *__restrict__ ch, const in
         const DChunk k = ch[c];
         const SysDev &D = sys[k.sys];
         if (!D.st->in_cycle) continue;
-        T *w = (T *)D.w, *t = (T *)D.t;
-        const T *invd = sizeof(T) == 8 ? (const T *)D.invd64 : (const T *)D.invd32;
-        constexpr int N = Pk<T>::N;
-        typename Pk<T>::type zero;
-#pragma unroll
-        for (int c = 0; c < N; ++c) zero.v[c] = (T)0;
-        for (int q = k.d0 + threadIdx.x * N; q < k.d1; q += blockDim.x * N) {
-            if (!precond_separate(D.precond)) {
-                auto tv = ld_pk(t + q);
-                if (D.precond == FG_PRECOND_DIAG) {
-                    auto iv = ld_pk(invd + q);
-#pragma unroll
-                    for (int c = 0; c < N; ++c) tv.v[c] *= iv.v[c];
-                }
-                st_pk(w + q, tv);
-            }
-            st_pk(t + q, zero);
-        }
+        const T *w = (const T *)D.w;
         __syncthreads();
         part_dots2<T, TV>(D, k, i, w, red);
         __syncthreads();

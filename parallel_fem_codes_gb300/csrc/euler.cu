@@ -679,8 +679,8 @@ int euler_mfdd_assemble_device(fg_system *s, const fg_euler_coeffs *c, const dou
     count_launches(1);
     if ((r = gather_residual(s, s->Fe.as<double>(), F_dev, st))) return r;
     s->blocks_ok = true;
-    s->csr_dirty = true;
-    return convert_blocks(s, st);
+    blocks_changed(s);
+    return FG_OK;
 }
 
 int euler_bubble_correct_device(fg_system *s, const double *Da_dev, double coef, double *DaB_dev, cudaStream_t st)
@@ -747,8 +747,8 @@ int euler_assemble_device(fg_system *s, const fg_euler_coeffs *c, const double *
     int r = gather_residual(s, s->Fe.as<double>(), R_dev, st);
     if (r) return r;
     s->blocks_ok = true;
-    s->csr_dirty = true;
-    return convert_blocks(s, st);
+    blocks_changed(s);
+    return FG_OK;
 }
 
 }  // namespace fg

@@ -51,15 +51,8 @@ struct Topology {
     std::vector<int> dofs;       // patch-local dof -> internal dof, bit 31 = shared with another patch
     std::vector<unsigned short> lm16;    // nel*S local indices (internal order), 0xFFFF = sink
     // x segment of each patch: its dofs lie in [xlo, xlo + xlen) (xlo and
-    // xlen multiples of 8, xlen <= kPatchXCap); lmx16: per element vertex
-    // its dof's position in that segment (0xFFFF = sink), for the matvec
-    // that copies the segment whole instead of gathering x dof by dof
+    // xlen multiples of 8); a 3x3 patch closes before xlen passes kPatchXCap
     std::vector<int> pt_xlo, pt_xlen;
-    std::vector<unsigned short> lmx16;
-    // 3x3: per patch one 16-byte aligned index blob (x-segment positions
-    // [3][W], dof list, incidence lists) at byte offset pt_boff[p]
-    std::vector<long long> pt_boff;
-    std::vector<unsigned char> blob;
     std::vector<int> pc_ptr, pc_list;    // patches grouped by patch colour
     // per-patch incidence lists: for patch p, at incl[pt_inc[p]] the list
     // starts (pnd + 1 entries) of each local dof, then the staged product
@@ -67,7 +60,15 @@ struct Topology {
     // element order; both parts padded to 8 entries (16-byte copies)
     std::vector<int> pt_inc;
     std::vector<unsigned short> incl;
+    // pattern of the assembled operator (rows.cu): units (ndof = 1: internal
+    // dofs, else nodes) in slices of kRowSlice; slice s holds the slots
+    // [rw_off[s], rw_off[s+1]), slot k of its unit l at rw_off[s] + k *
+    // kRowSlice + l, value = coupled unit (kRowPad set: unused slot)
+    int nunits = 0;
+    std::vector<int> rw_off, rw_col;
 };
+constexpr int kRowSlice = 32;
+constexpr int kRowPad = (int)0x80000000;
 
 // Assembled CSR form of a system (csr_Initialization.c), rows and columns
 // in the internal (RCM) numbering, which is the reference's CSR numbering.
@@ -179,8 +180,12 @@ struct SysDev {
     const unsigned short *pt_col;
     const int *pt_inc;                 // per-patch incidence lists (3x3 matvec)
     const unsigned short *incl;
-    const unsigned char *blob;         // per-patch index blobs (3x3 bulk-copy matvec)
     int maxdof;
+    // assembled operator in slices of units (rows.cu)
+    int nunits;
+    const int *rw_off, *rw_col;
+    const double *rw64;
+    const float *rw32;
     // assembled CSR operator and ILU(0) (op == 1)
     int op, csr_w;
     const int *csr_ia, *csr_ja, *csr_diag;
@@ -205,7 +210,7 @@ struct SysDev {
     const int *sp_piv;
     double *sp_g, *sp_h, *sp_x;
     const double *A64;         // [S*S][nel_pad]
-    const float *A32;
+    const float *A32;          // FP32 copy (3x3: blocked per patch), made when an FP32 element matvec asks for it
     const double *invd64;      // n_pad
     const float *invd32;
     const int *node_dof;       // [nnodes][ndof]
@@ -229,11 +234,6 @@ constexpr int kPartStride = 64;    // doubles per part (>= kmax + 2, kmax <= 60)
 __host__ __device__ constexpr bool precond_separate(int p) { return p >= 2; }
 
 struct EChunk { int sys, e0, e1; };
-// One 3x3 patch of a batched matvec launch for the bulk-copy pipeline:
-// system, first element, index-blob offset (16-byte units) and size
-// (bytes), x segment start, and packed counts (elements | dofs << 16,
-// incidence entries | x segment length << 16).
-struct alignas(32) MvRec { int sys, pe0, boff16, bsize, xlo, pn, nx, pad; };
 struct DChunk { int sys, part, d0, d1; };
 struct NChunk { int sys, n0, n1; };
 

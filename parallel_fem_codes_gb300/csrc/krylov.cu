@@ -10,9 +10,9 @@
 // (fixed part order, "last part reduces"), instead of 2(i+1) dependent
 // reductions.
 //
-// Work decomposition.  A batch holds any number of systems.  Element work
-// is cut into patches (grouped by patch colour), dof work into parts per
-// system; every
+// Work decomposition.  A batch holds any number of systems.  The operator
+// is the assembled one (rows.cu), cut into unit chunks, dof work into parts
+// per system; every
 // kernel walks its chunk table with a grid-stride loop and skips systems
 // that are not active.  A system's partial sums depend only on its own
 // parts, so a result is bit-identical whether the system is solved alone
@@ -490,263 +490,6 @@ k_ebe_mv3(const SysDev *__restrict__ sys, const EChunk *__restrict__ ch, const i
     }
 }
 
-// ---------------------------------------------------------------- 3x3 matvec, bulk-copy pipeline
-// The FP32-block 3x3 matvec of the batched engine as a warp-specialised
-// pipeline, one CTA of 1024 threads per SM.  Warp 0 is the producer: for
-// each patch of its CTA it waits until a stage of the three-stage
-// shared-memory ring is free, then one lane copies into it, with 1-D bulk
-// copies (cp.async.bulk, completion counted on the stage's "full"
-// mbarrier), everything the patch needs: its nine block rows, the three
-// rows of x-segment positions of its elements' vertices, its dof list and
-// incidence lists, and x itself -- the dofs of a patch lie in one short
-// segment of x (one contiguous band in the RCM numbering), so x arrives
-// as one copy instead of a dof-by-dof gather.  Warps 1..31 consume the
-// patches in order, with no global loads:
-//   products   each thread forms its elements' three row products from the
-//              staged blocks and x, and writes them over the first three
-//              block rows of its own elements (slots it alone reads);
-//   sums       the thread that owns a dof adds the products listed for it,
-//              in the fixed order of its incidence list, and writes it once
-//              (plain store, or red.add for a dof shared with patches of
-//              other colours, which run in other launches);
-// so each dof gets the same sum, in the same order, as in k_ebe_mv3.  The
-// consumers then release the stage on its "empty" mbarrier.
-// Every mbarrier wait is bounded (kMbarWaitCycles, ~2 s).  A consumer wait
-// that runs out marks the patch's system FG_ERR_TIMEOUT, stops the
-// producer, waits (bounded) for the copies in flight and ends the CTA; the
-// producer gives up on a free stage the same way.
-constexpr int kMv3pThreads = 1024;
-constexpr int kMv3pStages = 3;
-constexpr int kMv3pConsumers = kMv3pThreads - 32 * kMv3pStages;
-constexpr int kMv3pDofCap = 1536;                       // dofs per patch (the patch cap)
-constexpr int kMv3pIncCap = ((kMv3pDofCap + 1 + 7) / 8) * 8 + 3 * patch_elems(3);
-constexpr long long kMbarWaitCycles = 4000000000LL;     // ~2 s at 2 GHz
-// per-stage facts the producer leaves for the consumers (pne < 0: no patch)
-struct Mv3pMeta {
-    int pne, pnd, n, sys;
-    void *Y;
-    float vsci;
-    int W;             // block row / staged product row length (pne rounded up to 16)
-};
-template <typename TX>
-struct Mv3pSmem {
-    static constexpr int PE = patch_elems(3);
-    static constexpr size_t a = 0;                                   // [9][W] float, W <= PE
-    static constexpr size_t b = a + 9 * (size_t)PE * 4;              // index blob: [3][W] ushort, dofs, incidence
-    static constexpr size_t x = b + 6 * (size_t)PE + 4 * (size_t)kMv3pDofCap + 2 * (size_t)kMv3pIncCap;
-    static constexpr size_t meta = (x + (size_t)kPatchXCap * sizeof(TX) + 15) / 16 * 16;
-    static constexpr size_t stage = (meta + sizeof(Mv3pMeta) + 127) / 128 * 128;
-    static constexpr size_t full = kMv3pStages * stage;             // kMv3pStages mbarriers
-    static constexpr size_t empty = full + 8 * kMv3pStages;          // kMv3pStages mbarriers
-    static constexpr size_t abort = empty + 8 * kMv3pStages;         // consumers gave up
-    static constexpr size_t total = abort + 16;
-    static_assert(total <= 227 * 1024, "3x3 pipeline exceeds shared memory");
-    static_assert(x % 16 == 0, "x segment must stay 16-byte aligned");
-};
-static_assert(patch_elems(3) % 16 == 0, "patch rows must stay 16-byte aligned");
-
-__device__ __forceinline__ unsigned smem_u32(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void mbar_init(unsigned bar, unsigned count)
-{
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(bar), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(unsigned bar)
-{
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(unsigned bar, unsigned bytes)
-{
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void bulk_g2s(unsigned dst, const void *src, unsigned bytes, unsigned bar)
-{
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n"
-                 ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
-}
-// true when the phase with this parity has completed; false after ~2 s
-__device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity)
-{
-    const long long t0 = clock64();
-    for (;;) {
-        unsigned ok;
-        asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-                     " selp.u32 %0, 1, 0, p;\n}\n" : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-        if (ok) return true;
-        if (clock64() - t0 > kMbarWaitCycles) return false;
-    }
-}
-// barrier 1 over the consumer warps only; returns true in every consumer
-// thread when any of them passed true
-__device__ __forceinline__ bool consumers_sync_or(bool v)
-{
-    unsigned r;
-    asm volatile("{\n .reg .pred p, q;\n setp.ne.u32 p, %1, 0;\n bar.red.or.pred q, 1, %2, p;\n"
-                 " selp.u32 %0, 1, 0, q;\n}\n" : "=r"(r) : "r"((unsigned)v), "n"(kMv3pConsumers) : "memory");
-    return r != 0;
-}
-__device__ __forceinline__ void consumers_sync()
-{
-    asm volatile("bar.sync 1, %0;\n" ::"n"(kMv3pConsumers) : "memory");
-}
-// a staged x entry in FP32 (an FP16 basis vector is stored as sigma v)
-template <typename TX> __device__ __forceinline__ float staged_x(TX v, float vsci)
-{
-    if constexpr (std::is_same<TX, __half>::value) return __half2float(v) * vsci;
-    else return (float)v;
-}
-
-template <typename TX, typename TY>
-__global__ void __launch_bounds__(kMv3pThreads, 1)
-k_ebe_mv3p(const SysDev *__restrict__ sys, const MvRec *__restrict__ rec, const int *__restrict__ nch,
-           int gate, int in_sel, int out_sel, int step, const TX *aux_in, TY *aux_out)
-{
-    extern __shared__ __align__(128) unsigned char mv3p_smem[];
-    using L = Mv3pSmem<TX>;
-    using TA = float;
-    constexpr int NC = kMv3pConsumers, ST = kMv3pStages;
-    constexpr unsigned short kSink = 0xFFFF;
-    volatile int *s_abort = reinterpret_cast<volatile int *>(mv3p_smem + L::abort);
-    const unsigned full0 = smem_u32(mv3p_smem + L::full), empty0 = smem_u32(mv3p_smem + L::empty);
-    const int total = *nch;
-    const int tid = threadIdx.x;
-
-    if (tid == 0) {
-        for (int s = 0; s < ST; ++s) {
-            mbar_init(full0 + 8u * s, 1);
-            mbar_init(empty0 + 8u * s, 1);
-            reinterpret_cast<Mv3pMeta *>(mv3p_smem + s * L::stage + L::meta)->sys = 0;
-        }
-        *s_abort = 0;
-        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-    }
-    __syncthreads();
-
-    // ------------------------------------------------ producers (warps 0..ST-1)
-    // Producer warp w fills stage w with the CTA's patches k = w, w + ST,
-    // ...: it waits until the consumers released the stage, then lane 0
-    // arms the stage's full barrier and issues the patch's three bulk
-    // copies (blocks, index blob, x segment).  The next patch's record and
-    // system fields are loaded before the wait, so they overlap it.  A
-    // patch whose system is gated off is passed as an empty stage; past the
-    // CTA's last patch the producer leaves an end marker and stops.
-    if (tid < 32 * ST) {
-        if (tid & 31) return;
-        const int w = tid >> 5, s = w;
-        unsigned char *stg = mv3p_smem + s * L::stage;
-        Mv3pMeta *meta = reinterpret_cast<Mv3pMeta *>(stg + L::meta);
-        const unsigned full = full0 + 8u * s;
-        for (int k = w;; k += ST) {
-            const long long c = blockIdx.x + (long long)k * gridDim.x;
-            const bool have = c < total;
-            MvRec r = have ? rec[c] : MvRec{};
-            const SysDev &D = sys[r.sys];
-            const bool live = have && gated(D, gate);
-            const int pne = r.pn & 0xFFFF, pnd = r.pn >> 16, xlen = r.nx >> 16;
-            const int W = (pne + 15) & ~15;
-            const TX *X = in_sel == 0 ? (const TX *)D.x
-                        : in_sel == 1 ? (const TX *)D.V + (size_t)step * D.n_pad
-                    : in_sel == 3 ? (const TX *)D.r64 : aux_in;
-            void *Y = out_sel == 0 ? (void *)D.t64 : out_sel == 1 ? (void *)D.t : (void *)aux_out;
-            const int n = D.n;
-            const float vsci = D.vsci;
-            const TA *A = D.A32 + 9 * (size_t)r.pe0;
-            const unsigned char *blob = D.blob + 16 * (size_t)r.boff16;
-            if (k >= ST && !mbar_wait(empty0 + 8u * s, (unsigned)((k / ST - 1) & 1))) return;
-            if (*s_abort) return;
-            if (!have) {                                   // end of this CTA's patches
-                meta->pne = -1;
-                mbar_arrive(full);
-                return;
-            }
-            meta->sys = r.sys;
-            if (!live) {                                   // gated off: nothing to do
-                meta->pne = 0;
-                meta->pnd = 0;
-                mbar_arrive(full);
-                continue;
-            }
-            const unsigned ra = 9u * (unsigned)W * 4u, rb = (unsigned)r.bsize;
-            const unsigned rx = (unsigned)xlen * (unsigned)sizeof(TX);
-            meta->pne = pne;
-            meta->pnd = pnd;
-            meta->n = n;
-            meta->Y = Y;
-            meta->vsci = vsci;
-            meta->W = W;
-            mbar_expect_tx(full, ra + rb + rx);
-            bulk_g2s(smem_u32(stg + L::a), A, ra, full);
-            bulk_g2s(smem_u32(stg + L::b), blob, rb, full);
-            bulk_g2s(smem_u32(stg + L::x), X + r.xlo, rx, full);
-        }
-    }
-
-    // ------------------------------------------------ consumers (warps ST..31)
-    const int ct = tid - 32 * ST;
-    for (int j = 0;; ++j) {
-        const int s = j % ST;
-        unsigned char *stg = mv3p_smem + s * L::stage;
-        const Mv3pMeta *meta = reinterpret_cast<const Mv3pMeta *>(stg + L::meta);
-        const bool ok = mbar_wait(full0 + 8u * s, (unsigned)((j / ST) & 1));
-        const int pne = ok ? meta->pne : 0;
-        const int W = meta->W;
-        TA *sa = reinterpret_cast<TA *>(stg + L::a);
-        const unsigned short *sl = reinterpret_cast<const unsigned short *>(stg + L::b);
-        const TX *sx = reinterpret_cast<const TX *>(stg + L::x);
-        const float vsci = meta->vsci;
-        // products over the block rows 0..2 of the element's own slots
-        for (int q = ct; q < pne; q += NC) {
-            TA av[9], xv[3];
-#pragma unroll
-            for (int m = 0; m < 9; ++m) av[m] = sa[m * W + q];
-#pragma unroll
-            for (int a = 0; a < 3; ++a) {
-                const unsigned short li = sl[a * W + q];
-                xv[a] = li == kSink ? (TA)0 : staged_x(sx[li], vsci);
-            }
-#pragma unroll
-            for (int r = 0; r < 3; ++r) {
-                TA acc = av[3 * r] * xv[0];
-                acc += av[3 * r + 1] * xv[1];
-                acc += av[3 * r + 2] * xv[2];
-                sa[r * W + q] = acc;
-            }
-        }
-        if (consumers_sync_or(!ok)) {
-            // give up: record the timeout, stop the producer, wait (bounded)
-            // for the copies that may be in flight into the stages
-            if (ct == 0) {
-                *s_abort = 1;
-                SysState *st = sys[meta->sys].st;         // 0 until the stage was first filled
-                st->status = FG_ERR_TIMEOUT;
-                st->live = 0;
-                for (int q = j; q < j + ST; ++q) mbar_wait(full0 + 8u * (q % ST), (unsigned)((q / ST) & 1));
-            }
-            return;
-        }
-        if (pne < 0) break;                               // no more patches
-        const int pnd = meta->pnd, n = meta->n;
-        TY *Y = reinterpret_cast<TY *>(meta->Y);
-        const int head = (pnd + 1 + 7) & ~7;
-        const int *dl = reinterpret_cast<const int *>(stg + L::b + 6 * (size_t)W);
-        const unsigned short *ic = reinterpret_cast<const unsigned short *>(stg + L::b + 6 * (size_t)W + 4 * (size_t)pnd);
-        for (int jj = ct; jj < pnd; jj += NC) {
-            const int dd = dl[jj];
-            const int d = dd & 0x7fffffff;
-            if (d == n) continue;                         // dof-list padding
-            const int e0 = ic[jj], e1 = ic[jj + 1];
-            TA v = (TA)0;
-            for (int e = e0; e < e1; ++e) v += sa[ic[head + e]];
-            if (dd < 0) atomicAdd(Y + d, (TY)v);          // shared dof: reduction store
-            else Y[d] = (TY)v;
-        }
-        // this thread's shared-memory writes (the products) before the next
-        // bulk copy into the stage
-        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-        consumers_sync();                                 // stage s is free
-        if (ct == 0) mbar_arrive(empty0 + 8u * s);
-    }
-}
-
 // ---------------------------------------------------------------- CSR SpMV
 // y = A x for the assembled operator (csrmv.c:57-62), W lanes per row
 // (W = 4, 8 or 32 from the mean row length; rows of P1 transport hold ~7
@@ -785,35 +528,32 @@ k_csr_mv(const SysDev *__restrict__ sys, const DChunk *__restrict__ ch, const in
 // ---------------------------------------------------------------- block-diagonal apply
 // z[dofs of node] = invB(node) * p[dofs of node] (BlockDiag_precond.c:3-29,
 // BlockDiagDOF3_precond.c:3-27); dofs that are Dirichlet read 0 and are not
-// written.  sel: 0 = t64 -> u64 (FP64), 1 = t -> w (T), 2 = aux.
-template <int B, typename T>
+// written.  The cycle start's t64 -> u64; in the Arnoldi steps the matvec
+// applies it (rows.cu).
+template <int B>
 __global__ void __launch_bounds__(kThreads)
-k_blockdiag(const SysDev *__restrict__ sys, const NChunk *__restrict__ ch, const int *__restrict__ nch,
-            int gate, int sel, const T *aux_in, T *aux_out)
+k_blockdiag(const SysDev *__restrict__ sys, const NChunk *__restrict__ ch, const int *__restrict__ nch)
 {
     const int total = *nch;
     for (int c = blockIdx.x; c < total; c += gridDim.x) {
         const NChunk k = ch[c];
         const SysDev &D = sys[k.sys];
-        if (!gated(D, gate)) continue;
-        const T *P = sel == 0 ? (const T *)D.t64 : sel == 1 ? (const T *)D.t : aux_in;
-        T *Z = sel == 0 ? (T *)D.u64 : sel == 1 ? (T *)D.w : aux_out;
-        const T *M = sizeof(T) == 8 ? (const T *)D.ibd64 : (const T *)D.ibd32;
+        if (!D.st->live) continue;
         for (int nd = k.n0 + threadIdx.x; nd < k.n1; nd += blockDim.x) {
             int id[B];
-            T v[B];
+            double v[B];
 #pragma unroll
             for (int a = 0; a < B; ++a) {
                 id[a] = D.node_dof[nd * B + a];
-                v[a] = id[a] == D.n ? (T)0 : P[id[a]];
+                v[a] = id[a] == D.n ? 0.0 : D.t64[id[a]];
             }
-            const T *m = M + (size_t)nd * B * B;
+            const double *m = D.ibd64 + (size_t)nd * B * B;
 #pragma unroll
             for (int r = 0; r < B; ++r) {
-                T s = m[r * B] * v[0];
+                double s = m[r * B] * v[0];
 #pragma unroll
                 for (int q = 1; q < B; ++q) s += m[r * B + q] * v[q];
-                if (id[r] != D.n) Z[id[r]] = s;
+                if (id[r] != D.n) D.u64[id[r]] = s;
             }
         }
     }
@@ -823,7 +563,7 @@ k_blockdiag(const SysDev *__restrict__ sys, const NChunk *__restrict__ ch, const
 // FP64: u = M^-1 (A x) (t64 holds A x; for the block-diagonal case u64
 // already holds M^-1 t64), r = b - u (pgmres.c:64-75), partial ||r||^2,
 // true residual s = F - A x, partial ||s||^2, and on the first cycle ||b||^2
-// and ||F||^2.  t64 is cleared for the next use.
+// and ||F||^2.
 __global__ void __launch_bounds__(kThreads)
 k_start(const SysDev *__restrict__ sys, const DChunk *__restrict__ ch, const int *__restrict__ nch)
 {
@@ -845,7 +585,6 @@ k_start(const SysDev *__restrict__ sys, const DChunk *__restrict__ ch, const int
             double bd = D.b[d];
             double r = -1.0 * (u + -1.0 * bd);
             D.r64[d] = r;
-            D.t64[d] = 0.0;
             a0 += r * r;
             if (has_f) {
                 double s = D.ftrue[d] - t;
@@ -944,7 +683,6 @@ k_final(const SysDev *__restrict__ sys, const DChunk *__restrict__ ch, const int
         double a = 0;
         for (int d = k.d0 + threadIdx.x; d < k.d1; d += blockDim.x) {
             double t = D.t64[d];
-            D.t64[d] = 0.0;
             if (D.ftrue) { double s = D.ftrue[d] - t; a += s * s; }
         }
         a = warp_sum(a);
@@ -999,11 +737,6 @@ int sm_count()
 
 namespace {
 
-// FP32 3x3 blocks: the bulk-copy pipeline (k_ebe_mv3p) instead of k_ebe_mv3
-#ifndef FG_MV3_PIPELINE
-#define FG_MV3_PIPELINE 1
-#endif
-constexpr bool kMv3Pipeline = FG_MV3_PIPELINE != 0;
 // the matvec kernel of an S x S launch: 3x3, the pair kernel, or per element
 template <int S, typename TA, typename TX, typename TY, bool PAIRS>
 static auto pick_mv()
@@ -1067,29 +800,14 @@ struct MvLaunch {
         const int g = std::max(1, std::min(nitems, occ * sm_count()));
         kern<<<g, nt, smem, st>>>(sys, ch, nch, gate, in_sel, out_sel, step, ai, ao, maxdof);
     }
-    // the 3x3 FP32 bulk-copy pipeline: one CTA per SM, at most one per patch
-    template <typename TX, typename TY>
-    static void pipeline(int nitems, cudaStream_t st, const SysDev *sys, const MvRec *rec, const int *nch, int gate,
-                         int in_sel, int out_sel, int step, const TX *ai, TY *ao)
-    {
-        using L = Mv3pSmem<TX>;
-        static std::once_flag once;
-        std::call_once(once, [] {
-            cudaFuncSetAttribute(k_ebe_mv3p<TX, TY>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::total);
-        });
-        const int g = std::max(1, std::min(nitems, sm_count()));
-        k_ebe_mv3p<TX, TY><<<g, kMv3pThreads, L::total, st>>>(sys, rec, nch, gate, in_sel, out_sel, step, ai, ao);
-    }
 };
 
-template <typename T>
-void launch_blockdiag(int B, dim3 g, cudaStream_t st, const SysDev *sys, const NChunk *ch, const int *nch,
-                      int gate, int sel, const T *ai, T *ao)
+void launch_blockdiag(int B, dim3 g, cudaStream_t st, const SysDev *sys, const NChunk *ch, const int *nch)
 {
     switch (B) {
-    case 2: k_blockdiag<2, T><<<g, kThreads, 0, st>>>(sys, ch, nch, gate, sel, ai, ao); break;
-    case 3: k_blockdiag<3, T><<<g, kThreads, 0, st>>>(sys, ch, nch, gate, sel, ai, ao); break;
-    case 4: k_blockdiag<4, T><<<g, kThreads, 0, st>>>(sys, ch, nch, gate, sel, ai, ao); break;
+    case 2: k_blockdiag<2><<<g, kThreads, 0, st>>>(sys, ch, nch); break;
+    case 3: k_blockdiag<3><<<g, kThreads, 0, st>>>(sys, ch, nch); break;
+    case 4: k_blockdiag<4><<<g, kThreads, 0, st>>>(sys, ch, nch); break;
     }
 }
 
@@ -1164,17 +882,26 @@ int part_dofs_for(const std::vector<BatchMember> &mem, const SolveConfig &cfg)
     return (int)std::max<long long>(kPartMin, std::min<long long>(kPartMax, pd));
 }
 
+// Units per work item of the matvec: one row per thread (256 / ndof units)
+// while that leaves a wave of CTAs or less, so that small systems spread out,
+// else four rows per thread.  A tuned choice can pin either (mv3_pipeline 0:
+// always one row per thread); the sums are the same.
+int unit_chunk(const std::vector<BatchMember> &mem, const SolveConfig &cfg)
+{
+    fg_tune_choice tc;
+    const int B = mem[0].s->topo.ndof, one = 32 / B * (kThreads / 32);
+    if (tuned_choice(mem, cfg, tc) && tc.mv3_pipeline == 0) return one;
+    return batch_dofs(mem) > 8LL * kThreads * sm_count() ? 4 * one : one;
+}
+
 }  // namespace
 
 // Chunk tables of one batch (device copies + host counts).
 struct Plan {
-    int nsys = 0, ncol = 0, S = 3, B = 1, maxdof = 1;   // ncol: patch colours
-    int op = FG_OP_EBE, csr_w = 4, precond = FG_PRECOND_NONE, ilu_g = 4;
-    std::vector<int> ech_off;      // ncol+1 offsets into echunks
+    int nsys = 0, S = 3, B = 1;
+    int precond = FG_PRECOND_NONE, ilu_g = 4;
     int n_dch = 0, n_nch = 0, n_ilu = 0, n_ilub = 0, n_spb = 0, n_spi = 0;
-    DevMem sysdev, echunks, ecount, dchunks, dcount, nchunks, ncount, live;
-    DevMem mvrec;                                  // 3x3: per matvec work item, for the bulk-copy pipeline
-    bool mv3p = true;                              // 3x3 FP32: the bulk-copy pipeline (else the register kernel)
+    DevMem sysdev, dchunks, dcount, nchunks, ncount, live;
     bool rprec = false;                            // a right preconditioner (SGSe) before every matvec
     DevMem ilu_fwd, ilu_bwd, ilu_ctr;              // sync-free ILU(0) substitutions
     DevMem ilu_ws;                                 // block-Jacobi: (system, block) items, a warp each
@@ -1189,30 +916,12 @@ static int build_plan(Plan &P, std::vector<BatchMember> &mem, const SolveConfig 
     P.nsys = (int)mem.size();
     P.S = mem[0].s->topo.S;
     P.B = mem[0].s->topo.ndof;
-    P.ncol = 0;
-    P.maxdof = 1;
-    for (auto &m : mem) {
+    for (auto &m : mem)
         if (m.s->topo.S != P.S) { set_error("a batch must hold systems of one block size"); return FG_ERR_ARG; }
-        P.ncol = std::max(P.ncol, m.s->topo.npcol);
-        P.maxdof = std::max(P.maxdof, m.s->topo.maxdof);
-    }
-    // matvec work items: one per patch, grouped by patch colour
-    std::vector<EChunk> ech;
-    P.ech_off.assign(P.ncol + 1, 0);
-    for (int c = 0; c < P.ncol; ++c) {
-        for (int s = 0; s < P.nsys; ++s) {
-            const Topology &t = mem[s].s->topo;
-            if (c >= t.npcol) continue;
-            for (int q = t.pc_ptr[c]; q < t.pc_ptr[c + 1]; ++q) ech.push_back({s, t.pc_list[q], 0});
-        }
-        P.ech_off[c + 1] = (int)ech.size();
-    }
     std::vector<DChunk> dch;
     std::vector<NChunk> nch;
     const int pdofs = part_dofs_for(mem, cfg);
-    fg_tune_choice tc;
-    const bool tuned = tuned_choice(mem, cfg, tc);
-    P.mv3p = !(tuned && tc.mv3_pipeline == 0);
+    const int uchunk = unit_chunk(mem, cfg);
     P.rprec = cfg.precond == FG_PRECOND_SGSE;
     for (int s = 0; s < P.nsys; ++s) {
         int n = mem[s].s->topo.n;
@@ -1224,18 +933,14 @@ static int build_plan(Plan &P, std::vector<BatchMember> &mem, const SolveConfig 
             int d1 = p + 1 == np ? n : (int)((long long)n * (p + 1) / np) & ~7;
             dch.push_back({s, p, d0, d1});
         }
-        int nn = mem[s].s->topo.nnodes;
-        for (int a = 0; a < nn; a += 1024) nch.push_back({s, a, std::min(a + 1024, nn)});
+        const int nn = mem[s].s->topo.nunits;
+        for (int a = 0; a < nn; a += uchunk) nch.push_back({s, a, std::min(a + uchunk, nn)});
     }
     P.n_dch = (int)dch.size();
     P.n_nch = (int)nch.size();
-    P.op = mem[0].s->op;
     P.precond = cfg.precond;
-    P.csr_w = 4;
-    for (auto &m : mem) {
-        if (m.s->op != P.op) { set_error("a batch must use one operator kind"); return FG_ERR_ARG; }
-        P.csr_w = std::max(P.csr_w, m.s->csr_w);
-    }
+    for (auto &m : mem)
+        if (m.s->op != mem[0].s->op) { set_error("a batch must use one operator kind"); return FG_ERR_ARG; }
     // ILU(0) substitutions: one item per pass of a system's level order
     // (forward and backward lists), systems interleaved
     std::vector<int2> fwd, bwd;
@@ -1287,25 +992,8 @@ static int build_plan(Plan &P, std::vector<BatchMember> &mem, const SolveConfig 
         }
     P.n_spb = (int)spb.size();
     P.n_spi = (int)spi.size();
-    std::vector<int> ecounts(P.ncol);
-    for (int c = 0; c < P.ncol; ++c) ecounts[c] = P.ech_off[c + 1] - P.ech_off[c];
-    std::vector<MvRec> recs;
-    if (P.S == 3) {
-        recs.reserve(ech.size());
-        for (const EChunk &k : ech) {
-            const Topology &t = mem[k.sys].s->topo;
-            const int p = k.e0;
-            const int pne = t.pt_elem[p + 1] - t.pt_elem[p], pnd = t.pt_dof[p + 1] - t.pt_dof[p];
-            const int ni = t.pt_inc[p + 1] - t.pt_inc[p];
-            recs.push_back({k.sys, t.pt_elem[p], (int)(t.pt_boff[p] / 16), (int)(t.pt_boff[p + 1] - t.pt_boff[p]),
-                            t.pt_xlo[p], pne | (pnd << 16), ni | (t.pt_xlen[p] << 16), 0});
-        }
-    }
     int r;
     if ((r = P.sysdev.alloc(sizeof(SysDev) * hs.size())) ||
-        (r = P.echunks.alloc(sizeof(EChunk) * std::max<size_t>(1, ech.size()))) ||
-        (!recs.empty() && (r = P.mvrec.alloc(sizeof(MvRec) * recs.size()))) ||
-        (r = P.ecount.alloc(sizeof(int) * std::max(1, P.ncol))) ||
         (r = P.dchunks.alloc(sizeof(DChunk) * std::max<size_t>(1, dch.size()))) ||
         (r = P.dcount.alloc(sizeof(int))) ||
         (r = P.nchunks.alloc(sizeof(NChunk) * std::max<size_t>(1, nch.size()))) ||
@@ -1316,8 +1004,6 @@ static int build_plan(Plan &P, std::vector<BatchMember> &mem, const SolveConfig 
         (r = P.sp_blocks.alloc(sizeof(int2) * std::max<size_t>(1, spb.size()))) ||
         (r = P.sp_ifaces.alloc(sizeof(int2) * std::max<size_t>(1, spi.size()))))
         return r;
-    if (!recs.empty())
-        FG_CUDA(cudaMemcpyAsync(P.mvrec.p, recs.data(), sizeof(MvRec) * recs.size(), cudaMemcpyHostToDevice, st));
     if (!spb.empty())
         FG_CUDA(cudaMemcpyAsync(P.sp_blocks.p, spb.data(), sizeof(int2) * spb.size(), cudaMemcpyHostToDevice, st));
     if (!spi.empty())
@@ -1327,10 +1013,6 @@ static int build_plan(Plan &P, std::vector<BatchMember> &mem, const SolveConfig 
         FG_CUDA(cudaMemcpyAsync(P.ilu_bwd.p, bwd.data(), sizeof(int2) * bwd.size(), cudaMemcpyHostToDevice, st));
     }
     FG_CUDA(cudaMemcpyAsync(P.sysdev.p, hs.data(), sizeof(SysDev) * hs.size(), cudaMemcpyHostToDevice, st));
-    if (!ech.empty())
-        FG_CUDA(cudaMemcpyAsync(P.echunks.p, ech.data(), sizeof(EChunk) * ech.size(), cudaMemcpyHostToDevice, st));
-    if (P.ncol)
-        FG_CUDA(cudaMemcpyAsync(P.ecount.p, ecounts.data(), sizeof(int) * P.ncol, cudaMemcpyHostToDevice, st));
     FG_CUDA(cudaMemcpyAsync(P.dchunks.p, dch.data(), sizeof(DChunk) * dch.size(), cudaMemcpyHostToDevice, st));
     FG_CUDA(cudaMemcpyAsync(P.dcount.p, &P.n_dch, sizeof(int), cudaMemcpyHostToDevice, st));
     FG_CUDA(cudaMemcpyAsync(P.nchunks.p, nch.data(), sizeof(NChunk) * nch.size(), cudaMemcpyHostToDevice, st));
@@ -1339,25 +1021,9 @@ static int build_plan(Plan &P, std::vector<BatchMember> &mem, const SolveConfig 
     return FG_OK;
 }
 
-// Enqueue the matvec over all colours: mode 0 (x -> t64, FP64, gate live)
-// or mode 1 (V[step] -> t, T, gate in_cycle).
-template <typename TA, typename TX, typename TY>
-static void launch_csr_mv(const Plan &P, cudaStream_t st, int gate, int in_sel, int out_sel, int step)
-{
-    const SysDev *sys = P.sysdev.as<SysDev>();
-    dim3 g = grid_for(P.n_dch);
-    const DChunk *dc = P.dchunks.as<DChunk>();
-    const int *nd = P.dcount.as<int>();
-    if (P.csr_w == 4)
-        k_csr_mv<4, TA, TX, TY><<<g, kThreads, 0, st>>>(sys, dc, nd, gate, in_sel, out_sel, step, nullptr, nullptr);
-    else if (P.csr_w == 8)
-        k_csr_mv<8, TA, TX, TY><<<g, kThreads, 0, st>>>(sys, dc, nd, gate, in_sel, out_sel, step, nullptr, nullptr);
-    else
-        k_csr_mv<32, TA, TX, TY><<<g, kThreads, 0, st>>>(sys, dc, nd, gate, in_sel, out_sel, step, nullptr, nullptr);
-}
-
 // Enqueue the matvec: mode 0 (x -> t64, FP64, gate live), mode 1 (V[step]
-// -> t, T, gate in_cycle), mode 2 (V[0] -> t, T, every member), mode 3
+// -> w = M^-1 A v, T, gate in_cycle; a preconditioner with kernels of its own
+// gets t = A v instead), mode 2 (V[0] -> t, T, every member), mode 3
 // (x -> t64, FP64, every member).  Returns the number of kernels.
 // TV: storage type of the basis vector read in mode 1 (the Arnoldi step)
 template <typename T, typename TV = T>
@@ -1365,43 +1031,19 @@ static int enqueue_matvec(const Plan &P, int mode, int step, cudaStream_t st)
 {
     const bool f64 = mode == 0 || mode == 3;
     const int gate = mode == 0 ? 0 : mode == 1 ? 1 : -1;
-    const int sel = f64 ? 0 : 1;
+    const bool own = P.precond == FG_PRECOND_ILU0 || P.precond == FG_PRECOND_SPIKE || P.precond == FG_PRECOND_LUE ||
+                     P.precond == FG_PRECOND_SGSE;
     // pgmres.c:61,93: v = precondR(x or u_i) before the matvec (SGSe), into r64
-    int in0 = 0, in1 = 1, kr = 0;
+    int in = f64 ? 0 : 1, kr = 0;
     if (P.rprec && (mode == 0 || mode == 1)) {
         launch_elem_prec(P.sysdev.as<SysDev>(), P.nsys, 3, mode == 0 ? 0 : 1, step, st);
-        in0 = in1 = 3;
+        in = 3;
         kr = 1;
     }
-    if (P.op == FG_OP_CSR) {
-        if (f64) launch_csr_mv<double, double, double>(P, st, gate, sel, sel, step);
-        else launch_csr_mv<T, TV, T>(P, st, gate, sel, sel, step);
-        return 1;
-    }
-    const SysDev *sys = P.sysdev.as<SysDev>();
-    int k = 0;
-    for (int c = 0; c < P.ncol; ++c) {
-        int cnt = P.ech_off[c + 1] - P.ech_off[c];
-        if (!cnt) continue;
-        const EChunk *ch = P.echunks.as<EChunk>() + P.ech_off[c];
-        const int *nc = P.ecount.as<int>() + c;
-        bool done = false;
-        if (f64) {
-            MvLaunch::go<double, double, double>(P.S, cnt, st, sys, ch, nc, gate, in0, 0, 0, nullptr, nullptr,
-                                                 P.maxdof);
-            done = true;
-        }
-        if constexpr (sizeof(T) == 4) {
-            if (!done && P.S == 3 && kMv3Pipeline && P.mv3p && P.mvrec.p) {
-                MvLaunch::pipeline<TV, T>(cnt, st, sys, P.mvrec.as<MvRec>() + P.ech_off[c], nc, gate, 1, 1, step,
-                                          nullptr, nullptr);
-                done = true;
-            }
-        }
-        if (!done) MvLaunch::go<T, TV, T>(P.S, cnt, st, sys, ch, nc, gate, in1, 1, step, nullptr, nullptr, P.maxdof);
-        ++k;
-    }
-    return k + kr;
+    const int prec = f64 || sizeof(T) == 8 ? 64 : sizeof(TV) == 2 ? 16 : 32;
+    const int out = f64 ? 0 : mode == 1 && !own ? 2 : 1;
+    return kr + launch_rows_mv(P.B, prec, P.sysdev.as<SysDev>(), P.nchunks.as<NChunk>(), P.ncount.as<int>(), P.n_nch,
+                               gate, in, out, step, st);
 }
 
 // M^-1 applied after a matvec: sel 0 (t64 -> u64, FP64) or 1 (t -> w, T).
@@ -1410,12 +1052,8 @@ static int enqueue_precond(const Plan &P, int sel, cudaStream_t st)
 {
     const SysDev *sys = P.sysdev.as<SysDev>();
     if (P.precond == FG_PRECOND_BLOCKDIAG) {
-        if (sel == 0)
-            launch_blockdiag<double>(P.B, grid_for(P.n_nch), st, sys, P.nchunks.as<NChunk>(), P.ncount.as<int>(), 0,
-                                     0, nullptr, nullptr);
-        else
-            launch_blockdiag<T>(P.B, grid_for(P.n_nch), st, sys, P.nchunks.as<NChunk>(), P.ncount.as<int>(), 1, 1,
-                                nullptr, nullptr);
+        if (sel == 1) return 0;                       // in the matvec
+        launch_blockdiag(P.B, grid_for(P.n_nch), st, sys, P.nchunks.as<NChunk>(), P.ncount.as<int>());
         return 1;
     }
     if (P.precond == FG_PRECOND_LUE || P.precond == FG_PRECOND_SGSE) {   // FP64 only
@@ -1696,7 +1334,7 @@ size_t request_bytes(const fg_system *s, int kmax, int mixed, bool time_loop)
                             &w.counter, &w.state};
     size_t have = 0;
     for (auto *m : held) have += m->bytes;
-    size_t b = s->bytes() - std::min(have, s->bytes()) + workspace_bytes(s, kmax, mixed);
+    size_t b = s->bytes() - std::min(have, s->bytes()) + workspace_bytes(s, kmax, mixed) + rows_bytes(s, mixed != 0);
     if (time_loop) {
         const DevMem *loop[] = {&s->rhs_f, &s->rhs_b, &s->state_u, &s->state_a, &s->state_old};
         for (auto *m : loop)
@@ -1722,11 +1360,10 @@ int BatchRun::stage(const BatchMember &m)
     if (r) return r;
     if ((r = ensure_workspace(s, cfg.kmax, cfg.mixed + cfg.vhalf))) return r;
     if (s->op == FG_OP_CSR && (r = csr_refresh(s, st))) return r;
+    if ((r = rows_refresh(s, cfg.mixed != 0, st))) return r;
     Workspace &w = s->ws;
     size_t vb = 8 * (size_t)s->n_pad;
     FG_CUDA(cudaMemsetAsync(w.x.p, 0, vb, st));
-    FG_CUDA(cudaMemsetAsync(w.t64.p, 0, vb, st));
-    FG_CUDA(cudaMemsetAsync(w.t.p, 0, (cfg.mixed ? 4 : 8) * (size_t)s->n_pad, st));
     FG_CUDA(cudaMemsetAsync(w.V.p, 0, (cfg.vhalf ? 2 : cfg.mixed ? 4 : 8) * (size_t)s->n_pad * cfg.kmax, st));
     FG_CUDA(cudaMemsetAsync(w.small.p, 0, w.small.bytes, st));
     if (cfg.device_io) {
@@ -1900,6 +1537,10 @@ int matvec_device(fg_system *s, const double *x, double *y, int precision, cudaS
 {
     if (!s->blocks_ok) { set_error("matvec before element blocks were set"); return FG_ERR_STATE; }
     const Topology &t = s->topo;
+    if (precision == 32 && s->op != FG_OP_CSR) {
+        int rb = ensure_blocks32(s, st);
+        if (rb) return rb;
+    }
     SysDev D{};
     D.n = t.n; D.n_pad = s->n_pad; D.nel = t.nel; D.nel_pad = s->nel_pad; D.S = t.S;
     D.lm = s->lm.as<int>(); D.A64 = s->A64.as<double>(); D.A32 = s->A32.as<float>();
@@ -1977,12 +1618,13 @@ int bench_matvec(std::vector<fg_system *> &systems, int precision, int reps, dou
         if (!s->blocks_ok) { set_error("matvec before element blocks were set"); return FG_ERR_STATE; }
         int kk = std::max(2, s->ws.kmax);
         int r = ensure_workspace(s, kk, cfg.mixed);
-        if (r) return r;
+        if (r || (r = rows_refresh(s, cfg.mixed != 0, systems[0]->stream))) return r;
         cfg.kmax = kk;
         mem.push_back({s, nullptr, nullptr, nullptr});
         hs.push_back(make_desc(s, cfg, false));
         const Topology &t = s->topo;
-        b += (double)t.nel * (t.S * t.S * w + t.S * 4.0) + 2.0 * t.n * w;
+        // the assembled operator: values, columns, x once, y once
+        b += (double)t.rw_col.size() * (t.ndof * t.ndof * w + 4.0) + 2.0 * t.n * w;
     }
     cudaStream_t st = systems[0]->stream;
     Plan P;
@@ -2005,8 +1647,6 @@ int bench_matvec(std::vector<fg_system *> &systems, int precision, int reps, dou
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     if (ce != cudaSuccess) return cuda_fail(ce, "bench_matvec");
-    for (auto *s : systems)
-        FG_CUDA(cudaMemsetAsync(s->ws.t.p, 0, s->ws.t.bytes, st));
     FG_CUDA(cudaStreamSynchronize(st));
     *ms = t / reps;
     *bytes = b;

@@ -146,6 +146,7 @@ extern "C" int fg_matvec_noalloc(fg_system *s, const double *P_dev, double *Q_de
     double *d_x = reinterpret_cast<double *>(base + kOffX);
     double *d_y = reinterpret_cast<double *>(base + kOffY);
     cudaStream_t st = s->stream;
+    if (precision == 32 && (r = ensure_blocks32(s, st))) return r;
     FG_CUDA(cudaMemcpyAsync(d_desc, &D, sizeof(SysDev), cudaMemcpyHostToDevice, st));
     if (t.npcol) FG_CUDA(cudaMemcpyAsync(d_counts, counts, sizeof(int) * t.npcol, cudaMemcpyHostToDevice, st));
     // pageable source: staged before the call returns, while the lock is held

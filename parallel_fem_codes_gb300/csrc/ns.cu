@@ -386,8 +386,8 @@ int ns_assemble_device(fg_system *s, double reynolds, int form, const double *u_
     int r = gather_residual(s, s->Fe.as<double>(), F_dev, st);
     if (r) return r;
     s->blocks_ok = true;
-    s->csr_dirty = true;
-    return convert_blocks(s, st);
+    blocks_changed(s);
+    return FG_OK;
 }
 
 // ---------------------------------------------------------------- state updates

@@ -89,8 +89,15 @@ __global__ void k_to_f32_patches(const double *__restrict__ a, float *__restrict
     }
 }
 
-int convert_blocks(fg_system *s, cudaStream_t st)
+void blocks_changed(fg_system *s)
 {
+    s->csr_dirty = true;
+    s->rw64_ok = s->rw32_ok = s->a32_ok = false;
+}
+
+int ensure_blocks32(fg_system *s, cudaStream_t st)
+{
+    if (s->a32_ok) return FG_OK;
     if (s->topo.S == 3) {
         const int np = s->topo.npatch;
         if (np > 0)
@@ -103,6 +110,7 @@ int convert_blocks(fg_system *s, cudaStream_t st)
     }
     FG_CUDA(cudaGetLastError());
     count_launches(1);
+    s->a32_ok = true;
     return FG_OK;
 }
 
@@ -114,7 +122,8 @@ int upload_blocks_raw(fg_system *s, const double *raw_dev, cudaStream_t st)
                                                       s->nel_pad, s->topo.S * s->topo.S);
     FG_CUDA(cudaGetLastError());
     count_launches(1);
-    return convert_blocks(s, st);
+    blocks_changed(s);
+    return FG_OK;
 }
 
 int download_blocks_raw(const fg_system *s, double *raw_dev, cudaStream_t st)
@@ -582,8 +591,8 @@ int scale_device(fg_system *s, int kind, double *F_dev, cudaStream_t st)
         }
         s->scale_kind = kind;
         s->precond = FG_PRECOND_NONE;
-        s->csr_dirty = true;
-        return convert_blocks(s, st);
+        blocks_changed(s);
+        return FG_OK;
     }
     if ((r = precond_setup_device(s, FG_PRECOND_DIAG, FG_SETUP_ACCUMULATE, F_dev, st))) return r;
     double *invd = s->invd64.as<double>();
@@ -601,8 +610,8 @@ int scale_device(fg_system *s, int kind, double *F_dev, cudaStream_t st)
     }
     s->scale_kind = kind;
     s->precond = FG_PRECOND_NONE;                    // the scaled system is solved as it stands
-    s->csr_dirty = true;
-    return convert_blocks(s, st);
+    blocks_changed(s);
+    return FG_OK;
 }
 
 int unscale_device(fg_system *s, double *x_dev, cudaStream_t st)
@@ -1343,8 +1352,8 @@ int tt_assemble_device(fg_system *s, const fg_tt_coeffs *c, const double *u_dev,
     FG_CUDA(cudaGetLastError());
     count_launches(2);
     s->blocks_ok = true;
-    s->csr_dirty = true;
-    return convert_blocks(s, st);
+    blocks_changed(s);
+    return FG_OK;
 }
 
 // the bubble planes of a Predictor2 build with nb unknowns per element
@@ -1389,8 +1398,8 @@ int tt_mfdd_assemble_device(fg_system *s, const fg_tt_coeffs *c, const double *u
     FG_CUDA(cudaGetLastError());
     count_launches(2);
     s->blocks_ok = true;
-    s->csr_dirty = true;
-    return convert_blocks(s, st);
+    blocks_changed(s);
+    return FG_OK;
 }
 
 int tt_bubble_correct_device(fg_system *s, const double *Da_dev, double coef, double *DaB_dev, cudaStream_t st)
@@ -1464,8 +1473,8 @@ int transport_assemble_device(fg_system *s, const fg_transport_coeffs *c, const 
     FG_CUDA(cudaGetLastError());
     count_launches(1);
     s->blocks_ok = true;
-    s->csr_dirty = true;
-    return convert_blocks(s, st);
+    blocks_changed(s);
+    return FG_OK;
 }
 
 }  // namespace fg

@@ -39,7 +39,11 @@ struct fg_system {
     fg::DevMem lm, A64, A32;
     fg::DevMem dinc_ptr, dinc, ninc_ptr, ninc, node_dof, eorder, perm;
     fg::DevMem lm16, pt_elem, pt_dof, pt_col, pdofs, pt_inc, incl;   // matvec patch layout
-    fg::DevMem blob;                   // 3x3: per-patch index blobs of the bulk-copy matvec
+    // assembled operator of the Krylov engine (rows.cu): pattern, and values
+    // made from the element blocks when a solve first needs them
+    fg::DevMem rw_off, rw_col, rw64, rw32;
+    bool rw64_ok = false, rw32_ok = false;
+    bool a32_ok = false;               // A32 holds the current blocks
     // preconditioners
     fg::DevMem diag, invd64, invd32, bd, ibd64, ibd32;
     fg::DevMem pc_err;                 // set-up status word (singular nodal block)
@@ -163,7 +167,11 @@ inline void set_patch_fields(SysDev &D, const fg_system *s)
     D.dofs = s->pdofs.as<int>();
     D.pt_inc = s->pt_inc.as<int>();
     D.incl = s->incl.as<unsigned short>();
-    D.blob = s->blob.as<unsigned char>();
+    D.nunits = s->topo.nunits;
+    D.rw_off = s->rw_off.as<int>();
+    D.rw_col = s->rw_col.as<int>();
+    D.rw64 = s->rw64.as<double>();
+    D.rw32 = s->rw32.as<float>();
     D.maxdof = std::max(1, s->topo.maxdof);
 }
 
@@ -288,10 +296,23 @@ size_t request_bytes(const fg_system *s, int kmax, int mixed, bool time_loop);
 int euler_assemble_device(fg_system *s, const fg_euler_coeffs *c, const double *u_dev, const double *du_dev,
                           double *R_dev, cudaStream_t st);
 
+// Assembled operator (rows.cu): values from the current element blocks,
+// FP64 and (fp32) FP32; made on st when stale.
+int rows_refresh(fg_system *s, bool fp32, cudaStream_t st);
+size_t rows_bytes(const fg_system *s, bool fp32);
+// y = A x over unit chunks.  gate and in_sel as the element matvec; out 0:
+// t64 (FP64), 1: t, 2: w = M^-1 A x (preconditioners that act on one node:
+// none, Diag, BlockDiag).  prec 64 / 32, or 16: FP32 with an FP16 input.
+int launch_rows_mv(int B, int prec, const SysDev *sys, const NChunk *ch, const int *nch, int nchunks, int gate,
+                   int in_sel, int out, int step, cudaStream_t st);
+
 // Set-up kernels (setup.cu)
 int precond_setup_device(fg_system *s, int kind, int flags, double *F_dev, cudaStream_t st);
 int precond_apply_device(fg_system *s, const double *p, double *z, cudaStream_t st);
-int convert_blocks(fg_system *s, cudaStream_t st);
+// New element blocks in A64: everything made from the old ones is stale.
+void blocks_changed(fg_system *s);
+// FP32 copy of the blocks (FP32 element matvec), made on st when stale
+int ensure_blocks32(fg_system *s, cudaStream_t st);
 // Left / left-right diagonal scaling of the blocks and F (internal numbering)
 int scale_device(fg_system *s, int kind, double *F_dev, cudaStream_t st);
 int unscale_device(fg_system *s, double *x_dev, cudaStream_t st);

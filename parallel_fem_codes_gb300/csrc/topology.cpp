@@ -177,6 +177,58 @@ int matrix_bandwidth(int n, const int *IA, const int *JA)
     return std::max(bl, br);
 }
 
+// ---------------------------------------------------------------- rows
+// Pattern of the assembled operator in slices of kRowSlice units (ndof = 1:
+// internal dofs, whose adjacency is IB/JB; else mesh nodes): every unit of a
+// slice has the slice's width of slots, slot-major, so that consecutive
+// units read consecutive entries.  A node couples to the nodes it shares an
+// element with, itself included, where both have a free dof.  Unused slots
+// hold the unit itself with kRowPad set.
+static void build_rows(Topology &t, const std::vector<int> &IB, const std::vector<int> &JB)
+{
+    const int nu = t.nunits = t.ndof == 1 ? t.n : t.nnodes;
+    std::vector<int> ptr(1, 0), col;
+    const int *P = IB.data(), *C = JB.data();
+    if (t.ndof > 1) {
+        ptr.assign(nu + 1, 0);
+        col.reserve((size_t)nu * 8);
+        std::vector<char> free_node(nu, 0);
+        for (int i = 0; i < nu; ++i)
+            for (int k = 0; k < t.ndof; ++k)
+                if (t.type[(size_t)i * t.ndof + k] != 0) free_node[i] = 1;
+        std::vector<int> mark(nu, -1);
+        for (int i = 0; i < nu; ++i) {
+            const size_t b = col.size();
+            if (free_node[i])
+                for (int q = t.ninc_ptr[i]; q < t.ninc_ptr[i + 1]; ++q) {
+                    const int *v = &t.ien[3 * (size_t)t.eorder[t.ninc[q] >> 2]];
+                    for (int a = 0; a < 3; ++a)
+                        if (free_node[v[a]] && mark[v[a]] != i) { mark[v[a]] = i; col.push_back(v[a]); }
+                }
+            std::sort(col.begin() + b, col.end());
+            ptr[i + 1] = (int)col.size();
+        }
+        P = ptr.data();
+        C = col.data();
+    }
+    const int ns = (nu + kRowSlice - 1) / kRowSlice;
+    t.rw_off.assign(ns + 1, 0);
+    for (int s = 0; s < ns; ++s) {
+        int w = 0;
+        for (int u = s * kRowSlice; u < std::min(nu, (s + 1) * kRowSlice); ++u) w = std::max(w, P[u + 1] - P[u]);
+        t.rw_off[s + 1] = t.rw_off[s] + w * kRowSlice;
+    }
+    t.rw_col.resize(std::max(t.rw_off[ns], 1));
+    for (int s = 0; s < ns; ++s) {
+        const int w = (t.rw_off[s + 1] - t.rw_off[s]) / kRowSlice;
+        for (int l = 0; l < kRowSlice; ++l) {
+            const int u = s * kRowSlice + l, m = u < nu ? P[u + 1] - P[u] : 0;
+            for (int k = 0; k < w; ++k)
+                t.rw_col[t.rw_off[s] + k * kRowSlice + l] = k < m ? C[P[u] + k] : (std::min(u, std::max(nu - 1, 0)) | kRowPad);
+        }
+    }
+}
+
 // ---------------------------------------------------------------- topology
 int build_topology(Topology &t, int nnodes, int nel, int ndof, const int *ien,
                    const int *type, const int *invp, int neq, int reorder)
@@ -249,8 +301,10 @@ int build_topology(Topology &t, int nnodes, int nel, int ndof, const int *ien,
     for (int i = 0; i < n; ++i) t.iperm[t.perm[i]] = i;
     t.iperm[n] = n;
     t.band_after = t.band_before;
+    std::vector<int> IB, JB;           // the adjacency in the internal numbering
     if (n > 0 && reorder == FG_REORDER_RCM) {
-        std::vector<int> IB(n + 1, 0), JB(t.nnz);
+        IB.assign(n + 1, 0);
+        JB.resize(t.nnz);
         for (int i = 0; i < n; ++i) IB[i + 1] = IB[i] + IA[t.perm[i] + 1] - IA[t.perm[i]];
         for (int i = 0; i < n; ++i) {
             int o = IB[i];
@@ -258,6 +312,9 @@ int build_topology(Topology &t, int nnodes, int nel, int ndof, const int *ien,
             std::sort(JB.begin() + IB[i], JB.begin() + IB[i + 1]);
         }
         t.band_after = matrix_bandwidth(n, IB.data(), JB.data());
+    } else {
+        IB = std::move(IA);
+        JB = std::move(JA);
     }
 
     // greedy element colouring over the free dofs, in reference element order:
@@ -408,7 +465,6 @@ int build_topology(Topology &t, int nnodes, int nel, int ndof, const int *ien,
     for (int p = 0; p < nel; ++p) t.epos[t.eorder[p]] = p;
     // patch-local element maps (internal element order)
     t.lm16.assign((size_t)nel * S, 0xFFFF);
-    t.lmx16.assign((size_t)nel * S, 0xFFFF);
     for (int p = 0; p < t.npatch; ++p) {
         const int b = t.pt_elem[p], e = t.pt_elem[p + 1];
         for (int j = t.pt_dof[p]; j < t.pt_dof[p + 1]; ++j) local[t.dofs[j] & 0x7fffffff] = j - t.pt_dof[p];
@@ -416,7 +472,6 @@ int build_topology(Topology &t, int nnodes, int nel, int ndof, const int *ien,
             for (int a = 0; a < S; ++a) {
                 int r = t.lm[(size_t)t.eorder[q] * S + a];
                 t.lm16[(size_t)q * S + a] = r == n ? (unsigned short)0xFFFF : (unsigned short)local[t.iperm[r]];
-                t.lmx16[(size_t)q * S + a] = r == n ? (unsigned short)0xFFFF : (unsigned short)(t.iperm[r] - t.pt_xlo[p]);
             }
         for (int j = t.pt_dof[p]; j < t.pt_dof[p + 1]; ++j) local[t.dofs[j] & 0x7fffffff] = -1;
     }
@@ -452,26 +507,6 @@ int build_topology(Topology &t, int nnodes, int nel, int ndof, const int *ien,
                 }
         }
         t.pt_inc[t.npatch] = (int)t.incl.size();
-    }
-    // 3x3: one index blob per patch for the bulk-copy matvec, 16-byte
-    // aligned: x-segment positions [3][W] (W = element count rounded up to
-    // 16, padding 0xFFFF), the dof list, the incidence lists
-    if (S == 3) {
-        t.pt_boff.assign(t.npatch + 1, 0);
-        t.blob.clear();
-        for (int p = 0; p < t.npatch; ++p) {
-            const int b = t.pt_elem[p], e = t.pt_elem[p + 1], W = (e - b + 15) / 16 * 16;
-            t.pt_boff[p] = (long long)t.blob.size();
-            const size_t o = t.blob.size();
-            const size_t nd = t.pt_dof[p + 1] - t.pt_dof[p], ni = t.pt_inc[p + 1] - t.pt_inc[p];
-            t.blob.resize(o + 6 * (size_t)W + 4 * nd + 2 * ni);
-            unsigned short *lx = reinterpret_cast<unsigned short *>(t.blob.data() + o);
-            for (int a = 0; a < 3; ++a)
-                for (int i = 0; i < W; ++i) lx[a * W + i] = b + i < e ? t.lmx16[(size_t)(b + i) * 3 + a] : 0xFFFF;
-            std::memcpy(t.blob.data() + o + 6 * (size_t)W, t.dofs.data() + t.pt_dof[p], 4 * nd);
-            std::memcpy(t.blob.data() + o + 6 * (size_t)W + 4 * nd, t.incl.data() + t.pt_inc[p], 2 * ni);
-        }
-        t.pt_boff[t.npatch] = (long long)t.blob.size();
     }
     // patch colouring: patches that share a dof get different colours
     {
@@ -543,14 +578,13 @@ int build_topology(Topology &t, int nnodes, int nel, int ndof, const int *ien,
             if (pe0 % 16 || pne < 1 || pne > PE || pe0 + (pne + 15) / 16 * 16 > nel_pad || pd0 % 4 || pnd % 4 ||
                 pnd < 1 || pnd > dcap || i0 % 8 || ni % 8 || ni > icap ||
                 (S == 3 && (t.pt_xlo[p] % 8 || t.pt_xlen[p] % 8 || t.pt_xlen[p] < 8 || t.pt_xlen[p] > kPatchXCap ||
-                            t.pt_xlo[p] + t.pt_xlen[p] > (n + 1 + 31) / 32 * 32 || t.pt_boff[p] % 16 ||
-                            t.pt_boff[p + 1] - t.pt_boff[p] > 6LL * PE + 4LL * dcap + 2LL * icap ||
-                            t.pt_boff[p + 1] / 16 > 0x7fffffffLL))) {
+                            t.pt_xlo[p] + t.pt_xlen[p] > (n + 1 + 31) / 32 * 32))) {
                 set_error("internal: matvec patch layout out of its bounds");
                 return FG_ERR_UNSUPPORTED;
             }
         }
     }
+    build_rows(t, IB, JB);
     return FG_OK;
 }
 
