@@ -28,6 +28,7 @@ UNITS = [
     ("system.cu", []),
     ("krylov.cu", []),
     ("rows.cu", []),
+    ("cycle.cu", []),
     ("setup.cu", ["-fmad=false"]),
     ("noalloc.cu", []),
     ("server.cu", []),

@@ -66,6 +66,8 @@ struct Topology {
     // kRowSlice + l, value = coupled unit (kRowPad set: unused slot)
     int nunits = 0;
     std::vector<int> rw_off, rw_col;
+    int rw_lo = 0, rw_hi = 0;            // a unit u couples to units in [u - rw_lo, u + rw_hi]
+    int rw_w = 0;                        // widest slice (slots per unit)
 };
 constexpr int kRowSlice = 32;
 constexpr int kRowPad = (int)0x80000000;
@@ -182,7 +184,13 @@ struct SysDev {
     const unsigned short *incl;
     int maxdof;
     // assembled operator in slices of units (rows.cu)
-    int nunits;
+    int nunits, rw_lo, rw_hi, rw_w;
+    // gang of the on-chip restart cycle (cycle.cu): CTAs (0: streaming
+    // kernels), padded rows of each, exchange words, vector and epoch
+    int cy_g, cy_rows;
+    unsigned long long *cy_part;
+    void *cy_vb;
+    unsigned *cy_epoch;
     const int *rw_off, *rw_col;
     const double *rw64;
     const float *rw32;
@@ -234,6 +242,8 @@ constexpr int kPartStride = 64;    // doubles per part (>= kmax + 2, kmax <= 60)
 __host__ __device__ constexpr bool precond_separate(int p) { return p >= 2; }
 
 struct EChunk { int sys, e0, e1; };
+// One (system, rank) of a restart cycle on chip: the units [u0, u1) (cycle.cu)
+struct CycItem { int sys, rank, u0, u1; };
 struct DChunk { int sys, part, d0, d1; };
 struct NChunk { int sys, n0, n1; };
 

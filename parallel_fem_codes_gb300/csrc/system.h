@@ -26,6 +26,7 @@ struct DevMem {
 struct Workspace {
     int kmax = 0, mixed = -1;
     DevMem V, w, t, x, b, ftrue, r64, t64, u64, small, part, counter, state;
+    DevMem gang;                       // exchange block of the on-chip cycle
 };
 
 }  // namespace fg
@@ -168,6 +169,9 @@ inline void set_patch_fields(SysDev &D, const fg_system *s)
     D.pt_inc = s->pt_inc.as<int>();
     D.incl = s->incl.as<unsigned short>();
     D.nunits = s->topo.nunits;
+    D.rw_lo = s->topo.rw_lo;
+    D.rw_hi = s->topo.rw_hi;
+    D.rw_w = s->topo.rw_w;
     D.rw_off = s->rw_off.as<int>();
     D.rw_col = s->rw_col.as<int>();
     D.rw64 = s->rw64.as<double>();
@@ -221,6 +225,8 @@ private:
     int graph_nodes = 0;
     int *h_live = nullptr;
     size_t live_cap = 0;
+    std::vector<int> sched;            // live flags the on-chip work lists were made for (empty: every member)
+    int reschedule(const std::vector<int> &live);
 };
 
 int validate_member(fg_system *s, const SolveConfig &cfg);
@@ -305,6 +311,16 @@ size_t rows_bytes(const fg_system *s, bool fp32);
 // none, Diag, BlockDiag).  prec 64 / 32, or 16: FP32 with an FP16 input.
 int launch_rows_mv(int B, int prec, const SysDev *sys, const NChunk *ch, const int *nch, int nchunks, int gate,
                    int in_sel, int out, int step, cudaStream_t st);
+
+// Restart cycle on chip (cycle.cu)
+int gang_size(const fg_system *s, int kmax, bool f64, bool dense);
+int gang_ctas(int B, bool f64);   // CTAs of the on-chip cycle that are resident together
+size_t gang_bytes(const fg_system *s, int kmax, int g, bool f64);
+void set_gang_fields(SysDev &D, const fg_system *s, int kmax, int g, bool f64);
+void gang_schedule(const std::vector<SysDev> &hs, const std::vector<int> &live, int B, bool f64,
+                   std::vector<CycItem> &items, std::vector<int> &off, size_t &smem);
+int launch_cycle(int B, bool f64, const SysDev *sys, const CycItem *items, const int *off, int ctas, size_t smem,
+                 cudaStream_t st);
 
 // Set-up kernels (setup.cu)
 int precond_setup_device(fg_system *s, int kind, int flags, double *F_dev, cudaStream_t st);

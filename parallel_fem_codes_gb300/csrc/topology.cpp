@@ -211,12 +211,18 @@ static void build_rows(Topology &t, const std::vector<int> &IB, const std::vecto
         P = ptr.data();
         C = col.data();
     }
+    for (int u = 0; u < nu; ++u)
+        if (P[u] < P[u + 1]) {
+            t.rw_lo = std::max(t.rw_lo, u - C[P[u]]);
+            t.rw_hi = std::max(t.rw_hi, C[P[u + 1] - 1] - u);
+        }
     const int ns = (nu + kRowSlice - 1) / kRowSlice;
     t.rw_off.assign(ns + 1, 0);
     for (int s = 0; s < ns; ++s) {
         int w = 0;
         for (int u = s * kRowSlice; u < std::min(nu, (s + 1) * kRowSlice); ++u) w = std::max(w, P[u + 1] - P[u]);
         t.rw_off[s + 1] = t.rw_off[s] + w * kRowSlice;
+        t.rw_w = std::max(t.rw_w, w);
     }
     t.rw_col.resize(std::max(t.rw_off[ns], 1));
     for (int s = 0; s < ns; ++s) {

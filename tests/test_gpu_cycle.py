@@ -1,0 +1,78 @@
+"""The on-chip restart cycle (csrc/cycle.cu) at the edges of its gangs: one
+CTA, two, the largest gang whose CTAs sum all partials themselves and the next
+one, many CTAs; restart lengths below and above the CTA's lane groups; a batch
+that starts streaming and moves on chip as members converge.  FP64 solves
+against the oracle's GMRES (solution 1e-9, iterations within two), mixed
+precision against the same solution by its true residual.
+"""
+import numpy as np
+import pytest
+
+import oracle as O
+from parallel_fem_codes_gb300 import meshgen as G
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def fg():
+    from parallel_fem_codes_gb300 import femgpu
+    femgpu.lib()
+    return femgpu
+
+
+# 128 FP64 rows (512 FP32) a CTA: 100, 256, 961, 1089, 4096 equations
+@pytest.mark.parametrize("side,kmax", [(12, 30), (18, 30), (33, 30), (35, 30), (66, 30), (33, 3), (35, 33), (35, 60), (12, 60)])
+def test_matches_the_oracle(fg, side, kmax):
+    p = G.transport_problem(side, angle_deg=40.0, k=1e-3)
+    m = p.mesh
+    A, F = O.build_k_f_supg(p)
+    lm = O.fill_lm(m)
+    perm, inv, _ = O.permutation_of_lm(m)
+    X0, it0, _, _, _ = O.ebe_diag_solve(lm, A, m.neq, F, perm, inv, kmax=kmax, lmax=3000, tol=1e-10)
+    s = fg.System(m)
+    s.set_blocks(A)
+    B = s.precond_setup(fg.FG_PRECOND_DIAG, 0, F)
+    r = s.solve(B, kmax=kmax, lmax=3000, tol=1e-10, F_true=F)
+    assert r.stats["converged"] == 1 and r.stats["status"] == 0
+    assert abs(r.stats["iterations"] - it0) <= 2
+    n = np.linalg.norm
+    assert n(r.x[:-1] - X0[:-1]) <= 1e-9 * n(X0[:-1])
+    q = s.solve(B, kmax=kmax, lmax=3000, tol=1e-12, F_true=F, precision=fg.FG_PREC_MIXED)
+    assert q.stats["converged"] == 1 and q.stats["true_rel_residual"] <= 1e-12
+    assert n(q.x[:-1] - X0[:-1]) <= 1e-8 * n(X0[:-1])
+    again = s.solve(B, kmax=kmax, lmax=3000, tol=1e-12, F_true=F, precision=fg.FG_PREC_MIXED)
+    assert np.array_equal(again.x, q.x) and again.stats["iterations"] == q.stats["iterations"]
+
+
+@pytest.mark.parametrize("precision", [64, 32])
+def test_a_batch_moves_on_chip(fg, precision):
+    # together more CTAs than are resident: the first cycles stream
+    probs = [G.transport_problem(n, angle_deg=15.0 * n, k=10.0 ** -(2 + n % 5)) for n in (40, 300, 301, 45, 302, 120)]
+    systems = [fg.transport_system(p) for p in probs]
+    for s, p in zip(systems, probs):
+        s.transport_prepare(p)
+    st = fg.solve_resident(systems, tol=1e-11, lmax=3000, precision=precision)
+    for s, p, q in zip(systems, probs, st):
+        assert q["converged"] == 1 and q["status"] == 0
+        x = s.solution()
+        s.transport_prepare(p)
+        F = s.transport_assemble(p)
+        res = np.linalg.norm((F - s.matvec(x))[:-1]) / np.linalg.norm(F[:-1])
+        assert res <= (1e-11 if precision == 32 else 1e-9)
+
+
+def test_breakdown_and_zero_right_hand_side(fg):
+    p = G.transport_problem(40, k=1e-2)
+    s = fg.transport_system(p)
+    F = s.transport_assemble(p)
+    B = s.precond_setup(fg.FG_PRECOND_DIAG, 0, F)
+    for prec in (64, 32):
+        z = s.solve(np.zeros_like(B), F_true=np.zeros_like(F), precision=prec)
+        assert z.stats["converged"] == 1 and not z.x.any()
+        bad = B.copy()
+        bad[7] = np.nan
+        r = s.solve(bad, precision=prec)
+        assert r.stats["converged"] == 0 and r.stats["status"] == fg.FG_ERR_BREAKDOWN
+        ok = s.solve(B, F_true=F, precision=prec)
+        assert ok.stats["converged"] == 1

@@ -50,7 +50,7 @@ def _dense(m, A):
     return K
 
 
-@pytest.mark.parametrize("kind", [(1, 1), (4, 6), (5, 5), (31, 1), (13, 17), "wheel"])
+@pytest.mark.parametrize("kind", [(1, 1), (4, 6), (5, 5), (31, 1), (13, 17), (23, 19), "wheel"])
 @pytest.mark.parametrize("ndof,reorder", [(1, True), (1, False), (2, False), (3, False), (3, True), (4, False), (4, True)])
 def test_solves_match_a_dense_solve(fg, kind, ndof, reorder):
     m = _mesh(kind, ndof, 3 + ndof)
