@@ -1,17 +1,16 @@
-// Arnoldi step and cycle-end kernels of the batched GMRES engine
-// (included by krylov.cu).
+// Arnoldi step and cycle-end kernels of the streaming restart cycle
+// (included by krylov.cu): two passes over the basis per step, V read once in
+// each.
 //
-// Every dof kernel walks parts of kPartMin..kPartMax dofs (the size is
-// chosen per batch from its total dofs).  Within a part the work
-// is split in two shapes so that loads are never serialised behind
-// reductions:
-//   * update passes are thread-per-dof: w[d] -= sum_j h_j V[j][d] with the
-//     j loop unrolled, so a thread keeps several independent basis loads
-//     in flight;
-//   * dot passes are warp-per-basis-vector: warp w accumulates
-//     <V[j], w> for j = w, w+8, ... over the whole part with four
-//     independent accumulators per lane and reduces once at the end.
-// Part results are combined by the last part of the system in fixed order.
+// The basis is kept unscaled: V[j] is the vector as the step left it and
+// vscale[j] the reciprocal of its norm, known when the step's last part sums
+// it, so that no pass is spent on scaling (an FP16 basis is scaled when it is
+// stored, vscale[j] = 1 / sigma).  Both passes walk parts of kPartMin..kPartMax
+// dofs (the size is chosen per batch from its total dofs), one CTA a part, a
+// 16-byte pack of every vector per thread and several basis vectors in
+// flight.  Part results are combined by the last part of the system in fixed
+// order.  HBM-bound in FP32; in FP64 the FP64 pipe (2 FMA per clock and SM)
+// binds: 3 (i + 1) FMA per dof and step.
 
 // 16-byte packs along the dof direction: parts start at multiples of the
 // pack width and vectors are zero beyond n up to n_pad, so a pack never
@@ -90,342 +89,172 @@ __device__ __forceinline__ void st_v(TV *p, const T (&o)[VPk<TV>::G])
     }
 }
 
-// dots of V[0..i] with w over a part: warp-per-j, results to out[j]
-template <typename T>
-__device__ __forceinline__ void part_dots(const SysDev &D, const DChunk &k, int i, const T *__restrict__ w,
+// <V[j], w> and <V[j], V[i]> for j = 0..i over a part, raw (V and w as
+// stored).  A thread holds a pack of w and of V[i] and JB basis vectors' packs
+// at a time, so that JB + 2 loads are in flight and w is read from L1 after
+// the first group; the 2 JB sums are folded over the warp by halving (a
+// value's lanes drop out as the values do), then over the warps.
+template <typename T, typename TV>
+__device__ __forceinline__ void part_dots(const SysDev &D, const DChunk &k, int i, const T *__restrict__ w, T (*sw)[2 * kMaxRestart],
                                           double *out)
 {
-    constexpr int N = Pk<T>::N;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const T *V = (const T *)D.V;
-    for (int j = warp; j <= i; j += kThreads / 32) {
-        const T *vj = V + (size_t)j * D.n_pad;
-        T a0 = 0, a1 = 0, a2 = 0, a3 = 0;
-        int q = k.d0 + lane * N;
-        for (; q + 3 * 32 * N < k.d1; q += 4 * 32 * N) {
-            auto v0 = ld_pk(vj + q), v1 = ld_pk(vj + q + 32 * N), v2 = ld_pk(vj + q + 64 * N), v3 = ld_pk(vj + q + 96 * N);
-            auto w0 = ld_pk(w + q), w1 = ld_pk(w + q + 32 * N), w2 = ld_pk(w + q + 64 * N), w3 = ld_pk(w + q + 96 * N);
-#pragma unroll
-            for (int c = 0; c < N; ++c) {
-                a0 += v0.v[c] * w0.v[c];
-                a1 += v1.v[c] * w1.v[c];
-                a2 += v2.v[c] * w2.v[c];
-                a3 += v3.v[c] * w3.v[c];
-            }
-        }
-        for (; q < k.d1; q += 32 * N) {
-            auto v0 = ld_pk(vj + q), w0 = ld_pk(w + q);
-#pragma unroll
-            for (int c = 0; c < N; ++c) a0 += v0.v[c] * w0.v[c];
-        }
-        double s = (double)((a0 + a1) + (a2 + a3));
-        s = warp_sum(s);
-        if (lane == 0) out[j] = s;
-    }
-}
-
-// dots of V[0..i] with w and with v = V[i] over a part, in one sweep of the
-// basis.  With nv = i + 1 >= 8 vectors, warp w takes j = w, w+8, w+16, w+24
-// (i < 32) together over the whole part, so each pack of w and v is loaded
-// once per warp whatever the number of its vectors.  With fewer vectors
-// the idle warps split the dofs instead: S = 8 / nv warps per vector, each
-// on every S-th pack, their sums added in slice order (deterministic).
-// <V[j], w> to out[j], <V[j], v> to out[i + 1 + j].  Every thread of the
-// block must call it (it synchronises when the part is sliced).
-template <typename T, typename TV = T>
-__device__ __forceinline__ void part_dots2(const SysDev &D, const DChunk &k, int i, const T *__restrict__ w,
-                                           double *out)
-{
-    constexpr int G = VPk<TV>::G;
-    constexpr int NW = kThreads / 32;
-    __shared__ double sl[2 * NW];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int nv = i + 1;
-    const int S = nv >= NW ? 1 : NW / nv;                  // warps per vector
-    const int j0 = S == 1 ? warp : warp / S, sidx = S == 1 ? 0 : warp % S;
-    const int nj = S == 1 ? (warp <= i ? (i - warp) / NW + 1 : 0) : (j0 < nv ? 1 : 0);
+    constexpr int G = VPk<TV>::G, JB = sizeof(T) == 8 ? 4 : sizeof(TV) == 2 ? 4 : 8, NV = 2 * JB;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nv = i + 1;
     const TV *V = (const TV *)D.V;
-    const TV *vi = V + (size_t)i * D.n_pad;
-    const TV *vj[4];
+    const size_t ld = (size_t)D.n_pad;
+    const TV *vi = V + (size_t)i * ld;
+    for (int j0 = 0; j0 < nv; j0 += JB) {
+        T s[NV];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) vj[u] = V + (size_t)min(j0 + NW * u, i) * D.n_pad;
-    T a[4], b[4];
+        for (int u = 0; u < NV; ++u) s[u] = (T)0;
+        for (int q = k.d0 + threadIdx.x * G; q < k.d1; q += kThreads * G) {
+            T w0[G], u0[G], v[JB][G];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) a[u] = b[u] = (T)0;
-    if (nj > 0) {
-#pragma unroll 1
-        for (int q = k.d0 + (lane + 32 * sidx) * G; q < k.d1; q += 32 * G * S) {
-            T w0[G], u0[G], v0[4][G];
+            for (int u = 0; u < JB; ++u) ld_v<T, TV>(V + min(j0 + u, i) * ld + q, v[u]);
             ld_g<T, G>(w + q, w0);
             ld_v<T, TV>(vi + q, u0);
 #pragma unroll
-            for (int u = 0; u < 4; ++u)
-                if (u < nj) ld_v<T, TV>(vj[u] + q, v0[u]);
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                if (u >= nj) break;
+            for (int u = 0; u < JB; ++u)
 #pragma unroll
                 for (int c = 0; c < G; ++c) {
-                    a[u] += v0[u][c] * w0[c];
-                    b[u] += v0[u][c] * u0[c];
+                    s[u] += v[u][c] * w0[c];
+                    s[JB + u] += v[u][c] * u0[c];
                 }
-            }
         }
-    }
-    if (S == 1) {
+        int o = 16;
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            if (u >= nj) break;
-            const double sa = warp_sum((double)a[u]), sb = warp_sum((double)b[u]);
-            if (lane == 0) {
-                out[j0 + NW * u] = sa;
-                out[i + 1 + j0 + NW * u] = sb;
+        for (int m = NV / 2; m >= 1; m >>= 1, o >>= 1) {
+            const bool up = (lane & o) != 0;
+#pragma unroll
+            for (int u = 0; u < m; ++u) {
+                const T keep = up ? s[u + m] : s[u], give = up ? s[u] : s[u + m];
+                s[u] = keep + __shfl_xor_sync(0xffffffffu, give, o);
             }
         }
-        return;
-    }
-    const double sa = warp_sum((double)a[0]), sb = warp_sum((double)b[0]);
-    if (lane == 0 && nj > 0) {
-        sl[2 * warp] = sa;
-        sl[2 * warp + 1] = sb;
+        for (; o > 0; o >>= 1) s[0] += __shfl_xor_sync(0xffffffffu, s[0], o);
+        // value index: the lane's upper bits, most significant first
+        constexpr int SH = NV == 16 ? 1 : 2;
+        const int idx = lane >> SH, j = j0 + (idx & (JB - 1));
+        if ((lane & ((1 << SH) - 1)) == 0 && j < nv) sw[warp][(idx < JB ? 0 : nv) + j] = s[0];
     }
     __syncthreads();
-    if (threadIdx.x < nv) {
-        const int j = threadIdx.x;
-        double ta = sl[2 * (j * S)], tb = sl[2 * (j * S) + 1];
-        for (int q = 1; q < S; ++q) {
-            ta += sl[2 * (j * S + q)];
-            tb += sl[2 * (j * S + q) + 1];
-        }
-        out[j] = ta;
-        out[i + 1 + j] = tb;
+    for (int j = threadIdx.x; j < 2 * nv; j += kThreads) {
+        Sum<T> t;
+#pragma unroll
+        for (int q = 0; q < kThreads / 32; ++q) t.add(sw[q][j]);
+        out[j] = t.value();
     }
 }
 
-// w[d] -= sum_{j<=i} h[j] V[j][d] for the dofs of the part (a pack per
-// thread, four basis vectors in flight); returns this thread's sum of the
-// new w^2 when want_norm.  Entries past n stay zero.
-template <typename T, typename TV = T>
-__device__ __forceinline__ double part_update(const SysDev &D, const DChunk &k, int i, const T *h, T *w,
-                                              bool want_norm)
+// Pass 1 (classical Gram-Schmidt with a Gram correction): s = V^T w (w = M^-1 A
+// v_i from the matvec) and the new column g = V^T v_i of the basis' Gram
+// matrix G in one sweep.  The last part forms c = s + (s - G s): the
+// coefficients of the two classical passes of CGS2 (h1 = s, h2 = V^T (w - V s) =
+// s - G s) with the second one taken from G instead of a second sweep; c becomes
+// column i of H and, unscaled, the update that k_orth applies.
+template <typename T, typename TV>
+__global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 3 : 2)
+k_dots(const SysDev *__restrict__ sys, const DChunk *__restrict__ ch, const int *__restrict__ nch, int i)
 {
-    constexpr int G = VPk<TV>::G;
-    const TV *V = (const TV *)D.V;
-    const size_t ld = (size_t)D.n_pad;
-    double nrm = 0.0;
-    for (int q = k.d0 + threadIdx.x * G; q < k.d1; q += blockDim.x * G) {
-        T s0[G], s1[G], s2[G], s3[G];
-        ld_g<T, G>(w + q, s0);
-#pragma unroll
-        for (int c = 0; c < G; ++c) s1[c] = s2[c] = s3[c] = (T)0;
-        int j = 0;
-        for (; j + 3 <= i; j += 4) {
-            T v0[G], v1[G], v2[G], v3[G];
-            ld_v<T, TV>(V + j * ld + q, v0);
-            ld_v<T, TV>(V + (j + 1) * ld + q, v1);
-            ld_v<T, TV>(V + (j + 2) * ld + q, v2);
-            ld_v<T, TV>(V + (j + 3) * ld + q, v3);
-            const T h0 = h[j], h1 = h[j + 1], h2 = h[j + 2], h3 = h[j + 3];
-#pragma unroll
-            for (int c = 0; c < G; ++c) {
-                s0[c] -= h0 * v0[c];
-                s1[c] -= h1 * v1[c];
-                s2[c] -= h2 * v2[c];
-                s3[c] -= h3 * v3[c];
-            }
-        }
-        for (; j <= i; ++j) {
-            T v0[G];
-            ld_v<T, TV>(V + j * ld + q, v0);
-            const T h0 = h[j];
-#pragma unroll
-            for (int c = 0; c < G; ++c) s0[c] -= h0 * v0[c];
-        }
-#pragma unroll
-        for (int c = 0; c < G; ++c) {
-            T v = (s0[c] + s1[c]) + (s2[c] + s3[c]);
-            s0[c] = v;
-            if (want_norm) nrm += (double)(v * v);
-        }
-        st_g<T, G>(w + q, s0);
-    }
-    return nrm;
-}
-
-// pass 1: h1_j = <v_j, w>, j = 0..i (w = M^-1 A v_i from the matvec)
-template <typename T>
-__global__ void __launch_bounds__(kThreads)
-k_dots1(const SysDev *__restrict__ sys, const DChunk *__restrict__ ch, const int *__restrict__ nch, int i)
-{
-    __shared__ double red[kPartStride];
-    __shared__ double tot[kPartStride];
+    __shared__ T sw[kThreads / 32][2 * kMaxRestart];
+    __shared__ double tot[2 * kMaxRestart];
     const int total = *nch;
     for (int c = blockIdx.x; c < total; c += gridDim.x) {
         const DChunk k = ch[c];
         const SysDev &D = sys[k.sys];
         if (!D.st->in_cycle) continue;
-        const T *w = (const T *)D.w;
         __syncthreads();
-        part_dots<T>(D, k, i, w, red);
-        __syncthreads();
-        for (int j = threadIdx.x; j <= i; j += blockDim.x) D.part[k.part * kPartStride + j] = red[j];
-        if (last_part(D, 1)) {
-            reduce_parts(D, i + 1, tot);
-            for (int j = threadIdx.x; j <= i; j += blockDim.x) D.H[j * D.kmax + i] = tot[j];
-        }
-    }
-}
-
-// Mixed-precision pass 1 (classical Gram-Schmidt with a Gram correction):
-// s = V^T w (w = M^-1 A v_i) and the new column g = V^T v_i of the
-// basis' Gram matrix G = V^T V in one sweep.  The last part forms
-// c = s + (s - G s): the coefficients of the two classical passes of CGS2
-// (h1 = s, h2 = V^T (w - V s) = s - G s) with the second one taken from G
-// instead of a second sweep over the basis; c becomes column i of H and
-// the update that k_orth2 applies.  Used when kmax <= 32.
-template <typename T, typename TV = T>
-__global__ void __launch_bounds__(kThreads)
-k_dots1g(const SysDev *__restrict__ sys, const DChunk *__restrict__ ch, const int *__restrict__ nch, int i)
-{
-    __shared__ double red[kPartStride];
-    __shared__ double tot[kPartStride];
-    const int total = *nch;
-    for (int c = blockIdx.x; c < total; c += gridDim.x) {
-        const DChunk k = ch[c];
-        const SysDev &D = sys[k.sys];
-        if (!D.st->in_cycle) continue;
-        const T *w = (const T *)D.w;
-        __syncthreads();
-        part_dots2<T, TV>(D, k, i, w, red);
-        __syncthreads();
-        for (int j = threadIdx.x; j < 2 * (i + 1); j += blockDim.x) D.part[k.part * kPartStride + j] = red[j];
+        part_dots<T, TV>(D, k, i, (const T *)D.w, sw, D.part + k.part * kPartStride);
         if (last_part(D, 1)) {
             reduce_parts(D, 2 * (i + 1), tot);
             const int km = D.kmax;
-            // the stored basis is sigma V: dots carry 1 / sigma, Gram entries 1 / sigma^2
-            const double s1 = D.vsci, s2 = (double)D.vsci * D.vsci;
-            for (int j = threadIdx.x; j <= i; j += blockDim.x) {
-                D.G[j * km + i] = tot[i + 1 + j] * s2;
-                D.G[i * km + j] = tot[i + 1 + j] * s2;
+            const double *vs = D.vscale;
+            const double ws = std::is_same<T, TV>::value ? vs[i] : 1.0;   // the scale of w as stored
+            for (int j = threadIdx.x; j <= i; j += kThreads) {
+                const double g = tot[i + 1 + j] * vs[j] * vs[i];
+                D.G[j * km + i] = g;
+                D.G[i * km + j] = g;
+                tot[j] *= vs[j] * ws;
             }
             __syncthreads();
-            for (int j = threadIdx.x; j <= i; j += blockDim.x) {
+            for (int j = threadIdx.x; j <= i; j += kThreads) {
                 double gs = 0.0;
-                for (int l = 0; l <= i; ++l) gs += D.G[j * km + l] * (tot[l] * s1);
-                const double cj = tot[j] * s1 + (tot[j] * s1 - gs);
-                D.H[j * km + i] = cj;
-                D.hbuf[j] = cj;
+                for (int l = 0; l <= i; ++l) gs += D.G[l * km + j] * tot[l];
+                const double cj = tot[j] + (tot[j] - gs);
+                D.hcol[j] = cj;
+                D.hbuf[j] = cj * vs[j];
             }
         }
     }
 }
 
-// pass 2: w -= sum_j h1_j v_j ; h2_j = <v_j, w>
-template <typename T>
-__global__ void __launch_bounds__(kThreads)
-k_orth1(const SysDev *__restrict__ sys, const DChunk *__restrict__ ch, const int *__restrict__ nch, int i)
+// Pass 2: the new vector w - V c, unscaled, into V[i+1] (an FP16 basis: in
+// place, k_normalize stores it), and its norm; then, in the last part, the
+// Givens step and the cycle's stop test.
+template <typename T, typename TV>
+__global__ void __launch_bounds__(kThreads, 4)
+k_orth(const SysDev *__restrict__ sys, const DChunk *__restrict__ ch, const int *__restrict__ nch, int i)
 {
-    __shared__ double red[kPartStride];
-    __shared__ double tot[kPartStride];
-    __shared__ T hs[kPartStride];
-    const int total = *nch;
-    for (int c = blockIdx.x; c < total; c += gridDim.x) {
-        const DChunk k = ch[c];
-        const SysDev &D = sys[k.sys];
-        if (!D.st->in_cycle) continue;
-        T *w = (T *)D.w;
-        for (int j = threadIdx.x; j <= i; j += blockDim.x) hs[j] = (T)D.H[j * D.kmax + i];
-        __syncthreads();
-        part_update<T>(D, k, i, hs, w, false);
-        __syncthreads();
-        part_dots<T>(D, k, i, w, red);
-        __syncthreads();
-        for (int j = threadIdx.x; j <= i; j += blockDim.x) D.part[k.part * kPartStride + j] = red[j];
-        if (last_part(D, 2)) {
-            reduce_parts(D, i + 1, tot);
-            for (int j = threadIdx.x; j <= i; j += blockDim.x) {
-                D.hbuf[j] = tot[j];
-                D.H[j * D.kmax + i] += tot[j];
-            }
-        }
-    }
-}
-
-// Back-substitution of the cycle's least-squares problem (pgmres.c:163-171)
-// into D.y; one thread.
-__device__ __forceinline__ void solve_y(const SysDev &D, int m)
-{
-    const int km = D.kmax;
-    if (m <= 0) return;
-    int i = m - 1;
-    D.y[i] = D.g[i] / D.H[i * km + i];
-    for (int j = i - 1; j >= 0; --j) {
-        double s = 0.0;
-        for (int q = j + 1; q <= i; ++q) s = s + D.H[j * km + q] * D.y[q];
-        D.y[j] = (D.g[j] - s) / D.H[j * km + j];
-    }
-}
-
-// The last part's step after pass 3 (pgmres.c:111-157): h(i+1,i) = ||w||
-// from the summed squares, the earlier rotations applied to column i, the
-// new rotation, the residual estimate and the cycle's stop test; at the
-// end of a cycle the solution of the triangular system.  One thread.
-__device__ __forceinline__ void givens_step(const SysDev &D, int i, double sumsq)
-{
-    SysState *st = D.st;
-    const int km = D.kmax;
-    double *H = D.H, *cs = D.cs, *sn = D.sn, *g = D.g;
-    double hn = sqrt(sumsq);
-    st->hn = hn;
-    H[(i + 1) * km + i] = hn;
-    for (int j = 0; j <= i - 1; ++j) {
-        double h1 = cs[j] * H[j * km + i] + sn[j] * H[(j + 1) * km + i];
-        double h2 = -sn[j] * H[j * km + i] + cs[j] * H[(j + 1) * km + i];
-        H[j * km + i] = h1;
-        H[(j + 1) * km + i] = h2;
-    }
-    double r = sqrt(H[i * km + i] * H[i * km + i] + H[(i + 1) * km + i] * H[(i + 1) * km + i]);
-    cs[i] = H[i * km + i] / r;
-    sn[i] = H[(i + 1) * km + i] / r;
-    H[i * km + i] = r;
-    H[(i + 1) * km + i] = 0.0;
-    g[i + 1] = -sn[i] * g[i];
-    g[i] = cs[i] * g[i];
-    st->rho = fabs(g[i + 1]);
-    st->steps = i + 1;
-    st->iterations += 1;
-    double target = D.mixed ? st->target : st->eps;
-    if (!(r > 0.0) || !isfinite(st->rho)) {
-        st->status = FG_ERR_BREAKDOWN;
-        st->in_cycle = 0;
-        if (!(r > 0.0)) st->steps = i;     // column i unusable
-    } else if (!(st->rho > target) || i + 1 >= D.kmax - 1 || !(hn > 0.0)) {
-        st->in_cycle = 0;
-    }
-    if (!st->in_cycle) solve_y(D, st->steps);
-}
-
-// pass 3: w -= sum_j h2_j v_j ; ||w||; then, in the last part, the Givens
-// step (givens_step).
-template <typename T, typename TV = T>
-__global__ void __launch_bounds__(kThreads)
-k_orth2(const SysDev *__restrict__ sys, const DChunk *__restrict__ ch, const int *__restrict__ nch, int i)
-{
-    __shared__ double red[kThreads / 32];
-    __shared__ double tot[1];
-    __shared__ T hs[kPartStride];
+    constexpr int G = VPk<TV>::G, JB = sizeof(TV) == 2 ? 4 : 8;
+    __shared__ T hs[kMaxRestart + 4];
+    __shared__ double red[kThreads / 32], st_t[kMaxRestart + 4], st_a[kMaxRestart + 4], tot[2];
     const int total = *nch;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     for (int c = blockIdx.x; c < total; c += gridDim.x) {
         const DChunk k = ch[c];
         const SysDev &D = sys[k.sys];
         if (!D.st->in_cycle) continue;
-        T *w = (T *)D.w;
-        for (int j = threadIdx.x; j <= i; j += blockDim.x) hs[j] = (T)(D.hbuf[j] * D.vsci);
         __syncthreads();
-        double acc = part_update<T, TV>(D, k, i, hs, w, true);
-        acc = warp_sum(acc);
-        if (lane == 0) red[warp] = acc;
+        for (int j = threadIdx.x; j <= i; j += kThreads) hs[j] = (T)D.hbuf[j];
+        __syncthreads();
+        const TV *V = (const TV *)D.V;
+        const size_t ld = (size_t)D.n_pad;
+        const T *w = (const T *)D.w;
+        T *out = std::is_same<T, TV>::value ? (T *)D.V + (size_t)(i + 1) * ld : (T *)D.w;
+        const T ws = std::is_same<T, TV>::value ? (T)D.vscale[i] : (T)1;
+        Sum<T> nrm;
+        for (int q = k.d0 + threadIdx.x * G; q < k.d1; q += kThreads * G) {
+            T s0[G], s1[G];
+            ld_g<T, G>(w + q, s0);
+#pragma unroll
+            for (int u = 0; u < G; ++u) { s0[u] *= ws; s1[u] = (T)0; }
+            int j = 0;
+            for (; j + JB <= i + 1; j += JB) {
+                T v[JB][G];
+#pragma unroll
+                for (int u = 0; u < JB; ++u) ld_v<T, TV>(V + (j + u) * ld + q, v[u]);
+#pragma unroll
+                for (int u = 0; u < JB; u += 2) {
+                    const T h0 = hs[j + u], h1 = hs[j + u + 1];
+#pragma unroll
+                    for (int e = 0; e < G; ++e) {
+                        s0[e] -= h0 * v[u][e];
+                        s1[e] -= h1 * v[u + 1][e];
+                    }
+                }
+            }
+            if (j <= i) {                     // the rest: loads past i repeat V[i], unused
+                T v[JB][G];
+#pragma unroll
+                for (int u = 0; u < JB - 1; ++u) ld_v<T, TV>(V + min(j + u, i) * ld + q, v[u]);
+#pragma unroll
+                for (int u = 0; u < JB - 1; ++u) {
+                    if (j + u > i) break;
+                    const T h0 = hs[j + u];
+#pragma unroll
+                    for (int e = 0; e < G; ++e) s0[e] -= h0 * v[u][e];
+                }
+            }
+#pragma unroll
+            for (int e = 0; e < G; ++e) {
+                s0[e] = q + e < D.n ? s0[e] + s1[e] : (T)0;
+                nrm.add_square(s0[e]);
+            }
+            st_g<T, G>(out + q, s0);
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) nrm.fold(o);
+        if (lane == 0) red[warp] = nrm.value();
         __syncthreads();
         if (threadIdx.x == 0) {
             double s = 0;
@@ -434,13 +263,29 @@ k_orth2(const SysDev *__restrict__ sys, const DChunk *__restrict__ ch, const int
         }
         if (last_part(D, 3)) {
             reduce_parts(D, 1, tot);
-            if (threadIdx.x == 0) givens_step(D, i, tot[0]);
+            if (warp == 0) {
+                SysState *st = D.st;
+                const double hn = sqrt(tot[0]);
+                Rot R{D.cs, D.sn, D.g, st_t, st_a, 0, 0, 0, 0.0};
+                const bool stop = givens<double>(D.H, D.kmax, R, i, D.hcol, hn, D.mixed ? st->target : st->eps);
+                __syncwarp();
+                if (lane == 0) {
+                    st->hn = hn;
+                    D.vscale[i + 1] = std::is_same<T, TV>::value ? 1.0 / hn : (double)D.vsci;
+                    st->rho = R.rho;
+                    st->steps = R.steps;
+                    st->iterations += 1;
+                    if (R.breakdown) st->status = FG_ERR_BREAKDOWN;
+                    if (stop) st->in_cycle = 0;
+                }
+                if (stop) back_substitute(D.H, D.kmax, D.g, R.steps, D.y);
+            }
         }
     }
 }
 
-// v_{i+1} = w * (1 / h_{i+1,i}) (pgmres.c:117)
-template <typename T, typename TV = T>
+// FP16 basis: v_{i+1} = w * (1 / h_{i+1,i}) (pgmres.c:117), stored as sigma v
+template <typename T, typename TV>
 __global__ void __launch_bounds__(kThreads)
 k_normalize(const SysDev *__restrict__ sys, const DChunk *__restrict__ ch, const int *__restrict__ nch, int i)
 {
@@ -449,11 +294,11 @@ k_normalize(const SysDev *__restrict__ sys, const DChunk *__restrict__ ch, const
         const DChunk k = ch[c];
         const SysDev &D = sys[k.sys];
         if (!D.st->in_cycle) continue;
-        const T sc = (T)((double)D.vsc / D.st->hn);     // stored as sigma v
+        const T sc = (T)((double)D.vsc / D.st->hn);
         const T *w = (const T *)D.w;
         TV *v = (TV *)D.V + (size_t)(i + 1) * D.n_pad;
         constexpr int G = VPk<TV>::G;
-        for (int q = k.d0 + threadIdx.x * G; q < k.d1; q += blockDim.x * G) {
+        for (int q = k.d0 + threadIdx.x * G; q < k.d1; q += kThreads * G) {
             T p[G];
             ld_g<T, G>(w + q, p);
 #pragma unroll
@@ -464,13 +309,15 @@ k_normalize(const SysDev *__restrict__ sys, const DChunk *__restrict__ ch, const
 }
 
 // ---------------------------------------------------------------- cycle end
-// x += V y (pgmres.c:173-175) with y from k_orth2; the last part does the
-// restart bookkeeping (:177-179).
-template <typename T, typename TV = T>
+// x += V y (pgmres.c:173-175) with y from k_orth; the last part does the
+// restart bookkeeping (:177-179).  FP32: the sum of the products in error-free
+// FP32 pairs (an FP64 FMA and a conversion a value bound this pass).
+template <typename T, typename TV>
 __global__ void __launch_bounds__(kThreads)
 k_update(const SysDev *__restrict__ sys, const DChunk *__restrict__ ch, const int *__restrict__ nch)
 {
-    __shared__ double y[kPartStride];
+    __shared__ double y[kMaxRestart];
+    __shared__ float yh[kMaxRestart], yl[kMaxRestart];
     const int total = *nch;
     for (int c = blockIdx.x; c < total; c += gridDim.x) {
         const DChunk k = ch[c];
@@ -478,22 +325,26 @@ k_update(const SysDev *__restrict__ sys, const DChunk *__restrict__ ch, const in
         if (!D.st->live) continue;
         const int m = D.st->steps;
         __syncthreads();
-        for (int j = threadIdx.x; j < m; j += blockDim.x) y[j] = D.y[j] * D.vsci;
+        for (int j = threadIdx.x; j < m; j += kThreads) {
+            const double v = D.y[j] * D.vscale[j];
+            y[j] = v;
+            yh[j] = (float)v;
+            yl[j] = (float)(v - (double)(float)v);
+        }
         __syncthreads();
         const TV *V = (const TV *)D.V;
         const size_t ld = (size_t)D.n_pad;
-        // a 16-byte pack of the basis per thread and four vectors in flight;
-        // each dof still adds v_j y_j in j order (x and V are zero-padded to
-        // n_pad, so the pack past n adds zeros)
+        // (x and V are zero-padded to n_pad, so the pack past n adds zeros)
         constexpr int N = VPk<TV>::G;
-        for (int q = k.d0 + threadIdx.x * N; q < k.d1; q += blockDim.x * N) {
-            double xv[N];
+        for (int q = k.d0 + threadIdx.x * N; q < k.d1; q += kThreads * N) {
+            Sum<T> s[N];
+            auto take = [&](int j, const T (&v)[N]) {
 #pragma unroll
-            for (int c = 0; c < N; c += 2) {
-                const double2 x2 = *reinterpret_cast<const double2 *>(D.x + q + c);
-                xv[c] = x2.x;
-                xv[c + 1] = x2.y;
-            }
+                for (int e = 0; e < N; ++e) {
+                    if constexpr (sizeof(T) == 8) s[e].h += v[e] * y[j];
+                    else s[e].add_product(yh[j], yl[j], v[e]);
+                }
+            };
             int j = 0;
             for (; j + 3 < m; j += 4) {
                 T v0[N], v1[N], v2[N], v3[N];
@@ -501,25 +352,23 @@ k_update(const SysDev *__restrict__ sys, const DChunk *__restrict__ ch, const in
                 ld_v<T, TV>(V + (j + 1) * ld + q, v1);
                 ld_v<T, TV>(V + (j + 2) * ld + q, v2);
                 ld_v<T, TV>(V + (j + 3) * ld + q, v3);
-                const double y0 = y[j], y1 = y[j + 1], y2 = y[j + 2], y3 = y[j + 3];
-#pragma unroll
-                for (int c = 0; c < N; ++c) {
-                    xv[c] = xv[c] + (double)v0[c] * y0;
-                    xv[c] = xv[c] + (double)v1[c] * y1;
-                    xv[c] = xv[c] + (double)v2[c] * y2;
-                    xv[c] = xv[c] + (double)v3[c] * y3;
-                }
+                take(j, v0);
+                take(j + 1, v1);
+                take(j + 2, v2);
+                take(j + 3, v3);
             }
             for (; j < m; ++j) {
                 T v0[N];
                 ld_v<T, TV>(V + j * ld + q, v0);
-                const double y0 = y[j];
-#pragma unroll
-                for (int c = 0; c < N; ++c) xv[c] = xv[c] + (double)v0[c] * y0;
+                take(j, v0);
             }
 #pragma unroll
-            for (int c = 0; c < N; c += 2)
-                *reinterpret_cast<double2 *>(D.x + q + c) = make_double2(xv[c], xv[c + 1]);
+            for (int e = 0; e < N; e += 2) {
+                double2 x2 = *reinterpret_cast<const double2 *>(D.x + q + e);
+                x2.x += s[e].value();
+                x2.y += s[e + 1].value();
+                *reinterpret_cast<double2 *>(D.x + q + e) = x2;
+            }
         }
         if (last_part(D, 4)) {
             if (threadIdx.x == 0) {

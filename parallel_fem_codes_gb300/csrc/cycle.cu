@@ -55,7 +55,7 @@
 #include <mutex>
 #include <type_traits>
 
-#include "system.h"
+#include "sums.cuh"
 
 namespace fg {
 
@@ -133,64 +133,18 @@ template <typename T> __device__ __forceinline__ T from_words(const unsigned *v)
     else return __uint_as_float(v[0]);
 }
 
-// ---------------------------------------------------------------- sums
-// Running sum of T values with the error of a 48-bit (FP32) or plain (FP64)
-// accumulator: FP32 by error-free two-sums, because this part's FP64 pipe
-// issues one warp instruction in 16 cycles.
-template <typename T> struct Sum;
-template <> struct Sum<double> {
-    double h = 0.0;
-    __device__ __forceinline__ void put_pair(u64 *p, unsigned tag) const { put<double>(p, h, tag); }
-    __device__ __forceinline__ void add_pair(const unsigned *v) { h += from_words<double>(v); }
-    __device__ __forceinline__ double rounded() const { return h; }
-    __device__ __forceinline__ void add(double v) { h += v; }
-    __device__ __forceinline__ void add_square(double v) { h += v * v; }
-    __device__ __forceinline__ void fold(int o) { h += __shfl_xor_sync(0xffffffffu, h, o); }
-    __device__ __forceinline__ double value() const { return h; }
-};
-template <> struct Sum<float> {
-    float h = 0.f, l = 0.f;
-    __device__ __forceinline__ void put_pair(u64 *p, unsigned tag) const
-    {
-        put2(p, __float_as_uint(h), __float_as_uint(l), tag);
-    }
-    __device__ __forceinline__ void add_pair(const unsigned *v)
-    {
-        add(__uint_as_float(v[0]));
-        l = __fadd_rn(l, __uint_as_float(v[1]));
-    }
-    __device__ __forceinline__ float rounded() const { return __fadd_rn(h, l); }
-    __device__ __forceinline__ void add(float v)
-    {
-        const float s = __fadd_rn(h, v), t = __fsub_rn(s, h);
-        l = __fadd_rn(l, __fadd_rn(__fsub_rn(h, __fsub_rn(s, t)), __fsub_rn(v, t)));
-        h = s;
-    }
-    __device__ __forceinline__ void add_square(float v)
-    {
-        const float p = __fmul_rn(v, v);
-        l = __fadd_rn(l, __fmaf_rn(v, v, -p));
-        add(p);
-    }
-    // h += a b, exact product of a float pair and a float
-    __device__ __forceinline__ void add_product(float ah, float al, float b)
-    {
-        const float p = __fmul_rn(ah, b);
-        l = __fadd_rn(l, __fmaf_rn(al, b, __fmaf_rn(ah, b, -p)));
-        add(p);
-    }
-    __device__ __forceinline__ void fold(int o)
-    {
-        const float oh = __shfl_xor_sync(0xffffffffu, h, o), ol = __shfl_xor_sync(0xffffffffu, l, o);
-        // the two partners add in the same order, so both hold the same sum
-        const bool up = (threadIdx.x & o) != 0;
-        const float ah = up ? oh : h, al = up ? ol : l, bh = up ? h : oh, bl = up ? l : ol;
-        h = ah;
-        l = __fadd_rn(al, bl);
-        add(bh);
-    }
-    __device__ __forceinline__ double value() const { return (double)h + (double)l; }
-};
+// a sum as two words of the exchange
+__device__ __forceinline__ void put_pair(u64 *p, const Sum<double> &t, unsigned tag) { put<double>(p, t.h, tag); }
+__device__ __forceinline__ void put_pair(u64 *p, const Sum<float> &t, unsigned tag)
+{
+    put2(p, __float_as_uint(t.h), __float_as_uint(t.l), tag);
+}
+__device__ __forceinline__ void add_pair(Sum<double> &t, const unsigned *v) { t.add(from_words<double>(v)); }
+__device__ __forceinline__ void add_pair(Sum<float> &t, const unsigned *v)
+{
+    t.add(__uint_as_float(v[0]));
+    t.l = __fadd_rn(t.l, __uint_as_float(v[1]));
+}
 
 // ---------------------------------------------------------------- rows
 template <int B, typename T> __device__ __forceinline__ void load_vals(const T *p, T (&a)[B])
@@ -283,82 +237,6 @@ __device__ __forceinline__ T row_times_x(const int *__restrict__ off, const int 
 
 __device__ __forceinline__ void sync_workers() { asm volatile("bar.sync 1, %0;\n" ::"n"(kWorkers) : "memory"); }
 
-// Givens step i (pgmres.c:111-157) by one warp of rank 0: the coefficients
-// h[0..i] and h(i+1, i) = hn of column i; rotations and right-hand side in
-// shared memory, the rotated column to D.H.  The recurrence down the column
-// is one FMA a row (its products are formed by the lanes).  Returns true when
-// the cycle ends.
-template <typename T> struct Rot {
-    double *cs, *sn, *g, *t, *a;    // kmax each (g: + 1); t, a: scratch
-    int iters, steps, breakdown;
-    double rho;
-};
-template <typename T>
-__device__ __forceinline__ bool givens(const SysDev &D, Rot<T> &R, int i, const T *h, double hn, double target)
-{
-    const int km = D.kmax, lane = threadIdx.x & 31;
-    for (int j = lane; j < i; j += 32) R.t[j] = R.cs[j] * (double)h[j + 1];
-    __syncwarp();
-    if (lane == 0) {
-        double a = (double)h[0];
-        for (int j = 0; j < i; ++j) {
-            R.a[j] = a;
-            a = fma(-R.sn[j], a, R.t[j]);
-        }
-        R.a[i] = a;
-    }
-    __syncwarp();
-    for (int j = lane; j < i; j += 32) D.H[j * km + i] = R.cs[j] * R.a[j] + R.sn[j] * (double)h[j + 1];
-    const double a = R.a[i], q = a * a + hn * hn, ri = rsqrt(q), r = q * ri;
-    const double cs = a * ri, sn = hn * ri, gi = R.g[i];
-    __syncwarp();
-    if (lane == 0) {
-        R.cs[i] = cs;
-        R.sn[i] = sn;
-        D.H[i * km + i] = r;
-        R.g[i + 1] = -sn * gi;
-        R.g[i] = cs * gi;
-    }
-    __syncwarp();
-    R.rho = fabs(sn * gi);
-    R.iters = R.steps = i + 1;
-    if (!(q > 0.0) || !isfinite(R.rho)) {
-        R.breakdown = 1;
-        if (!(q > 0.0)) R.steps = i;         // column i unusable
-        return true;
-    }
-    return !(R.rho > target) || i + 1 >= km - 1 || !(hn > 0.0);
-}
-
-// y of the cycle's triangular system (pgmres.c:163-171) by one warp: columns
-// from the last to the first, each lane keeping two rows of the right-hand side
-template <typename T> __device__ __forceinline__ void back_substitute(const SysDev &D, const Rot<T> &R, int m, double *y)
-{
-    const int lane = threadIdx.x & 31, km = D.kmax;
-    double g0 = lane < m ? R.g[lane] : 0.0, g1 = lane + 32 < m ? R.g[lane + 32] : 0.0;
-    const double d0 = lane < m ? 1.0 / D.H[lane * km + lane] : 0.0;
-    const double d1 = lane + 32 < m ? 1.0 / D.H[(lane + 32) * km + lane + 32] : 0.0;
-    for (int c1 = m - 1; c1 >= 0; c1 -= 4) {
-        double h0[4], h1[4];                 // four columns' loads together
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int c = c1 - q;
-            h0[q] = lane < c ? D.H[lane * km + c] : 0.0;
-            h1[q] = lane + 32 < c ? D.H[(lane + 32) * km + c] : 0.0;
-        }
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int c = c1 - q;
-            if (c < 0) break;
-            const double yc = __shfl_sync(0xffffffffu, c < 32 ? g0 * d0 : g1 * d1, c & 31);
-            if (lane == 0) y[c] = yc;
-            g0 -= h0[q] * yc;
-            g1 -= h1[q] * yc;
-        }
-    }
-    __syncwarp();
-}
-
 // 1 / sqrt(n2) in T
 __device__ __forceinline__ float inv_norm(const Sum<float> &n2) { return rsqrtf(n2.rounded()); }
 __device__ __forceinline__ double inv_norm(const Sum<double> &n2) { return rsqrt(n2.h); }
@@ -375,7 +253,7 @@ template <typename T, int B>
 __global__ void __launch_bounds__(kCycThreads, 2)
 k_cycle(const SysDev *__restrict__ sys, const CycItem *__restrict__ items, const int *__restrict__ ioff, int smem)
 {
-    constexpr int N = Pack<T>::N, KM = kPartStride, WP = kWords<T>;
+    constexpr int N = Pack<T>::N, KM = kMaxRestart + 4, WP = kWords<T>;
     extern __shared__ __align__(16) unsigned char cyc_smem[];
     T *V = reinterpret_cast<T *>(cyc_smem);
     __shared__ double s_cs[KM], s_sn[KM], s_g[KM + 1], s_t[KM], s_a[KM];
@@ -409,7 +287,7 @@ k_cycle(const SysDev *__restrict__ sys, const CycItem *__restrict__ items, const
         const bool direct = g <= (sizeof(T) == 8 ? kDirect64 : kDirect32);
         const int pre = D.precond;
         const double target = D.mixed ? D.st->target : D.st->eps;
-        Rot<T> R{s_cs, s_sn, s_g, s_t, s_a, 0, 0, 0, 0.0};
+        Rot R{s_cs, s_sn, s_g, s_t, s_a, 0, 0, 0, 0.0};
         const int lo = max(k.u0 - D.rw_lo, 0), hi = min(k.u1 + D.rw_hi, D.nunits);
         const int nhl = (k.u0 - lo) * B, nh = nhl + (hi - k.u1) * B;
         Newest<T> X{V, halo, k.u0, k.u1, lo};
@@ -580,7 +458,7 @@ k_cycle(const SysDev *__restrict__ sys, const CycItem *__restrict__ items, const
 #pragma unroll
                 for (int o = 16; o > 0; o >>= 1) n2.fold(o);
                 if (g > 1 && lane == 0) {
-                    n2.put_pair(norm + 2 * rank, tag);
+                    put_pair(norm + 2 * rank, n2, tag);
                     if (rank == 0) put1(note + (i & 1), (unsigned)s_stop, tag);
                 }
             }
@@ -655,16 +533,16 @@ k_cycle(const SysDev *__restrict__ sys, const CycItem *__restrict__ items, const
 #pragma unroll
                             for (int q = 0; q < K; ++q) {
                                 const unsigned v[2] = {lw[q], hw[q]};
-                                t.add_pair(v);
+                                add_pair(t, v);
                             }
                         }
 #pragma unroll
                         for (int o = 16; o > 0; o >>= 1) t.fold(o);
-                        if (!direct && lane == 0) t.put_pair(total + (size_t)2 * km * WP, tag);
+                        if (!direct && lane == 0) put_pair(total + (size_t)2 * km * WP, t, tag);
                     } else {
                         unsigned v[2];
                         poll<2>(total + (size_t)2 * km * WP, 1, 2, tag, v, gave_up);
-                        t.add_pair(v);
+                        add_pair(t, v);
                     }
                     n2 = t;
                 }
@@ -763,7 +641,7 @@ k_cycle(const SysDev *__restrict__ sys, const CycItem *__restrict__ items, const
                 // ---- the rotations of column i - 1, beside the rest of the step
                 asm volatile("bar.sync 2, %0;\n" ::"n"(kCycThreads) : "memory");
                 if (rank == 0 && i > 0) {
-                    const bool stop = givens<T>(D, R, i - 1, s_c[(i - 1) & 1], 1.0 / (double)sc, target);
+                    const bool stop = givens<T>(D.H, km, R, i - 1, s_c[(i - 1) & 1], 1.0 / (double)sc, target);
                     if (lane == 0) s_stop = stop;
                 }
             }
@@ -782,7 +660,7 @@ k_cycle(const SysDev *__restrict__ sys, const CycItem *__restrict__ items, const
 #pragma unroll
                 for (int o = 8; o > 0; o >>= 1) t.fold(o);
                 if (rank != 0) {
-                    if (lane == 0) t.put_pair(norm2 + (i & 1) * (2 * (size_t)g) + 2 * rank, ntag);
+                    if (lane == 0) put_pair(norm2 + (i & 1) * (2 * (size_t)g) + 2 * rank, t, ntag);
                 } else {
                     Sum<T> u;
                     if (lane == 0) u = t;
@@ -790,18 +668,18 @@ k_cycle(const SysDev *__restrict__ sys, const CycItem *__restrict__ items, const
                         if (q == 0) continue;
                         unsigned v[2];
                         poll<2>(norm2 + (i & 1) * (2 * (size_t)g) + 2 * q, 1, 2, ntag, v, gave_up);
-                        u.add_pair(v);
+                        add_pair(u, v);
                     }
 #pragma unroll
                     for (int o = 16; o > 0; o >>= 1) u.fold(o);
                     __syncwarp();
-                    if (!s_stop) givens<T>(D, R, i - 1, s_c[(i - 1) & 1], sqrt(u.value()), target);
+                    if (!s_stop) givens<T>(D.H, km, R, i - 1, s_c[(i - 1) & 1], sqrt(u.value()), target);
                 }
             }
             if (rank == 0) {
                 const int m = R.steps;
                 __syncwarp();
-                back_substitute<T>(D, R, m, y);
+                back_substitute(D.H, km, s_g, m, y);
                 if (g > 1)
                     for (int j = lane; j < m; j += 32) put<double>(note + 3 + 2 * j, y[j], ytag);
                 if (lane == 0) {

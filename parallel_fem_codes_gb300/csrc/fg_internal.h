@@ -228,14 +228,15 @@ struct SysDev {
     void *V;                   // kmax vectors of T, stride n_pad
     void *w, *t;               // T vectors
     double *H;                 // (kmax+1) x kmax, H[j*kmax + i]
-    double *g, *cs, *sn, *hbuf, *y;  // kmax+1 each
-    double *G;                 // kmax x kmax Gram matrix of the basis (mixed precision)
+    double *g, *cs, *sn, *hbuf, *y, *hcol, *vscale;  // kmax+1 each
+    double *G;                 // kmax x kmax Gram matrix of the basis
     double *part;              // nparts x kPartStride
     unsigned *counter;         // 4 counters (one per reduction kernel kind)
     SysState *st;
 };
 constexpr int kIluWsChunk = 8;      // rows per staged chunk of the warp-per-block ILU substitutions
-constexpr int kPartStride = 64;    // doubles per part (>= kmax + 2, kmax <= 60)
+constexpr int kMaxRestart = 60;     // largest kmax
+constexpr int kPartStride = 128;    // doubles per part (>= 2 kmax)
 
 // Preconditioners applied by kernels of their own between the matvec and
 // the Arnoldi pass (the others are fused into the vector kernels).

@@ -5,10 +5,11 @@
 // Arnoldi steps per cycle (pgmres.c:159), Givens rotations (:120-155),
 // back-substitution (:163-171) and X += V y (:173-175).  The reference's
 // modified Gram-Schmidt with one MPI_Allreduce per dot becomes classical
-// Gram-Schmidt with reorthogonalisation (CGS2): three streaming passes over
-// the basis per step, each ending in a deterministic device-wide reduction
-// (fixed part order, "last part reduces"), instead of 2(i+1) dependent
-// reductions.
+// Gram-Schmidt with a Gram correction (the second classical pass' coefficients
+// from the basis' Gram matrix): two streaming passes over the basis per step,
+// each ending in a deterministic device-wide reduction (fixed part order, "last
+// part reduces"), instead of 2(i+1) dependent reductions; batches that fit it
+// run their cycles on chip (cycle.cu).
 //
 // Work decomposition.  A batch holds any number of systems.  The operator
 // is the assembled one (rows.cu), cut into unit chunks, dof work into parts
@@ -30,7 +31,7 @@
 #include <mutex>
 #include <tuple>
 
-#include "system.h"
+#include "sums.cuh"
 
 namespace fg {
 
@@ -75,18 +76,33 @@ __device__ __forceinline__ bool last_part(const SysDev &D, int slot)
     return s_last != 0;
 }
 
-// Deterministic sum over parts of slots [0, nv): warp w reduces slots
-// w, w+8, ...; lane l adds parts l, l+32, ... in order, then a fixed
-// butterfly.  Results to out[] (shared or global).
+// Deterministic sum over parts of slots [0, nv), nv <= kPartStride: thread
+// (sub, slot) adds parts sub, sub + S, ... in order (consecutive slots are
+// consecutive addresses; the fewest FP64 instructions), then the S subs in
+// order.  Results to out[] (shared).
 __device__ __forceinline__ void reduce_parts(const SysDev &D, int nv, double *out)
 {
-    int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int j = warp; j < nv; j += kThreads / 32) {
-        double s = 0.0;
-        for (int p = lane; p < D.nparts; p += 32) s += __ldcg(&D.part[p * kPartStride + j]);
-        s = warp_sum(s);
-        if (lane == 0) out[j] = s;
+    __shared__ double sub_sum[kThreads];
+    const int L = nv <= 4 ? 4 : nv <= 64 ? 64 : kPartStride, S = kThreads / L;
+    const int slot = threadIdx.x % L, sub = threadIdx.x / L;
+    double s = 0.0;
+    if (slot < nv) {
+        const double *p = D.part + slot;
+        int q = sub;
+        for (; q + 3 * S < D.nparts; q += 4 * S) {
+            const double a = __ldcg(p + (size_t)q * kPartStride), b = __ldcg(p + (size_t)(q + S) * kPartStride);
+            const double c = __ldcg(p + (size_t)(q + 2 * S) * kPartStride), d = __ldcg(p + (size_t)(q + 3 * S) * kPartStride);
+            s += (a + b) + (c + d);
+        }
+        for (; q < D.nparts; q += S) s += __ldcg(p + (size_t)q * kPartStride);
     }
+    sub_sum[threadIdx.x] = s;
+    __syncthreads();
+    for (int w = S / 2; w >= 1; w >>= 1) {
+        if (sub < w) sub_sum[threadIdx.x] += sub_sum[threadIdx.x + w * L];
+        __syncthreads();
+    }
+    if (threadIdx.x < nv) out[threadIdx.x] = sub_sum[threadIdx.x];
     __syncthreads();
 }
 
@@ -660,6 +676,7 @@ k_scale_v0(const SysDev *__restrict__ sys, const DChunk *__restrict__ ch, const 
         if (!D.st->in_cycle) continue;
         const double sc = 1.0 / D.st->r0;
         TV *V0 = (TV *)D.V;
+        if (k.part == 0 && threadIdx.x == 0) D.vscale[0] = D.vsci;
         for (int d = k.d0 + threadIdx.x; d < k.d1; d += blockDim.x) {
             const T v = (T)(sc * D.r64[d]);
             V0[d] = to_basis<TV>((double)D.vsc * (double)v);
@@ -811,11 +828,8 @@ void launch_blockdiag(int B, dim3 g, cudaStream_t st, const SysDev *sys, const N
     }
 }
 
-inline dim3 grid_for(int nchunks)
-{
-    int cap = 8 * sm_count();
-    return dim3((unsigned)std::max(1, std::min(nchunks, cap)));
-}
+// a CTA a chunk: the hardware hands them out as CTAs finish
+inline dim3 grid_for(int nchunks) { return dim3((unsigned)std::max(1, nchunks)); }
 
 int parts_for(int n, int part_dofs = kPartMax)
 {
@@ -1110,9 +1124,6 @@ static int enqueue_cycle(const Plan &P, const SolveConfig &cfg, cudaStream_t st)
     const SysDev *sys = P.sysdev.as<SysDev>();
     const DChunk *dc = P.dchunks.as<DChunk>();
     const int *nd = P.dcount.as<int>();
-    // mixed precision: one sweep fewer per step (Gram-corrected CGS); the
-    // FP64 reference method keeps two full classical passes
-    const bool gram = cfg.mixed && cfg.kmax <= 32;   // 2 (i + 1) partial sums fit a part slot
     int k = enqueue_matvec<T>(P, 0, 0, st);
     k += enqueue_precond<T>(P, 0, st);
     k_start<<<grid_for(P.n_dch), kThreads, 0, st>>>(sys, dc, nd);
@@ -1128,20 +1139,13 @@ static int enqueue_cycle(const Plan &P, const SolveConfig &cfg, cudaStream_t st)
         for (int i = 0; i < cfg.kmax - 1; ++i) {
             k += enqueue_matvec<T, TV>(P, 1, i, st);
             k += enqueue_precond<T>(P, 1, st);
-            if constexpr (std::is_same<T, TV>::value) {
-                if (gram) {
-                    k_dots1g<T><<<gd, kThreads, 0, st>>>(sys, dc, nd, i);
-                } else {
-                    k_dots1<T><<<gd, kThreads, 0, st>>>(sys, dc, nd, i);
-                    k_orth1<T><<<gd, kThreads, 0, st>>>(sys, dc, nd, i);
-                    ++k;
-                }
-            } else {
-                k_dots1g<T, TV><<<gd, kThreads, 0, st>>>(sys, dc, nd, i);   // narrow basis: Gram path only
+            k_dots<T, TV><<<gd, kThreads, 0, st>>>(sys, dc, nd, i);
+            k_orth<T, TV><<<gd, kThreads, 0, st>>>(sys, dc, nd, i);
+            k += 2;
+            if constexpr (!std::is_same<T, TV>::value) {
+                k_normalize<T, TV><<<gd, kThreads, 0, st>>>(sys, dc, nd, i);
+                ++k;
             }
-            k_orth2<T, TV><<<gd, kThreads, 0, st>>>(sys, dc, nd, i);
-            k_normalize<T, TV><<<gd, kThreads, 0, st>>>(sys, dc, nd, i);
-            k += 3;
         }
         k_update<T, TV><<<gd, kThreads, 0, st>>>(sys, dc, nd);
         ++k;
@@ -1174,7 +1178,7 @@ static int ensure_workspace(fg_system *s, int kmax, int mode)
     if ((r = w.w.alloc(ts * np)) || (r = w.t.alloc(ts * np)) ||
         (r = w.x.alloc(8 * np)) || (r = w.b.alloc(8 * np)) || (r = w.ftrue.alloc(8 * np)) ||
         (r = w.r64.alloc(8 * np)) || (r = w.t64.alloc(8 * np)) || (r = w.u64.alloc(8 * np)) ||
-        (r = w.small.alloc(8 * ((size_t)(kmax + 1) * kmax + 5 * (kmax + 1) + (size_t)kmax * kmax))) ||
+        (r = w.small.alloc(8 * ((size_t)(kmax + 1) * kmax + 7 * (kmax + 1) + (size_t)kmax * kmax))) ||
         (r = w.part.alloc(8 * (size_t)kMaxParts * kPartStride)) ||
         (r = w.counter.alloc(sizeof(unsigned) * 8)) || (r = w.state.alloc(sizeof(SysState))))
         return r;
@@ -1220,7 +1224,9 @@ static SysDev make_desc(fg_system *s, const SolveConfig &cfg, bool has_f)
     D.sn = D.cs + (cfg.kmax + 1);
     D.hbuf = D.sn + (cfg.kmax + 1);
     D.y = D.hbuf + (cfg.kmax + 1);
-    D.G = D.y + (cfg.kmax + 1);
+    D.hcol = D.y + (cfg.kmax + 1);
+    D.vscale = D.hcol + (cfg.kmax + 1);
+    D.G = D.vscale + (cfg.kmax + 1);
     D.part = w.part.as<double>();
     D.counter = w.counter.as<unsigned>();
     D.st = w.state.as<SysState>();
@@ -1229,7 +1235,7 @@ static SysDev make_desc(fg_system *s, const SolveConfig &cfg, bool has_f)
 
 int validate_member(fg_system *s, const SolveConfig &cfg)
 {
-    if (cfg.kmax < 2 || cfg.kmax > kPartStride - 4) { set_error("kmax must be in [2, 60]"); return FG_ERR_ARG; }
+    if (cfg.kmax < 2 || cfg.kmax > kMaxRestart) { set_error("kmax must be in [2, 60]"); return FG_ERR_ARG; }
     if (cfg.lmax < 1) { set_error("lmax must be >= 1"); return FG_ERR_ARG; }
     if (!s->blocks_ok) { set_error("solve before element blocks were set"); return FG_ERR_STATE; }
     if (cfg.precond != FG_PRECOND_NONE && s->precond != cfg.precond) {
@@ -1257,7 +1263,7 @@ size_t workspace_bytes(const fg_system *s, int kmax, int mixed)
 {
     size_t np = (size_t)s->n_pad, ts = mixed ? 4 : 8;
     return ts * np * (kmax + 2) + 8 * np * 6 +
-           8 * ((size_t)(kmax + 1) * kmax + 5 * (kmax + 1) + (size_t)kmax * kmax) +
+           8 * ((size_t)(kmax + 1) * kmax + 7 * (kmax + 1) + (size_t)kmax * kmax) +
            8 * (size_t)kMaxParts * kPartStride + 256 + (mixed ? 4 : 8) * ((size_t)s->topo.nunits * s->topo.ndof + (size_t)4 * kmax * 304) ;
 }
 

@@ -335,7 +335,7 @@ int fg_server_create(fg_server **out, const fg_server_opts *opts)
     if (opts->precision == FG_PREC_MIXED16 && opts->kmax > 32) {
         set_error("FG_PREC_MIXED16 needs kmax <= 32"); return FG_ERR_ARG;
     }
-    if (opts->kmax < 2 || opts->kmax > kPartStride - 4 || opts->lmax < 1) {
+    if (opts->kmax < 2 || opts->kmax > kMaxRestart || opts->lmax < 1) {
         set_error("kmax must be in [2, 60] and lmax >= 1"); return FG_ERR_ARG;
     }
     fg_server *sv = new (std::nothrow) fg_server();
