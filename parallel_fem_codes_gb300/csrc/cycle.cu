@@ -46,10 +46,9 @@
 // warp instruction in 16 cycles, so sums across CTAs are error-free FP32
 // pairs.
 //
-// The launch is cooperative, so all CTAs are resident; every CTA works
-// through its list of (system, rank) items, all lists in one global order, so
-// a gang never waits on a CTA that waits on it.  Polls are bounded (~2 s):
-// a CTA that gives up marks the system FG_ERR_TIMEOUT and leaves.
+// The launch is cooperative, so all CTAs are resident; a CTA is one rank of
+// one system's gang.  Polls are bounded (~2 s): a CTA that gives up marks the
+// system FG_ERR_TIMEOUT and leaves.
 #include <algorithm>
 #include <cstring>
 #include <mutex>
@@ -251,7 +250,7 @@ __device__ __forceinline__ double gram_diag(const Sum<double> &n2, double sc) { 
 // ---------------------------------------------------------------- the cycle
 template <typename T, int B>
 __global__ void __launch_bounds__(kCycThreads, 2)
-k_cycle(const SysDev *__restrict__ sys, const CycItem *__restrict__ items, const int *__restrict__ ioff, int smem)
+k_cycle(const SysDev *__restrict__ sys, const CycItem *__restrict__ items, int smem)
 {
     constexpr int N = Pack<T>::N, KM = kMaxRestart + 4, WP = kWords<T>;
     extern __shared__ __align__(16) unsigned char cyc_smem[];
@@ -266,11 +265,10 @@ k_cycle(const SysDev *__restrict__ sys, const CycItem *__restrict__ items, const
     const bool worker = tid < kWorkers;
     if (tid == 0) s_gave_up = 0;
 
-    for (int it = ioff[blockIdx.x]; it < ioff[blockIdx.x + 1]; ++it) {
-        const CycItem k = items[it];
+    {
+        const CycItem k = items[blockIdx.x];
         const SysDev &D = sys[k.sys];
-        if (!D.st->in_cycle) continue;
-        __syncthreads();                          // shared memory of the previous item is free
+        if (!D.st->in_cycle) return;
         const int km = D.kmax, rank = k.rank, g = D.cy_g, Rp = D.cy_rows, n = D.n;
         const int nrow = (k.u1 - k.u0) * B, np = Rp / N;
         const unsigned base = *D.cy_epoch;
@@ -838,61 +836,29 @@ void set_gang_fields(SysDev &D, const fg_system *s, int kmax, int g, bool f64)
     D.cy_vb = p + gang_head(kmax, g, f64);
 }
 
-// Work lists of a cycle launch: the live systems (all: empty) in descending size, each on the
-// g least loaded CTAs (in CTA order), so every list is in one global order.
-void gang_schedule(const std::vector<SysDev> &hs, const std::vector<int> &live, int B, bool f64,
-                   std::vector<CycItem> &items, std::vector<int> &off, size_t &smem)
+// The CTAs of a cycle launch: every rank of every live system (live empty:
+// all) that has a gang, and the shared memory of the largest.
+void gang_items(const std::vector<SysDev> &hs, const std::vector<int> &live, int B, bool f64,
+                std::vector<CycItem> &items, size_t &smem)
 {
-    const Residency dev = residency(B, f64);
-    std::vector<int> order;
-    smem = 0;
-    int most = 0;
-    for (int i = 0; i < (int)hs.size(); ++i)
-        if (hs[i].cy_g > 0 && (live.empty() || live[i])) {
-            order.push_back(i);
-            most = std::max(most, hs[i].cy_g);
-            // and the operator's rows, as far as they fit
-            const size_t w = f64 ? 8 : 4;
-            smem = std::max(smem, std::min(dev.smem, cycle_smem(hs[i].kmax, hs[i].cy_rows, std::min(hs[i].nunits, hs[i].rw_lo + hs[i].rw_hi) * B, w) +
-                                                                    (size_t)hs[i].cy_rows * hs[i].rw_w * (B * w + 2) + 16));
-        }
+    const size_t w = f64 ? 8 : 4, cap = residency(B, f64).smem;
     items.clear();
-    off.assign(1, 0);
-    if (order.empty()) return;
-    std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return hs[a].nunits > hs[b].nunits; });
-    const int ctas = std::max(most, dev.ctas);
-    std::vector<double> load(ctas, 0.0);
-    std::vector<std::vector<CycItem>> list(ctas);
-    std::vector<int> idx(ctas);
-    for (int i : order) {
+    smem = 0;
+    for (int i = 0; i < (int)hs.size(); ++i) {
         const SysDev &D = hs[i];
-        const int g = D.cy_g;
-        for (int c = 0; c < ctas; ++c) idx[c] = c;
-        if (g < ctas)
-            std::nth_element(idx.begin(), idx.begin() + g, idx.end(),
-                             [&](int a, int b) { return load[a] != load[b] ? load[a] < load[b] : a < b; });
-        std::sort(idx.begin(), idx.begin() + g);
-        double t = 0.0;
-        for (int r = 0; r < g; ++r) t = std::max(t, load[idx[r]]);
-        t += 4.0 + D.cy_rows * (f64 ? 0.013 : 0.002);        // us a step, about
-        for (int r = 0; r < g; ++r) {
-            list[idx[r]].push_back({i, r, (int)((long long)D.nunits * r / g), (int)((long long)D.nunits * (r + 1) / g)});
-            load[idx[r]] = t;
-        }
-    }
-    int used = ctas;
-    while (used > 0 && list[used - 1].empty()) --used;
-    for (int c = 0; c < used; ++c) {
-        items.insert(items.end(), list[c].begin(), list[c].end());
-        off.push_back((int)items.size());
+        if (D.cy_g == 0 || (!live.empty() && !live[i])) continue;
+        for (int r = 0; r < D.cy_g; ++r)
+            items.push_back({i, r, (int)((long long)D.nunits * r / D.cy_g), (int)((long long)D.nunits * (r + 1) / D.cy_g)});
+        // and the operator's rows, as far as they fit
+        const size_t need = cycle_smem(D.kmax, D.cy_rows, std::min(D.nunits, D.rw_lo + D.rw_hi) * B, w);
+        smem = std::max(smem, std::min(cap, need + (size_t)D.cy_rows * D.rw_w * (B * w + 2) + 16));
     }
 }
 
-int launch_cycle(int B, bool f64, const SysDev *sys, const CycItem *items, const int *off, int ctas, size_t smem,
-                 cudaStream_t st)
+int launch_cycle(int B, bool f64, const SysDev *sys, const CycItem *items, int ctas, size_t smem, cudaStream_t st)
 {
     int bytes = (int)smem;
-    void *args[] = {(void *)&sys, (void *)&items, (void *)&off, (void *)&bytes};
+    void *args[] = {(void *)&sys, (void *)&items, (void *)&bytes};
     const void *k = f64 ? cycle_kernel<double>(B) : cycle_kernel<float>(B);
     cudaError_t e = cudaLaunchCooperativeKernel(k, dim3(ctas), dim3(kCycThreads), args, smem, st);
     if (e != cudaSuccess) cuda_fail(e, "cudaLaunchCooperativeKernel");

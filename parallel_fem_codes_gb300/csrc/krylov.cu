@@ -732,11 +732,18 @@ __global__ void k_init_state(const SysDev *__restrict__ sys, int nsys)
     for (int c = 0; c < 8; ++c) sys[s].counter[c] = 0u;
 }
 
-// live flags of all systems into one array (one small copy per cycle)
+// live flags of all systems into one array (pinned host memory)
 __global__ void k_live(const SysDev *__restrict__ sys, int nsys, int *out)
 {
     int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s < nsys) out[s] = sys[s].st->live;
+}
+
+// states of all systems into one array (pinned host memory)
+__global__ void k_states(const SysDev *__restrict__ sys, int nsys, SysState *out)
+{
+    int s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s < nsys) out[s] = *sys[s].st;
 }
 
 // ---------------------------------------------------------------- host side
@@ -915,16 +922,21 @@ struct Plan {
     int nsys = 0, S = 3, B = 1;
     int precond = FG_PRECOND_NONE, ilu_g = 4;
     int n_dch = 0, n_nch = 0, n_ilu = 0, n_ilub = 0, n_spb = 0, n_spi = 0;
-    DevMem sysdev, dchunks, dcount, nchunks, ncount, live;
-    DevMem cyc_items, cyc_off;                     // on-chip cycle: work lists of its CTAs
+    // device tables, all in one block of the run's arena
+    struct Span {
+        void *p = nullptr;
+        template <class T> T *as() const { return static_cast<T *>(p); }
+    };
+    Span sysdev, dchunks, dcount, nchunks, ncount;
+    Span cyc_items;                                // on-chip cycle: (system, rank) of its CTAs
     int n_cyc = 0;                                 // its CTAs (0: the cycle streams)
     size_t cyc_smem = 0;
     bool rprec = false;                            // a right preconditioner (SGSe) before every matvec
-    DevMem ilu_fwd, ilu_bwd, ilu_ctr;              // sync-free ILU(0) substitutions
-    DevMem ilu_ws;                                 // block-Jacobi: (system, block) items, a warp each
+    Span ilu_fwd, ilu_bwd, ilu_ctr;                // sync-free ILU(0) substitutions
+    Span ilu_ws;                                 // block-Jacobi: (system, block) items, a warp each
     int n_ilw = 0, ilu_wx = 0, ilu_we = 0;         // items, rows of the largest block (0: level-scheduled
                                                    // path), entries of the longest chunk
-    DevMem sp_blocks, sp_ifaces;                   // SPIKE (system, block) and (system, interface) items
+    Span sp_blocks, sp_ifaces;                   // SPIKE (system, block) and (system, interface) items
 };
 
 static int choose_engine(const std::vector<BatchMember> &mem, const SolveConfig &cfg, std::vector<SysDev> &hs,
@@ -932,7 +944,7 @@ static int choose_engine(const std::vector<BatchMember> &mem, const SolveConfig 
 
 // cycles: restart cycles will run (else only residuals)
 static int build_plan(Plan &P, std::vector<BatchMember> &mem, const SolveConfig &cfg, std::vector<SysDev> &hs,
-                      bool cycles, cudaStream_t st)
+                      bool cycles, PlanArena &arena, cudaStream_t st)
 {
     int r;
     P.nsys = (int)mem.size();
@@ -960,9 +972,8 @@ static int build_plan(Plan &P, std::vector<BatchMember> &mem, const SolveConfig 
         for (int a = 0; a < nn; a += uchunk) nch.push_back({s, a, std::min(a + uchunk, nn)});
     }
     std::vector<CycItem> cyc;
-    std::vector<int> cyc_off;
-    if (cycles) gang_schedule(hs, {}, P.B, !cfg.mixed, cyc, cyc_off, P.cyc_smem);
-    P.n_cyc = std::max(0, (int)cyc_off.size() - 1);
+    if (cycles) gang_items(hs, {}, P.B, !cfg.mixed, cyc, P.cyc_smem);
+    P.n_cyc = (int)cyc.size();
     P.n_dch = (int)dch.size();
     P.n_nch = (int)nch.size();
     P.precond = cfg.precond;
@@ -970,10 +981,8 @@ static int build_plan(Plan &P, std::vector<BatchMember> &mem, const SolveConfig 
         if (m.s->op != mem[0].s->op) { set_error("a batch must use one operator kind"); return FG_ERR_ARG; }
     // ILU(0) substitutions: one item per pass of a system's level order
     // (forward and backward lists), systems interleaved
-    std::vector<int2> fwd, bwd;
+    std::vector<int2> fwd, bwd, wit;
     if (cfg.precond == FG_PRECOND_ILU0) {
-        int r0;
-        if ((r0 = P.ilu_ctr.alloc(64))) return r0;
         int maxp = 0;
         for (int s = 0; s < P.nsys; ++s) {
             maxp = std::max({maxp, mem[s].s->ilu_nfpass, mem[s].s->ilu_nbpass});
@@ -997,13 +1006,10 @@ static int build_plan(Plan &P, std::vector<BatchMember> &mem, const SolveConfig 
         }
         we *= kIluWsChunk;
         if (ws && P.nsys > 0) {
-            std::vector<int2> wit;
             for (int s = 0; s < P.nsys; ++s) {
                 const int np = std::max(1, std::min(mem[s].s->ilu_blocks, mem[s].s->topo.n));
                 for (int q = 0; q < np; ++q) wit.push_back(make_int2(s, q));
             }
-            if ((r0 = P.ilu_ws.alloc(sizeof(int2) * wit.size()))) return r0;
-            FG_CUDA(cudaMemcpyAsync(P.ilu_ws.p, wit.data(), sizeof(int2) * wit.size(), cudaMemcpyHostToDevice, st));
             P.n_ilw = (int)wit.size();
             P.ilu_wx = wx;
             P.ilu_we = we;
@@ -1019,38 +1025,55 @@ static int build_plan(Plan &P, std::vector<BatchMember> &mem, const SolveConfig 
         }
     P.n_spb = (int)spb.size();
     P.n_spi = (int)spi.size();
-    if ((r = P.sysdev.alloc(sizeof(SysDev) * hs.size())) ||
-        (r = P.dchunks.alloc(sizeof(DChunk) * std::max<size_t>(1, dch.size()))) ||
-        (r = P.dcount.alloc(sizeof(int))) ||
-        (r = P.nchunks.alloc(sizeof(NChunk) * std::max<size_t>(1, nch.size()))) ||
-        (r = P.ncount.alloc(sizeof(int))) ||
-        (r = P.cyc_items.alloc(sizeof(CycItem) * std::max<size_t>(1, cyc.size()))) ||
-        (r = P.cyc_off.alloc(sizeof(int) * std::max<size_t>(cyc_off.size(), 4 * (size_t)sm_count()))) ||
-        (r = P.live.alloc(sizeof(int) * P.nsys)) ||
-        (r = P.ilu_fwd.alloc(sizeof(int2) * std::max<size_t>(1, fwd.size()))) ||
-        (r = P.ilu_bwd.alloc(sizeof(int2) * std::max<size_t>(1, bwd.size()))) ||
-        (r = P.sp_blocks.alloc(sizeof(int2) * std::max<size_t>(1, spb.size()))) ||
-        (r = P.sp_ifaces.alloc(sizeof(int2) * std::max<size_t>(1, spi.size()))))
-        return r;
-    if (!spb.empty())
-        FG_CUDA(cudaMemcpyAsync(P.sp_blocks.p, spb.data(), sizeof(int2) * spb.size(), cudaMemcpyHostToDevice, st));
-    if (!spi.empty())
-        FG_CUDA(cudaMemcpyAsync(P.sp_ifaces.p, spi.data(), sizeof(int2) * spi.size(), cudaMemcpyHostToDevice, st));
-    if (!fwd.empty()) {
-        FG_CUDA(cudaMemcpyAsync(P.ilu_fwd.p, fwd.data(), sizeof(int2) * fwd.size(), cudaMemcpyHostToDevice, st));
-        FG_CUDA(cudaMemcpyAsync(P.ilu_bwd.p, bwd.data(), sizeof(int2) * bwd.size(), cudaMemcpyHostToDevice, st));
+    // one block, one copy: the tables in pinned staging, in order
+    struct Piece { Plan::Span *to; const void *from; size_t bytes, room; };
+    const int zeros[16] = {0};
+    auto piece = [](Plan::Span &to, const auto &v, size_t least = 0) {
+        const size_t e = sizeof(v[0]);
+        return Piece{&to, v.data(), e * v.size(), e * std::max(v.size(), least)};
+    };
+    const Piece all[] = {
+        piece(P.sysdev, hs), piece(P.dchunks, dch), {&P.dcount, &P.n_dch, sizeof(int), sizeof(int)},
+        piece(P.nchunks, nch), {&P.ncount, &P.n_nch, sizeof(int), sizeof(int)},
+        piece(P.cyc_items, cyc, cycles ? gang_ctas(P.B, !cfg.mixed) : 0), piece(P.ilu_fwd, fwd), piece(P.ilu_bwd, bwd),
+        {&P.ilu_ctr, zeros, sizeof(zeros), sizeof(zeros)}, piece(P.ilu_ws, wit), piece(P.sp_blocks, spb),
+        piece(P.sp_ifaces, spi)};
+    size_t bytes = 0;
+    for (const Piece &q : all) bytes += (q.room + 255) & ~(size_t)255;
+    if ((r = arena.ensure(bytes, P.nsys))) return r;
+    size_t at = 0;
+    for (const Piece &q : all) {
+        q.to->p = arena.dev.as<unsigned char>() + at;
+        if (q.bytes) std::memcpy(arena.host + at, q.from, q.bytes);
+        at += (q.room + 255) & ~(size_t)255;
     }
-    FG_CUDA(cudaMemcpyAsync(P.sysdev.p, hs.data(), sizeof(SysDev) * hs.size(), cudaMemcpyHostToDevice, st));
-    FG_CUDA(cudaMemcpyAsync(P.dchunks.p, dch.data(), sizeof(DChunk) * dch.size(), cudaMemcpyHostToDevice, st));
-    FG_CUDA(cudaMemcpyAsync(P.dcount.p, &P.n_dch, sizeof(int), cudaMemcpyHostToDevice, st));
-    if (!cyc.empty())
-        FG_CUDA(cudaMemcpyAsync(P.cyc_items.p, cyc.data(), sizeof(CycItem) * cyc.size(), cudaMemcpyHostToDevice, st));
-    if (!cyc_off.empty())
-        FG_CUDA(cudaMemcpyAsync(P.cyc_off.p, cyc_off.data(), sizeof(int) * cyc_off.size(), cudaMemcpyHostToDevice, st));
-    FG_CUDA(cudaMemcpyAsync(P.nchunks.p, nch.data(), sizeof(NChunk) * nch.size(), cudaMemcpyHostToDevice, st));
-    FG_CUDA(cudaMemcpyAsync(P.ncount.p, &P.n_nch, sizeof(int), cudaMemcpyHostToDevice, st));
-    FG_CUDA(cudaStreamSynchronize(st));   // host vectors above go out of scope
+    FG_CUDA(cudaMemcpyAsync(arena.dev.p, arena.host, at, cudaMemcpyHostToDevice, st));
     return FG_OK;
+}
+
+// Room for `bytes` of tables and the flags and states of n members.  The
+// staging is rewritten only between runs of the batch, with nothing in flight.
+int PlanArena::ensure(size_t bytes, int n)
+{
+    int r;
+    if (dev.bytes < bytes || host_bytes < bytes || members < n) {
+        bytes = std::max(bytes + bytes / 2, (size_t)16384);
+        n = std::max(n, 8);
+        if ((r = dev.alloc(bytes))) return r;
+        if (host) cudaFreeHost(host);
+        host = nullptr;
+        const size_t tail = 2 * sizeof(int) * (size_t)n + sizeof(SysState) * (size_t)n + 64;
+        FG_CUDA(cudaMallocHost(&host, bytes + tail));
+        host_bytes = bytes;
+        members = n;
+        states = reinterpret_cast<SysState *>(host + (bytes + 15) / 16 * 16);
+        live = reinterpret_cast<int *>(states + n);
+    }
+    return FG_OK;
+}
+PlanArena::~PlanArena()
+{
+    if (host) cudaFreeHost(host);
 }
 
 // Enqueue the matvec: mode 0 (x -> t64, FP64, gate live), mode 1 (V[step]
@@ -1119,7 +1142,7 @@ static int enqueue_precond(const Plan &P, int sel, cudaStream_t st)
 // whose bases fit the chip together runs its Arnoldi steps in one kernel
 // (cycle.cu), any other streams through the pass kernels below.
 template <typename T, typename TV = T>
-static int enqueue_cycle(const Plan &P, const SolveConfig &cfg, cudaStream_t st)
+static int enqueue_cycle(const Plan &P, const SolveConfig &cfg, int *live, cudaStream_t st)
 {
     const SysDev *sys = P.sysdev.as<SysDev>();
     const DChunk *dc = P.dchunks.as<DChunk>();
@@ -1130,7 +1153,7 @@ static int enqueue_cycle(const Plan &P, const SolveConfig &cfg, cudaStream_t st)
     ++k;
     if (P.n_cyc > 0) {
         constexpr bool f64 = sizeof(T) == 8;
-        k += launch_cycle(P.B, f64, sys, P.cyc_items.as<CycItem>(), P.cyc_off.as<int>(), P.n_cyc, P.cyc_smem, st);
+        k += launch_cycle(P.B, f64, sys, P.cyc_items.as<CycItem>(), P.n_cyc, P.cyc_smem, st);
     }
     else {
         const dim3 gd = grid_for(P.n_dch);
@@ -1150,7 +1173,7 @@ static int enqueue_cycle(const Plan &P, const SolveConfig &cfg, cudaStream_t st)
         k_update<T, TV><<<gd, kThreads, 0, st>>>(sys, dc, nd);
         ++k;
     }
-    k_live<<<(P.nsys + 255) / 256, 256, 0, st>>>(sys, P.nsys, P.live.as<int>());
+    k_live<<<(P.nsys + 255) / 256, 256, 0, st>>>(sys, P.nsys, live);
     return k + 1;
 }
 
@@ -1394,12 +1417,13 @@ size_t request_bytes(const fg_system *s, int kmax, int mixed, bool time_loop)
     return b;
 }
 
-BatchRun::BatchRun(const SolveConfig &c, cudaStream_t s) : cfg(c), st(s) {}
+BatchRun::BatchRun(const SolveConfig &c, cudaStream_t s, PlanArena *a) : cfg(c), st(s), arena(a ? a : &own) {}
 
 BatchRun::~BatchRun()
 {
     if (exec) cudaGraphExecDestroy(exec);
-    if (h_live) cudaFreeHost(h_live);
+    for (cudaEvent_t e : done)
+        if (e) cudaEventDestroy(e);
 }
 
 // Workspace, cleared vectors and right-hand side of a new member (queued on
@@ -1480,7 +1504,7 @@ int BatchRun::commit()
     sched.clear();
     if (mem.empty()) { pending = 0; return FG_OK; }
     P = std::make_unique<Plan>();
-    int r = build_plan(*P, mem, cfg, hs, true, st);
+    int r = build_plan(*P, mem, cfg, hs, true, *arena, st);
     if (r) return r;
     if (pending > 0) {
         int first = (int)mem.size() - pending;
@@ -1489,27 +1513,23 @@ int BatchRun::commit()
         count_launches(1);
     }
     pending = 0;
-    if ((int)live_cap < (int)mem.size()) {
-        if (h_live) cudaFreeHost(h_live);
-        live_cap = std::max<size_t>(mem.size(), 2 * live_cap);
-        FG_CUDA(cudaMallocHost(&h_live, sizeof(int) * live_cap));
-    }
     return FG_OK;
 }
 
-// One restart cycle of every member; live[i] tells whether member i goes on.
-int BatchRun::cycle(bool use_graph, std::vector<int> &live)
+// One restart cycle of every member queued, its live flags to `flags`.
+int BatchRun::enqueue(bool use_graph, int *flags)
 {
-    live.assign(mem.size(), 0);
-    if (mem.empty()) return FG_OK;
     const Plan &Pl = *P;
     cudaError_t ce = cudaSuccess;
+    auto queue = [&] {
+        return cfg.vhalf ? enqueue_cycle<float, __half>(Pl, cfg, flags, st)
+               : cfg.mixed ? enqueue_cycle<float>(Pl, cfg, flags, st) : enqueue_cycle<double>(Pl, cfg, flags, st);
+    };
     if (Pl.n_cyc > 0) use_graph = false;           // on chip: a few launches
     if (use_graph && !exec) {
         cudaGraph_t graph = nullptr;
         FG_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-        graph_nodes = cfg.vhalf ? enqueue_cycle<float, __half>(Pl, cfg, st)
-                             : cfg.mixed ? enqueue_cycle<float>(Pl, cfg, st) : enqueue_cycle<double>(Pl, cfg, st);
+        graph_nodes = queue();
         ce = cudaStreamEndCapture(st, &graph);
         if (ce != cudaSuccess) return cuda_fail(ce, "cudaStreamEndCapture");
         ce = cudaGraphInstantiate(&exec, graph, 0);
@@ -1520,16 +1540,60 @@ int BatchRun::cycle(bool use_graph, std::vector<int> &live)
         ce = cudaGraphLaunch(exec, st);
         count_launches(graph_nodes);
     } else {
-        count_launches(cfg.vhalf ? enqueue_cycle<float, __half>(Pl, cfg, st)
-                             : cfg.mixed ? enqueue_cycle<float>(Pl, cfg, st) : enqueue_cycle<double>(Pl, cfg, st));
+        count_launches(queue());
         ce = cudaGetLastError();
     }
-    if (ce == cudaSuccess) ce = cudaMemcpyAsync(h_live, Pl.live.p, sizeof(int) * mem.size(), cudaMemcpyDeviceToHost, st);
-    if (ce == cudaSuccess) ce = cudaStreamSynchronize(st);
+    return ce == cudaSuccess ? FG_OK : cuda_fail(ce, "GMRES cycle");
+}
+
+// One restart cycle of every member; live[i] tells whether member i goes on.
+int BatchRun::cycle(bool use_graph, std::vector<int> &live)
+{
+    live.assign(mem.size(), 0);
+    if (mem.empty()) return FG_OK;
+    int r = enqueue(use_graph, arena->live);
+    if (r) return r;
+    cudaError_t ce = cudaStreamSynchronize(st);
     if (ce != cudaSuccess) return cuda_fail(ce, "GMRES cycle");
-    for (size_t i = 0; i < mem.size(); ++i) live[i] = h_live[i];
+    for (size_t i = 0; i < mem.size(); ++i) live[i] = arena->live[i];
     return reschedule(live);
 }
+
+// Restart cycles until every member stopped, at most `limit`.  A single
+// system's next cycle is queued before its flag is read, so that the host's
+// round trip does not show between cycles; the one queued last finds the
+// system stopped and does nothing.
+int BatchRun::run(bool use_graph, int limit)
+{
+    int r;
+    if (mem.size() != 1 || use_graph_streams(use_graph)) {
+        std::vector<int> live;
+        for (int c = 0; c < limit; ++c) {
+            if ((r = cycle(use_graph, live))) return r;
+            int any = 0;
+            for (int v : live) any |= v;
+            if (!any) break;
+        }
+        return FG_OK;
+    }
+    for (cudaEvent_t &e : done)
+        if (!e) FG_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    for (int c = 0; c <= limit; ++c) {
+        if (c < limit) {
+            if ((r = enqueue(false, arena->live + (c & 1)))) return r;
+            FG_CUDA(cudaEventRecord(done[c & 1], st));
+        }
+        if (c > 0) {
+            FG_CUDA(cudaEventSynchronize(done[(c - 1) & 1]));
+            if (!arena->live[(c - 1) & 1]) break;
+        }
+    }
+    FG_CUDA(cudaStreamSynchronize(st));
+    return FG_OK;
+}
+
+// whether a cycle is a graph, whose nodes hold the address of the flags
+bool BatchRun::use_graph_streams(bool use_graph) const { return use_graph && P && P->n_cyc == 0; }
 
 // Once members stopped: the remaining ones spread over all CTAs again, or move
 // on chip now that they fit.  Nothing is in flight.
@@ -1545,15 +1609,17 @@ int BatchRun::reschedule(const std::vector<int> &live)
     int r = choose_engine(mem, cfg, hs, live, P->B);
     if (r) return r;
     std::vector<CycItem> cyc;
-    std::vector<int> off;
-    gang_schedule(hs, live, P->B, !cfg.mixed, cyc, off, P->cyc_smem);
-    P->n_cyc = (int)off.size() - 1;
+    gang_items(hs, live, P->B, !cfg.mixed, cyc, P->cyc_smem);
+    P->n_cyc = (int)cyc.size();
     if (P->n_cyc == 0) return FG_OK;               // still streaming
-    if (P->cyc_items.bytes < sizeof(CycItem) * cyc.size() && (r = P->cyc_items.alloc(sizeof(CycItem) * cyc.size()))) return r;
-    FG_CUDA(cudaMemcpyAsync(P->sysdev.p, hs.data(), sizeof(SysDev) * hs.size(), cudaMemcpyHostToDevice, st));
-    FG_CUDA(cudaMemcpyAsync(P->cyc_items.p, cyc.data(), sizeof(CycItem) * cyc.size(), cudaMemcpyHostToDevice, st));
-    FG_CUDA(cudaMemcpyAsync(P->cyc_off.p, off.data(), sizeof(int) * off.size(), cudaMemcpyHostToDevice, st));
-    FG_CUDA(cudaStreamSynchronize(st));            // host vectors go out of scope
+    unsigned char *d = arena->dev.as<unsigned char>();
+    auto put = [&](const Plan::Span &to, const void *from, size_t bytes) -> cudaError_t {
+        unsigned char *h = arena->host + (to.as<unsigned char>() - d);
+        std::memcpy(h, from, bytes);
+        return cudaMemcpyAsync(to.p, h, bytes, cudaMemcpyHostToDevice, st);
+    };
+    FG_CUDA(put(P->sysdev, hs.data(), sizeof(SysDev) * hs.size()));
+    FG_CUDA(put(P->cyc_items, cyc.data(), sizeof(CycItem) * cyc.size()));
     return FG_OK;
 }
 
@@ -1562,21 +1628,27 @@ int BatchRun::finish(const std::vector<int> &idx, std::vector<SysState> &out)
 {
     out.assign(idx.size(), SysState{});
     if (idx.empty()) return FG_OK;
+    // every member: the run's own tables; some: tables of their own
     std::vector<BatchMember> sub;
     std::vector<SysDev> shs;
+    const bool all = idx.size() == mem.size() && P;
     for (int i : idx) { sub.push_back(mem[i]); shs.push_back(hs[i]); }
     Plan F;
-    int r = build_plan(F, sub, cfg, shs, false, st);
-    if (r) return r;
-    const SysDev *sys = F.sysdev.as<SysDev>();
-    if (F.rprec) launch_elem_prec(sys, F.nsys, 3, 2, 0, st);   // pgmres.c:186: X = precondR(X)
-    count_launches(enqueue_matvec<double>(F, 3, 0, st));
-    k_final<<<grid_for(F.n_dch), kThreads, 0, st>>>(sys, F.dchunks.as<DChunk>(), F.dcount.as<int>());
+    PlanArena &ar = all ? *arena : sub_arena;
+    if (!all) {
+        int r = build_plan(F, sub, cfg, shs, false, sub_arena, st);
+        if (r) return r;
+    }
+    const Plan &T = all ? *P : F;
+    const SysDev *sys = T.sysdev.as<SysDev>();
+    if (T.rprec) launch_elem_prec(sys, T.nsys, 3, 2, 0, st);   // pgmres.c:186: X = precondR(X)
+    count_launches(enqueue_matvec<double>(T, 3, 0, st));
+    k_final<<<grid_for(T.n_dch), kThreads, 0, st>>>(sys, T.dchunks.as<DChunk>(), T.dcount.as<int>());
+    k_states<<<(T.nsys + 127) / 128, 128, 0, st>>>(sys, T.nsys, ar.states);
     FG_CUDA(cudaGetLastError());
-    count_launches(1);
-    for (size_t q = 0; q < idx.size(); ++q)
-        FG_CUDA(cudaMemcpyAsync(&out[q], sub[q].s->ws.state.p, sizeof(SysState), cudaMemcpyDeviceToHost, st));
+    count_launches(2);
     FG_CUDA(cudaStreamSynchronize(st));
+    for (size_t q = 0; q < idx.size(); ++q) out[q] = ar.states[all ? idx[q] : (int)q];
     return FG_OK;
 }
 
@@ -1613,18 +1685,11 @@ int solve_batch(std::vector<BatchMember> &mem, const SolveConfig &cfg, fg_solve_
         if (r) return r;
     }
     auto t0 = std::chrono::steady_clock::now();
-    BatchRun run(cfg, st);
+    BatchRun run(cfg, st, &mem[0].s->arena);
     int r;
     for (auto &m : mem)
         if ((r = run.stage(m))) return r;
-    if ((r = run.commit())) return r;
-    std::vector<int> live;
-    for (int cyc = 0; cyc < cfg.lmax + 2; ++cyc) {
-        if ((r = run.cycle(cfg.use_graph != 0, live))) return r;
-        int any = 0;
-        for (int v : live) any |= v;
-        if (!any) break;
-    }
+    if ((r = run.commit()) || (r = run.run(cfg.use_graph != 0, cfg.lmax + 2))) return r;
     std::vector<int> all(mem.size());
     for (size_t i = 0; i < all.size(); ++i) all[i] = (int)i;
     std::vector<SysState> sts;
@@ -1743,7 +1808,8 @@ int bench_matvec(std::vector<fg_system *> &systems, int precision, int reps, dou
     }
     cudaStream_t st = systems[0]->stream;
     Plan P;
-    int r = build_plan(P, mem, cfg, hs, false, st);
+    PlanArena arena;
+    int r = build_plan(P, mem, cfg, hs, false, arena, st);
     if (r) return r;
     cudaEvent_t e0, e1;
     FG_CUDA(cudaEventCreate(&e0));

@@ -458,13 +458,20 @@ __global__ void k_lincomb(int n, double c1, const double *x1, double c2, const d
         y[i] = c1 * x1[i] - c2 * x2[i];
 }
 
+// one warp: a lane per 32nd part, in order, then a fixed butterfly
 __global__ void k_sum_parts(const double *__restrict__ part, int nb, double *__restrict__ out)
 {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
     double a = 0.0, b = 0.0;
-    for (int k = 0; k < nb; ++k) { a += part[2 * k]; b += part[2 * k + 1]; }
-    out[0] = a;
-    out[1] = b;
+    for (int k = threadIdx.x; k < nb; k += 32) { a += part[2 * k]; b += part[2 * k + 1]; }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        a += __shfl_xor_sync(0xffffffffu, a, o);
+        b += __shfl_xor_sync(0xffffffffu, b, o);
+    }
+    if (threadIdx.x == 0) {
+        out[0] = a;
+        out[1] = b;
+    }
 }
 
 int axpy_norms_device(int n, double a, const double *x, double *y, double *part, double *out, cudaStream_t st)

@@ -1008,7 +1008,10 @@ static int time_loop(fg_system *s, double dt, double alpha, Assemble &&assemble,
             gmres += st.iterations;
             last_res = st.true_rel_residual;
             const double *Da = s->ws.x.as<double>();
-            if ((rr = axpy_norms_device(n, 1, Da, da, part, norms, s->stream))) return rr;   // a += Da
+            // a += Da (and the norms, where the stop test reads them)
+            if ((rr = to->stop_by_norm ? axpy_norms_device(n, 1, Da, da, part, norms, s->stream)
+                                       : axpy_device(n, 1, Da, da, s->stream)))
+                return rr;
             if ((rr = axpy_device(n, coef, Da, du, s->stream))) return rr;                 // u += coef Da
             if (hooks && hooks->corrected && (rr = hooks->corrected(Da, coef))) return rr;
             if (to->stop_by_norm) {

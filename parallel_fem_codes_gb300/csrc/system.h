@@ -29,6 +29,23 @@ struct Workspace {
     DevMem gang;                       // exchange block of the on-chip cycle
 };
 
+// Tables of a batch run on the device with their pinned staging, and the
+// members' live flags and final states in pinned memory; kept by the run's
+// owner between runs (a system for its own solves, the server for its batch).
+struct PlanArena {
+    DevMem dev;
+    unsigned char *host = nullptr;
+    size_t host_bytes = 0;
+    int members = 0;
+    SysState *states = nullptr;
+    int *live = nullptr;       // two per member
+    PlanArena() = default;
+    PlanArena(const PlanArena &) = delete;
+    PlanArena &operator=(const PlanArena &) = delete;
+    ~PlanArena();
+    int ensure(size_t bytes, int n);
+};
+
 }  // namespace fg
 
 struct fg_system {
@@ -94,6 +111,7 @@ struct fg_system {
     // host staging (pinned)
     double *h_vec = nullptr;   // 2*(n+1) doubles
     fg::Workspace ws;
+    fg::PlanArena arena;       // tables of the runs this system leads
     size_t bytes() const;
     ~fg_system();
 };
@@ -205,11 +223,12 @@ struct Plan;
 // removed.  solve_batch and the request server are built on it.
 class BatchRun {
 public:
-    BatchRun(const SolveConfig &cfg, cudaStream_t st);
+    BatchRun(const SolveConfig &cfg, cudaStream_t st, PlanArena *arena = nullptr);
     ~BatchRun();
     int stage(const BatchMember &m);
     int commit();
     int cycle(bool use_graph, std::vector<int> &live);
+    int run(bool use_graph, int limit);
     int finish(const std::vector<int> &idx, std::vector<SysState> &out);
     void remove(std::vector<int> idx);
     size_t size() const { return mem.size(); }
@@ -223,10 +242,12 @@ private:
     int pending = 0;
     cudaGraphExec_t exec = nullptr;
     int graph_nodes = 0;
-    int *h_live = nullptr;
-    size_t live_cap = 0;
-    std::vector<int> sched;            // live flags the on-chip work lists were made for (empty: every member)
+    PlanArena own, sub_arena, *arena;
+    cudaEvent_t done[2] = {nullptr, nullptr};
+    std::vector<int> sched;            // live flags the cycle's engine was chosen for (empty: every member)
+    int enqueue(bool use_graph, int *flags);
     int reschedule(const std::vector<int> &live);
+    bool use_graph_streams(bool use_graph) const;
 };
 
 int validate_member(fg_system *s, const SolveConfig &cfg);
@@ -317,10 +338,9 @@ int gang_size(const fg_system *s, int kmax, bool f64, bool dense);
 int gang_ctas(int B, bool f64);   // CTAs of the on-chip cycle that are resident together
 size_t gang_bytes(const fg_system *s, int kmax, int g, bool f64);
 void set_gang_fields(SysDev &D, const fg_system *s, int kmax, int g, bool f64);
-void gang_schedule(const std::vector<SysDev> &hs, const std::vector<int> &live, int B, bool f64,
-                   std::vector<CycItem> &items, std::vector<int> &off, size_t &smem);
-int launch_cycle(int B, bool f64, const SysDev *sys, const CycItem *items, const int *off, int ctas, size_t smem,
-                 cudaStream_t st);
+void gang_items(const std::vector<SysDev> &hs, const std::vector<int> &live, int B, bool f64,
+                std::vector<CycItem> &items, size_t &smem);
+int launch_cycle(int B, bool f64, const SysDev *sys, const CycItem *items, int ctas, size_t smem, cudaStream_t st);
 
 // Set-up kernels (setup.cu)
 int precond_setup_device(fg_system *s, int kind, int flags, double *F_dev, cudaStream_t st);
