@@ -6,9 +6,10 @@
 // vscale[j] the reciprocal of its norm, known when the step's last part sums
 // it, so that no pass is spent on scaling (an FP16 basis is scaled when it is
 // stored, vscale[j] = 1 / sigma).  Both passes walk parts of kPartMin..kPartMax
-// dofs (the size is chosen per batch from its total dofs), one CTA a part, a
-// 16-byte pack of every vector per thread and several basis vectors in
-// flight.  Part results are combined by the last part of the system in fixed
+// dofs (the size is chosen per batch from its total dofs), a 16-byte pack of
+// every vector per thread and several basis vectors in flight.  A part is one
+// CTA's, or, where a batch has few parts, gridDim.y CTAs': pass 1 splits the
+// basis vectors among them, pass 2 the dofs.  Part results are combined by the last part of the system in fixed
 // order.  HBM-bound in FP32; in FP64 the FP64 pipe (2 FMA per clock and SM)
 // binds: 3 (i + 1) FMA per dof and step.
 
@@ -89,8 +90,10 @@ __device__ __forceinline__ void st_v(TV *p, const T (&o)[VPk<TV>::G])
     }
 }
 
-// <V[j], w> and <V[j], V[i]> for j = 0..i over a part, raw (V and w as
-// stored).  A thread holds a pack of w and of V[i] and JB basis vectors' packs
+constexpr int kMaxSplit = 8;        // CTAs of a part in pass 2
+
+// <V[j], w> and <V[j], V[i]> over a part for this CTA's share of j = 0..i, raw
+// (V and w as stored).  A thread holds a pack of w and of V[i] and JB basis vectors' packs
 // at a time, so that JB + 2 loads are in flight and w is read from L1 after
 // the first group; the 2 JB sums are folded over the warp by halving (a
 // value's lanes drop out as the values do), then over the warps.
@@ -103,7 +106,9 @@ __device__ __forceinline__ void part_dots(const SysDev &D, const DChunk &k, int 
     const TV *V = (const TV *)D.V;
     const size_t ld = (size_t)D.n_pad;
     const TV *vi = V + (size_t)i * ld;
-    for (int j0 = 0; j0 < nv; j0 += JB) {
+    const int ng = (nv + JB - 1) / JB;
+    const int ja = JB * (int)(ng * blockIdx.y / gridDim.y), jb = min(nv, JB * (int)(ng * (blockIdx.y + 1) / gridDim.y));
+    for (int j0 = ja; j0 < jb; j0 += JB) {
         T s[NV];
 #pragma unroll
         for (int u = 0; u < NV; ++u) s[u] = (T)0;
@@ -138,7 +143,8 @@ __device__ __forceinline__ void part_dots(const SysDev &D, const DChunk &k, int 
         if ((lane & ((1 << SH) - 1)) == 0 && j < nv) sw[warp][(idx < JB ? 0 : nv) + j] = s[0];
     }
     __syncthreads();
-    for (int j = threadIdx.x; j < 2 * nv; j += kThreads) {
+    for (int h = threadIdx.x; h < 2 * (jb - ja); h += kThreads) {
+        const int j = h < jb - ja ? ja + h : nv + ja + h - (jb - ja);
         Sum<T> t;
 #pragma unroll
         for (int q = 0; q < kThreads / 32; ++q) t.add(sw[q][j]);
@@ -153,7 +159,7 @@ __device__ __forceinline__ void part_dots(const SysDev &D, const DChunk &k, int 
 // s - G s) with the second one taken from G instead of a second sweep; c becomes
 // column i of H and, unscaled, the update that k_orth applies.
 template <typename T, typename TV>
-__global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 3 : 2)
+__global__ void __launch_bounds__(kThreads, 3)
 k_dots(const SysDev *__restrict__ sys, const DChunk *__restrict__ ch, const int *__restrict__ nch, int i)
 {
     __shared__ T sw[kThreads / 32][2 * kMaxRestart];
@@ -165,7 +171,7 @@ k_dots(const SysDev *__restrict__ sys, const DChunk *__restrict__ ch, const int 
         if (!D.st->in_cycle) continue;
         __syncthreads();
         part_dots<T, TV>(D, k, i, (const T *)D.w, sw, D.part + k.part * kPartStride);
-        if (last_part(D, 1)) {
+        if (last_part(D, 1, gridDim.y)) {
             reduce_parts(D, 2 * (i + 1), tot);
             const int km = D.kmax;
             const double *vs = D.vscale;
@@ -197,7 +203,7 @@ k_orth(const SysDev *__restrict__ sys, const DChunk *__restrict__ ch, const int 
 {
     constexpr int G = VPk<TV>::G, JB = sizeof(TV) == 2 ? 4 : 8;
     __shared__ T hs[kMaxRestart + 4];
-    __shared__ double red[kThreads / 32], st_t[kMaxRestart + 4], st_a[kMaxRestart + 4], tot[2];
+    __shared__ double red[kThreads / 32], st_t[kMaxRestart + 4], st_a[kMaxRestart + 4], tot[kMaxSplit];
     const int total = *nch;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     for (int c = blockIdx.x; c < total; c += gridDim.x) {
@@ -213,7 +219,10 @@ k_orth(const SysDev *__restrict__ sys, const DChunk *__restrict__ ch, const int 
         T *out = std::is_same<T, TV>::value ? (T *)D.V + (size_t)(i + 1) * ld : (T *)D.w;
         const T ws = std::is_same<T, TV>::value ? (T)D.vscale[i] : (T)1;
         Sum<T> nrm;
-        for (int q = k.d0 + threadIdx.x * G; q < k.d1; q += kThreads * G) {
+        const int len = k.d1 - k.d0;
+        const int d0 = k.d0 + ((int)((long long)len * blockIdx.y / gridDim.y) & ~7);
+        const int d1 = blockIdx.y + 1 == gridDim.y ? k.d1 : k.d0 + ((int)((long long)len * (blockIdx.y + 1) / gridDim.y) & ~7);
+        for (int q = d0 + threadIdx.x * G; q < d1; q += kThreads * G) {
             T s0[G], s1[G];
             ld_g<T, G>(w + q, s0);
 #pragma unroll
@@ -259,13 +268,15 @@ k_orth(const SysDev *__restrict__ sys, const DChunk *__restrict__ ch, const int 
         if (threadIdx.x == 0) {
             double s = 0;
             for (int w8 = 0; w8 < kThreads / 32; ++w8) s += red[w8];
-            D.part[k.part * kPartStride] = s;
+            D.part[k.part * kPartStride + blockIdx.y] = s;
         }
-        if (last_part(D, 3)) {
-            reduce_parts(D, 1, tot);
+        if (last_part(D, 3, gridDim.y)) {
+            reduce_parts(D, gridDim.y, tot);
             if (warp == 0) {
                 SysState *st = D.st;
-                const double hn = sqrt(tot[0]);
+                double n2 = tot[0];
+                for (int y = 1; y < gridDim.y; ++y) n2 += tot[y];
+                const double hn = sqrt(n2);
                 Rot R{D.cs, D.sn, D.g, st_t, st_a, 0, 0, 0, 0.0};
                 const bool stop = givens<double>(D.H, D.kmax, R, i, D.hcol, hn, D.mixed ? st->target : st->eps);
                 __syncwarp();

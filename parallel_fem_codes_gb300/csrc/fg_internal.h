@@ -148,11 +148,10 @@ constexpr int kMaxColours = 64;
 constexpr int kElemChunk = 1024;   // elements per matvec work item
 constexpr int kMaxParts = 1024;    // dof parts (reduction partials) per system
 // Dofs per part of the Krylov dof kernels, chosen per batch (unless the
-// autotuner cached a choice): 2 sqrt(batch dofs), rounded to the nearest
-// power of two, within [kPartMin, kPartMax], so small systems spread over
-// many SMs and large batches keep the per-part overhead low.  Fitted to measured optima on GB300 (one
-// restart cycle): 16k dofs -> 256-dof parts, 65k -> 512, 147k -> 1024,
-// 3.1M (one NS system) -> ~3k, the 24.8M-dof served batch -> 8k-16k.
+// autotuner cached a choice): 2 sqrt(batch dofs) up to 64k dofs, 4 sqrt above,
+// rounded to the nearest power of two, within [kPartMin, kPartMax], so small
+// systems spread over many SMs and large batches keep the per-part overhead
+// low.
 constexpr int kPartMin = 256;
 constexpr int kPartMax = 16384;
 constexpr int kThreads = 256;

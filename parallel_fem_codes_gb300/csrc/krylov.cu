@@ -60,15 +60,16 @@ __device__ __forceinline__ bool gated(const SysDev &D, int gate)
 }
 
 // Last-part election: returns true in the CTA that completed the final part
-// of system D for counter slot `slot` (all threads of the CTA agree).
-__device__ __forceinline__ bool last_part(const SysDev &D, int slot)
+// of system D (`split` CTAs a part) for counter slot `slot` (all threads of the
+// CTA agree).
+__device__ __forceinline__ bool last_part(const SysDev &D, int slot, unsigned split = 1)
 {
     __shared__ int s_last;
     __syncthreads();
     if (threadIdx.x == 0) {
         __threadfence();
         unsigned prev = atomicAdd(&D.counter[slot], 1u);
-        s_last = (prev == (unsigned)D.nparts - 1u);
+        s_last = (prev == split * (unsigned)D.nparts - 1u);
         if (s_last) D.counter[slot] = 0u;
     }
     __syncthreads();
@@ -891,15 +892,16 @@ static bool tuned_choice(const std::vector<BatchMember> &mem, const SolveConfig 
 namespace {
 
 // part size of a batch (multiple of 8 dofs): the tuned one, else
-// 2 sqrt(batch dofs) rounded to the nearest power of two, within
-// [kPartMin, kPartMax] (powers of two: a system solved alone and inside a
+// 2 sqrt(batch dofs) up to 64k dofs and 4 sqrt above (where a part's sums are
+// split among CTAs), rounded to the nearest power of two, within [kPartMin,
+// kPartMax] (powers of two: a system solved alone and inside a
 // batch of similar size get the same parts, hence bit-identical results)
 int part_dofs_for(const std::vector<BatchMember> &mem, const SolveConfig &cfg)
 {
     fg_tune_choice tc;
     if (tuned_choice(mem, cfg, tc) && tc.part_dofs > 0) return tc.part_dofs & ~7;
     const double tot = (double)std::max(1LL, batch_dofs(mem));
-    const long long pd = 1LL << (int)std::lround(std::log2(2.0 * std::sqrt(tot)));
+    const long long pd = 1LL << (int)std::lround(std::log2((tot > 65536.0 ? 4.0 : 2.0) * std::sqrt(tot)));
     return (int)std::max<long long>(kPartMin, std::min<long long>(kPartMax, pd));
 }
 
@@ -1157,13 +1159,15 @@ static int enqueue_cycle(const Plan &P, const SolveConfig &cfg, int *live, cudaS
     }
     else {
         const dim3 gd = grid_for(P.n_dch);
+        // few parts: several CTAs each, up to eight CTAs an SM in all
+        const int split = std::max(1, std::min(16, 8 * sm_count() / std::max(1, P.n_dch)));
         k_scale_v0<T, TV><<<gd, kThreads, 0, st>>>(sys, dc, nd);
         ++k;
         for (int i = 0; i < cfg.kmax - 1; ++i) {
             k += enqueue_matvec<T, TV>(P, 1, i, st);
             k += enqueue_precond<T>(P, 1, st);
-            k_dots<T, TV><<<gd, kThreads, 0, st>>>(sys, dc, nd, i);
-            k_orth<T, TV><<<gd, kThreads, 0, st>>>(sys, dc, nd, i);
+            k_dots<T, TV><<<dim3(gd.x, std::min(split, (i + 4) / 4)), kThreads, 0, st>>>(sys, dc, nd, i);
+            k_orth<T, TV><<<dim3(gd.x, std::min(split, kMaxSplit)), kThreads, 0, st>>>(sys, dc, nd, i);
             k += 2;
             if constexpr (!std::is_same<T, TV>::value) {
                 k_normalize<T, TV><<<gd, kThreads, 0, st>>>(sys, dc, nd, i);
