@@ -86,7 +86,121 @@ __device__ __forceinline__ double a0_norm2(const double A0[10], const double w[4
            w[3] * A0[9] * w[3];
 }
 
-__global__ void __launch_bounds__(128) k_euler_elem(int nel, int ld, int n, const int *__restrict__ gien,
+// Structure of the Jacobians: 0 zero, 1 one, 2 a value.
+constexpr int kAx[4][4] = {{0, 1, 0, 0}, {2, 2, 2, 2}, {2, 2, 2, 0}, {2, 2, 2, 2}};
+constexpr int kAy[4][4] = {{0, 0, 1, 0}, {2, 2, 2, 0}, {2, 2, 2, 2}, {2, 2, 2, 2}};
+// value of structure s times x of structure t; the caller knows neither is 0
+template <int S, int T> __device__ __forceinline__ double eu_mul(double v, double x)
+{
+    if constexpr (S == 1) return x;
+    else if constexpr (T == 1) return v;
+    else return v * x;
+}
+// (NAME: sum over k ascending of M[R][k] N[k][Q] without the terms of a zero
+// factor; NAME_any: whether there are others)
+#define EU_PROD(NAME, SM, SN)                                                                                        \
+    template <int R, int Q> constexpr bool NAME##_any()                                                              \
+    {                                                                                                                \
+        for (int k = 0; k < 4; ++k)                                                                                  \
+            if (SM[R][k] && SN[k][Q]) return true;                                                                   \
+        return false;                                                                                                \
+    }                                                                                                                \
+    template <int R, int Q, int K = 0, bool ANY = false>                                                             \
+    __device__ __forceinline__ double NAME(const double (&M)[4][4], const double (&N)[4][4], double s = 0.0)         \
+    {                                                                                                                \
+        if constexpr (K == 4) return s;                                                                              \
+        else if constexpr (SM[R][K] == 0 || SN[K][Q] == 0) return NAME<R, Q, K + 1, ANY>(M, N, s);                    \
+        else {                                                                                                       \
+            const double t = eu_mul<SM[R][K], SN[K][Q]>(M[R][K], N[K][Q]);                                           \
+            return NAME<R, Q, K + 1, true>(M, N, ANY ? s + t : t);                                                   \
+        }                                                                                                            \
+    }
+EU_PROD(eu_xx, kAx, kAx)
+EU_PROD(eu_xy, kAx, kAy)
+EU_PROD(eu_yx, kAy, kAx)
+EU_PROD(eu_yy, kAy, kAy)
+#undef EU_PROD
+
+// s x + t y where x and y may be structural zeros or ones
+template <int SX, int SY> __device__ __forceinline__ double eu_comb(double s, double x, double t, double y)
+{
+    if constexpr (SX == 0 && SY == 0) return 0.0;
+    else if constexpr (SY == 0) return eu_mul<2, SX>(s, x);
+    else if constexpr (SX == 0) return eu_mul<2, SY>(t, y);
+    else return eu_mul<2, SX>(s, x) + eu_mul<2, SY>(t, y);
+}
+
+struct EuElem { double Mg1, Mg2, t4a, Kc01, Kc02, Kc12, tau, adt; };
+
+// Rows r of the three node blocks of Me + alpha dt Ke and of the residual.
+// The FP64 pipe bounds this kernel (two operations a cycle and SM), so what
+// does not depend on the row's node -- the products' row r and the Galerkin
+// row -- is formed once for the three, and terms with a structural zero or
+// one of Ax, Ay are not computed: 2.4k operations an element instead of 4.6k.
+template <int r>
+__device__ __forceinline__ void eu_rows(const EuElem &e, const double (&Ax)[4][4], const double (&Ay)[4][4], const double (&b)[3],
+                                        const double (&c)[3], const double (&Ue)[12], const double (&dUe)[12], double *a,
+                                        double *fe, int ld)
+{
+    const double sixth = 1.0 / 6.0;
+    // row r of AxAx, AxAy, AyAx, AyAy (sums over k ascending)
+    const double pxx[4] = {eu_xx<r, 0>(Ax, Ax), eu_xx<r, 1>(Ax, Ax), eu_xx<r, 2>(Ax, Ax), eu_xx<r, 3>(Ax, Ax)};
+    const double pxy[4] = {eu_xy<r, 0>(Ax, Ay), eu_xy<r, 1>(Ax, Ay), eu_xy<r, 2>(Ax, Ay), eu_xy<r, 3>(Ax, Ay)};
+    const double pyx[4] = {eu_yx<r, 0>(Ay, Ax), eu_yx<r, 1>(Ay, Ax), eu_yx<r, 2>(Ay, Ax), eu_yx<r, 3>(Ay, Ax)};
+    const double pyy[4] = {eu_yy<r, 0>(Ay, Ay), eu_yy<r, 1>(Ay, Ay), eu_yy<r, 2>(Ay, Ay), eu_yy<r, 3>(Ay, Ay)};
+    double kg[3][4];
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+        kg[j][0] = eu_comb<kAx[r][0], kAy[r][0]>(b[j], Ax[r][0], c[j], Ay[r][0]) * sixth;
+        kg[j][1] = eu_comb<kAx[r][1], kAy[r][1]>(b[j], Ax[r][1], c[j], Ay[r][1]) * sixth;
+        kg[j][2] = eu_comb<kAx[r][2], kAy[r][2]>(b[j], Ax[r][2], c[j], Ay[r][2]) * sixth;
+        kg[j][3] = eu_comb<kAx[r][3], kAy[r][3]>(b[j], Ax[r][3], c[j], Ay[r][3]) * sixth;
+    }
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        const int o1 = i == 0 ? 1 : 0, o2 = i == 2 ? 1 : 2;     // the other two nodes, ascending
+        const double kcd = i == 0 ? e.Kc01 + e.Kc02 : i == 1 ? e.Kc01 + e.Kc12 : e.Kc02 + e.Kc12;
+        const int R = 4 * i + r;
+        double mpg[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) mpg[q] = kg[i][q] * e.tau;   // (b_i Ax + c_i Ay) / 6 tau
+        const double ax[4] = {eu_comb<eu_xx_any<r, 0>() ? 2 : 0, eu_yx_any<r, 0>() ? 2 : 0>(b[i], pxx[0], c[i], pyx[0]),
+                              eu_comb<eu_xx_any<r, 1>() ? 2 : 0, eu_yx_any<r, 1>() ? 2 : 0>(b[i], pxx[1], c[i], pyx[1]),
+                              eu_comb<eu_xx_any<r, 2>() ? 2 : 0, eu_yx_any<r, 2>() ? 2 : 0>(b[i], pxx[2], c[i], pyx[2]),
+                              eu_comb<eu_xx_any<r, 3>() ? 2 : 0, eu_yx_any<r, 3>() ? 2 : 0>(b[i], pxx[3], c[i], pyx[3])};
+        const double ay[4] = {eu_comb<eu_xy_any<r, 0>() ? 2 : 0, eu_yy_any<r, 0>() ? 2 : 0>(b[i], pxy[0], c[i], pyy[0]),
+                              eu_comb<eu_xy_any<r, 1>() ? 2 : 0, eu_yy_any<r, 1>() ? 2 : 0>(b[i], pxy[1], c[i], pyy[1]),
+                              eu_comb<eu_xy_any<r, 2>() ? 2 : 0, eu_yy_any<r, 2>() ? 2 : 0>(b[i], pxy[2], c[i], pyy[2]),
+                              eu_comb<eu_xy_any<r, 3>() ? 2 : 0, eu_yy_any<r, 3>() ? 2 : 0>(b[i], pxy[3], c[i], pyy[3])};
+        double m = 0, k = 0;
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            const double kij = j == i ? 0.0 : (i + j == 1 ? e.Kc01 : i + j == 2 ? e.Kc02 : e.Kc12);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const double Me = r == q ? (i == j ? e.Mg1 : e.Mg2) + mpg[q] : mpg[q];
+                double Ke;
+                if (i == j) {
+                    const double p1 = e.t4a * (b[o1] * ax[q] + c[o1] * ay[q]);
+                    const double p2 = e.t4a * (b[o2] * ax[q] + c[o2] * ay[q]);
+                    const double kk = kg[j][q] - (p1 + p2);
+                    Ke = r == q ? kk - kcd : kk;
+                } else {
+                    const double p = e.t4a * (b[j] * ax[q] + c[j] * ay[q]);
+                    Ke = r == q ? kg[j][q] + p + kij : kg[j][q] + p;
+                }
+                const int Q = 4 * j + q;
+                m += Me * dUe[Q];
+                k += Ke * Ue[Q];
+                a[(size_t)(R * 12 + Q) * ld] = Me + e.adt * Ke;
+            }
+        }
+        fe[(size_t)R * ld] = -m - k;
+    }
+}
+
+// (CTAs of 64: on a small mesh they spread over more SMs)
+__global__ void __launch_bounds__(64) k_euler_elem(int nel, int ld, int n, const int *__restrict__ gien,
                                                     const double *__restrict__ gx, const double *__restrict__ gy,
                                                     const int *__restrict__ node_dof, const double *__restrict__ up,
                                                     const double *__restrict__ u, const double *__restrict__ du,
@@ -184,62 +298,13 @@ __global__ void __launch_bounds__(128) k_euler_elem(int nel, int ld, int n, cons
     const double Kc01 = d4a * (b[0] * b[1] + c[0] * c[1]);
     const double Kc02 = d4a * (b[0] * b[2] + c[0] * c[2]);
     const double Kc12 = d4a * (b[1] * b[2] + c[1] * c[2]);
-    const double adt = cf.alpha * cf.dt;
+    const EuElem e{Mg1, Mg2, t4a, Kc01, Kc02, Kc12, tau, cf.alpha * cf.dt};
     double *a = A64 + pos;
     double *fe = Fe + pos;
-#pragma unroll 1
-    for (int i = 0; i < 3; ++i) {
-        const int o1 = i == 0 ? 1 : 0, o2 = i == 2 ? 1 : 2;     // the other two nodes, ascending
-        const double kcd = i == 0 ? Kc01 + Kc02 : i == 1 ? Kc01 + Kc12 : Kc02 + Kc12;
-#pragma unroll
-        for (int r = 0; r < 4; ++r) {
-            // row r of AxAx, AxAy, AyAx, AyAy (sums over k ascending)
-            double pxx[4], pxy[4], pyx[4], pyy[4];
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                double s1 = Ax[r][0] * Ax[0][q], s2 = Ax[r][0] * Ay[0][q];
-                double s3 = Ay[r][0] * Ax[0][q], s4 = Ay[r][0] * Ay[0][q];
-#pragma unroll
-                for (int k = 1; k < 4; ++k) {
-                    s1 += Ax[r][k] * Ax[k][q];
-                    s2 += Ax[r][k] * Ay[k][q];
-                    s3 += Ay[r][k] * Ax[k][q];
-                    s4 += Ay[r][k] * Ay[k][q];
-                }
-                pxx[q] = s1; pxy[q] = s2; pyx[q] = s3; pyy[q] = s4;
-            }
-            const int R = 4 * i + r;
-            double m = 0, k = 0;
-#pragma unroll
-            for (int j = 0; j < 3; ++j) {
-                const double kij = j == i ? 0.0 : (i + j == 1 ? Kc01 : i + j == 2 ? Kc02 : Kc12);
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    const double Ci = (b[i] * Ax[r][q] + c[i] * Ay[r][q]) * sixth;
-                    const double mpg = Ci * tau;
-                    const double Me = r == q ? (i == j ? Mg1 : Mg2) + mpg : mpg;
-                    const double kg = (b[j] * Ax[r][q] + c[j] * Ay[r][q]) * sixth;
-                    const double ax = b[i] * pxx[q] + c[i] * pyx[q];
-                    const double ay = b[i] * pxy[q] + c[i] * pyy[q];
-                    double Ke;
-                    if (i == j) {
-                        const double p1 = t4a * (b[o1] * ax + c[o1] * ay);
-                        const double p2 = t4a * (b[o2] * ax + c[o2] * ay);
-                        const double kk = kg - (p1 + p2);
-                        Ke = r == q ? kk - kcd : kk;
-                    } else {
-                        const double p = t4a * (b[j] * ax + c[j] * ay);
-                        Ke = r == q ? kg + p + kij : kg + p;
-                    }
-                    const int Q = 4 * j + q;
-                    m += Me * dUe[Q];
-                    k += Ke * Ue[Q];
-                    a[(size_t)(R * 12 + Q) * ld] = Me + adt * Ke;
-                }
-            }
-            fe[(size_t)R * ld] = -m - k;
-        }
-    }
+    eu_rows<0>(e, Ax, Ay, b, c, Ue, dUe, a, fe, ld);
+    eu_rows<1>(e, Ax, Ay, b, c, Ue, dUe, a, fe, ld);
+    eu_rows<2>(e, Ax, Ay, b, c, Ue, dUe, a, fe, ld);
+    eu_rows<3>(e, Ax, Ay, b, c, Ue, dUe, a, fe, ld);
 }
 
 // ---------------------------------------------------------------- DD form
@@ -738,7 +803,7 @@ int euler_assemble_device(fg_system *s, const fg_euler_coeffs *c, const double *
                                                                 s->shock_state.as<double>() + s->nel_pad,
                                                                 s->A64.as<double>(), s->Fe.as<double>());
     } else if (t.nel > 0)
-        k_euler_elem<<<(t.nel + 127) / 128, 128, 0, st>>>(t.nel, s->nel_pad, t.n, s->gien.as<int>(),
+        k_euler_elem<<<(t.nel + 63) / 64, 64, 0, st>>>(t.nel, s->nel_pad, t.n, s->gien.as<int>(),
                                                          s->gx.as<double>(), s->gy.as<double>(),
                                                          s->node_dof.as<int>(), s->gup.as<double>(), u_dev, du_dev,
                                                          *c, s->A64.as<double>(), s->Fe.as<double>());
