@@ -248,7 +248,11 @@ __device__ __forceinline__ float gram_diag(const Sum<float> &n2, float sc)
 __device__ __forceinline__ double gram_diag(const Sum<double> &n2, double sc) { return fma(sc * n2.h, sc, -1.0); }
 
 // ---------------------------------------------------------------- the cycle
-template <typename T, int B>
+// SPILL: a system alone on the GPU whose basis passes its shared memory by up
+// to a few times: the older basis vectors stay in shared memory, the others in
+// global memory (L2), where only the CTA that owns the rows reads them; the two
+// newest vectors have shared-memory slots of their own.
+template <typename T, int B, bool SPILL>
 __global__ void __launch_bounds__(kCycThreads, 2)
 k_cycle(const SysDev *__restrict__ sys, const CycItem *__restrict__ items, int smem)
 {
@@ -280,7 +284,12 @@ k_cycle(const SysDev *__restrict__ sys, const CycItem *__restrict__ items, int s
         u64 *const total = norm2 + 4 * (size_t)g;            // [slot], WP words; the norm's 2 words
         u64 *const note = total + (size_t)2 * km * WP + 2;   // stop flag [parity], m, y [km][2]
         u64 *vb = (u64 *)D.cy_vb;                            // [row], WP words
-        T *E = V + (size_t)km * Rp;                          // Gram matrix less I, km x km
+        const int js = SPILL ? D.cy_js : km;                 // basis vectors in shared memory
+        T *const W2 = V + (size_t)js * Rp;                   // SPILL: the two newest vectors
+        T *const gV = SPILL ? (T *)D.cy_spill + (size_t)rank * Rp : nullptr;
+        const size_t gs = (size_t)g * Rp;
+        auto slot = [&](int j) -> T * { return !SPILL || j < js ? V + (size_t)j * Rp : gV + (j - js) * gs; };
+        T *E = W2 + (SPILL ? 2 * (size_t)Rp : 0);             // Gram matrix less I, km x km
         T *halo = E + ((km * km + N - 1) & ~(N - 1));
         const bool direct = g <= (sizeof(T) == 8 ? kDirect64 : kDirect32);
         const int pre = D.precond;
@@ -288,7 +297,7 @@ k_cycle(const SysDev *__restrict__ sys, const CycItem *__restrict__ items, int s
         Rot R{s_cs, s_sn, s_g, s_t, s_a, 0, 0, 0, 0.0};
         const int lo = max(k.u0 - D.rw_lo, 0), hi = min(k.u1 + D.rw_hi, D.nunits);
         const int nhl = (k.u0 - lo) * B, nh = nhl + (hi - k.u1) * B;
-        Newest<T> X{V, halo, k.u0, k.u1, lo};
+        Newest<T> X{SPILL ? W2 : V, halo, k.u0, k.u1, lo};
         // rows [0, nc) of the operator: values [slot][row][B], local units [slot][row]
         const int W = D.rw_w;
         T *rv = halo + ((nh + N - 1) & ~(N - 1));
@@ -321,7 +330,7 @@ k_cycle(const SysDev *__restrict__ sys, const CycItem *__restrict__ items, int s
             Sum<T> t;
             for (int q = tid; q < Rp; q += kWorkers) {
                 const T v = q < nrow ? v0(k.u0 * B + q) : (T)0;
-                V[q] = v;
+                (SPILL ? W2 : V)[q] = v;
                 t.add_square(v);
             }
             for (int q = tid; q < nh; q += kWorkers) {
@@ -341,7 +350,8 @@ k_cycle(const SysDev *__restrict__ sys, const CycItem *__restrict__ items, int s
             const int nv = i + 1;
             const unsigned tag = base + (unsigned)i + 1u;
             u64 *part = part2 + (i & 1) * ((size_t)2 * km * g * WP), *norm = norm2 + (i & 1) * (2 * (size_t)g);
-            T *vi = V + (size_t)i * Rp, *w = vi + Rp;
+            T *vi = SPILL ? W2 + (i & 1) * Rp : V + (size_t)i * Rp;
+            T *w = SPILL ? W2 + ((i + 1) & 1) * Rp : vi + Rp;
             X.own = vi;
             if (worker) {
                 const int nsl = dot_slices(np, nv);
@@ -351,7 +361,7 @@ k_cycle(const SysDev *__restrict__ sys, const CycItem *__restrict__ items, int s
                         const int j = h % nv, sl = h / nv;
                         T a = (T)0, a2 = (T)0;
                         if (sl < nsl) {
-                            const T *vj = V + (size_t)j * Rp;
+                            const T *vj = SPILL && j == i ? vi : slot(j);
 #pragma unroll 4
                             for (int p = sl * 8 + l8; p < np; p += 8 * nsl) {
                                 const auto x = ldp(vj + p * N), z = ldp(y + p * N);
@@ -587,18 +597,19 @@ k_cycle(const SysDev *__restrict__ sys, const CycItem *__restrict__ items, int s
                 Sum<T> t;
                 const int keep_l = D.rw_hi * B, keep_r = nrow - D.rw_lo * B;
                 constexpr int R = sizeof(T) == 4 ? 4 : 1;
-                for (int q = tid * R; q < nrow; q += kWorkers * R) {
+                for (int q = tid * R; q < (SPILL ? Rp : nrow); q += kWorkers * R) {   // (SPILL: zeros behind the rows too)
                     T s0[R], s1[R], v[R];
 #pragma unroll
                     for (int r = 0; r < R; ++r) {
                         v[r] = sc * vi[q + r];
                         s0[r] = sc * w[q + r];
                         s1[r] = -c[i] * v[r];
-                        vi[q + r] = v[r];
+                        (SPILL ? slot(i) : vi)[q + r] = v[r];
                     }
                     int j = 0;
+                    const int in = SPILL ? min(i, js) : i;
 #pragma unroll 4
-                    for (; j + 1 < i; j += 2) {
+                    for (; j + 1 < in; j += 2) {
                         const T c0 = c[j], c1 = c[j + 1];
                         T a[R], b[R];
                         if constexpr (R == 4) {
@@ -615,9 +626,34 @@ k_cycle(const SysDev *__restrict__ sys, const CycItem *__restrict__ items, int s
                             s1[r] -= c1 * b[r];
                         }
                     }
-                    if (j < i)
+                    if (j < in)
 #pragma unroll
                         for (int r = 0; r < R; ++r) s0[r] -= c[j] * V[(size_t)j * Rp + q + r];
+                    if constexpr (SPILL) {
+                        for (int h = js; h < i; h += 8) {    // eight loads in flight
+                            T a[8][R];
+#pragma unroll
+                            for (int m = 0; m < 8; ++m) {
+                                const T *p = gV + (min(h + m, i - 1) - js) * gs + q;
+                                if constexpr (R == 4) {
+                                    const auto x = ldp(p);
+#pragma unroll
+                                    for (int r = 0; r < R; ++r) a[m][r] = x.v[r];
+                                } else {
+                                    a[m][0] = p[0];
+                                }
+                            }
+#pragma unroll
+                            for (int m = 0; m < 8; ++m) {
+                                if (h + m >= i) break;
+#pragma unroll
+                                for (int r = 0; r < R; ++r) {
+                                    if (m & 1) s1[r] -= c[h + m] * a[m][r];
+                                    else s0[r] -= c[h + m] * a[m][r];
+                                }
+                            }
+                        }
+                    }
 #pragma unroll
                     for (int r = 0; r < R; ++r) {
                         s0[r] += s1[r];
@@ -718,8 +754,9 @@ k_cycle(const SysDev *__restrict__ sys, const CycItem *__restrict__ items, int s
                 if (id == n) continue;
                 Sum<T> t;
                 for (int j = 0; j < m; ++j) {
-                    if constexpr (sizeof(T) == 8) t.h += y[j] * V[(size_t)j * Rp + q];
-                    else t.add_product(s_tot[2 * j], s_tot[2 * j + 1], V[(size_t)j * Rp + q]);
+                    const T v = slot(j)[q];
+                    if constexpr (sizeof(T) == 8) t.h += y[j] * v;
+                    else t.add_product(s_tot[2 * j], s_tot[2 * j + 1], v);
                 }
                 D.x[id] += t.value();
             }
@@ -745,30 +782,36 @@ size_t cycle_smem(int km, int rows, int halo_rows, size_t w)
 {
     return w * ((size_t)km * rows + (((size_t)km * km + 3) & ~(size_t)3) + ((halo_rows + 3) & ~3));
 }
-template <typename T> const void *cycle_kernel(int B)
+template <typename T, bool SPILL> const void *cycle_kernel(int B)
 {
     switch (B) {
-    case 1: return (const void *)k_cycle<T, 1>;
-    case 2: return (const void *)k_cycle<T, 2>;
-    case 3: return (const void *)k_cycle<T, 3>;
-    default: return (const void *)k_cycle<T, 4>;
+    case 1: return (const void *)k_cycle<T, 1, SPILL>;
+    case 2: return (const void *)k_cycle<T, 2, SPILL>;
+    case 3: return (const void *)k_cycle<T, 3, SPILL>;
+    default: return (const void *)k_cycle<T, 4, SPILL>;
     }
+}
+const void *cycle_kernel(int B, bool f64, bool spill)
+{
+    return f64 ? (spill ? cycle_kernel<double, true>(B) : cycle_kernel<double, false>(B))
+               : (spill ? cycle_kernel<float, true>(B) : cycle_kernel<float, false>(B));
 }
 
 // What k_cycle<T, B> has on this device: the dynamic shared memory with which
 // two CTAs share an SM, and the CTAs that are then resident together (0:
 // none).  Looked up once per kernel; raises its shared-memory limit.
 struct Residency { int ctas; size_t smem; };
-Residency residency(int B, bool f64)
+Residency residency(int B, bool f64, bool spill = false)
 {
     static std::mutex mu;
-    static bool known[2][5];
-    static Residency found[2][5];
+    static bool known[4][5];
+    static Residency found[4][5];
     std::lock_guard<std::mutex> l(mu);
-    Residency &v = found[f64 ? 1 : 0][B];
-    if (!known[f64 ? 1 : 0][B]) {
-        known[f64 ? 1 : 0][B] = true;
-        const void *k = f64 ? cycle_kernel<double>(B) : cycle_kernel<float>(B);
+    const int w = (f64 ? 1 : 0) + (spill ? 2 : 0);
+    Residency &v = found[w][B];
+    if (!known[w][B]) {
+        known[w][B] = true;
+        const void *k = cycle_kernel(B, f64, spill);
         int dev = 0, coop = 0, occ = 0, sm = 0, own = 0;
         cudaFuncAttributes fa{};
         v = {0, 0};
@@ -797,6 +840,7 @@ Residency residency(int B, bool f64)
 // apart for the halo.
 constexpr int kRows32 = 512, kRows64 = 128;
 static int halo_units(const fg_system *s) { return std::min(s->topo.nunits, s->topo.rw_lo + s->topo.rw_hi); }
+int gang_rows(const fg_system *s, int g);
 int gang_size(const fg_system *s, int kmax, bool f64, bool dense)
 {
     const int B = s->topo.ndof, nu = s->topo.nunits;
@@ -810,7 +854,21 @@ int gang_size(const fg_system *s, int kmax, bool f64, bool dense)
     const int g = std::max((nu + cap_u - 1) / cap_u, std::min(ctas, (nu + want_u - 1) / want_u));
     return g <= ctas ? g : 0;
 }
-int gang_ctas(int B, bool f64) { return residency(B, f64).ctas; }
+int gang_ctas(int B, bool f64, bool spill) { return residency(B, f64, spill).ctas; }
+// Basis vectors that stay in shared memory when a system that does not fit
+// runs alone on every CTA (0: fewer than a fifth, or none; it streams).
+// Measured on FP64 systems (a step, streaming -> spilling): 147k equations,
+// GMRES(30), 23 vectors inside 55 -> 34 us; 198k, GMRES(50), 12 inside 103 -> 65.
+int gang_spill(const fg_system *s, int kmax, bool f64)
+{
+    const int B = s->topo.ndof;
+    const Residency dev = residency(B, f64, true);
+    if (dev.ctas == 0 || s->topo.nunits < dev.ctas) return 0;
+    const size_t w = f64 ? 8 : 4, fixed = cycle_smem(kmax, 0, halo_units(s) * B, w);
+    if (fixed >= dev.smem) return 0;
+    const int js = std::min(kmax - 2, (int)((dev.smem - fixed) / (w * gang_rows(s, dev.ctas))) - 2);
+    return js >= 2 && 5 * js >= kmax ? js : 0;
+}
 int gang_rows(const fg_system *s, int g) { return ((s->topo.nunits + g - 1) / g * s->topo.ndof + 3) & ~3; }
 
 // Exchange block of a gang: the epoch (16 bytes), the exchange words, the
@@ -825,8 +883,14 @@ size_t gang_bytes(const fg_system *s, int kmax, int g, bool f64)
 {
     return gang_head(kmax, g, f64) + (size_t)s->topo.nunits * s->topo.ndof * (f64 ? 16 : 8);
 }
-void set_gang_fields(SysDev &D, const fg_system *s, int kmax, int g, bool f64)
+size_t gang_spill_bytes(const fg_system *s, int kmax, int g, int js, bool f64)
 {
+    return js ? (size_t)(kmax - js) * g * gang_rows(s, g) * (f64 ? 8 : 4) : 0;
+}
+void set_gang_fields(SysDev &D, const fg_system *s, int kmax, int g, int js, bool f64)
+{
+    D.cy_js = js;
+    D.cy_spill = s->ws.spill.p;
     D.cy_g = g;
     if (!g) return;
     D.cy_rows = gang_rows(s, g);
@@ -841,7 +905,7 @@ void set_gang_fields(SysDev &D, const fg_system *s, int kmax, int g, bool f64)
 void gang_items(const std::vector<SysDev> &hs, const std::vector<int> &live, int B, bool f64,
                 std::vector<CycItem> &items, size_t &smem)
 {
-    const size_t w = f64 ? 8 : 4, cap = residency(B, f64).smem;
+    const size_t w = f64 ? 8 : 4;
     items.clear();
     smem = 0;
     for (int i = 0; i < (int)hs.size(); ++i) {
@@ -850,16 +914,19 @@ void gang_items(const std::vector<SysDev> &hs, const std::vector<int> &live, int
         for (int r = 0; r < D.cy_g; ++r)
             items.push_back({i, r, (int)((long long)D.nunits * r / D.cy_g), (int)((long long)D.nunits * (r + 1) / D.cy_g)});
         // and the operator's rows, as far as they fit
-        const size_t need = cycle_smem(D.kmax, D.cy_rows, std::min(D.nunits, D.rw_lo + D.rw_hi) * B, w);
+        const size_t cap = residency(B, f64, D.cy_js > 0).smem;
+        const size_t need = cycle_smem(D.kmax, 0, 0, w) + w * (D.cy_js > 0 ? D.cy_js + 2 : D.kmax) * D.cy_rows +
+                            cycle_smem(0, 0, std::min(D.nunits, D.rw_lo + D.rw_hi) * B, w);
         smem = std::max(smem, std::min(cap, need + (size_t)D.cy_rows * D.rw_w * (B * w + 2) + 16));
     }
 }
 
-int launch_cycle(int B, bool f64, const SysDev *sys, const CycItem *items, int ctas, size_t smem, cudaStream_t st)
+int launch_cycle(int B, bool f64, bool spill, const SysDev *sys, const CycItem *items, int ctas, size_t smem,
+                 cudaStream_t st)
 {
     int bytes = (int)smem;
     void *args[] = {(void *)&sys, (void *)&items, (void *)&bytes};
-    const void *k = f64 ? cycle_kernel<double>(B) : cycle_kernel<float>(B);
+    const void *k = cycle_kernel(B, f64, spill);
     cudaError_t e = cudaLaunchCooperativeKernel(k, dim3(ctas), dim3(kCycThreads), args, smem, st);
     if (e != cudaSuccess) cuda_fail(e, "cudaLaunchCooperativeKernel");
     return 1;

@@ -187,6 +187,8 @@ struct SysDev {
     // gang of the on-chip restart cycle (cycle.cu): CTAs (0: streaming
     // kernels), padded rows of each, exchange words, vector and epoch
     int cy_g, cy_rows;
+    int cy_js;                 // > 0: basis vectors in shared memory, the others in cy_spill
+    void *cy_spill;
     unsigned long long *cy_part;
     void *cy_vb;
     unsigned *cy_epoch;

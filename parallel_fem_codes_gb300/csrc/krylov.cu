@@ -933,6 +933,7 @@ struct Plan {
     Span cyc_items;                                // on-chip cycle: (system, rank) of its CTAs
     int n_cyc = 0;                                 // its CTAs (0: the cycle streams)
     size_t cyc_smem = 0;
+    bool cyc_spill = false;                        // one system, part of its basis in global memory
     bool rprec = false;                            // a right preconditioner (SGSe) before every matvec
     Span ilu_fwd, ilu_bwd, ilu_ctr;                // sync-free ILU(0) substitutions
     Span ilu_ws;                                 // block-Jacobi: (system, block) items, a warp each
@@ -976,6 +977,7 @@ static int build_plan(Plan &P, std::vector<BatchMember> &mem, const SolveConfig 
     std::vector<CycItem> cyc;
     if (cycles) gang_items(hs, {}, P.B, !cfg.mixed, cyc, P.cyc_smem);
     P.n_cyc = (int)cyc.size();
+    P.cyc_spill = P.n_cyc > 0 && hs[cyc[0].sys].cy_js > 0;
     P.n_dch = (int)dch.size();
     P.n_nch = (int)nch.size();
     P.precond = cfg.precond;
@@ -1155,7 +1157,7 @@ static int enqueue_cycle(const Plan &P, const SolveConfig &cfg, int *live, cudaS
     ++k;
     if (P.n_cyc > 0) {
         constexpr bool f64 = sizeof(T) == 8;
-        k += launch_cycle(P.B, f64, sys, P.cyc_items.as<CycItem>(), P.n_cyc, P.cyc_smem, st);
+        k += launch_cycle(P.B, f64, P.cyc_spill, sys, P.cyc_items.as<CycItem>(), P.n_cyc, P.cyc_smem, st);
     }
     else {
         const dim3 gd = grid_for(P.n_dch);
@@ -1184,12 +1186,14 @@ static int enqueue_cycle(const Plan &P, const SolveConfig &cfg, int *live, cudaS
 // The gang of a member's on-chip restart cycle (0: it streams): the
 // preconditioner must act on one node, the basis must be kept in the
 // arithmetic's type and fit.
+static bool chip_config(const SolveConfig &cfg)
+{
+    return !cfg.vhalf && (cfg.precond == FG_PRECOND_NONE || cfg.precond == FG_PRECOND_DIAG ||
+                          cfg.precond == FG_PRECOND_BLOCKDIAG);
+}
 static int member_gang(const fg_system *s, const SolveConfig &cfg, bool dense)
 {
-    if (cfg.vhalf || (cfg.precond != FG_PRECOND_NONE && cfg.precond != FG_PRECOND_DIAG &&
-                      cfg.precond != FG_PRECOND_BLOCKDIAG))
-        return 0;
-    return gang_size(s, cfg.kmax, !cfg.mixed, dense);
+    return chip_config(cfg) ? gang_size(s, cfg.kmax, !cfg.mixed, dense) : 0;
 }
 
 // mode: 0 FP64, 1 FP32 basis, 2 FP16 basis (mixed precision in both)
@@ -1409,7 +1413,7 @@ size_t request_bytes(const fg_system *s, int kmax, int mixed, bool time_loop)
 {
     const Workspace &w = s->ws;
     const DevMem *held[] = {&w.V, &w.w, &w.t, &w.x, &w.b, &w.ftrue, &w.r64, &w.t64, &w.u64, &w.small, &w.part,
-                            &w.counter, &w.state, &w.gang};
+                            &w.counter, &w.state, &w.gang, &w.spill};
     size_t have = 0;
     for (auto *m : held) have += m->bytes;
     size_t b = s->bytes() - std::min(have, s->bytes()) + workspace_bytes(s, kmax, mixed) + rows_bytes(s, mixed != 0);
@@ -1438,17 +1442,12 @@ int BatchRun::stage(const BatchMember &m)
     int r = validate_member(s, cfg);
     if (r) return r;
     if ((r = ensure_workspace(s, cfg.kmax, cfg.mixed + cfg.vhalf))) return r;
-    const int gang = member_gang(s, cfg, false);    // the largest it is run with
     if (s->op == FG_OP_CSR && (r = csr_refresh(s, st))) return r;
     if ((r = rows_refresh(s, cfg.mixed != 0, st))) return r;
     Workspace &w = s->ws;
     size_t vb = 8 * (size_t)s->n_pad;
     FG_CUDA(cudaMemsetAsync(w.x.p, 0, vb, st));
-    if (gang > 0) {
-        const size_t gb = gang_bytes(s, cfg.kmax, gang, !cfg.mixed);
-        if (w.gang.bytes < gb && (r = w.gang.alloc(gb))) return r;
-        FG_CUDA(cudaMemsetAsync(w.gang.p, 0, gb, st));
-    }
+    if (w.gang.p) FG_CUDA(cudaMemsetAsync(w.gang.p, 0, w.gang.bytes, st));
     FG_CUDA(cudaMemsetAsync(w.small.p, 0, w.small.bytes, st));
     if (cfg.device_io) {
         FG_CUDA(cudaMemcpyAsync(w.b.p, m.B, 8 * (size_t)(s->topo.n + 1), cudaMemcpyDeviceToDevice, st));
@@ -1471,8 +1470,8 @@ int BatchRun::stage(const BatchMember &m)
 
 // Where the batch's restart cycles run, for the live members (all: empty): on
 // chip when their gangs are resident together (CTAs of about kRows rows if
-// those fit, else as few as hold the systems), else streaming through global
-// memory.  Measured on 32 transport instances, 3.1 M equations: one Arnoldi
+// those fit, else as few as hold the systems), or partly on chip for a system
+// alone, else streaming through global memory.  Measured on 32 transport instances, 3.1 M equations: one Arnoldi
 // step of all 201 us on chip in 19 rounds, 171 us streaming; a single one of
 // them of 261k equations 12 us on chip, 55 us streaming.
 static int choose_engine(const std::vector<BatchMember> &mem, const SolveConfig &cfg, std::vector<SysDev> &hs,
@@ -1491,11 +1490,27 @@ static int choose_engine(const std::vector<BatchMember> &mem, const SolveConfig 
             chip = g[i] > 0 && sum <= room;
         }
     }
+    // a system alone may keep part of its basis outside
+    int alone = -1, js = 0;
+    for (size_t i = 0; i < mem.size(); ++i)
+        if (live.empty() || live[i]) alone = alone == -1 ? (int)i : -2;
+    if (!chip && alone >= 0 && chip_config(cfg) && (js = gang_spill(mem[alone].s, cfg.kmax, !cfg.mixed)) > 0) {
+        chip = true;
+        g[alone] = gang_ctas(B, !cfg.mixed, true);
+    }
     for (size_t i = 0; i < mem.size(); ++i) {
         int r;
-        if (!chip && (r = ensure_basis(mem[i].s))) return r;
-        hs[i].V = mem[i].s->ws.V.p;
-        set_gang_fields(hs[i], mem[i].s, cfg.kmax, chip ? g[i] : 0, !cfg.mixed);
+        fg_system *s = mem[i].s;
+        Workspace &w = s->ws;
+        const int my_js = (int)i == alone ? js : 0;
+        if (!chip && (r = ensure_basis(s))) return r;
+        if (chip && g[i] > 0) {
+            const size_t gb = gang_bytes(s, cfg.kmax, g[i], !cfg.mixed);
+            const size_t sb = gang_spill_bytes(s, cfg.kmax, g[i], my_js, !cfg.mixed);
+            if ((w.gang.bytes < gb && (r = w.gang.alloc(gb))) || (w.spill.bytes < sb && (r = w.spill.alloc(sb)))) return r;
+        }
+        hs[i].V = w.V.p;
+        set_gang_fields(hs[i], s, cfg.kmax, chip ? g[i] : 0, my_js, !cfg.mixed);
     }
     return FG_OK;
 }
@@ -1615,6 +1630,7 @@ int BatchRun::reschedule(const std::vector<int> &live)
     std::vector<CycItem> cyc;
     gang_items(hs, live, P->B, !cfg.mixed, cyc, P->cyc_smem);
     P->n_cyc = (int)cyc.size();
+    P->cyc_spill = P->n_cyc > 0 && hs[cyc[0].sys].cy_js > 0;
     if (P->n_cyc == 0) return FG_OK;               // still streaming
     unsigned char *d = arena->dev.as<unsigned char>();
     auto put = [&](const Plan::Span &to, const void *from, size_t bytes) -> cudaError_t {

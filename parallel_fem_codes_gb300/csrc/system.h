@@ -26,7 +26,7 @@ struct DevMem {
 struct Workspace {
     int kmax = 0, mixed = -1;
     DevMem V, w, t, x, b, ftrue, r64, t64, u64, small, part, counter, state;
-    DevMem gang;                       // exchange block of the on-chip cycle
+    DevMem gang, spill;                // exchange block of the on-chip cycle, basis vectors it has no room for
 };
 
 // Tables of a batch run on the device with their pinned staging, and the
@@ -335,12 +335,15 @@ int launch_rows_mv(int B, int prec, const SysDev *sys, const NChunk *ch, const i
 
 // Restart cycle on chip (cycle.cu)
 int gang_size(const fg_system *s, int kmax, bool f64, bool dense);
-int gang_ctas(int B, bool f64);   // CTAs of the on-chip cycle that are resident together
+int gang_spill(const fg_system *s, int kmax, bool f64);
+size_t gang_spill_bytes(const fg_system *s, int kmax, int g, int js, bool f64);
+int gang_ctas(int B, bool f64, bool spill = false);   // CTAs of the on-chip cycle that are resident together
 size_t gang_bytes(const fg_system *s, int kmax, int g, bool f64);
-void set_gang_fields(SysDev &D, const fg_system *s, int kmax, int g, bool f64);
+void set_gang_fields(SysDev &D, const fg_system *s, int kmax, int g, int js, bool f64);
 void gang_items(const std::vector<SysDev> &hs, const std::vector<int> &live, int B, bool f64,
                 std::vector<CycItem> &items, size_t &smem);
-int launch_cycle(int B, bool f64, const SysDev *sys, const CycItem *items, int ctas, size_t smem, cudaStream_t st);
+int launch_cycle(int B, bool f64, bool spill, const SysDev *sys, const CycItem *items, int ctas, size_t smem,
+                 cudaStream_t st);
 
 // Set-up kernels (setup.cu)
 int precond_setup_device(fg_system *s, int kind, int flags, double *F_dev, cudaStream_t st);

@@ -76,3 +76,16 @@ def test_breakdown_and_zero_right_hand_side(fg):
         assert r.stats["converged"] == 0 and r.stats["status"] == fg.FG_ERR_BREAKDOWN
         ok = s.solve(B, F_true=F, precision=prec)
         assert ok.stats["converged"] == 1
+
+
+@pytest.mark.parametrize("side,kmax,precision", [(370, 30, 64), (387, 30, 64), (560, 30, 32), (230, 60, 64)])
+def test_a_system_beyond_shared_memory(fg, side, kmax, precision):
+    # part of the basis in global memory; true residual by the element matvec
+    p = G.transport_problem(side, angle_deg=40.0, k=1e-3)
+    s = fg.transport_system(p)
+    s.transport_prepare(p)
+    st = fg.solve_resident([s], kmax=kmax, tol=1e-11, lmax=3000, precision=precision)[0]
+    assert st["converged"] == 1 and st["status"] == 0
+    x = s.solution()
+    F = s.transport_assemble(p)
+    assert np.linalg.norm((F - s.matvec(x))[:-1]) <= (1e-11 if precision == 32 else 1e-9) * np.linalg.norm(F[:-1])
