@@ -5,7 +5,7 @@
 // to 260k equations) is launch and latency bound: 30 to 80 us for work that
 // the chip's shared memory does in 1 or 2.  The basis of a whole restart
 // cycle fits it: 152 SMs x 218 KB hold 30 vectors of 268k FP32 (134k FP64)
-// entries.  So a gang of g CTAs (two per SM) owns a system for a cycle, CTA
+// entries.  So a gang of g CTAs (one per SM) owns a system for a cycle, CTA
 // `rank` the units [u0, u1) and their rows of every basis vector, and keeps
 // as many of their operator rows beside them as fit; the other rows are read
 // from L2 each step, and only the newest vector and the reductions pass
@@ -37,8 +37,8 @@
 // exchange that follows its reading.
 //
 // Measured (GB300), a whole solve with the pass kernels -> on chip, and an
-// Arnoldi step: 961 equations FP64 8.8 -> 2.4 ms (8 us a step), 16k FP64 26.5 ->
-// 6.7 ms (9 us), 16k FP32 21.9 -> 5.4 ms (7 us), 261k FP32 94 -> 31 ms (14 us).
+// Arnoldi step: 961 equations FP64 8.8 -> 1.9 ms (6 us a step), 16k FP64 26.5 ->
+// 5.8 ms (7 us), 16k FP32 21.9 -> 4.2 ms (5 us), 261k FP32 94 -> 24 ms (9 us).
 // What is left of a step is mostly the two trips through L2 of the exchange
 // (2 to 5 us with the CTAs' skew); the basis sweeps take 2 to 3 us.
 //
@@ -50,6 +50,7 @@
 // one system's gang.  Polls are bounded (~2 s): a CTA that gives up marks the
 // system FG_ERR_TIMEOUT and leaves.
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 #include <mutex>
 #include <type_traits>
@@ -60,7 +61,12 @@ namespace fg {
 
 namespace {
 
-constexpr int kWorkers = 256;                 // threads per CTA besides the Givens warp
+// Threads per CTA besides the Givens warp, one CTA an SM.  Halving the ranks
+// halves the words that a reduction polls, and the rank with a whole SM's rows
+// keeps as many threads: 148k equations FP64 38.8 -> 33.7 ms a solve (two CTAs of
+// 256 -> one of 512), 263k FP32 31.7 -> 24.1, 16k FP32 4.9 -> 4.2; one of 384
+// 36.9, 28.3, 4.5 (where 512 took 35.7, 26.4, 4.3), one of 256 39.0, 31.8, 4.4.
+constexpr int kWorkers = 512;
 constexpr int kCycThreads = kWorkers + 32;
 constexpr int kGroups = kWorkers / 8;         // 8-lane groups
 constexpr int kMaxSlices = 8;
@@ -253,7 +259,7 @@ __device__ __forceinline__ double gram_diag(const Sum<double> &n2, double sc) { 
 // global memory (L2), where only the CTA that owns the rows reads them; the two
 // newest vectors have shared-memory slots of their own.
 template <typename T, int B, bool SPILL>
-__global__ void __launch_bounds__(kCycThreads, 2)
+__global__ void __launch_bounds__(kCycThreads, 1)
 k_cycle(const SysDev *__restrict__ sys, const CycItem *__restrict__ items, int smem)
 {
     constexpr int N = Pack<T>::N, KM = kMaxRestart + 4, WP = kWords<T>;
@@ -798,7 +804,7 @@ const void *cycle_kernel(int B, bool f64, bool spill)
 }
 
 // What k_cycle<T, B> has on this device: the dynamic shared memory with which
-// two CTAs share an SM, and the CTAs that are then resident together (0:
+// one CTA fills an SM, and the CTAs that are then resident together (0:
 // none).  Looked up once per kernel; raises its shared-memory limit.
 struct Residency { int ctas; size_t smem; };
 Residency residency(int B, bool f64, bool spill = false)
@@ -819,11 +825,11 @@ Residency residency(int B, bool f64, bool spill = false)
             cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) == cudaSuccess && coop &&
             cudaDeviceGetAttribute(&sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev) == cudaSuccess &&
             cudaDeviceGetAttribute(&own, cudaDevAttrReservedSharedMemoryPerBlock, dev) == cudaSuccess &&
-            cudaFuncGetAttributes(&fa, k) == cudaSuccess && (size_t)sm / 2 > own + fa.sharedSizeBytes + 4096) {
-            const size_t cap = ((size_t)sm / 2 - own - fa.sharedSizeBytes) & ~(size_t)127;
+            cudaFuncGetAttributes(&fa, k) == cudaSuccess && (size_t)sm > own + fa.sharedSizeBytes + 4096) {
+            const size_t cap = ((size_t)sm - own - fa.sharedSizeBytes) & ~(size_t)127;
             if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cap) == cudaSuccess &&
                 cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, kCycThreads, cap) == cudaSuccess && occ > 0)
-                v = {std::min(occ, 2) * sm_count(), cap};
+                v = {sm_count(), cap};
         }
         cudaGetLastError();
     }
@@ -833,12 +839,19 @@ Residency residency(int B, bool f64, bool spill = false)
 }  // namespace
 
 // CTAs of a system's gang: enough for its rows to fit shared memory, and,
-// unless the batch is dense, while CTAs are left no more than kRows32 (FP32)
-// or kRows64 (FP64) rows each: below that a step is bound by the exchanges, and
-// the FP64 pipe (52 FMA a row and step at kmax 30, two a cycle) wants every
-// SM.  0: the system does not fit, or its numbering couples units too far
-// apart for the halo.
-constexpr int kRows32 = 512, kRows64 = 128;
+// unless the batch is dense, while CTAs are left no more than gang_want rows
+// each: below that a step is bound by the exchanges, whose words grow with the
+// gang, above it by the rows (FP64: 52 FMA a row and step at kmax 30, two a
+// cycle), so FP64 CTAs get rows as the square root of the units.  0: the system
+// does not fit, or its numbering couples units too far apart for the halo.
+// Measured with 512 / 256 / 128 rows FP32: 16k equations 4.70 / 4.32 / 4.46 ms a
+// solve; with 128 / 96 / 64 rows FP64: 961 equations 2.02 / 1.99 / 1.89, a
+// four-step process of 9k 19.1 / 17.0 / 18.2, 16k 5.62 / 5.69 / 5.69, Euler with
+// 4k nodes 5.02 / 4.71 / 4.73; with 32 rows 961 equations 1.87, 9k 19.9.
+static int gang_want(const fg_system *s, bool f64)
+{
+    return f64 ? std::max(64, (int)std::sqrt((double)s->topo.nunits)) : 256;
+}
 static int halo_units(const fg_system *s) { return std::min(s->topo.nunits, s->topo.rw_lo + s->topo.rw_hi); }
 int gang_rows(const fg_system *s, int g);
 int gang_size(const fg_system *s, int kmax, bool f64, bool dense)
@@ -850,7 +863,7 @@ int gang_size(const fg_system *s, int kmax, bool f64, bool dense)
     const size_t w = f64 ? 8 : 4, fixed = cycle_smem(kmax, 0, halo_units(s) * B, w);
     if (fixed + (size_t)kmax * w * 64 > dev.smem) return 0;
     const int cap = (int)((dev.smem - fixed) / (kmax * w)) & ~3;
-    const int cap_u = cap / B, want_u = dense ? cap_u : std::max(1, std::min(cap_u, (f64 ? kRows64 : kRows32) / B));
+    const int cap_u = cap / B, want_u = dense ? cap_u : std::max(1, std::min(cap_u, gang_want(s, f64) / B));
     const int g = std::max((nu + cap_u - 1) / cap_u, std::min(ctas, (nu + want_u - 1) / want_u));
     return g <= ctas ? g : 0;
 }

@@ -21,8 +21,8 @@ def fg():
     return femgpu
 
 
-# 128 FP64 rows (512 FP32) a CTA: 100, 256, 961, 1089, 4096 equations
-@pytest.mark.parametrize("side,kmax", [(12, 30), (18, 30), (33, 30), (35, 30), (66, 30), (33, 3), (35, 33), (35, 60), (12, 60)])
+# 64 FP64 rows (256 FP32) a CTA: 64, 100, 256, 484, 529, 961, 1089, 4096 equations
+@pytest.mark.parametrize("side,kmax", [(10, 30), (12, 30), (18, 30), (24, 30), (25, 30), (33, 30), (35, 30), (66, 30), (33, 3), (35, 33), (35, 60), (12, 60)])
 def test_matches_the_oracle(fg, side, kmax):
     p = G.transport_problem(side, angle_deg=40.0, k=1e-3)
     m = p.mesh
