@@ -913,24 +913,32 @@ void set_gang_fields(SysDev &D, const fg_system *s, int kmax, int g, int js, boo
     D.cy_vb = p + gang_head(kmax, g, f64);
 }
 
-// The CTAs of a cycle launch: every rank of every live system (live empty:
-// all) that has a gang, and the shared memory of the largest.
+// The CTAs of a cycle's launches: every rank of every live system (live empty:
+// all) that has a gang, bin by bin, and the shared memory of a bin's largest.
 void gang_items(const std::vector<SysDev> &hs, const std::vector<int> &live, int B, bool f64,
-                std::vector<CycItem> &items, size_t &smem)
+                std::vector<CycItem> &items, std::vector<CycBin> &bins)
 {
     const size_t w = f64 ? 8 : 4;
     items.clear();
-    smem = 0;
-    for (int i = 0; i < (int)hs.size(); ++i) {
-        const SysDev &D = hs[i];
-        if (D.cy_g == 0 || (!live.empty() && !live[i])) continue;
-        for (int r = 0; r < D.cy_g; ++r)
-            items.push_back({i, r, (int)((long long)D.nunits * r / D.cy_g), (int)((long long)D.nunits * (r + 1) / D.cy_g)});
-        // and the operator's rows, as far as they fit
-        const size_t cap = residency(B, f64, D.cy_js > 0).smem;
-        const size_t need = cycle_smem(D.kmax, 0, 0, w) + w * (D.cy_js > 0 ? D.cy_js + 2 : D.kmax) * D.cy_rows +
-                            cycle_smem(0, 0, std::min(D.nunits, D.rw_lo + D.rw_hi) * B, w);
-        smem = std::max(smem, std::min(cap, need + (size_t)D.cy_rows * D.rw_w * (B * w + 2) + 16));
+    bins.clear();
+    int nbin = 0;
+    for (const SysDev &D : hs) nbin = std::max(nbin, D.cy_bin + 1);
+    for (int b = 0; b < nbin; ++b) {
+        CycBin bin{(int)items.size(), 0, 0, false};
+        for (int i = 0; i < (int)hs.size(); ++i) {
+            const SysDev &D = hs[i];
+            if (D.cy_g == 0 || D.cy_bin != b || (!live.empty() && !live[i])) continue;
+            for (int r = 0; r < D.cy_g; ++r)
+                items.push_back({i, r, (int)((long long)D.nunits * r / D.cy_g), (int)((long long)D.nunits * (r + 1) / D.cy_g)});
+            // and the operator's rows, as far as they fit
+            const size_t cap = residency(B, f64, D.cy_js > 0).smem;
+            const size_t need = cycle_smem(D.kmax, 0, 0, w) + w * (D.cy_js > 0 ? D.cy_js + 2 : D.kmax) * D.cy_rows +
+                                cycle_smem(0, 0, std::min(D.nunits, D.rw_lo + D.rw_hi) * B, w);
+            bin.smem = std::max(bin.smem, std::min(cap, need + (size_t)D.cy_rows * D.rw_w * (B * w + 2) + 16));
+            bin.spill = bin.spill || D.cy_js > 0;
+        }
+        bin.ctas = (int)items.size() - bin.first;
+        if (bin.ctas) bins.push_back(bin);
     }
 }
 

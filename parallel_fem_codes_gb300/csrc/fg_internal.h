@@ -187,6 +187,7 @@ struct SysDev {
     // gang of the on-chip restart cycle (cycle.cu): CTAs (0: streaming
     // kernels), padded rows of each, exchange words, vector and epoch
     int cy_g, cy_rows;
+    int cy_bin;                // its launch among a cycle's
     int cy_js;                 // > 0: basis vectors in shared memory, the others in cy_spill
     void *cy_spill;
     unsigned long long *cy_part;
@@ -246,6 +247,8 @@ __host__ __device__ constexpr bool precond_separate(int p) { return p >= 2; }
 struct EChunk { int sys, e0, e1; };
 // One (system, rank) of a restart cycle on chip: the units [u0, u1) (cycle.cu)
 struct CycItem { int sys, rank, u0, u1; };
+// One launch of on-chip cycles: the CTAs [first, first + ctas) of the items
+struct CycBin { int first, ctas; size_t smem; bool spill; };
 struct DChunk { int sys, part, d0, d1; };
 struct NChunk { int sys, n0, n1; };
 

@@ -931,9 +931,7 @@ struct Plan {
     };
     Span sysdev, dchunks, dcount, nchunks, ncount;
     Span cyc_items;                                // on-chip cycle: (system, rank) of its CTAs
-    int n_cyc = 0;                                 // its CTAs (0: the cycle streams)
-    size_t cyc_smem = 0;
-    bool cyc_spill = false;                        // one system, part of its basis in global memory
+    std::vector<CycBin> bins;                      // its launches (none: the cycle streams)
     bool rprec = false;                            // a right preconditioner (SGSe) before every matvec
     Span ilu_fwd, ilu_bwd, ilu_ctr;                // sync-free ILU(0) substitutions
     Span ilu_ws;                                 // block-Jacobi: (system, block) items, a warp each
@@ -944,6 +942,7 @@ struct Plan {
 
 static int choose_engine(const std::vector<BatchMember> &mem, const SolveConfig &cfg, std::vector<SysDev> &hs,
                          const std::vector<int> &live, int B);
+static size_t items_room(const std::vector<BatchMember> &mem, const SolveConfig &cfg, int B);
 
 // cycles: restart cycles will run (else only residuals)
 static int build_plan(Plan &P, std::vector<BatchMember> &mem, const SolveConfig &cfg, std::vector<SysDev> &hs,
@@ -975,9 +974,7 @@ static int build_plan(Plan &P, std::vector<BatchMember> &mem, const SolveConfig 
         for (int a = 0; a < nn; a += uchunk) nch.push_back({s, a, std::min(a + uchunk, nn)});
     }
     std::vector<CycItem> cyc;
-    if (cycles) gang_items(hs, {}, P.B, !cfg.mixed, cyc, P.cyc_smem);
-    P.n_cyc = (int)cyc.size();
-    P.cyc_spill = P.n_cyc > 0 && hs[cyc[0].sys].cy_js > 0;
+    if (cycles) gang_items(hs, {}, P.B, !cfg.mixed, cyc, P.bins);
     P.n_dch = (int)dch.size();
     P.n_nch = (int)nch.size();
     P.precond = cfg.precond;
@@ -1039,7 +1036,7 @@ static int build_plan(Plan &P, std::vector<BatchMember> &mem, const SolveConfig 
     const Piece all[] = {
         piece(P.sysdev, hs), piece(P.dchunks, dch), {&P.dcount, &P.n_dch, sizeof(int), sizeof(int)},
         piece(P.nchunks, nch), {&P.ncount, &P.n_nch, sizeof(int), sizeof(int)},
-        piece(P.cyc_items, cyc, cycles ? gang_ctas(P.B, !cfg.mixed) : 0), piece(P.ilu_fwd, fwd), piece(P.ilu_bwd, bwd),
+        piece(P.cyc_items, cyc, cycles ? items_room(mem, cfg, P.B) : 0), piece(P.ilu_fwd, fwd), piece(P.ilu_bwd, bwd),
         {&P.ilu_ctr, zeros, sizeof(zeros), sizeof(zeros)}, piece(P.ilu_ws, wit), piece(P.sp_blocks, spb),
         piece(P.sp_ifaces, spi)};
     size_t bytes = 0;
@@ -1143,8 +1140,8 @@ static int enqueue_precond(const Plan &P, int sel, cudaStream_t st)
 
 // One restart cycle for every member; returns the number of kernels.  TV
 // is the basis' storage type (T, or FP16 under FP32 arithmetic).  A batch
-// whose bases fit the chip together runs its Arnoldi steps in one kernel
-// (cycle.cu), any other streams through the pass kernels below.
+// whose bases fit the chip runs its Arnoldi steps in a kernel, or a few
+// (cycle.cu, choose_engine), any other streams through the pass kernels below.
 template <typename T, typename TV = T>
 static int enqueue_cycle(const Plan &P, const SolveConfig &cfg, int *live, cudaStream_t st)
 {
@@ -1155,11 +1152,9 @@ static int enqueue_cycle(const Plan &P, const SolveConfig &cfg, int *live, cudaS
     k += enqueue_precond<T>(P, 0, st);
     k_start<<<grid_for(P.n_dch), kThreads, 0, st>>>(sys, dc, nd);
     ++k;
-    if (P.n_cyc > 0) {
-        constexpr bool f64 = sizeof(T) == 8;
-        k += launch_cycle(P.B, f64, P.cyc_spill, sys, P.cyc_items.as<CycItem>(), P.n_cyc, P.cyc_smem, st);
-    }
-    else {
+    for (const CycBin &b : P.bins)
+        k += launch_cycle(P.B, sizeof(T) == 8, b.spill, sys, P.cyc_items.as<CycItem>() + b.first, b.ctas, b.smem, st);
+    if (P.bins.empty()) {
         const dim3 gd = grid_for(P.n_dch);
         // few parts: several CTAs each, up to eight CTAs an SM in all
         const int split = std::max(1, std::min(16, 8 * sm_count() / std::max(1, P.n_dch)));
@@ -1194,6 +1189,18 @@ static bool chip_config(const SolveConfig &cfg)
 static int member_gang(const fg_system *s, const SolveConfig &cfg, bool dense)
 {
     return chip_config(cfg) ? gang_size(s, cfg.kmax, !cfg.mixed, dense) : 0;
+}
+
+// CTAs that the members' on-chip launches may hold at most, now or as members stop
+static size_t items_room(const std::vector<BatchMember> &mem, const SolveConfig &cfg, int B)
+{
+    const size_t room = gang_ctas(B, !cfg.mixed);
+    size_t sum = 0;
+    for (const BatchMember &m : mem) {
+        const int g = member_gang(m.s, cfg, true);
+        sum += g ? g : room;
+    }
+    return chip_config(cfg) ? std::max(room, sum) : 0;
 }
 
 // mode: 0 FP64, 1 FP32 basis, 2 FP16 basis (mixed precision in both)
@@ -1468,49 +1475,64 @@ int BatchRun::stage(const BatchMember &m)
     return FG_OK;
 }
 
-// Where the batch's restart cycles run, for the live members (all: empty): on
-// chip when their gangs are resident together (CTAs of about kRows rows if
-// those fit, else as few as hold the systems), or partly on chip for a system
-// alone, else streaming through global memory.  Measured on 32 transport instances, 3.1 M equations: one Arnoldi
-// step of all 201 us on chip in 19 rounds, 171 us streaming; a single one of
-// them of 261k equations 12 us on chip, 55 us streaming.
+// Where the batch's restart cycles run, for the live members (all: empty).  On
+// chip when gangs of the CTAs they like (gang_want) are resident together.
+// Else as up to kMaxBins launches one behind the other, in which gangs are as
+// small as their rows allow and a member that fits no chip has all of one with
+// part of its basis outside.  Else streaming through global memory, all at once:
+// a launch is about 9 us a step (FP64 20 to 50) whatever it holds up to 276k
+// equations, while streaming takes 25 us (FP64 55) and little more for each
+// further member.  Measured, streaming -> launches: 2 transport instances 55.6 ->
+// 33.8 ms (FP64 101 -> 75), 4 67.7 -> 41.5, 10 in 4 launches 88.4 -> 76.6 (FP64 139 ->
+// 129), 16 in 7 141.1 -> 144.6, 64 in up to 24 480 -> 544.
+constexpr int kMaxBins = 4;
 static int choose_engine(const std::vector<BatchMember> &mem, const SolveConfig &cfg, std::vector<SysDev> &hs,
                          const std::vector<int> &live, int B)
 {
-    const int room = gang_ctas(B, !cfg.mixed);
-    bool chip = false;
-    std::vector<int> g(mem.size(), 0);
-    for (int dense = 0; dense < 2 && !chip; ++dense) {
-        long long sum = 0;
-        chip = true;
-        for (size_t i = 0; i < mem.size() && chip; ++i) {
-            if (!live.empty() && !live[i]) continue;
-            g[i] = member_gang(mem[i].s, cfg, dense != 0);
-            sum += g[i];
+    const int room = gang_ctas(B, !cfg.mixed), n = (int)mem.size();
+    std::vector<int> g(n, 0), js(n, 0), bin(n, 0);
+    std::vector<int> todo;
+    for (int i = 0; i < n; ++i)
+        if (live.empty() || live[i]) todo.push_back(i);
+    bool chip = chip_config(cfg) && room > 0;
+    long long sum = 0;
+    for (int i : todo)
+        if (chip) {
+            sum += g[i] = member_gang(mem[i].s, cfg, false);
             chip = g[i] > 0 && sum <= room;
         }
-    }
-    // a system alone may keep part of its basis outside
-    int alone = -1, js = 0;
-    for (size_t i = 0; i < mem.size(); ++i)
-        if (live.empty() || live[i]) alone = alone == -1 ? (int)i : -2;
-    if (!chip && alone >= 0 && chip_config(cfg) && (js = gang_spill(mem[alone].s, cfg.kmax, !cfg.mixed)) > 0) {
+    if (!chip && chip_config(cfg) && room > 0) {
+        // launches of dense gangs, the largest first
         chip = true;
-        g[alone] = gang_ctas(B, !cfg.mixed, true);
+        for (int i : todo) {
+            g[i] = member_gang(mem[i].s, cfg, true);
+            if (!g[i] && (js[i] = gang_spill(mem[i].s, cfg.kmax, !cfg.mixed)) > 0) g[i] = gang_ctas(B, !cfg.mixed, true);
+            chip = chip && g[i] > 0;
+        }
+        std::stable_sort(todo.begin(), todo.end(), [&](int a, int b) { return g[a] > g[b]; });
+        std::vector<int> left;
+        for (int i : todo) {
+            size_t b = 0;
+            while (b < left.size() && (js[i] || left[b] < g[i])) ++b;
+            if (b == left.size()) left.push_back(room);
+            bin[i] = (int)b;
+            left[b] = js[i] ? 0 : left[b] - g[i];
+        }
+        chip = chip && (int)left.size() <= kMaxBins;
     }
-    for (size_t i = 0; i < mem.size(); ++i) {
+    for (int i = 0; i < n; ++i) {
         int r;
         fg_system *s = mem[i].s;
         Workspace &w = s->ws;
-        const int my_js = (int)i == alone ? js : 0;
         if (!chip && (r = ensure_basis(s))) return r;
         if (chip && g[i] > 0) {
             const size_t gb = gang_bytes(s, cfg.kmax, g[i], !cfg.mixed);
-            const size_t sb = gang_spill_bytes(s, cfg.kmax, g[i], my_js, !cfg.mixed);
+            const size_t sb = gang_spill_bytes(s, cfg.kmax, g[i], js[i], !cfg.mixed);
             if ((w.gang.bytes < gb && (r = w.gang.alloc(gb))) || (w.spill.bytes < sb && (r = w.spill.alloc(sb)))) return r;
         }
         hs[i].V = w.V.p;
-        set_gang_fields(hs[i], s, cfg.kmax, chip ? g[i] : 0, my_js, !cfg.mixed);
+        hs[i].cy_bin = bin[i];
+        set_gang_fields(hs[i], s, cfg.kmax, chip ? g[i] : 0, chip ? js[i] : 0, !cfg.mixed);
     }
     return FG_OK;
 }
@@ -1544,7 +1566,7 @@ int BatchRun::enqueue(bool use_graph, int *flags)
         return cfg.vhalf ? enqueue_cycle<float, __half>(Pl, cfg, flags, st)
                : cfg.mixed ? enqueue_cycle<float>(Pl, cfg, flags, st) : enqueue_cycle<double>(Pl, cfg, flags, st);
     };
-    if (Pl.n_cyc > 0) use_graph = false;           // on chip: a few launches
+    if (!Pl.bins.empty()) use_graph = false;           // on chip: a few launches
     if (use_graph && !exec) {
         cudaGraph_t graph = nullptr;
         FG_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
@@ -1612,7 +1634,7 @@ int BatchRun::run(bool use_graph, int limit)
 }
 
 // whether a cycle is a graph, whose nodes hold the address of the flags
-bool BatchRun::use_graph_streams(bool use_graph) const { return use_graph && P && P->n_cyc == 0; }
+bool BatchRun::use_graph_streams(bool use_graph) const { return use_graph && P && P->bins.empty(); }
 
 // Once members stopped: the remaining ones spread over all CTAs again, or move
 // on chip now that they fit.  Nothing is in flight.
@@ -1628,10 +1650,8 @@ int BatchRun::reschedule(const std::vector<int> &live)
     int r = choose_engine(mem, cfg, hs, live, P->B);
     if (r) return r;
     std::vector<CycItem> cyc;
-    gang_items(hs, live, P->B, !cfg.mixed, cyc, P->cyc_smem);
-    P->n_cyc = (int)cyc.size();
-    P->cyc_spill = P->n_cyc > 0 && hs[cyc[0].sys].cy_js > 0;
-    if (P->n_cyc == 0) return FG_OK;               // still streaming
+    gang_items(hs, live, P->B, !cfg.mixed, cyc, P->bins);
+    if (P->bins.empty()) return FG_OK;               // still streaming
     unsigned char *d = arena->dev.as<unsigned char>();
     auto put = [&](const Plan::Span &to, const void *from, size_t bytes) -> cudaError_t {
         unsigned char *h = arena->host + (to.as<unsigned char>() - d);

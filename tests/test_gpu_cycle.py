@@ -89,3 +89,19 @@ def test_a_system_beyond_shared_memory(fg, side, kmax, precision):
     x = s.solution()
     F = s.transport_assemble(p)
     assert np.linalg.norm((F - s.matvec(x))[:-1]) <= (1e-11 if precision == 32 else 1e-9) * np.linalg.norm(F[:-1])
+
+
+# 376 x 376 equations fit 152 CTAs in FP64, 525 x 525 in FP32; up to four launches, then streaming
+@pytest.mark.parametrize("sides,precision", [((380, 40, 300, 35), 64), ((200, 290, 210, 300, 220), 64), ((340, 350, 360, 365, 370), 64),
+                                             ((513, 37, 400), 32), ((530, 36), 32), ((500, 505, 510, 513, 37, 500), 32)])
+def test_a_batch_in_several_launches(fg, sides, precision):
+    probs = [G.transport_problem(n, angle_deg=11.0 * n, k=10.0 ** -(2 + n % 3)) for n in sides]
+    systems = [fg.transport_system(p) for p in probs]
+    for s, p in zip(systems, probs):
+        s.transport_prepare(p)
+    st = fg.solve_resident(systems, tol=1e-11, lmax=3000, precision=precision)
+    for s, p, q in zip(systems, probs, st):
+        assert q["converged"] == 1 and q["status"] == 0
+        x = s.solution()
+        F = s.transport_assemble(p)
+        assert np.linalg.norm((F - s.matvec(x))[:-1]) <= (1e-11 if precision == 32 else 1e-9) * np.linalg.norm(F[:-1])
