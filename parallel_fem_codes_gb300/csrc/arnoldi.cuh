@@ -55,12 +55,20 @@ template <typename T, int G> __device__ __forceinline__ void st_g(T *p, const T 
         st_pk(p + h * N, v);
     }
 }
-// one basis pack as T
-template <typename T, typename TV>
+// 16 bytes of the basis, which passes through: L1 is left to the vectors that
+// every group of basis vectors reads again
+__device__ __forceinline__ uint4 ld_stream(const void *p)
+{
+    uint4 r;
+    asm volatile("ld.global.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];\n" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(p));
+    return r;
+}
+// one basis pack as T (KEEP: read again soon)
+template <typename T, typename TV, bool KEEP = false>
 __device__ __forceinline__ void ld_v(const TV *p, T (&o)[VPk<TV>::G])
 {
     if constexpr (std::is_same<TV, __half>::value) {
-        const uint4 r = *reinterpret_cast<const uint4 *>(p);
+        const uint4 r = KEEP ? *reinterpret_cast<const uint4 *>(p) : ld_stream(p);
         const unsigned u[4] = {r.x, r.y, r.z, r.w};
 #pragma unroll
         for (int h = 0; h < 4; ++h) {
@@ -71,7 +79,8 @@ __device__ __forceinline__ void ld_v(const TV *p, T (&o)[VPk<TV>::G])
             o[2 * h + 1] = (T)f.y;
         }
     } else {
-        ld_g<T, VPk<TV>::G>(reinterpret_cast<const T *>(p), o);
+        const uint4 r = KEEP ? *reinterpret_cast<const uint4 *>(p) : ld_stream(p);
+        memcpy(&o[0], &r, 16);
     }
 }
 template <typename T, typename TV>
@@ -115,9 +124,13 @@ __device__ __forceinline__ void part_dots(const SysDev &D, const DChunk &k, int 
         for (int q = k.d0 + threadIdx.x * G; q < k.d1; q += kThreads * G) {
             T w0[G], u0[G], v[JB][G];
 #pragma unroll
-            for (int u = 0; u < JB; ++u) ld_v<T, TV>(V + min(j0 + u, i) * ld + q, v[u]);
+            for (int u = 0; u < JB; ++u)
+                if (j0 + u <= i) ld_v<T, TV>(V + (j0 + u) * ld + q, v[u]);
+                else
+#pragma unroll
+                    for (int c = 0; c < G; ++c) v[u][c] = (T)0;
             ld_g<T, G>(w + q, w0);
-            ld_v<T, TV>(vi + q, u0);
+            ld_v<T, TV, true>(vi + q, u0);
 #pragma unroll
             for (int u = 0; u < JB; ++u)
 #pragma unroll
@@ -198,7 +211,7 @@ k_dots(const SysDev *__restrict__ sys, const DChunk *__restrict__ ch, const int 
 // place, k_normalize stores it), and its norm; then, in the last part, the
 // Givens step and the cycle's stop test.
 template <typename T, typename TV>
-__global__ void __launch_bounds__(kThreads, 4)
+__global__ void __launch_bounds__(kThreads, 3)
 k_orth(const SysDev *__restrict__ sys, const DChunk *__restrict__ ch, const int *__restrict__ nch, int i)
 {
     constexpr int G = VPk<TV>::G, JB = sizeof(TV) == 2 ? 4 : 8;
@@ -207,7 +220,7 @@ k_orth(const SysDev *__restrict__ sys, const DChunk *__restrict__ ch, const int 
     const int total = *nch;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     for (int c = blockIdx.x; c < total; c += gridDim.x) {
-        const DChunk k = ch[c];
+        const DChunk k = ch[total - 1 - c];      // pass 1's last parts first: those are in L2
         const SysDev &D = sys[k.sys];
         if (!D.st->in_cycle) continue;
         __syncthreads();
@@ -242,10 +255,11 @@ k_orth(const SysDev *__restrict__ sys, const DChunk *__restrict__ ch, const int 
                     }
                 }
             }
-            if (j <= i) {                     // the rest: loads past i repeat V[i], unused
+            if (j <= i) {                     // the rest
                 T v[JB][G];
 #pragma unroll
-                for (int u = 0; u < JB - 1; ++u) ld_v<T, TV>(V + min(j + u, i) * ld + q, v[u]);
+                for (int u = 0; u < JB - 1; ++u)
+                    if (j + u <= i) ld_v<T, TV>(V + (j + u) * ld + q, v[u]);
 #pragma unroll
                 for (int u = 0; u < JB - 1; ++u) {
                     if (j + u > i) break;

@@ -66,6 +66,8 @@ struct Topology {
     // kRowSlice + l, value = coupled unit (kRowPad set: unused slot)
     int nunits = 0;
     std::vector<int> rw_off, rw_col;
+    std::vector<short> rw_dc;            // coupled unit - unit per slot (unused: 0); empty where a difference has no 16 bits
+    int rw_u = 0;                        // > 0: every slice has this width, rw_off[s] = s * rw_u * kRowSlice
     int rw_lo = 0, rw_hi = 0;            // a unit u couples to units in [u - rw_lo, u + rw_hi]
     int rw_w = 0;                        // widest slice (slots per unit)
 };
@@ -194,6 +196,8 @@ struct SysDev {
     void *cy_vb;
     unsigned *cy_epoch;
     const int *rw_off, *rw_col;
+    const short *rw_dc;        // null: rw_col only
+    int rw_u;
     const double *rw64;
     const float *rw32;
     // assembled CSR operator and ILU(0) (op == 1)

@@ -894,13 +894,27 @@ namespace {
 // part size of a batch (multiple of 8 dofs): the tuned one, else
 // 2 sqrt(batch dofs) up to 64k dofs and 4 sqrt above (where a part's sums are
 // split among CTAs), rounded to the nearest power of two, within [kPartMin,
-// kPartMax] (powers of two: a system solved alone and inside a
-// batch of similar size get the same parts, hence bit-identical results)
+// kPartMax] (powers of two: a system solved alone and inside a batch of similar
+// size get the same parts, hence bit-identical results).  A batch that gives
+// every resident CTA (3 an SM; FP64, which splits the sums, 4) a part of 1024 dofs
+// (a pass of its threads) takes the smallest multiple of that with which the
+// parts fill whole rounds of CTAs: 4.0 M dofs FP32 on 152 SMs, a step with 8192
+// dofs in 506 parts 173 us, with 9216 in 452 parts 156; 3 M FP64 391 -> 362.
 int part_dofs_for(const std::vector<BatchMember> &mem, const SolveConfig &cfg)
 {
     fg_tune_choice tc;
     if (tuned_choice(mem, cfg, tc) && tc.part_dofs > 0) return tc.part_dofs & ~7;
-    const double tot = (double)std::max(1LL, batch_dofs(mem));
+    const long long dofs = std::max(1LL, batch_dofs(mem)), round = (cfg.mixed ? 3LL : 4LL) * sm_count();
+    if (dofs > 1024 * round) {
+        for (long long rounds = 1;; ++rounds)
+            for (int pd = 1024; pd <= kPartMax; pd += 1024) {
+                if (dofs > rounds * round * pd) continue;
+                long long parts = 0;
+                for (auto &m : mem) parts += parts_for(m.s->topo.n, pd);
+                if (parts <= rounds * round) return pd;
+            }
+    }
+    const double tot = (double)dofs;
     const long long pd = 1LL << (int)std::lround(std::log2((tot > 65536.0 ? 4.0 : 2.0) * std::sqrt(tot)));
     return (int)std::max<long long>(kPartMin, std::min<long long>(kPartMax, pd));
 }
@@ -1156,15 +1170,21 @@ static int enqueue_cycle(const Plan &P, const SolveConfig &cfg, int *live, cudaS
         k += launch_cycle(P.B, sizeof(T) == 8, b.spill, sys, P.cyc_items.as<CycItem>() + b.first, b.ctas, b.smem, st);
     if (P.bins.empty()) {
         const dim3 gd = grid_for(P.n_dch);
-        // few parts: several CTAs each, up to eight CTAs an SM in all
-        const int split = std::max(1, std::min(16, 8 * sm_count() / std::max(1, P.n_dch)));
+        // Few parts: several CTAs each, up to eight CTAs an SM in all.  FP32: none
+        // once parts fill two CTAs an SM (4.0 M dofs in 452 parts, CTAs a part in
+        // the two passes 1 and 1: 156 us a step, 2 and 2: 163, 4 and 4: 174); FP64 is bound by
+        // its pipe and wants it evenly loaded (3 M dofs in 600 parts, 1 and 1: 397,
+        // 2 and 2: 373, 4 and 2: 362).
+        const int fill = 8 * sm_count() / std::max(1, P.n_dch), ways = std::min(16, fill * (sizeof(T) == 8 ? 2 : 1));
+        const bool split = sizeof(T) == 8 || P.n_dch < 2 * sm_count();
+        const int yd = split ? std::max(1, ways) : 1, yo = split ? std::max(1, std::min(kMaxSplit, fill)) : 1;
         k_scale_v0<T, TV><<<gd, kThreads, 0, st>>>(sys, dc, nd);
         ++k;
         for (int i = 0; i < cfg.kmax - 1; ++i) {
             k += enqueue_matvec<T, TV>(P, 1, i, st);
             k += enqueue_precond<T>(P, 1, st);
-            k_dots<T, TV><<<dim3(gd.x, std::min(split, (i + 4) / 4)), kThreads, 0, st>>>(sys, dc, nd, i);
-            k_orth<T, TV><<<dim3(gd.x, std::min(split, kMaxSplit)), kThreads, 0, st>>>(sys, dc, nd, i);
+            k_dots<T, TV><<<dim3(gd.x, std::min(yd, (i + 4) / 4)), kThreads, 0, st>>>(sys, dc, nd, i);
+            k_orth<T, TV><<<dim3(gd.x, yo), kThreads, 0, st>>>(sys, dc, nd, i);
             k += 2;
             if constexpr (!std::is_same<T, TV>::value) {
                 k_normalize<T, TV><<<gd, kThreads, 0, st>>>(sys, dc, nd, i);
@@ -1482,10 +1502,10 @@ int BatchRun::stage(const BatchMember &m)
 // part of its basis outside.  Else streaming through global memory, all at once:
 // a launch is about 9 us a step (FP64 20 to 50) whatever it holds up to 276k
 // equations, while streaming takes 25 us (FP64 55) and little more for each
-// further member.  Measured, streaming -> launches: 2 transport instances 55.6 ->
-// 33.8 ms (FP64 101 -> 75), 4 67.7 -> 41.5, 10 in 4 launches 88.4 -> 76.6 (FP64 139 ->
-// 129), 16 in 7 141.1 -> 144.6, 64 in up to 24 480 -> 544.
-constexpr int kMaxBins = 4;
+// further member.  Measured, streaming -> launches: 2 transport instances 53.9 ->
+// 33.7 ms (FP64 100 -> 74), 4 65.9 -> 41.7, 10 in up to 3 launches 74.8 -> 71.5 (FP64
+// 132 -> 126), in up to 4 74.9 (FP64 127), 16 119.5 -> 117.3, in up to 6 125.2.
+constexpr int kMaxBins = 3;
 static int choose_engine(const std::vector<BatchMember> &mem, const SolveConfig &cfg, std::vector<SysDev> &hs,
                          const std::vector<int> &live, int B)
 {
@@ -1844,7 +1864,7 @@ int bench_matvec(std::vector<fg_system *> &systems, int precision, int reps, dou
         hs.push_back(make_desc(s, cfg, false));
         const Topology &t = s->topo;
         // the assembled operator: values, columns, x once, y once
-        b += (double)t.rw_col.size() * (t.ndof * t.ndof * w + 4.0) + 2.0 * t.n * w;
+        b += (double)t.rw_col.size() * (t.ndof * t.ndof * w + (t.rw_dc.empty() ? 4.0 : 2.0)) + 2.0 * t.n * w;
     }
     cudaStream_t st = systems[0]->stream;
     Plan P;

@@ -8,9 +8,9 @@
 // summed.  Assembled it is about 7 coupled nodes per node, B^2 values and one
 // column each, summed by the thread that owns the row: one launch, no
 // staging, no atomics.  Bytes per node and matvec, FP32 (FP64):
-//   1 dof   105 (177) by elements,   64  (92) assembled
-//   3 dofs  756 (1404),             304 (556)
-//   4 dofs 1296 (2448),             508 (956)
+//   1 dof   105 (177) by elements,   50  (78) assembled
+//   3 dofs  756 (1404),             290 (542)
+//   4 dofs 1296 (2448),             494 (942)
 // The same holds for the FP64 pipe (about 2 FMA per clock and SM on this
 // part): 12 x 12 blocks take 288 FMA per node by elements, 112 assembled.
 // The sums differ from the element order by rounding only; an FP32 entry is
@@ -24,9 +24,11 @@
 //
 // Layout: units (1 dof per node: the internal dofs; else the mesh nodes) in
 // slices of kRowSlice; slot k of unit l of a slice starts at entry
-// e = off[slice] + k * kRowSlice + l: its column (a unit) at col[e], its
+// e = off[slice] + k * kRowSlice + l: its column (a unit) at col[e], the
+// column's distance from the unit at dc[e] where 16 bits hold all of them, its
 // B x B block, row-major, at value e * B * B.  A slice is as wide as its
-// widest unit.  Rows and columns of prescribed dofs are zero.
+// widest unit, or, where that pads by an eighth at most, as the widest of all.
+// Rows and columns of prescribed dofs are zero.
 #include <algorithm>
 #include <type_traits>
 
@@ -191,6 +193,54 @@ k_rows_mv(const SysDev *__restrict__ sys, const NChunk *__restrict__ ch, const i
         const TA *A = sizeof(TA) == 8 ? (const TA *)D.rw64 : (const TA *)D.rw32;
         const int n = D.n;
         const int *col = D.rw_col, *nd = D.node_dof;
+        const short *dc = D.rw_dc;
+        const int ru = D.rw_u;
+        if constexpr (B == 1 && sizeof(TA) == 4) {
+            // Slices of one width, at most U: two rows a thread, in 8- and 4-byte
+            // loads.  The pass waits on its loads: half the instructions carry the
+            // same bytes, and 1.7 times the rows are in flight (4.0 M dofs:
+            // one row a thread and 32-bit columns 63 us, 16-bit and twice the
+            // CTAs 52, two rows 38; 33 at copy bandwidth).
+            if (dc && ru > 0 && ru <= U) {
+                for (int u = k.n0 + 2 * threadIdx.x; u < k.n1; u += 2 * kThreads) {
+                    const bool two = u + 1 < k.n1;
+                    const int e = u / kRowSlice * ru * kRowSlice + u % kRowSlice;
+                    short2 m[U];
+                    float2 a[U];
+#pragma unroll
+                    for (int q = 0; q < U; ++q) {
+                        m[q] = make_short2(0, 0);
+                        a[q] = make_float2(0.0f, 0.0f);
+                        if (q < ru) {
+                            m[q] = __ldcs(reinterpret_cast<const short2 *>(dc + e + q * kRowSlice));
+                            a[q] = __ldcs(reinterpret_cast<const float2 *>(A + e + q * kRowSlice));
+                        }
+                    }
+                    const float2 pc = out == 2 && D.precond == FG_PRECOND_DIAG
+                                          ? make_float2(((const float *)D.invd32)[u], ((const float *)D.invd32)[two ? u + 1 : u])
+                                          : make_float2(1.0f, 1.0f);
+                    float x0[U], x1[U], y0 = 0.0f, y1 = 0.0f;
+#pragma unroll
+                    for (int q = 0; q < U; ++q) {
+                        x0[q] = row_x<TA, TX>(X[u + m[q].x], D);
+                        x1[q] = row_x<TA, TX>(X[two ? u + 1 + m[q].y : u], D);
+                    }
+#pragma unroll
+                    for (int q = 0; q < U; ++q) { y0 += a[q].x * x0[q]; y1 += a[q].y * x1[q]; }
+                    y0 *= pc.x;
+                    y1 *= pc.y;
+                    if (out == 0) {
+                        D.t64[u] = (double)y0;
+                        if (two) D.t64[u + 1] = (double)y1;
+                    } else {
+                        float *o = (float *)(out == 2 ? D.w : D.t);
+                        if (two) *reinterpret_cast<float2 *>(o + u) = make_float2(y0, y1);
+                        else o[u] = y0;
+                    }
+                }
+                continue;
+            }
+        }
         for (int u0 = k.n0; u0 < k.n1; u0 += UC) {
             const int u = u0 + warp * UW + lu;
             const bool on = lu < UW && u < k.n1;
@@ -199,23 +249,27 @@ k_rows_mv(const SysDev *__restrict__ sys, const NChunk *__restrict__ ch, const i
             if (on) {
                 id = B == 1 ? u : nd[(size_t)u * B + r];
                 const int s = u / kRowSlice;
-                const int e1 = D.rw_off[s + 1];
-                for (int e = D.rw_off[s] + u % kRowSlice; e < e1; e += U * kRowSlice) {
+                const int e0 = ru ? s * ru * kRowSlice : __ldg(D.rw_off + s), e1 = ru ? e0 + ru * kRowSlice : __ldg(D.rw_off + s + 1);
+                for (int e = e0 + u % kRowSlice; e < e1; e += U * kRowSlice) {
                     int m[U];
                     TA a[U][B], x[U][B];
+                    if (dc) {
 #pragma unroll
-                    for (int q = 0; q < U; ++q) {
-                        const bool in = e + q * kRowSlice < e1;
-                        m[q] = in ? __ldcs(col + e + q * kRowSlice) & ~kRowPad : u;
-                        if (in) row_vals<B, TA>(A + ((size_t)(e + q * kRowSlice) * B + r) * B, a[q]);
+                        for (int q = 0; q < U; ++q) m[q] = e + q * kRowSlice < e1 ? __ldcs(dc + e + q * kRowSlice) : 0;
+                    } else {
+#pragma unroll
+                        for (int q = 0; q < U; ++q) m[q] = e + q * kRowSlice < e1 ? (__ldcs(col + e + q * kRowSlice) & ~kRowPad) - u : 0;
+                    }
+#pragma unroll
+                    for (int q = 0; q < U; ++q)
+                        if (e + q * kRowSlice < e1) row_vals<B, TA>(A + ((size_t)(e + q * kRowSlice) * B + r) * B, a[q]);
                         else
 #pragma unroll
                             for (int w = 0; w < B; ++w) a[q][w] = (TA)0;
-                    }
 #pragma unroll
                     for (int q = 0; q < U; ++q) {
                         int d[B];
-                        unit_dofs<B>(nd, m[q], d);
+                        unit_dofs<B>(nd, u + m[q], d);
 #pragma unroll
                         for (int w = 0; w < B; ++w) x[q][w] = row_x<TA, TX>(X[d[w]], D);
                     }
@@ -265,7 +319,7 @@ static void rows_mv(int prec, dim3 g, const SysDev *sys, const NChunk *ch, const
 int launch_rows_mv(int B, int prec, const SysDev *sys, const NChunk *ch, const int *nch, int nchunks, int gate,
                    int in_sel, int out, int step, cudaStream_t st)
 {
-    const dim3 g((unsigned)std::max(1, std::min(nchunks, 8 * sm_count())));
+    const dim3 g((unsigned)std::max(1, std::min(nchunks, 16 * sm_count())));
     switch (B) {
     case 1: rows_mv<1>(prec, g, sys, ch, nch, gate, in_sel, out, step, st); break;
     case 2: rows_mv<2>(prec, g, sys, ch, nch, gate, in_sel, out, step, st); break;

@@ -59,7 +59,7 @@ struct fg_system {
     fg::DevMem lm16, pt_elem, pt_dof, pt_col, pdofs, pt_inc, incl;   // matvec patch layout
     // assembled operator of the Krylov engine (rows.cu): pattern, and values
     // made from the element blocks when a solve first needs them
-    fg::DevMem rw_off, rw_col, rw64, rw32;
+    fg::DevMem rw_off, rw_col, rw_dc, rw64, rw32;
     bool rw64_ok = false, rw32_ok = false;
     bool a32_ok = false;               // A32 holds the current blocks
     // preconditioners
@@ -192,6 +192,8 @@ inline void set_patch_fields(SysDev &D, const fg_system *s)
     D.rw_w = s->topo.rw_w;
     D.rw_off = s->rw_off.as<int>();
     D.rw_col = s->rw_col.as<int>();
+    D.rw_dc = s->topo.rw_dc.empty() ? nullptr : s->rw_dc.as<short>();
+    D.rw_u = s->topo.rw_u;
     D.rw64 = s->rw64.as<double>();
     D.rw32 = s->rw32.as<float>();
     D.maxdof = std::max(1, s->topo.maxdof);

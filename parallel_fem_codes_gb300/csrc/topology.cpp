@@ -224,6 +224,11 @@ static void build_rows(Topology &t, const std::vector<int> &IB, const std::vecto
         t.rw_off[s + 1] = t.rw_off[s] + w * kRowSlice;
         t.rw_w = std::max(t.rw_w, w);
     }
+    // one width for all where that pads little: the matvec then needs no offset
+    if (8LL * ((long long)ns * t.rw_w * kRowSlice - t.rw_off[ns]) <= t.rw_off[ns]) {
+        t.rw_u = t.rw_w;
+        for (int s = 0; s < ns; ++s) t.rw_off[s + 1] = (s + 1) * t.rw_w * kRowSlice;
+    }
     t.rw_col.resize(std::max(t.rw_off[ns], 1));
     for (int s = 0; s < ns; ++s) {
         const int w = (t.rw_off[s + 1] - t.rw_off[s]) / kRowSlice;
@@ -232,6 +237,12 @@ static void build_rows(Topology &t, const std::vector<int> &IB, const std::vecto
             for (int k = 0; k < w; ++k)
                 t.rw_col[t.rw_off[s] + k * kRowSlice + l] = k < m ? C[P[u] + k] : (std::min(u, std::max(nu - 1, 0)) | kRowPad);
         }
+    }
+    if (std::max(t.rw_lo, t.rw_hi) < 32768) {
+        t.rw_dc.assign(t.rw_col.size(), 0);
+        for (int s = 0; s < ns; ++s)
+            for (int e = t.rw_off[s]; e < t.rw_off[s + 1]; ++e)
+                if (t.rw_col[e] >= 0) t.rw_dc[e] = (short)(t.rw_col[e] - (s * kRowSlice + (e - t.rw_off[s]) % kRowSlice));
     }
 }
 

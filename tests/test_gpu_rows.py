@@ -88,3 +88,22 @@ def test_new_blocks_are_assembled_again(fg):
         # the element matvec in FP32 sees the new blocks too
         y = s.matvec(r.x, precision=32)
         assert np.linalg.norm(y[:-1] - F[:-1]) <= 1e-5 * np.linalg.norm(F)
+
+
+# Streaming sweeps (FP16 bases; a numbering too wide for the chip): rows in
+# pairs (slices of one width), single rows (a wheel's hub, 2 dofs per node),
+# columns within 2^15 units and beyond
+@pytest.mark.parametrize("kind,ndof", [((4, 6), 1), ((5, 5), 1), ((31, 1), 1), ((13, 17), 1), ((40, 37), 1), ("wheel", 1),
+                                       ((13, 17), 2), ("wheel", 2), ((32000, 1), 2), ((33000, 1), 2)])
+def test_streamed_solves(fg, kind, ndof):
+    m = _mesh(kind, ndof, 7)
+    A = G.random_blocks(m.nel, 3 * ndof, seed=2, dominance=6.0 * ndof)
+    F = np.append(np.random.Generator(np.random.PCG64(9)).uniform(-1.0, 1.0, m.neq), 0.0)
+    s = fg.System(m, reorder=False)
+    s.set_blocks(A)
+    B = s.precond_setup(fg.FG_PRECOND_DIAG, 0, F)
+    for prec in (fg.FG_PREC_MIXED16, fg.FG_PREC_MIXED, fg.FG_PREC_FP64):
+        r = s.solve(B, tol=1e-11, F_true=F, precision=prec)
+        assert r.stats["converged"] == 1, r.stats
+        res = np.linalg.norm((F - s.matvec(r.x))[:-1]) / np.linalg.norm(F[:-1])
+        assert res <= 1e-9, prec
