@@ -210,21 +210,23 @@ template <int B, typename T> __device__ __forceinline__ T row_add(T y, const T (
     return y + z;
 }
 
-// a row of the operator from global memory times the newest vector
+// A row of the operator from global memory times the newest vector: 16-bit
+// columns, no slice offset where slices have one width (263k equations FP32, a
+// fifth of the rows on chip: 26.2 -> 25.7 ms a solve; rows in pairs 26.3).
 template <int B, typename T>
-__device__ __forceinline__ T row_times_x(const int *__restrict__ off, const int *__restrict__ col,
+__device__ __forceinline__ T row_times_x(const int *__restrict__ off, const short *__restrict__ dc, int ru,
                                          const T *__restrict__ A, const Newest<T> &x, int u, int r)
 {
     constexpr int U = B == 1 ? 8 : 4;
-    const int s = u / kRowSlice, e1 = __ldg(off + s + 1);
+    const int s = u / kRowSlice, e0 = ru ? s * ru * kRowSlice : __ldg(off + s), e1 = ru ? e0 + ru * kRowSlice : __ldg(off + s + 1);
     T y = (T)0;
-    for (int e = __ldg(off + s) + u % kRowSlice; e < e1; e += U * kRowSlice) {
+    for (int e = e0 + u % kRowSlice; e < e1; e += U * kRowSlice) {
         int m[U];
         T a[U][B];
 #pragma unroll
         for (int q = 0; q < U; ++q) {
             const bool in = e + q * kRowSlice < e1;
-            m[q] = in ? __ldg(col + e + q * kRowSlice) & ~kRowPad : u;
+            m[q] = in ? u + __ldg(dc + e + q * kRowSlice) : u;
             if (in) load_vals<B, T>(A + ((size_t)(e + q * kRowSlice) * B + r) * B, a[q]);
             else
 #pragma unroll
@@ -309,7 +311,9 @@ k_cycle(const SysDev *__restrict__ sys, const CycItem *__restrict__ items, int s
         T *rv = halo + ((nh + N - 1) & ~(N - 1));
         const int nc = max(0, min(nrow, (int)((smem - (int)((unsigned char *)rv - cyc_smem)) / (max(W, 1) * (int)(B * sizeof(T) + 2))) & ~7));
         unsigned short *ri = reinterpret_cast<unsigned short *>(rv + (size_t)W * nc * B);
-        const int *off = D.rw_off, *col = D.rw_col, *nd = D.node_dof;
+        const int *off = D.rw_off, *nd = D.node_dof;
+        const short *dc = D.rw_dc;
+        const int ru = D.rw_u;
         const T *M = B > 1 && pre == FG_PRECOND_BLOCKDIAG ? (sizeof(T) == 8 ? (const T *)D.ibd64 : (const T *)D.ibd32)
                    : pre == FG_PRECOND_DIAG ? (sizeof(T) == 8 ? (const T *)D.invd64 : (const T *)D.invd32) : nullptr;
 
@@ -319,7 +323,7 @@ k_cycle(const SysDev *__restrict__ sys, const CycItem *__restrict__ items, int s
                 const int e0 = __ldg(off + s) + u % kRowSlice, e1 = __ldg(off + s + 1);
                 for (int w = 0; w < W; ++w) {
                     const int e = e0 + w * kRowSlice;
-                    const int m = e < e1 ? __ldg(col + e) & ~kRowPad : u;
+                    const int m = e < e1 ? u + __ldg(dc + e) : u;
                     T a[B];
                     if (e < e1) load_vals<B, T>(A + ((size_t)e * B + r) * B, a);
 #pragma unroll
@@ -421,7 +425,7 @@ k_cycle(const SysDev *__restrict__ sys, const CycItem *__restrict__ items, int s
                                 load_x<B, T>(X.template at<B>(ri[s * nc + q]), x);
                                 y = row_add<B, T>(y, a, x);
                             }
-                        } else y = row_times_x<B, T>(off, col, A, X, u, r);
+                        } else y = row_times_x<B, T>(off, dc, ru, A, X, u, r);
                         const int id = B == 1 ? u : __ldg(nd + (size_t)u * B + r);
                         if (id == n) y = (T)0;
                         else if (pre == FG_PRECOND_DIAG) y *= __ldg(M + id);
@@ -861,7 +865,7 @@ int gang_size(const fg_system *s, int kmax, bool f64, bool dense)
     const int ctas = dev.ctas;
     if (ctas == 0 || nu == 0) return 0;
     const size_t w = f64 ? 8 : 4, fixed = cycle_smem(kmax, 0, halo_units(s) * B, w);
-    if (fixed + (size_t)kmax * w * 64 > dev.smem) return 0;
+    if (fixed + (size_t)kmax * w * 64 > dev.smem || s->topo.rw_dc.empty()) return 0;   // (couplings that far fit no halo either)
     const int cap = (int)((dev.smem - fixed) / (kmax * w)) & ~3;
     const int cap_u = cap / B, want_u = dense ? cap_u : std::max(1, std::min(cap_u, gang_want(s, f64) / B));
     const int g = std::max((nu + cap_u - 1) / cap_u, std::min(ctas, (nu + want_u - 1) / want_u));
@@ -876,7 +880,7 @@ int gang_spill(const fg_system *s, int kmax, bool f64)
 {
     const int B = s->topo.ndof;
     const Residency dev = residency(B, f64, true);
-    if (dev.ctas == 0 || s->topo.nunits < dev.ctas) return 0;
+    if (dev.ctas == 0 || s->topo.nunits < dev.ctas || s->topo.rw_dc.empty()) return 0;
     const size_t w = f64 ? 8 : 4, fixed = cycle_smem(kmax, 0, halo_units(s) * B, w);
     if (fixed >= dev.smem) return 0;
     const int js = std::min(kmax - 2, (int)((dev.smem - fixed) / (w * gang_rows(s, dev.ctas))) - 2);

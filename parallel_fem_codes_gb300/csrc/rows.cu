@@ -16,9 +16,9 @@
 // The sums differ from the element order by rounding only; an FP32 entry is
 // the FP64 sum rounded once.
 // One matvec, by elements -> assembled (GB300, FP32 / FP64):
-//   48 transport systems, 5.6 M dofs   119 -> 74 us / 427 -> 109 us
-//   Euler 513 x 513 (4 dofs a node)    103 -> 47 us / 262 -> 95 us
-//   Navier-Stokes 513 x 513 (3 dofs)    72 -> 27 us / 162 -> 80 us
+//   48 transport systems, 5.6 M dofs   119 -> 46 us / 427 -> 95 us
+//   Euler 513 x 513 (4 dofs a node)    103 -> 43 us / 262 -> 82 us
+//   Navier-Stokes 513 x 513 (3 dofs)    72 -> 25 us / 162 -> 70 us
 // The values cost about one element matvec per solve.  A single matvec
 // (fg_matvec, fg_matvec_noalloc) stays with the element blocks.
 //
