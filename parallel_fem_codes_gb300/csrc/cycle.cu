@@ -4,7 +4,7 @@
 // Why.  As one kernel per pass an Arnoldi step of the systems served here (1k
 // to 260k equations) is launch and latency bound: 30 to 80 us for work that
 // the chip's shared memory does in 1 or 2.  The basis of a whole restart
-// cycle fits it: 152 SMs x 218 KB hold 30 vectors of 268k FP32 (134k FP64)
+// cycle fits it: 152 SMs x 227 KB hold 30 vectors of 276k FP32 (138k FP64)
 // entries.  So a gang of g CTAs (one per SM) owns a system for a cycle, CTA
 // `rank` the units [u0, u1) and their rows of every basis vector, and keeps
 // as many of their operator rows beside them as fit; the other rows are read

@@ -136,7 +136,8 @@ struct EuElem { double Mg1, Mg2, t4a, Kc01, Kc02, Kc12, tau, adt; };
 // The FP64 pipe bounds this kernel (two operations a cycle and SM), so what
 // does not depend on the row's node -- the products' row r and the Galerkin
 // row -- is formed once for the three, and terms with a structural zero or
-// one of Ax, Ay are not computed: 2.4k operations an element instead of 4.6k.
+// one of Ax, Ay are not computed: 131k elements 1043 -> 750 us, the pipe 80%
+// active, about 2.9k operations an element.
 template <int r>
 __device__ __forceinline__ void eu_rows(const EuElem &e, const double (&Ax)[4][4], const double (&Ay)[4][4], const double (&b)[3],
                                         const double (&c)[3], const double (&Ue)[12], const double (&dUe)[12], double *a,

@@ -151,9 +151,9 @@ constexpr int kElemChunk = 1024;   // elements per matvec work item
 constexpr int kMaxParts = 1024;    // dof parts (reduction partials) per system
 // Dofs per part of the Krylov dof kernels, chosen per batch (unless the
 // autotuner cached a choice): 2 sqrt(batch dofs) up to 64k dofs, 4 sqrt above,
-// rounded to the nearest power of two, within [kPartMin, kPartMax], so small
-// systems spread over many SMs and large batches keep the per-part overhead
-// low.
+// rounded to the nearest power of two, so small systems spread over many SMs;
+// large batches in whole rounds of resident CTAs (part_dofs_for); within
+// [kPartMin, kPartMax].
 constexpr int kPartMin = 256;
 constexpr int kPartMax = 16384;
 constexpr int kThreads = 256;

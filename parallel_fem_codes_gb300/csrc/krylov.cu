@@ -13,8 +13,7 @@
 //
 // Work decomposition.  A batch holds any number of systems.  The operator
 // is the assembled one (rows.cu), cut into unit chunks, dof work into parts
-// per system; every
-// kernel walks its chunk table with a grid-stride loop and skips systems
+// per system; every kernel walks its chunk table with a grid-stride loop and skips systems
 // that are not active.  A system's partial sums depend only on its own
 // parts, so a result is bit-identical whether the system is solved alone
 // or inside a batch.
@@ -139,7 +138,7 @@ template <typename TA, typename TX> __device__ __forceinline__ TA in_value(TX v,
 // the write-back none.
 // The patch sizes (patch_elems) and this kernel shape were chosen by a
 // measured sweep: an L2 prefetch of the next patch, one thread per block
-// row with small patches, and a two-stage bulk-copy pipeline through shared
+// row with small patches, and a two-stage copy pipeline through shared
 // memory were all slower.  The sink (index n) is never written.
 // in_sel: 0 = x (FP64), 1 = V[step] (T), 2 = aux (TX); out_sel: 0 = t64,
 // 1 = t, 2 = aux.
@@ -851,8 +850,8 @@ int parts_for(int n, int part_dofs = kPartMax)
 // Measured launch shapes of a batch, chosen by fg_autotune and cached per
 // (block size, precision, batch-size class = floor(log2(batch dofs))) for
 // the process: the dof-part size of the Krylov kernels and, for 3x3
-// blocks in FP32, the matvec kernel (bulk-copy pipeline or the register
-// kernel).  A batch with no cached choice uses the built-in rule.
+// blocks in FP32, the matvec's work items (four rows a thread or one).  A batch
+// with no cached choice uses the built-in rule.
 struct TuneKey {
     int S, mixed, vhalf, cls;
     bool operator<(const TuneKey &o) const
