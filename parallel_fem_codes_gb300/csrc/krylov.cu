@@ -1321,7 +1321,8 @@ size_t workspace_bytes(const fg_system *s, int kmax, int mixed)
     size_t np = (size_t)s->n_pad, ts = mixed ? 4 : 8;
     return ts * np * (kmax + 2) + 8 * np * 6 +
            8 * ((size_t)(kmax + 1) * kmax + 7 * (kmax + 1) + (size_t)kmax * kmax) +
-           8 * (size_t)kMaxParts * kPartStride + 256 + (mixed ? 4 : 8) * ((size_t)s->topo.nunits * s->topo.ndof + (size_t)4 * kmax * 304) ;
+           8 * (size_t)kMaxParts * kPartStride + 256 +
+           (mixed ? 8 : 16) * ((size_t)s->topo.nunits * s->topo.ndof + (size_t)4 * kmax * 152);   // (a gang's exchange words)
 }
 
 int autotune(std::vector<fg_system *> &sys, const SolveConfig &cfg0, bool remeasure, bool lookup_only,
@@ -1539,16 +1540,23 @@ static int choose_engine(const std::vector<BatchMember> &mem, const SolveConfig 
         }
         chip = chip && (int)left.size() <= kMaxBins;
     }
+    // no memory for the gangs: stream (a basis that streamed before has room for
+    // what a gang keeps outside)
+    for (int i = 0; i < n && chip; ++i) {
+        if (g[i] == 0) continue;
+        Workspace &w = mem[i].s->ws;
+        const size_t gb = gang_bytes(mem[i].s, cfg.kmax, g[i], !cfg.mixed);
+        const size_t sb = gang_spill_bytes(mem[i].s, cfg.kmax, g[i], js[i], !cfg.mixed);
+        chip = (w.gang.bytes >= gb || w.gang.alloc(gb) == FG_OK) &&
+               (std::max(w.V.bytes, w.spill.bytes) >= sb || w.spill.alloc(sb) == FG_OK);
+    }
+    if (!chip) cudaGetLastError();
     for (int i = 0; i < n; ++i) {
         int r;
         fg_system *s = mem[i].s;
         Workspace &w = s->ws;
+        if (!chip) w.spill.release();
         if (!chip && (r = ensure_basis(s))) return r;
-        if (chip && g[i] > 0) {
-            const size_t gb = gang_bytes(s, cfg.kmax, g[i], !cfg.mixed);
-            const size_t sb = gang_spill_bytes(s, cfg.kmax, g[i], js[i], !cfg.mixed);
-            if ((w.gang.bytes < gb && (r = w.gang.alloc(gb))) || (w.spill.bytes < sb && (r = w.spill.alloc(sb)))) return r;
-        }
         hs[i].V = w.V.p;
         hs[i].cy_bin = bin[i];
         set_gang_fields(hs[i], s, cfg.kmax, chip ? g[i] : 0, chip ? js[i] : 0, !cfg.mixed);

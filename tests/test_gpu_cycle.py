@@ -92,7 +92,7 @@ def test_a_system_beyond_shared_memory(fg, side, kmax, precision):
 
 
 # 376 x 376 equations fit 152 CTAs in FP64, 525 x 525 in FP32; up to four launches, then streaming
-@pytest.mark.parametrize("sides,precision", [((380, 40, 300, 35), 64), ((200, 290, 210, 300, 220), 64), ((340, 350, 360, 365, 370), 64),
+@pytest.mark.parametrize("sides,precision", [((380, 40, 300, 35), 64), ((200, 290, 210, 300, 220), 64), ((340, 350, 360, 365, 370), 64), ((378, 380, 382, 385, 387), 64),
                                              ((513, 37, 400), 32), ((530, 36), 32), ((500, 505, 510, 513, 37, 500), 32)])
 def test_a_batch_in_several_launches(fg, sides, precision):
     probs = [G.transport_problem(n, angle_deg=11.0 * n, k=10.0 ** -(2 + n % 3)) for n in sides]
@@ -105,3 +105,24 @@ def test_a_batch_in_several_launches(fg, sides, precision):
         x = s.solution()
         F = s.transport_assemble(p)
         assert np.linalg.norm((F - s.matvec(x))[:-1]) <= (1e-11 if precision == 32 else 1e-9) * np.linalg.norm(F[:-1])
+
+
+def test_streams_where_memory_for_the_gang_is_short(fg):
+    # five systems too large for the chip stream one cycle and so have a basis; then no more may be allocated
+    probs = [G.transport_problem(n, angle_deg=40.0, k=1e-2) for n in (380, 381, 382, 383, 384)]
+    systems = [fg.transport_system(p) for p in probs]
+    for s, p in zip(systems, probs):
+        s.transport_prepare(p)
+    fg.solve_resident(systems, tol=1e-11, lmax=1, precision=64)
+    used = fg.memory_in_use()
+    xs = []
+    for limit in (used + 4096, 0):
+        fg.set_memory_limit(limit)
+        try:
+            st = fg.solve_resident(systems[:1], tol=1e-11, lmax=3000, precision=64)[0]
+        finally:
+            fg.set_memory_limit(0)
+        assert st["converged"] == 1 and st["status"] == 0
+        assert (fg.memory_in_use() == used) == (limit > 0)
+        xs.append(systems[0].solution())
+    assert np.linalg.norm(xs[0] - xs[1]) <= 1e-8 * np.linalg.norm(xs[1])
