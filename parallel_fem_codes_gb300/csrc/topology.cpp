@@ -184,7 +184,7 @@ int matrix_bandwidth(int n, const int *IA, const int *JA)
 // units read consecutive entries.  A node couples to the nodes it shares an
 // element with, itself included, where both have a free dof.  Unused slots
 // hold the unit itself with kRowPad set.
-static void build_rows(Topology &t, const std::vector<int> &IB, const std::vector<int> &JB)
+static int build_rows(Topology &t, const std::vector<int> &IB, const std::vector<int> &JB)
 {
     const int nu = t.nunits = t.ndof == 1 ? t.n : t.nnodes;
     std::vector<int> ptr(1, 0), col;
@@ -218,14 +218,18 @@ static void build_rows(Topology &t, const std::vector<int> &IB, const std::vecto
         }
     const int ns = (nu + kRowSlice - 1) / kRowSlice;
     t.rw_off.assign(ns + 1, 0);
+    long long slots = 0;
     for (int s = 0; s < ns; ++s) {
         int w = 0;
         for (int u = s * kRowSlice; u < std::min(nu, (s + 1) * kRowSlice); ++u) w = std::max(w, P[u + 1] - P[u]);
-        t.rw_off[s + 1] = t.rw_off[s] + w * kRowSlice;
+        slots += (long long)w * kRowSlice;
+        if (slots > 0x7fffffffLL) { set_error("the operator's pattern has more entries than 32 bits count"); return FG_ERR_UNSUPPORTED; }
+        t.rw_off[s + 1] = (int)slots;
         t.rw_w = std::max(t.rw_w, w);
     }
     // one width for all where that pads little: the matvec then needs no offset
-    if (8LL * ((long long)ns * t.rw_w * kRowSlice - t.rw_off[ns]) <= t.rw_off[ns]) {
+    const long long wide = (long long)ns * t.rw_w * kRowSlice;
+    if (wide <= 0x7fffffffLL && 8 * (wide - slots) <= slots) {
         t.rw_u = t.rw_w;
         for (int s = 0; s < ns; ++s) t.rw_off[s + 1] = (s + 1) * t.rw_w * kRowSlice;
     }
@@ -244,6 +248,7 @@ static void build_rows(Topology &t, const std::vector<int> &IB, const std::vecto
             for (int e = t.rw_off[s]; e < t.rw_off[s + 1]; ++e)
                 if (t.rw_col[e] >= 0) t.rw_dc[e] = (short)(t.rw_col[e] - (s * kRowSlice + (e - t.rw_off[s]) % kRowSlice));
     }
+    return FG_OK;
 }
 
 // ---------------------------------------------------------------- topology
@@ -601,8 +606,7 @@ int build_topology(Topology &t, int nnodes, int nel, int ndof, const int *ien,
             }
         }
     }
-    build_rows(t, IB, JB);
-    return FG_OK;
+    return build_rows(t, IB, JB);
 }
 
 }  // namespace fg
