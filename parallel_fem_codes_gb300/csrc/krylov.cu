@@ -954,7 +954,7 @@ struct Plan {
 };
 
 static int choose_engine(const std::vector<BatchMember> &mem, const SolveConfig &cfg, std::vector<SysDev> &hs,
-                         const std::vector<int> &live, int B);
+                         const std::vector<int> &live, int B, cudaStream_t st);
 static size_t items_room(const std::vector<BatchMember> &mem, const SolveConfig &cfg, int B);
 
 // cycles: restart cycles will run (else only residuals)
@@ -972,7 +972,7 @@ static int build_plan(Plan &P, std::vector<BatchMember> &mem, const SolveConfig 
     const int pdofs = part_dofs_for(mem, cfg);
     const int uchunk = unit_chunk(mem, cfg);
     P.rprec = cfg.precond == FG_PRECOND_SGSE;
-    if (cycles && (r = choose_engine(mem, cfg, hs, {}, P.B))) return r;
+    if (cycles && (r = choose_engine(mem, cfg, hs, {}, P.B, st))) return r;
     for (int s = 0; s < P.nsys; ++s) {
         int n = mem[s].s->topo.n;
         hs[s].nparts = parts_for(n, pdofs);
@@ -1248,7 +1248,9 @@ static int ensure_basis(fg_system *s)
 {
     Workspace &w = s->ws;
     const size_t need = (w.mixed == 0 ? 8 : w.mixed == 2 ? 2 : 4) * (size_t)s->n_pad * w.kmax;
-    return w.V.bytes >= need ? FG_OK : w.V.alloc(need);
+    if (w.V.bytes >= need) return FG_OK;
+    w.v_lent = false;
+    return w.V.alloc(need);
 }
 
 static SysDev make_desc(fg_system *s, const SolveConfig &cfg, bool has_f)
@@ -1507,7 +1509,7 @@ int BatchRun::stage(const BatchMember &m)
 // 132 -> 126), in up to 4 74.9 (FP64 127), 16 119.5 -> 117.3, in up to 6 125.2.
 constexpr int kMaxBins = 3;
 static int choose_engine(const std::vector<BatchMember> &mem, const SolveConfig &cfg, std::vector<SysDev> &hs,
-                         const std::vector<int> &live, int B)
+                         const std::vector<int> &live, int B, cudaStream_t st)
 {
     const int room = gang_ctas(B, !cfg.mixed), n = (int)mem.size();
     std::vector<int> g(n, 0), js(n, 0), bin(n, 0);
@@ -1557,9 +1559,16 @@ static int choose_engine(const std::vector<BatchMember> &mem, const SolveConfig 
         Workspace &w = s->ws;
         if (!chip) w.spill.release();
         if (!chip && (r = ensure_basis(s))) return r;
+        // the streaming sweeps read packs across n and the sink at n: zeros, but
+        // not where a gang kept its vectors
+        if (!chip && w.v_lent) {
+            FG_CUDA(cudaMemsetAsync(w.V.p, 0, w.V.bytes, st));
+            w.v_lent = false;
+        }
         hs[i].V = w.V.p;
         hs[i].cy_bin = bin[i];
         set_gang_fields(hs[i], s, cfg.kmax, chip ? g[i] : 0, chip ? js[i] : 0, !cfg.mixed);
+        if (hs[i].cy_js > 0 && hs[i].cy_spill == w.V.p) w.v_lent = true;
     }
     return FG_OK;
 }
@@ -1674,7 +1683,7 @@ int BatchRun::reschedule(const std::vector<int> &live)
     }
     if (now == was || now == 0) return FG_OK;
     sched = live;
-    int r = choose_engine(mem, cfg, hs, live, P->B);
+    int r = choose_engine(mem, cfg, hs, live, P->B, st);
     if (r) return r;
     std::vector<CycItem> cyc;
     gang_items(hs, live, P->B, !cfg.mixed, cyc, P->bins);

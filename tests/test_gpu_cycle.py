@@ -126,3 +126,20 @@ def test_streams_where_memory_for_the_gang_is_short(fg):
         assert (fg.memory_in_use() == used) == (limit > 0)
         xs.append(systems[0].solution())
     assert np.linalg.norm(xs[0] - xs[1]) <= 1e-8 * np.linalg.norm(xs[1])
+
+
+@pytest.mark.parametrize("sides", [(381, 383, 385, 40, 120), (40, 381, 383, 385, 387, 120)])
+def test_streaming_again_after_a_basis_was_lent(fg, sides):
+    # odd counts of equations: the batch streams, then large members keep basis vectors where it streamed
+    probs = [G.transport_problem(n, angle_deg=11.0 * n, k=10.0 ** -(2 + n % 3)) for n in sides]
+    systems = [fg.transport_system(p) for p in probs]
+    first = None
+    for _ in range(3):
+        for s, p in zip(systems, probs):
+            s.transport_prepare(p)
+        st = fg.solve_resident(systems, tol=1e-11, lmax=3000, precision=64)
+        got = [(q["converged"], q["iterations"], s.solution()) for s, q in zip(systems, st)]
+        first = first or got
+        for a, b in zip(first, got):
+            assert a[:2] == b[:2] and a[0] == 1
+            assert np.array_equal(a[2], b[2]) and b[2][-1] == 0.0
