@@ -907,8 +907,7 @@ size_t gang_spill_bytes(const fg_system *s, int kmax, int g, int js, bool f64)
 void set_gang_fields(SysDev &D, const fg_system *s, int kmax, int g, int js, bool f64)
 {
     D.cy_js = js;
-    const size_t sb = gang_spill_bytes(s, kmax, g, js, f64);
-    D.cy_spill = js && s->ws.spill.bytes < sb ? s->ws.V.p : s->ws.spill.p;
+    D.cy_spill = s->ws.V.p;            // (free while the cycle is on chip)
     D.cy_g = g;
     if (!g) return;
     D.cy_rows = gang_rows(s, g);

@@ -1222,17 +1222,29 @@ static size_t items_room(const std::vector<BatchMember> &mem, const SolveConfig 
     return chip_config(cfg) ? std::max(room, sum) : 0;
 }
 
-// mode: 0 FP64, 1 FP32 basis, 2 FP16 basis (mixed precision in both)
+// The basis in global memory: kmax vectors, which the streaming kernels
+// use, or those that a gang of the whole chip keeps outside (more where
+// prescribed dofs count among the units).
+static size_t basis_bytes(const fg_system *s, int kmax, int mode)
+{
+    const size_t w = mode == 0 ? 8 : mode == 2 ? 2 : 4, all = w * (size_t)s->n_pad * kmax;
+    const int js = mode == 2 ? 0 : gang_spill(s, kmax, mode == 0);
+    return std::max(all, gang_spill_bytes(s, kmax, gang_ctas(s->topo.ndof, mode == 0, true), js, mode == 0));
+}
+
+// mode: 0 FP64, 1 FP32 basis, 2 FP16 basis (mixed precision in both).  All
+// that a cycle may need is allocated before the first one, wherever it runs,
+// but the exchange blocks of the gangs (choose_engine).
 static int ensure_workspace(fg_system *s, int kmax, int mode)
 {
     Workspace &w = s->ws;
     if (w.kmax >= kmax && w.mixed == mode) return FG_OK;
     w.kmax = 0;
     w.mixed = -1;
-    w.V.release();
+    w.v_lent = false;
     size_t np = (size_t)s->n_pad, ts = mode ? sizeof(float) : sizeof(double);
     int r;
-    if ((r = w.w.alloc(ts * np)) || (r = w.t.alloc(ts * np)) ||
+    if ((r = w.V.alloc(basis_bytes(s, kmax, mode))) || (r = w.w.alloc(ts * np)) || (r = w.t.alloc(ts * np)) ||
         (r = w.x.alloc(8 * np)) || (r = w.b.alloc(8 * np)) || (r = w.ftrue.alloc(8 * np)) ||
         (r = w.r64.alloc(8 * np)) || (r = w.t64.alloc(8 * np)) || (r = w.u64.alloc(8 * np)) ||
         (r = w.small.alloc(8 * ((size_t)(kmax + 1) * kmax + 7 * (kmax + 1) + (size_t)kmax * kmax))) ||
@@ -1243,16 +1255,6 @@ static int ensure_workspace(fg_system *s, int kmax, int mode)
     w.mixed = mode;
     return FG_OK;
 }
-// the basis in global memory, of a system whose cycles stream
-static int ensure_basis(fg_system *s)
-{
-    Workspace &w = s->ws;
-    const size_t need = (w.mixed == 0 ? 8 : w.mixed == 2 ? 2 : 4) * (size_t)s->n_pad * w.kmax;
-    if (w.V.bytes >= need) return FG_OK;
-    w.v_lent = false;
-    return w.V.alloc(need);
-}
-
 static SysDev make_desc(fg_system *s, const SolveConfig &cfg, bool has_f)
 {
     const Topology &t = s->topo;
@@ -1324,7 +1326,7 @@ size_t workspace_bytes(const fg_system *s, int kmax, int mixed)
     return ts * np * (kmax + 2) + 8 * np * 6 +
            8 * ((size_t)(kmax + 1) * kmax + 7 * (kmax + 1) + (size_t)kmax * kmax) +
            8 * (size_t)kMaxParts * kPartStride + 256 +
-           (mixed ? 8 : 16) * ((size_t)s->topo.nunits * s->topo.ndof + (size_t)4 * kmax * 152);   // (a gang's exchange words)
+           gang_bytes(s, kmax, gang_ctas(s->topo.ndof, !mixed), !mixed);
 }
 
 int autotune(std::vector<fg_system *> &sys, const SolveConfig &cfg0, bool remeasure, bool lookup_only,
@@ -1442,7 +1444,7 @@ size_t request_bytes(const fg_system *s, int kmax, int mixed, bool time_loop)
 {
     const Workspace &w = s->ws;
     const DevMem *held[] = {&w.V, &w.w, &w.t, &w.x, &w.b, &w.ftrue, &w.r64, &w.t64, &w.u64, &w.small, &w.part,
-                            &w.counter, &w.state, &w.gang, &w.spill};
+                            &w.counter, &w.state, &w.gang};
     size_t have = 0;
     for (auto *m : held) have += m->bytes;
     size_t b = s->bytes() - std::min(have, s->bytes()) + workspace_bytes(s, kmax, mixed) + rows_bytes(s, mixed != 0);
@@ -1508,6 +1510,10 @@ int BatchRun::stage(const BatchMember &m)
 // 33.7 ms (FP64 100 -> 74), 4 65.9 -> 41.7, 10 in up to 3 launches 74.8 -> 71.5 (FP64
 // 132 -> 126), in up to 4 74.9 (FP64 127), 16 119.5 -> 117.3, in up to 6 125.2.
 constexpr int kMaxBins = 3;
+// The choice for the live members (all: empty), written to hs where it
+// changes.  Members with live given are in mid-solve: those on chip stay there (a
+// gang's block has room for the largest gang that its system can get), those that
+// stream move on chip if they now fit and their gangs' blocks can be had.
 static int choose_engine(const std::vector<BatchMember> &mem, const SolveConfig &cfg, std::vector<SysDev> &hs,
                          const std::vector<int> &live, int B, cudaStream_t st)
 {
@@ -1542,23 +1548,22 @@ static int choose_engine(const std::vector<BatchMember> &mem, const SolveConfig 
         }
         chip = chip && (int)left.size() <= kMaxBins;
     }
-    // no memory for the gangs: stream (a basis that streamed before has room for
-    // what a gang keeps outside)
-    for (int i = 0; i < n && chip; ++i) {
-        if (g[i] == 0) continue;
+    // no memory for the gangs: stream
+    for (int i : todo) {
+        if (!chip) break;
         Workspace &w = mem[i].s->ws;
-        const size_t gb = gang_bytes(mem[i].s, cfg.kmax, g[i], !cfg.mixed);
-        const size_t sb = gang_spill_bytes(mem[i].s, cfg.kmax, g[i], js[i], !cfg.mixed);
+        const int most = std::max(g[i], member_gang(mem[i].s, cfg, false));
+        const size_t gb = gang_bytes(mem[i].s, cfg.kmax, most, !cfg.mixed);
         chip = (w.gang.bytes >= gb || w.gang.alloc(gb) == FG_OK) &&
-               (std::max(w.V.bytes, w.spill.bytes) >= sb || w.spill.alloc(sb) == FG_OK);
+               w.V.bytes >= gang_spill_bytes(mem[i].s, cfg.kmax, g[i], js[i], !cfg.mixed);
     }
-    if (!chip) cudaGetLastError();
+    if (!chip) {
+        cudaGetLastError();
+        if (!live.empty()) return FG_OK;              // as they are
+    }
     for (int i = 0; i < n; ++i) {
-        int r;
         fg_system *s = mem[i].s;
         Workspace &w = s->ws;
-        if (!chip) w.spill.release();
-        if (!chip && (r = ensure_basis(s))) return r;
         // the streaming sweeps read packs across n and the sink at n: zeros, but
         // not where a gang kept its vectors
         if (!chip && w.v_lent) {
@@ -1568,7 +1573,7 @@ static int choose_engine(const std::vector<BatchMember> &mem, const SolveConfig 
         hs[i].V = w.V.p;
         hs[i].cy_bin = bin[i];
         set_gang_fields(hs[i], s, cfg.kmax, chip ? g[i] : 0, chip ? js[i] : 0, !cfg.mixed);
-        if (hs[i].cy_js > 0 && hs[i].cy_spill == w.V.p) w.v_lent = true;
+        if (hs[i].cy_js > 0) w.v_lent = true;
     }
     return FG_OK;
 }
@@ -1687,7 +1692,7 @@ int BatchRun::reschedule(const std::vector<int> &live)
     if (r) return r;
     std::vector<CycItem> cyc;
     gang_items(hs, live, P->B, !cfg.mixed, cyc, P->bins);
-    if (P->bins.empty()) return FG_OK;               // still streaming
+    if (P->bins.empty()) return FG_OK;               // still streaming: nothing changed
     unsigned char *d = arena->dev.as<unsigned char>();
     auto put = [&](const Plan::Span &to, const void *from, size_t bytes) -> cudaError_t {
         unsigned char *h = arena->host + (to.as<unsigned char>() - d);
@@ -1874,7 +1879,7 @@ int bench_matvec(std::vector<fg_system *> &systems, int precision, int reps, dou
         if (!s->blocks_ok) { set_error("matvec before element blocks were set"); return FG_ERR_STATE; }
         int kk = std::max(2, s->ws.kmax);
         int r = ensure_workspace(s, kk, cfg.mixed);
-        if (r || (r = ensure_basis(s)) || (r = rows_refresh(s, cfg.mixed != 0, systems[0]->stream))) return r;
+        if (r || (r = rows_refresh(s, cfg.mixed != 0, systems[0]->stream))) return r;
         cfg.kmax = kk;
         mem.push_back({s, nullptr, nullptr, nullptr});
         hs.push_back(make_desc(s, cfg, false));

@@ -108,7 +108,7 @@ size_t fg_system::bytes() const
                            &sp_B, &sp_C, &sp_S, &sp_piv, &sp_g, &sp_h, &sp_x, &sp_tw, &sp_err, &sp_items, &sp_sysdev,
                            &diag, &invd64, &invd32, &bd, &ibd64, &ibd32, &gx, &gy, &gup, &gien, &gtype,
                            &ginvp, &Fe, &F64, &gf1, &gf2, &state_u, &state_a, &state_old, &state_u1, &state_u2, &shock_state, &bubble, &norm_part, &ws.V, &ws.w, &ws.t, &ws.x, &ws.b, &ws.ftrue, &ws.r64,
-                           &ws.t64, &ws.u64, &ws.small, &ws.part, &ws.counter, &ws.state, &ws.gang, &ws.spill, &ep_lmi, &ep_coef};
+                           &ws.t64, &ws.u64, &ws.small, &ws.part, &ws.counter, &ws.state, &ws.gang, &ep_lmi, &ep_coef};
     size_t b = 0;
     for (auto *m : all) b += m->bytes;
     return b;

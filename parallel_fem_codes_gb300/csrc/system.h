@@ -26,8 +26,8 @@ struct DevMem {
 struct Workspace {
     int kmax = 0, mixed = -1;
     DevMem V, w, t, x, b, ftrue, r64, t64, u64, small, part, counter, state;
-    DevMem gang, spill;                // exchange block of the on-chip cycle, basis vectors it has no room for
-    bool v_lent = false;               // a gang kept such vectors in V since it was last cleared
+    DevMem gang;                       // exchange block of the on-chip cycle
+    bool v_lent = false;               // a gang kept basis vectors in V since it was last cleared
 };
 
 // Tables of a batch run on the device with their pinned staging, and the

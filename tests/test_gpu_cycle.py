@@ -143,3 +143,36 @@ def test_streaming_again_after_a_basis_was_lent(fg, sides):
         for a, b in zip(first, got):
             assert a[:2] == b[:2] and a[0] == 1
             assert np.array_equal(a[2], b[2]) and b[2][-1] == 0.0
+
+
+@pytest.mark.parametrize("kmax,lmax", [(30, 2000), (2, 12)])
+def test_every_memory_limit_solves_or_refuses(fg, kmax, lmax):
+    # members stop at different cycles, so that the others' gangs grow; a limit in between must not strand a cycle
+    probs = [G.transport_problem(n, angle_deg=40.0, k=k) for n, k in ((150, 1e-1), (210, 1e-3), (200, 1e-2), (60, 1e-1))]
+
+    def solve(extra):
+        systems = [fg.transport_system(p) for p in probs]
+        for s, p in zip(systems, probs):
+            s.transport_prepare(p)
+        before = fg.memory_in_use()
+        fg.set_memory_limit(before + extra if extra else 0)
+        try:
+            st = fg.solve_resident(systems, kmax=kmax, tol=1e-10, lmax=lmax, precision=64)
+            return fg.memory_in_use() - before, [s.solution() for s in systems], st
+        except fg.FemGpuError as e:
+            assert extra and e.code == fg.FG_ERR_NOMEM
+            return None
+        finally:
+            fg.set_memory_limit(0)
+
+    need, ref, _ = solve(0)
+    outcomes = []
+    for short in (0, 1, 2, 3, 4, 6, 8, 12, 16, 32, 64, 256):
+        got = solve(need - short * need // 1024)
+        outcomes.append(got is not None)
+        if got is None:
+            continue
+        for x, y, q in zip(ref, got[1], got[2]):
+            assert q["status"] in (fg.FG_OK, fg.FG_ERR_NOTCONV)
+            assert np.linalg.norm(x - y) <= 1e-7 * np.linalg.norm(x)
+    assert outcomes[0] and not outcomes[-1]
