@@ -1066,7 +1066,9 @@ static int build_plan(Plan &P, std::vector<BatchMember> &mem, const SolveConfig 
 }
 
 // Room for `bytes` of tables and the flags and states of n members.  The
-// staging is rewritten only between runs of the batch, with nothing in flight.
+// staging is rewritten only between cycles: a copy of it that may still be in
+// flight then (tables of a batch that changed twice) is followed by one of the
+// new tables before any kernel reads them.
 int PlanArena::ensure(size_t bytes, int n)
 {
     int r;
@@ -1076,6 +1078,8 @@ int PlanArena::ensure(size_t bytes, int n)
         if ((r = dev.alloc(bytes))) return r;
         if (host) cudaFreeHost(host);
         host = nullptr;
+        host_bytes = 0;                    // (should the next line fail, the next run asks again)
+        members = 0;
         const size_t tail = 2 * sizeof(int) * (size_t)n + sizeof(SysState) * (size_t)n + 64;
         FG_CUDA(cudaMallocHost(&host, bytes + tail));
         host_bytes = bytes;
