@@ -186,9 +186,12 @@ int fg_set_ilu_fill(fg_system *s, int p);
  * substitutions' dependency depth drops about blocks-fold.  1 (the
  * default) is the global ILU(p). */
 int fg_set_ilu_blocks(fg_system *s, int blocks);
-/* Polls (>= 1) a device-side dependency wait of the ILU kernels makes
- * before it gives up and the call returns FG_ERR_TIMEOUT (default 2^24,
- * about half a second); applies to the current device. */
+/* Polls (>= 1) a device-side wait makes before it gives up: the dependency
+ * waits of the ILU kernels, whose call then returns FG_ERR_TIMEOUT, and the
+ * exchanges between the CTAs of an on-chip restart cycle, whose solve then
+ * reports FG_ERR_TIMEOUT as its status.  Default 2^24 (about half a second in
+ * the ILU kernels; an exchange also gives up after about two seconds);
+ * applies to the current device. */
 int fg_set_wait_limit(long long polls);
 /* Cap (bytes) on the device memory the library allocates in this process;
  * an allocation that would pass it fails with FG_ERR_NOMEM and the call

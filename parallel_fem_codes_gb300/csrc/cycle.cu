@@ -47,8 +47,9 @@
 // pairs.
 //
 // The launch is cooperative, so all CTAs are resident; a CTA is one rank of
-// one system's gang.  Polls are bounded (~2 s): a CTA that gives up marks the
-// system FG_ERR_TIMEOUT and leaves.
+// one system's gang.  Polls are bounded (~2 s, or the number fg_set_wait_limit
+// gives): a CTA that gives up marks the system FG_ERR_TIMEOUT and leaves at the
+// step's next barrier, all its threads together.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -73,6 +74,7 @@ constexpr int kMaxSlices = 8;
 // slices of the CTA's rows in the dots: while every lane keeps 8 packs
 __device__ __forceinline__ int dot_slices(int np, int nv) { return max(1, min(min(kMaxSlices, np / 64), kGroups / nv)); }
 constexpr long long kPollCycles = 4000000000LL;   // ~2 s
+__device__ int g_gang_polls = 1 << 24;            // fg_set_wait_limit
 // gangs up to this size sum all partials in every CTA
 // (129 x 129 FP32, 32 CTAs: 5.3 ms a solve in two trips, 6.4 ms in one)
 constexpr int kDirect32 = 8, kDirect64 = 8;
@@ -103,11 +105,16 @@ __device__ __forceinline__ u64 peek(const u64 *p)
     return w;
 }
 // The values of NW words p[k * stride], k < cnt, once each carries the tag.
-// All loads of a round are in flight together.  Gives up after ~2 s, or when
-// the CTA already did (values are then garbage).
+// All loads of a round are in flight together.  Gives up after ~2 s or `polls`
+// rounds, looked at every 32 (limits below that: every) rounds, or when the CTA
+// already did (values are then garbage).
+struct Bound {
+    volatile int *gave_up;
+    int mask;
+};
 template <int NW>
 __device__ __forceinline__ void poll(const u64 *p, size_t stride, int cnt, unsigned tag, unsigned (&v)[NW],
-                                     volatile int *gave_up)
+                                     const Bound &bound)
 {
     u64 w[NW];
     const long long t0 = clock64();
@@ -118,7 +125,10 @@ __device__ __forceinline__ void poll(const u64 *p, size_t stride, int cnt, unsig
 #pragma unroll
         for (int k = 0; k < NW; ++k) ok = ok && (unsigned)(w[k] >> 32) == tag;
         if (ok) break;
-        if ((it & 31) == 31 && (*gave_up || clock64() - t0 > kPollCycles)) { *gave_up = 1; break; }
+        if ((it & bound.mask) == bound.mask && (*bound.gave_up || it + 1 >= g_gang_polls || clock64() - t0 > kPollCycles)) {
+            *bound.gave_up = 1;
+            break;
+        }
     }
 #pragma unroll
     for (int k = 0; k < NW; ++k) v[k] = (unsigned)w[k];
@@ -272,7 +282,7 @@ k_cycle(const SysDev *__restrict__ sys, const CycItem *__restrict__ items, int s
     __shared__ T s_n2h[kWorkers / 32], s_n2l[kWorkers / 32];
     __shared__ T s_sc, s_dg;                      // 1 / norm of the newest vector, its Gram diagonal less 1
     __shared__ int s_stop, s_gave_up, s_m;
-    volatile int *gave_up = &s_gave_up;
+    const Bound bound{&s_gave_up, g_gang_polls < 32 ? 0 : 31};
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, l8 = tid & 7, gid = tid >> 3;
     const bool worker = tid < kWorkers;
     if (tid == 0) s_gave_up = 0;
@@ -396,12 +406,12 @@ k_cycle(const SysDev *__restrict__ sys, const CycItem *__restrict__ items, int s
                         const int q2 = q + kWorkers, p = q < nhl ? q : q + nrow, p2 = q2 < nhl ? q2 : q2 + nrow;
                         const u64 *src = vb + (size_t)lo * B * WP;
                         unsigned v[2 * WP];
-                        if constexpr (WP == 1) poll<2>(src + p, p2 - p, q2 < nh ? 2 : 1, tag - 1u, v, gave_up);
+                        if constexpr (WP == 1) poll<2>(src + p, p2 - p, q2 < nh ? 2 : 1, tag - 1u, v, bound);
                         else {
                             unsigned a[2], b[2];
                             const int cnt = q2 < nh ? 2 : 1;
-                            poll<2>(src + 2 * (size_t)p, 2 * (size_t)(p2 - p), cnt, tag - 1u, a, gave_up);
-                            poll<2>(src + 2 * (size_t)p + 1, 2 * (size_t)(p2 - p), cnt, tag - 1u, b, gave_up);
+                            poll<2>(src + 2 * (size_t)p, 2 * (size_t)(p2 - p), cnt, tag - 1u, a, bound);
+                            poll<2>(src + 2 * (size_t)p + 1, 2 * (size_t)(p2 - p), cnt, tag - 1u, b, bound);
                             v[0] = a[0];
                             v[1] = b[0];
                             v[2] = a[1];
@@ -489,13 +499,13 @@ k_cycle(const SysDev *__restrict__ sys, const CycItem *__restrict__ items, int s
                             if constexpr (WP == 1) {
                                 unsigned v[kDirect32 / 8];
                                 const int cnt = (g - l8 + 7) / 8;
-                                poll<kDirect32 / 8>(p + l8, 8, cnt, tag, v, gave_up);
+                                poll<kDirect32 / 8>(p + l8, 8, cnt, tag, v, bound);
 #pragma unroll
                                 for (int q = 0; q < kDirect32 / 8; ++q) t.add(__uint_as_float(v[q]));
                             } else {
                                 for (int q = l8; q < g; q += 8) {
                                     unsigned v[2];
-                                    poll<2>(p + 2 * q, 1, 2, tag, v, gave_up);
+                                    poll<2>(p + 2 * q, 1, 2, tag, v, bound);
                                     t.add(from_words<T>(v));
                                 }
                             }
@@ -514,13 +524,13 @@ k_cycle(const SysDev *__restrict__ sys, const CycItem *__restrict__ items, int s
                         for (int q0 = lane; q0 < g; q0 += 32 * K) {
                             if constexpr (WP == 1) {
                                 unsigned v[K];
-                                poll<K>(p + q0, 32, (g - q0 + 31) / 32, tag, v, gave_up);
+                                poll<K>(p + q0, 32, (g - q0 + 31) / 32, tag, v, bound);
 #pragma unroll
                                 for (int q = 0; q < K; ++q) t.add(__uint_as_float(v[q]));
                             } else {
                                 unsigned lo[K], hi[K];
-                                poll<K>(p + 2 * q0, 64, (g - q0 + 31) / 32, tag, lo, gave_up);
-                                poll<K>(p + 2 * q0 + 1, 64, (g - q0 + 31) / 32, tag, hi, gave_up);
+                                poll<K>(p + 2 * q0, 64, (g - q0 + 31) / 32, tag, lo, bound);
+                                poll<K>(p + 2 * q0 + 1, 64, (g - q0 + 31) / 32, tag, hi, bound);
 #pragma unroll
                                 for (int q = 0; q < K; ++q) {
                                     const unsigned v[2] = {lo[q], hi[q]};
@@ -534,7 +544,7 @@ k_cycle(const SysDev *__restrict__ sys, const CycItem *__restrict__ items, int s
                     }
                     if (tid < 2 * nv) {
                         unsigned v[WP];
-                        poll<WP>(total + tid * WP, 1, WP, tag, v, gave_up);
+                        poll<WP>(total + tid * WP, 1, WP, tag, v, bound);
                         s_tot[tid] = from_words<T>(v);
                     }
                 }
@@ -546,8 +556,8 @@ k_cycle(const SysDev *__restrict__ sys, const CycItem *__restrict__ items, int s
                         constexpr int K = 5;
                         for (int q0 = lane; q0 < g; q0 += 32 * K) {
                             unsigned lw[K], hw[K];
-                            poll<K>(norm + 2 * q0, 64, (g - q0 + 31) / 32, tag, lw, gave_up);
-                            poll<K>(norm + 2 * q0 + 1, 64, (g - q0 + 31) / 32, tag, hw, gave_up);
+                            poll<K>(norm + 2 * q0, 64, (g - q0 + 31) / 32, tag, lw, bound);
+                            poll<K>(norm + 2 * q0 + 1, 64, (g - q0 + 31) / 32, tag, hw, bound);
 #pragma unroll
                             for (int q = 0; q < K; ++q) {
                                 const unsigned v[2] = {lw[q], hw[q]};
@@ -559,7 +569,7 @@ k_cycle(const SysDev *__restrict__ sys, const CycItem *__restrict__ items, int s
                         if (!direct && lane == 0) put_pair(total + (size_t)2 * km * WP, t, tag);
                     } else {
                         unsigned v[2];
-                        poll<2>(total + (size_t)2 * km * WP, 1, 2, tag, v, gave_up);
+                        poll<2>(total + (size_t)2 * km * WP, 1, 2, tag, v, bound);
                         add_pair(t, v);
                     }
                     n2 = t;
@@ -571,11 +581,10 @@ k_cycle(const SysDev *__restrict__ sys, const CycItem *__restrict__ items, int s
                 }
             } else if (g > 1 && tid == kWorkers - 1 && rank != 0) {
                 unsigned v[1];
-                poll<1>(note + (i & 1), 0, 1, tag, v, gave_up);
+                poll<1>(note + (i & 1), 0, 1, tag, v, bound);
                 s_stop = (int)v[0];
             }
-            __syncthreads();
-            if (s_stop || s_gave_up) break;
+            if (__syncthreads_or(s_stop | s_gave_up)) break;   // (the flags may still change: one answer for all)
             const T sc = s_sc;
             T *c = s_c[i & 1];
             if (worker) {
@@ -711,7 +720,7 @@ k_cycle(const SysDev *__restrict__ sys, const CycItem *__restrict__ items, int s
                     for (int q = lane; q < g; q += 32) {
                         if (q == 0) continue;
                         unsigned v[2];
-                        poll<2>(norm2 + (i & 1) * (2 * (size_t)g) + 2 * q, 1, 2, ntag, v, gave_up);
+                        poll<2>(norm2 + (i & 1) * (2 * (size_t)g) + 2 * q, 1, 2, ntag, v, bound);
                         add_pair(u, v);
                     }
 #pragma unroll
@@ -732,10 +741,10 @@ k_cycle(const SysDev *__restrict__ sys, const CycItem *__restrict__ items, int s
                 }
             } else {
                 unsigned v[1];
-                poll<1>(note + 2, 0, 1, ytag, v, gave_up);
+                poll<1>(note + 2, 0, 1, ytag, v, bound);
                 for (int j = lane; j < (int)v[0] && j < km; j += 32) {
                     unsigned w2[2];
-                    poll<2>(note + 3 + 2 * j, 1, 2, ytag, w2, gave_up);
+                    poll<2>(note + 3 + 2 * j, 1, 2, ytag, w2, bound);
                     y[j] = from_words<double>(w2);
                 }
                 if (lane == 0) s_m = min((int)v[0], km);
@@ -749,10 +758,9 @@ k_cycle(const SysDev *__restrict__ sys, const CycItem *__restrict__ items, int s
                     s_tot[2 * j + 1] = (float)(y[j] - (double)yh);
                 }
         }
-        __syncthreads();
-        if (s_gave_up) {
+        if (__syncthreads_or(s_gave_up)) {
             if (tid == 0) {
-                D.st->status = FG_ERR_TIMEOUT;
+                atomicExch(&D.st->status, FG_ERR_TIMEOUT);
                 D.st->live = D.st->in_cycle = 0;
             }
             return;
@@ -780,7 +788,7 @@ k_cycle(const SysDev *__restrict__ sys, const CycItem *__restrict__ items, int s
             if (R.breakdown) { st->status = FG_ERR_BREAKDOWN; st->live = 0; }
             else if (!D.mixed) {
                 if (!(st->rho > st->eps)) { st->converged = 1; st->live = 0; }
-                else if (st->cycles >= D.lmax) { st->status = FG_ERR_NOTCONV; st->live = 0; }
+                else if (st->cycles >= D.lmax) { atomicCAS(&st->status, FG_OK, FG_ERR_NOTCONV); st->live = 0; }
             }
             *D.cy_epoch = base + (unsigned)km + 4u;
         }
@@ -870,6 +878,12 @@ int gang_size(const fg_system *s, int kmax, bool f64, bool dense)
     const int cap_u = cap / B, want_u = dense ? cap_u : std::max(1, std::min(cap_u, gang_want(s, f64) / B));
     const int g = std::max((nu + cap_u - 1) / cap_u, std::min(ctas, (nu + want_u - 1) / want_u));
     return g <= ctas ? g : 0;
+}
+int set_gang_polls(long long polls)
+{
+    const int n = (int)std::min(polls, 0x7fffffffLL);
+    FG_CUDA(cudaMemcpyToSymbol(g_gang_polls, &n, sizeof(n)));
+    return FG_OK;
 }
 int gang_ctas(int B, bool f64, bool spill) { return residency(B, f64, spill).ctas; }
 // Basis vectors that stay in shared memory when a system that does not fit

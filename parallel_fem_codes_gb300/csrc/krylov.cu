@@ -1754,7 +1754,7 @@ void fill_stats(const SysState &s, double secs, fg_solve_stats &o)
 {
     o.iterations = s.iterations;
     o.cycles = s.cycles;
-    o.converged = s.converged;
+    o.converged = s.status == FG_ERR_TIMEOUT ? 0 : s.converged;   // (another CTA of its gang may have set it)
     o.status = s.status;
     o.rho = s.rho;
     o.eps = s.eps;

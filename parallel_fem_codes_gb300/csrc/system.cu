@@ -591,7 +591,8 @@ size_t fg_memory_in_use(void) { return g_dev_bytes.load(); }
 int fg_set_wait_limit(long long polls)
 {
     if (polls < 1) { set_error("wait limit must be >= 1 poll"); return FG_ERR_ARG; }
-    return set_wait_limit(polls);
+    const int r = set_wait_limit(polls);
+    return r ? r : set_gang_polls(polls);
 }
 
 int fg_get_csr(const fg_system *s, int *nnz, int *IA, int *JA, double *AA)

@@ -345,6 +345,7 @@ size_t gang_bytes(const fg_system *s, int kmax, int g, bool f64);
 void set_gang_fields(SysDev &D, const fg_system *s, int kmax, int g, int js, bool f64);
 void gang_items(const std::vector<SysDev> &hs, const std::vector<int> &live, int B, bool f64,
                 std::vector<CycItem> &items, std::vector<CycBin> &bins);
+int set_gang_polls(long long polls);   // bounded waits of a gang's exchanges
 int launch_cycle(int B, bool f64, bool spill, const SysDev *sys, const CycItem *items, int ctas, size_t smem,
                  cudaStream_t st);
 

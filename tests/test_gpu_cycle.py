@@ -176,3 +176,22 @@ def test_every_memory_limit_solves_or_refuses(fg, kmax, lmax):
             assert q["status"] in (fg.FG_OK, fg.FG_ERR_NOTCONV)
             assert np.linalg.norm(x - y) <= 1e-7 * np.linalg.norm(x)
     assert outcomes[0] and not outcomes[-1]
+
+
+@pytest.mark.parametrize("precision", [64, 32])
+def test_wait_limit_times_out_and_recovers(fg, precision):
+    # one poll an exchange: some CTA looks before its neighbour has published
+    p = G.transport_problem(129, angle_deg=40.0, k=1e-3)
+    s = fg.transport_system(p)
+    s.transport_prepare(p)
+    good = fg.solve_resident([s], tol=1e-10, precision=precision)[0]
+    x = s.solution()
+    try:
+        fg.set_wait_limit(1)
+        st = fg.solve_resident([s], tol=1e-10, precision=precision)[0]
+    finally:
+        fg.set_wait_limit()
+    assert good["converged"] == 1 and st["converged"] == 0 and st["status"] == fg.FG_ERR_TIMEOUT
+    again = fg.solve_resident([s], tol=1e-10, precision=precision)[0]
+    assert again["converged"] == 1 and again["iterations"] == good["iterations"]
+    assert np.array_equal(s.solution(), x)
