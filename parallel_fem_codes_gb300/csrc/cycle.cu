@@ -53,7 +53,9 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <map>
 #include <mutex>
+#include <tuple>
 #include <type_traits>
 
 #include "sums.cuh"
@@ -815,37 +817,36 @@ const void *cycle_kernel(int B, bool f64, bool spill)
                : (spill ? cycle_kernel<float, true>(B) : cycle_kernel<float, false>(B));
 }
 
-// What k_cycle<T, B> has on this device: the dynamic shared memory with which
-// one CTA fills an SM, and the CTAs that are then resident together (0:
-// none).  Looked up once per kernel; raises its shared-memory limit.
+// What k_cycle<T, B> has on the current device: the dynamic shared memory with
+// which one CTA fills an SM, and the CTAs that are then resident together (0:
+// none).  Looked up once per device and kernel; raises the kernel's
+// shared-memory limit there.
 struct Residency { int ctas; size_t smem; };
 Residency residency(int B, bool f64, bool spill = false)
 {
     static std::mutex mu;
-    static bool known[4][5];
-    static Residency found[4][5];
+    static std::map<std::tuple<int, int, bool, bool>, Residency> found;
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) { cudaGetLastError(); return {0, 0}; }
     std::lock_guard<std::mutex> l(mu);
-    const int w = (f64 ? 1 : 0) + (spill ? 2 : 0);
-    Residency &v = found[w][B];
-    if (!known[w][B]) {
-        known[w][B] = true;
-        const void *k = cycle_kernel(B, f64, spill);
-        int dev = 0, coop = 0, occ = 0, sm = 0, own = 0;
-        cudaFuncAttributes fa{};
-        v = {0, 0};
-        if (cudaGetDevice(&dev) == cudaSuccess &&
-            cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) == cudaSuccess && coop &&
-            cudaDeviceGetAttribute(&sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev) == cudaSuccess &&
-            cudaDeviceGetAttribute(&own, cudaDevAttrReservedSharedMemoryPerBlock, dev) == cudaSuccess &&
-            cudaFuncGetAttributes(&fa, k) == cudaSuccess && (size_t)sm > own + fa.sharedSizeBytes + 4096) {
-            const size_t cap = ((size_t)sm - own - fa.sharedSizeBytes) & ~(size_t)127;
-            if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cap) == cudaSuccess &&
-                cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, kCycThreads, cap) == cudaSuccess && occ > 0)
-                v = {sm_count(), cap};
-        }
-        cudaGetLastError();
+    const auto key = std::make_tuple(dev, B, f64, spill);
+    const auto it = found.find(key);
+    if (it != found.end()) return it->second;
+    Residency v{0, 0};
+    const void *k = cycle_kernel(B, f64, spill);
+    int coop = 0, occ = 0, sm = 0, own = 0;
+    cudaFuncAttributes fa{};
+    if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) == cudaSuccess && coop &&
+        cudaDeviceGetAttribute(&sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev) == cudaSuccess &&
+        cudaDeviceGetAttribute(&own, cudaDevAttrReservedSharedMemoryPerBlock, dev) == cudaSuccess &&
+        cudaFuncGetAttributes(&fa, k) == cudaSuccess && (size_t)sm > own + fa.sharedSizeBytes + 4096) {
+        const size_t cap = ((size_t)sm - own - fa.sharedSizeBytes) & ~(size_t)127;
+        if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cap) == cudaSuccess &&
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, kCycThreads, cap) == cudaSuccess && occ > 0)
+            v = {sm_count(), cap};
     }
-    return v;
+    cudaGetLastError();
+    return found[key] = v;
 }
 
 }  // namespace

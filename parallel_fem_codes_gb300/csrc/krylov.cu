@@ -749,13 +749,14 @@ __global__ void k_states(const SysDev *__restrict__ sys, int nsys, SysState *out
 // ---------------------------------------------------------------- host side
 int sm_count()
 {
-    static int n = 0;
-    if (!n) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-        if (n <= 0) n = 1;
-    }
+    constexpr int kKnown = 64;
+    static std::atomic<int> known[kKnown];
+    int dev = 0, n = 0;
+    cudaGetDevice(&dev);
+    if (dev >= 0 && dev < kKnown && (n = known[dev].load(std::memory_order_relaxed)) > 0) return n;
+    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+    if (n <= 0) return 1;
+    if (dev >= 0 && dev < kKnown) known[dev].store(n, std::memory_order_relaxed);
     return n;
 }
 
