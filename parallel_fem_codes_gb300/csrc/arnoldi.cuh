@@ -5,7 +5,8 @@
 // The basis is kept unscaled: V[j] is the vector as the step left it and
 // vscale[j] the reciprocal of its norm, known when the step's last part sums
 // it, so that no pass is spent on scaling (an FP16 basis is scaled when it is
-// stored, vscale[j] = 1 / sigma).  Both passes walk parts of kPartMin..kPartMax
+// stored, vscale[j] = 1 / sigma).  A step leaves its vector times vscale[kmax], a
+// power of two that the cycle's first step finds (unit_scale).  Both passes walk parts of kPartMin..kPartMax
 // dofs (the size is chosen per batch from its total dofs), a 16-byte pack of
 // every vector per thread and several basis vectors in flight.  A part is one
 // CTA's, or, where a batch has few parts, gridDim.y CTAs': pass 1 splits the
@@ -169,14 +170,15 @@ __device__ __forceinline__ void part_dots(const SysDev &D, const DChunk &k, int 
 // v_i from the matvec) and the new column g = V^T v_i of the basis' Gram
 // matrix G in one sweep.  The last part forms c = s + (s - G s): the
 // coefficients of the two classical passes of CGS2 (h1 = s, h2 = V^T (w - V s) =
-// s - G s) with the second one taken from G instead of a second sweep; c becomes
-// column i of H and, unscaled, the update that k_orth applies.
+// s - G s, but for rounding) with the second one taken from G instead of a second sweep; c becomes
+// column i of H and, unscaled, the update that k_orth applies, the scale of w behind it.
 template <typename T, typename TV>
 __global__ void __launch_bounds__(kThreads, 3)
 k_dots(const SysDev *__restrict__ sys, const DChunk *__restrict__ ch, const int *__restrict__ nch, int i)
 {
-    __shared__ T sw[kThreads / 32][2 * kMaxRestart];
+    __shared__ T sw[kThreads / 32][2 * kMaxRestart], mx[kThreads / 32];
     __shared__ double tot[2 * kMaxRestart];
+    constexpr bool kUnscaled = std::is_same<T, TV>::value;
     const int total = *nch;
     for (int c = blockIdx.x; c < total; c += gridDim.x) {
         const DChunk k = ch[c];
@@ -184,11 +186,30 @@ k_dots(const SysDev *__restrict__ sys, const DChunk *__restrict__ ch, const int 
         if (!D.st->in_cycle) continue;
         __syncthreads();
         part_dots<T, TV>(D, k, i, (const T *)D.w, sw, D.part + k.part * kPartStride);
+        if (kUnscaled && i == 0) {               // the part's largest |w| (one CTA a part here)
+            constexpr int G = VPk<TV>::G;
+            T m = (T)0;
+            for (int q = k.d0 + threadIdx.x * G; q < k.d1; q += kThreads * G) {
+                T v[G];
+                ld_g<T, G>((const T *)D.w + q, v);
+#pragma unroll
+                for (int e = 0; e < G; ++e) m = max(m, abs(v[e]));
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+            if ((threadIdx.x & 31) == 0) mx[threadIdx.x >> 5] = m;
+            __syncthreads();
+            if (threadIdx.x == 0) {
+                for (int q = 1; q < kThreads / 32; ++q) m = max(m, mx[q]);
+                D.part[k.part * kPartStride + 2] = (double)m;
+            }
+        }
         if (last_part(D, 1, gridDim.y)) {
-            reduce_parts(D, 2 * (i + 1), tot);
+            reduce_parts(D, 2 * (i + 1) + (kUnscaled && i == 0), tot);
             const int km = D.kmax;
             const double *vs = D.vscale;
-            const double ws = std::is_same<T, TV>::value ? vs[i] : 1.0;   // the scale of w as stored
+            const double ws = kUnscaled ? vs[i] : 1.0;   // the scale of w as stored
+            if (i == 0 && threadIdx.x == 0) D.vscale[km] = kUnscaled ? (double)unit_scale((T)tot[2]) : 1.0;
             for (int j = threadIdx.x; j <= i; j += kThreads) {
                 const double g = tot[i + 1 + j] * vs[j] * vs[i];
                 D.G[j * km + i] = g;
@@ -196,12 +217,13 @@ k_dots(const SysDev *__restrict__ sys, const DChunk *__restrict__ ch, const int 
                 tot[j] *= vs[j] * ws;
             }
             __syncthreads();
+            if (threadIdx.x == 0) D.hbuf[i + 1] = ws * vs[km];
             for (int j = threadIdx.x; j <= i; j += kThreads) {
                 double gs = 0.0;
                 for (int l = 0; l <= i; ++l) gs += D.G[l * km + j] * tot[l];
                 const double cj = tot[j] + (tot[j] - gs);
                 D.hcol[j] = cj;
-                D.hbuf[j] = cj * vs[j];
+                D.hbuf[j] = cj * vs[j] * vs[km];
             }
         }
     }
@@ -224,13 +246,13 @@ k_orth(const SysDev *__restrict__ sys, const DChunk *__restrict__ ch, const int 
         const SysDev &D = sys[k.sys];
         if (!D.st->in_cycle) continue;
         __syncthreads();
-        for (int j = threadIdx.x; j <= i; j += kThreads) hs[j] = (T)D.hbuf[j];
+        for (int j = threadIdx.x; j <= i + 1; j += kThreads) hs[j] = (T)D.hbuf[j];
         __syncthreads();
         const TV *V = (const TV *)D.V;
         const size_t ld = (size_t)D.n_pad;
         const T *w = (const T *)D.w;
         T *out = std::is_same<T, TV>::value ? (T *)D.V + (size_t)(i + 1) * ld : (T *)D.w;
-        const T ws = std::is_same<T, TV>::value ? (T)D.vscale[i] : (T)1;
+        const T ws = hs[i + 1];
         Sum<T> nrm;
         const int len = k.d1 - k.d0;
         const int d0 = k.d0 + ((int)((long long)len * blockIdx.y / gridDim.y) & ~7);
@@ -290,13 +312,13 @@ k_orth(const SysDev *__restrict__ sys, const DChunk *__restrict__ ch, const int 
                 SysState *st = D.st;
                 double n2 = tot[0];
                 for (int y = 1; y < gridDim.y; ++y) n2 += tot[y];
-                const double hn = sqrt(n2);
+                const double vn = sqrt(n2), hn = vn / D.vscale[D.kmax];
                 Rot R{D.cs, D.sn, D.g, st_t, st_a, 0, 0, 0, 0.0};
                 const bool stop = givens<double>(D.H, D.kmax, R, i, D.hcol, hn, D.mixed ? st->target : st->eps);
                 __syncwarp();
                 if (lane == 0) {
                     st->hn = hn;
-                    D.vscale[i + 1] = std::is_same<T, TV>::value ? 1.0 / hn : (double)D.vsci;
+                    D.vscale[i + 1] = std::is_same<T, TV>::value ? 1.0 / vn : (double)D.vsci;
                     st->rho = R.rho;
                     st->steps = R.steps;
                     st->iterations += 1;
@@ -335,13 +357,12 @@ k_normalize(const SysDev *__restrict__ sys, const DChunk *__restrict__ ch, const
 
 // ---------------------------------------------------------------- cycle end
 // x += V y (pgmres.c:173-175) with y from k_orth; the last part does the
-// restart bookkeeping (:177-179).  FP32: the sum of the products in error-free
-// FP32 pairs (an FP64 FMA and a conversion a value bound this pass).
+// restart bookkeeping (:177-179).  FP32: the sum of the products in FP32 pairs (split_y).
 template <typename T, typename TV>
 __global__ void __launch_bounds__(kThreads)
 k_update(const SysDev *__restrict__ sys, const DChunk *__restrict__ ch, const int *__restrict__ nch)
 {
-    __shared__ double y[kMaxRestart];
+    __shared__ double y[kMaxRestart], back;
     __shared__ float yh[kMaxRestart], yl[kMaxRestart];
     const int total = *nch;
     for (int c = blockIdx.x; c < total; c += gridDim.x) {
@@ -350,12 +371,9 @@ k_update(const SysDev *__restrict__ sys, const DChunk *__restrict__ ch, const in
         if (!D.st->live) continue;
         const int m = D.st->steps;
         __syncthreads();
-        for (int j = threadIdx.x; j < m; j += kThreads) {
-            const double v = D.y[j] * D.vscale[j];
-            y[j] = v;
-            yh[j] = (float)v;
-            yl[j] = (float)(v - (double)(float)v);
-        }
+        if constexpr (sizeof(T) == 8) {
+            for (int j = threadIdx.x; j < m; j += kThreads) y[j] = D.y[j] * D.vscale[j];
+        } else if (threadIdx.x < 32) split_y(D.y, D.vscale, m, yh, yl, 1, &back);
         __syncthreads();
         const TV *V = (const TV *)D.V;
         const size_t ld = (size_t)D.n_pad;
@@ -390,8 +408,8 @@ k_update(const SysDev *__restrict__ sys, const DChunk *__restrict__ ch, const in
 #pragma unroll
             for (int e = 0; e < N; e += 2) {
                 double2 x2 = *reinterpret_cast<const double2 *>(D.x + q + e);
-                x2.x += s[e].value();
-                x2.y += s[e + 1].value();
+                x2.x += sizeof(T) == 8 ? s[e].value() : s[e].value() * back;
+                x2.y += sizeof(T) == 8 ? s[e + 1].value() : s[e + 1].value() * back;
                 *reinterpret_cast<double2 *>(D.x + q + e) = x2;
             }
         }

@@ -14,8 +14,9 @@
 // A step (classical Gram-Schmidt with a Gram correction: with G = V^T V the
 // coefficients of the two classical passes are s + (s - G s), s = V^T w, so
 // one pass over the basis gives both; FP64 systems too).  The newest vector
-// is kept unscaled until its norm is known, so that the norm travels with the
-// next step's dots and a step has a single reduction over the gang:
+// is kept unscaled until its norm is known (but for a power of two that a cycle's
+// first step finds, unit_scale), so that the norm travels with the next step's
+// dots and a step has a single reduction over the gang:
 //   1. the Gram column V^T v_i over the CTA's rows, 8 lanes per basis vector,
 //      while the newest vector's entries of neighbouring CTAs (the halo)
 //      arrive: polled from the exchange vector vb into shared memory;
@@ -283,6 +284,7 @@ k_cycle(const SysDev *__restrict__ sys, const CycItem *__restrict__ items, int s
     __shared__ T s_tot[2 * KM], s_red[2 * KM], s_c[2][KM];     // c of this and the previous step
     __shared__ T s_n2h[kWorkers / 32], s_n2l[kWorkers / 32];
     __shared__ T s_sc, s_dg;                      // 1 / norm of the newest vector, its Gram diagonal less 1
+    __shared__ T s_sg, s_ss;                      // the newest vector's power of two, times s_sc
     __shared__ int s_stop, s_gave_up, s_m;
     const Bound bound{&s_gave_up, g_gang_polls < 32 ? 0 : 31};
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, l8 = tid & 7, gid = tid >> 3;
@@ -402,8 +404,8 @@ k_cycle(const SysDev *__restrict__ sys, const CycItem *__restrict__ items, int s
                     }
                 };
                 // ---- g = V^T v_i (v_i not scaled yet) while the halo arrives
-                dot(vi, s_red + KM);
                 if (i > 0) {
+                    dot(vi, s_red + KM);
                     for (int q = tid; q < nh; q += 2 * kWorkers) {
                         const int q2 = q + kWorkers, p = q < nhl ? q : q + nrow, p2 = q2 < nhl ? q2 : q2 + nrow;
                         const u64 *src = vb + (size_t)lo * B * WP;
@@ -465,8 +467,15 @@ k_cycle(const SysDev *__restrict__ sys, const CycItem *__restrict__ items, int s
                     }
                     sync_workers();
                 }
-                // ---- s = V^T w over this CTA's rows
+                // ---- s = V^T w over this CTA's rows; the first step's largest |w| in g's place
                 dot(w, s_red);
+                if (i == 0) {
+                    T m = (T)0;
+                    for (int q = tid; q < nrow; q += kWorkers) m = max(m, abs(w[q]));
+#pragma unroll
+                    for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+                    if (lane == 0) s_red[KM + warp] = m;
+                }
             }
             __syncthreads();                      // the Givens warp is done with column i - 2 too
             // ---- exchange: 2 nv sums (s_j, g_j), ||v_i||^2 and the stop flag
@@ -474,7 +483,10 @@ k_cycle(const SysDev *__restrict__ sys, const CycItem *__restrict__ items, int s
                 const int nsl = dot_slices(np, nv);
                 const T *red = s_red + (tid & 1) * KM + (tid >> 1);
                 T s = red[0];
-                for (int q = 1; q < nsl; ++q) s += red[q * nv];
+                if (i == 0 && tid == 1)
+                    for (int q = 1; q < kWorkers / 32; ++q) s = max(s, red[q]);
+                else
+                    for (int q = 1; q < nsl; ++q) s += red[q * nv];
                 if (g == 1) s_tot[tid] = s;
                 else put<T>(part + ((size_t)tid * g + rank) * WP, s, tag);
             }
@@ -579,6 +591,7 @@ k_cycle(const SysDev *__restrict__ sys, const CycItem *__restrict__ items, int s
                 if (lane == 0) {
                     const T sc = i == 0 ? (T)1 : inv_norm(n2);     // v_0 is taken as it is
                     s_sc = sc;
+                    if (i > 0) s_ss = sc * s_sg;
                     s_dg = gram_diag(n2, sc);
                 }
             } else if (g > 1 && tid == kWorkers - 1 && rank != 0) {
@@ -590,7 +603,9 @@ k_cycle(const SysDev *__restrict__ sys, const CycItem *__restrict__ items, int s
             const T sc = s_sc;
             T *c = s_c[i & 1];
             if (worker) {
-                // ---- c = s - (G - I) s; the new Gram column from this step's sums
+                const T ss = i == 0 ? unit_scale(s_tot[1]) : s_ss;
+                if (i == 0 && tid == 0) s_sg = ss;
+                // ---- c = s - (G - I) s (times sg); the new Gram column from this step's sums
                 for (int j = gid; j < ((nv + 3) & ~3); j += kGroups) {
                     T d = (T)0;
                     if (j < nv) {
@@ -608,11 +623,11 @@ k_cycle(const SysDev *__restrict__ sys, const CycItem *__restrict__ items, int s
                     d += __shfl_xor_sync(0xffffffffu, d, 4);
                     d += __shfl_xor_sync(0xffffffffu, d, 2);
                     d += __shfl_xor_sync(0xffffffffu, d, 1);
-                    if (l8 == 0 && j < nv) c[j] = sc * ((j == i ? sc * s_tot[2 * j] : s_tot[2 * j]) - d);
+                    if (l8 == 0 && j < nv) c[j] = ss * ((j == i ? sc * s_tot[2 * j] : s_tot[2 * j]) - d);
                 }
                 sync_workers();
                 asm volatile("bar.arrive 2, %0;\n" ::"n"(kCycThreads) : "memory");
-                // ---- v_i and w scaled, w -= V c, ||w||^2; what neighbours need to vb
+                // ---- v_i scaled, w scaled and times sg, w -= V c, ||w||^2; what neighbours need to vb
                 // (FP32: four rows a thread, so that a coefficient is read once for
                 // four; FP64: one, to keep every quarter of its pipe busy)
                 Sum<T> t;
@@ -623,7 +638,7 @@ k_cycle(const SysDev *__restrict__ sys, const CycItem *__restrict__ items, int s
 #pragma unroll
                     for (int r = 0; r < R; ++r) {
                         v[r] = sc * vi[q + r];
-                        s0[r] = sc * w[q + r];
+                        s0[r] = ss * w[q + r];
                         s1[r] = -c[i] * v[r];
                         (SPILL ? slot(i) : vi)[q + r] = v[r];
                     }
@@ -693,7 +708,7 @@ k_cycle(const SysDev *__restrict__ sys, const CycItem *__restrict__ items, int s
                 }
                 sync_workers();                   // w complete (and the norm's shares)
             } else {
-                // ---- the rotations of column i - 1, beside the rest of the step
+                // ---- the rotations of column i - 1 (H times s_sg), beside the rest of the step
                 asm volatile("bar.sync 2, %0;\n" ::"n"(kCycThreads) : "memory");
                 if (rank == 0 && i > 0) {
                     const bool stop = givens<T>(D.H, km, R, i - 1, s_c[(i - 1) & 1], 1.0 / (double)sc, target);
@@ -735,6 +750,7 @@ k_cycle(const SysDev *__restrict__ sys, const CycItem *__restrict__ items, int s
                 const int m = R.steps;
                 __syncwarp();
                 back_substitute(D.H, km, s_g, m, y);
+                for (int j = lane; j < m; j += 32) y[j] *= s_sg;
                 if (g > 1)
                     for (int j = lane; j < m; j += 32) put<double>(note + 3 + 2 * j, y[j], ytag);
                 if (lane == 0) {
@@ -752,13 +768,7 @@ k_cycle(const SysDev *__restrict__ sys, const CycItem *__restrict__ items, int s
                 if (lane == 0) s_m = min((int)v[0], km);
             }
             __syncwarp();
-            // FP32: y as pairs
-            if constexpr (sizeof(T) == 4)
-                for (int j = lane; j < s_m; j += 32) {
-                    const float yh = (float)y[j];
-                    s_tot[2 * j] = yh;
-                    s_tot[2 * j + 1] = (float)(y[j] - (double)yh);
-                }
+            if constexpr (sizeof(T) == 4) split_y(y, nullptr, s_m, s_tot, s_tot + 1, 2, s_a);
         }
         if (__syncthreads_or(s_gave_up)) {
             if (tid == 0) {
@@ -778,7 +788,7 @@ k_cycle(const SysDev *__restrict__ sys, const CycItem *__restrict__ items, int s
                     if constexpr (sizeof(T) == 8) t.h += y[j] * v;
                     else t.add_product(s_tot[2 * j], s_tot[2 * j + 1], v);
                 }
-                D.x[id] += t.value();
+                D.x[id] += sizeof(T) == 8 ? t.value() : t.value() * s_a[0];
             }
         if (rank == 0 && tid == kWorkers) {       // restart bookkeeping (pgmres.c:177-179)
             SysState *st = D.st;

@@ -52,6 +52,23 @@ template <> struct Sum<float> {
     __device__ __forceinline__ double value() const { return (double)h + (double)l; }
 };
 
+// The power of two that brings m into [1, 2) (1 where m is 0 or not finite): what
+// is kept in FP32 is kept times it, so that its range is FP64's.  The
+// newest basis vector is stored unscaled, times this for an m of the size of
+// M^-1 A v_0: its products with the basis then grow with the operator's scale,
+// not with its cube, and a power of two changes no rounding.
+// (A power whose reciprocal is normal too; by the exponent's bits.)
+__device__ __forceinline__ float unit_scale(float m)
+{
+    const int e = (__float_as_int(m) >> 23) & 0xff;
+    return m == 0.f || e == 0xff ? 1.f : __int_as_float((254 - max(1, min(e, 253))) << 23);
+}
+__device__ __forceinline__ double unit_scale(double m)
+{
+    const int e = (__double2hiint(m) >> 20) & 0x7ff;
+    return m == 0.0 || e == 0x7ff ? 1.0 : __hiloint2double((2046 - max(1, min(e, 2045))) << 20, 0);
+}
+
 // Givens step i (pgmres.c:111-157) by one warp: the coefficients h[0..i] and
 // h(i+1, i) = hn of column i; rotations and right-hand side in cs, sn, g
 // (kmax, kmax, kmax + 1), the rotated column to H; t, a: scratch of kmax.  The
@@ -126,6 +143,37 @@ __device__ __forceinline__ void back_substitute(const double *H, int km, const d
         }
     }
     __syncwarp();
+}
+
+// y as FP32 pairs times a power of two, by one warp, m <= 64: yh, yl and the
+// power's reciprocal.  Sums of V y are then formed in error-free FP32 pairs (the
+// FP64 FMA and the conversion a value would bind: 513 x 513 FP32 26.0 -> 27.4 ms a solve, 32
+// streaming systems 229 -> 256), with the range of FP64.  The solution is off from the exact
+// one by as much as with FP64 sums (432 solves of 961 to 25k equations, FP64 /
+// pairs 1.00 where the last bits show, 1.0 to 1.2 at a tolerance of 1e-11).
+__device__ __forceinline__ void split_y(const double *y, const double *scale, int m, float *yh, float *yl, int stride, double *back)
+{
+    const int lane = threadIdx.x & 31;
+    double a = lane < m ? y[lane] : 0.0, b = lane + 32 < m ? y[lane + 32] : 0.0;
+    if (scale) {
+        if (lane < m) a *= scale[lane];
+        if (lane + 32 < m) b *= scale[lane + 32];
+    }
+    double t = fmax(fabs(a), fabs(b));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) t = fmax(t, __shfl_xor_sync(0xffffffffu, t, o));
+    const double u = unit_scale(t);
+    a *= u;
+    b *= u;
+    if (lane < m) {
+        yh[stride * lane] = (float)a;
+        yl[stride * lane] = (float)(a - (double)(float)a);
+    }
+    if (lane + 32 < m) {
+        yh[stride * (lane + 32)] = (float)b;
+        yl[stride * (lane + 32)] = (float)(b - (double)(float)b);
+    }
+    if (lane == 0) *back = 1.0 / u;
 }
 
 }  // namespace fg

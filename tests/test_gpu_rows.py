@@ -107,3 +107,25 @@ def test_streamed_solves(fg, kind, ndof):
         assert r.stats["converged"] == 1, r.stats
         res = np.linalg.norm((F - s.matvec(r.x))[:-1]) / np.linalg.norm(F[:-1])
         assert res <= 1e-9, prec
+
+
+# Operators and right-hand sides far from 1, by powers of two: the same solve but
+# for the scale, on chip and streaming.  (The tolerance is the solves', 1e-11, times
+# a condition below 100.)
+@pytest.mark.parametrize("kind,ndof", [((23, 19), 1), ((33000, 1), 2)])
+@pytest.mark.parametrize("precision,ea,ef", [(32, 50, 0), (32, -50, 0), (32, 0, 150), (32, -40, -150), (64, 400, 0), (64, -400, 0)])
+def test_scaled_systems(fg, kind, ndof, precision, ea, ef):
+    m = _mesh(kind, ndof, 7)
+    A = G.random_blocks(m.nel, 3 * ndof, seed=2, dominance=6.0 * ndof)
+    F = np.append(np.random.Generator(np.random.PCG64(9)).uniform(-1.0, 1.0, m.neq), 0.0)
+    xs, its = [], []
+    for a, f in ((0, 0), (ea, ef)):
+        s = fg.System(m, reorder=False)
+        s.set_blocks(A * 2.0 ** a)
+        B = s.precond_setup(fg.FG_PRECOND_NONE, 0, F * 2.0 ** f)
+        r = s.solve(B, tol=1e-11, F_true=F * 2.0 ** f, precision=precision)
+        assert r.stats["converged"] == 1 and r.stats["true_rel_residual"] <= 1e-10, r.stats
+        xs.append(r.x * 2.0 ** (a - f))
+        its.append(r.stats["iterations"])
+    assert its[0] == its[1]
+    assert np.linalg.norm(xs[1] - xs[0]) <= 1e-9 * np.linalg.norm(xs[0])
