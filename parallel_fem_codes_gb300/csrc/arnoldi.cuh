@@ -106,7 +106,8 @@ constexpr int kMaxSplit = 8;        // CTAs of a part in pass 2
 // (V and w as stored).  A thread holds a pack of w and of V[i] and JB basis vectors' packs
 // at a time, so that JB + 2 loads are in flight and w is read from L1 after
 // the first group; the 2 JB sums are folded over the warp by halving (a
-// value's lanes drop out as the values do), then over the warps.
+// value's lanes drop out as the values do), then over the warps (FP32: in
+// pairs).
 template <typename T, typename TV>
 __device__ __forceinline__ void part_dots(const SysDev &D, const DChunk &k, int i, const T *__restrict__ w, T (*sw)[2 * kMaxRestart],
                                           double *out)
@@ -140,21 +141,25 @@ __device__ __forceinline__ void part_dots(const SysDev &D, const DChunk &k, int 
                     s[JB + u] += v[u][c] * u0[c];
                 }
         }
+        Sum<T> t[NV];
+#pragma unroll
+        for (int u = 0; u < NV; ++u) t[u].h = s[u];
         int o = 16;
 #pragma unroll
         for (int m = NV / 2; m >= 1; m >>= 1, o >>= 1) {
             const bool up = (lane & o) != 0;
 #pragma unroll
             for (int u = 0; u < m; ++u) {
-                const T keep = up ? s[u + m] : s[u], give = up ? s[u] : s[u + m];
-                s[u] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+                const Sum<T> give = up ? t[u] : t[u + m];
+                if (up) t[u] = t[u + m];
+                t[u].take(give, o);
             }
         }
-        for (; o > 0; o >>= 1) s[0] += __shfl_xor_sync(0xffffffffu, s[0], o);
+        for (; o > 0; o >>= 1) t[0].fold(o);
         // value index: the lane's upper bits, most significant first
         constexpr int SH = NV == 16 ? 1 : 2;
         const int idx = lane >> SH, j = j0 + (idx & (JB - 1));
-        if ((lane & ((1 << SH) - 1)) == 0 && j < nv) sw[warp][(idx < JB ? 0 : nv) + j] = s[0];
+        if ((lane & ((1 << SH) - 1)) == 0 && j < nv) sw[warp][(idx < JB ? 0 : nv) + j] = t[0].rounded();
     }
     __syncthreads();
     for (int h = threadIdx.x; h < 2 * (jb - ja); h += kThreads) {

@@ -379,27 +379,34 @@ k_cycle(const SysDev *__restrict__ sys, const CycItem *__restrict__ items, int s
             X.own = vi;
             if (worker) {
                 const int nsl = dot_slices(np, nv);
-                // nsl groups a basis vector (more vectors than groups: in rounds)
+                // nsl groups a basis vector; FP32: a lane's four chains, the lanes and the
+                // slices are added in pairs
                 auto dot = [&](const T *y, T *red) {
                     for (int h = gid; h - (gid & 3) < nv * nsl; h += kGroups) {
                         const int j = h % nv, sl = h / nv;
-                        T a = (T)0, a2 = (T)0;
+                        T s4[N];
+#pragma unroll
+                        for (int c = 0; c < N; ++c) s4[c] = (T)0;
                         if (sl < nsl) {
                             const T *vj = SPILL && j == i ? vi : slot(j);
 #pragma unroll 4
                             for (int p = sl * 8 + l8; p < np; p += 8 * nsl) {
                                 const auto x = ldp(vj + p * N), z = ldp(y + p * N);
 #pragma unroll
-                                for (int c = 0; c < N; c += 2) {
-                                    a += x.v[c] * z.v[c];
-                                    a2 += x.v[c + 1] * z.v[c + 1];
-                                }
+                                for (int c = 0; c < N; ++c) s4[c] += x.v[c] * z.v[c];
                             }
                         }
-                        a += a2;
-                        a += __shfl_xor_sync(0xffffffffu, a, 4);
-                        a += __shfl_xor_sync(0xffffffffu, a, 2);
-                        a += __shfl_xor_sync(0xffffffffu, a, 1);
+                        Sum<T> t;
+                        if constexpr (N == 4) {
+                            t.h = s4[0];
+                            t.add(s4[1]);
+                            t.add(s4[N - 2]);
+                            t.add(s4[N - 1]);
+                        } else t.h = s4[0] + s4[1];
+                        t.fold(4);
+                        t.fold(2);
+                        t.fold(1);
+                        const T a = t.rounded();
                         if (sl < nsl && l8 == 0) red[sl * nv + j] = a;
                     }
                 };
@@ -486,7 +493,11 @@ k_cycle(const SysDev *__restrict__ sys, const CycItem *__restrict__ items, int s
                 if (i == 0 && tid == 1)
                     for (int q = 1; q < kWorkers / 32; ++q) s = max(s, red[q]);
                 else
-                    for (int q = 1; q < nsl; ++q) s += red[q * nv];
+                {
+                    Sum<T> t;
+                    for (int q = 0; q < nsl; ++q) t.add(red[q * nv]);
+                    s = t.rounded();
+                }
                 if (g == 1) s_tot[tid] = s;
                 else put<T>(part + ((size_t)tid * g + rank) * WP, s, tag);
             }

@@ -14,6 +14,8 @@ template <> struct Sum<double> {
     __device__ __forceinline__ void add(double v) { h += v; }
     __device__ __forceinline__ void add_square(double v) { h += v * v; }
     __device__ __forceinline__ void fold(int o) { h += __shfl_xor_sync(0xffffffffu, h, o); }
+    // plus what lane ^ o gives
+    __device__ __forceinline__ void take(const Sum &give, int o) { h += __shfl_xor_sync(0xffffffffu, give.h, o); }
     __device__ __forceinline__ double rounded() const { return h; }
     __device__ __forceinline__ double value() const { return h; }
 };
@@ -47,6 +49,11 @@ template <> struct Sum<float> {
         h = ah;
         l = __fadd_rn(al, bl);
         add(bh);
+    }
+    __device__ __forceinline__ void take(const Sum &give, int o)
+    {
+        l = __fadd_rn(l, __shfl_xor_sync(0xffffffffu, give.l, o));
+        add(__shfl_xor_sync(0xffffffffu, give.h, o));
     }
     __device__ __forceinline__ float rounded() const { return __fadd_rn(h, l); }
     __device__ __forceinline__ double value() const { return (double)h + (double)l; }
