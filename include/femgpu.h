@@ -274,9 +274,13 @@ int fg_solve(fg_system *s, const fg_solver_opts *opts, const double *B, double *
              const double *F_true, fg_solve_stats *stats);
 
 /* Solve many systems together (same block size and preconditioner kind):
- * one CUDA-graph launch per restart cycle advances every member, members
- * stop independently, and each result is bit-identical to solving that
- * system alone.  B[i], X[i], F_true[i] are host vectors of system i
+ * each restart cycle (a few kernels on chip, or one CUDA-graph launch)
+ * advances every member, and members stop independently.  A batch always gives
+ * the same result, bit for bit.  Members of a batch with fewer than 32768
+ * equations in all, each of which can run on chip (or none of which can: an
+ * ILU, SPIKE or element preconditioner), get the bits that they get alone; in
+ * larger batches the order of the sums follows the batch, and results agree to
+ * rounding.  B[i], X[i], F_true[i] are host vectors of system i
  * (F_true may be NULL, or F_true[i] NULL).  stats has count entries. */
 int fg_solve_batch(fg_system *const *systems, int count, const fg_solver_opts *opts,
                    const double *const *B, double *const *X, const double *const *F_true,
@@ -606,7 +610,8 @@ int fg_bubble_state(fg_system *s, double *uB, double *aB);
  * assembles them on the device (SUPG/CAU at u = 0, fresh Diag), and every
  * cycle advances all admitted solves together; a solve leaves the batch as
  * soon as it converges.  Meshes and Krylov state stay on the device.  A
- * result is bit-identical to solving the same system alone. */
+ * result has the bits of the same solve alone while fewer than 32768 equations
+ * are active (see fg_solve_batch), and agrees with it to rounding otherwise. */
 typedef struct fg_server fg_server;
 typedef struct {
     int kmax, lmax;

@@ -33,8 +33,8 @@
 // one trip through L2 (small gangs: every CTA sums all partials; vb) or two
 // (large gangs: CTA m sums slot m, everyone reads the totals) and no barrier
 // or fence.  Partials are summed in rank order: results are the same run to
-// run, and depend on the gang only through its size, which is the system's
-// (gang_size).  A word is rewritten only after every CTA published the
+// run, and depend on the gang only through its size (gang_size: the system's, or
+// in larger batches the room's too).  A word is rewritten only after every CTA published the
 // exchange that follows its reading.
 //
 // Measured (GB300), a whole solve with the pass kernels -> on chip, and an

@@ -14,9 +14,11 @@
 // Work decomposition.  A batch holds any number of systems.  The operator
 // is the assembled one (rows.cu), cut into unit chunks, dof work into parts
 // per system; every kernel walks its chunk table with a grid-stride loop and skips systems
-// that are not active.  A system's partial sums depend only on its own
-// parts, so a result is bit-identical whether the system is solved alone
-// or inside a batch.
+// that are not active.  A system's sums depend on its own parts and gang only.
+// In a batch of fewer than kSoloDofs equations these are the ones that the system
+// has alone, so that a result has the same bits alone and in the batch; in a
+// larger one part sizes, gangs and the engine follow the batch (and who has
+// stopped), and results agree to rounding.
 #include <algorithm>
 #include <atomic>
 #include <chrono>
@@ -839,6 +841,10 @@ void launch_blockdiag(int B, dim3 g, cudaStream_t st, const SysDev *sys, const N
 // a CTA a chunk: the hardware hands them out as CTAs finish
 inline dim3 grid_for(int nchunks) { return dim3((unsigned)std::max(1, nchunks)); }
 
+// Batches below this: what a member's sums depend on follows its own size only
+// (parts of kPartMin, part_dofs_for).
+constexpr long long kSoloDofs = 32768;
+
 int parts_for(int n, int part_dofs = kPartMax)
 {
     int p = (n + part_dofs - 1) / part_dofs;
@@ -914,6 +920,7 @@ int part_dofs_for(const std::vector<BatchMember> &mem, const SolveConfig &cfg)
                 if (parts <= rounds * round) return pd;
             }
     }
+    if (dofs < kSoloDofs) return kPartMin;
     const double tot = (double)dofs;
     const long long pd = 1LL << (int)std::lround(std::log2((tot > 65536.0 ? 4.0 : 2.0) * std::sqrt(tot)));
     return (int)std::max<long long>(kPartMin, std::min<long long>(kPartMax, pd));
@@ -946,6 +953,7 @@ struct Plan {
     Span sysdev, dchunks, dcount, nchunks, ncount;
     Span cyc_items;                                // on-chip cycle: (system, rank) of its CTAs
     std::vector<CycBin> bins;                      // its launches (none: the cycle streams)
+    bool solo = false;                             // fewer than kSoloDofs equations
     bool rprec = false;                            // a right preconditioner (SGSe) before every matvec
     Span ilu_fwd, ilu_bwd, ilu_ctr;                // sync-free ILU(0) substitutions
     Span ilu_ws;                                 // block-Jacobi: (system, block) items, a warp each
@@ -973,6 +981,7 @@ static int build_plan(Plan &P, std::vector<BatchMember> &mem, const SolveConfig 
     const int pdofs = part_dofs_for(mem, cfg);
     const int uchunk = unit_chunk(mem, cfg);
     P.rprec = cfg.precond == FG_PRECOND_SGSE;
+    P.solo = batch_dofs(mem) < kSoloDofs;
     if (cycles && (r = choose_engine(mem, cfg, hs, {}, P.B, st))) return r;
     for (int s = 0; s < P.nsys; ++s) {
         int n = mem[s].s->topo.n;
@@ -1181,7 +1190,9 @@ static int enqueue_cycle(const Plan &P, const SolveConfig &cfg, int *live, cudaS
         // 2 and 2: 373, 4 and 2: 362).
         const int fill = 8 * sm_count() / std::max(1, P.n_dch), ways = std::min(16, fill * (sizeof(T) == 8 ? 2 : 1));
         const bool split = sizeof(T) == 8 || P.n_dch < 2 * sm_count();
-        const int yd = split ? std::max(1, ways) : 1, yo = split ? std::max(1, std::min(kMaxSplit, fill)) : 1;
+        // (a part's norm depends on the CTAs it is split among in pass 2, not on those of pass 1)
+        const int yd = split ? std::max(1, ways) : 1;
+        const int yo = P.solo ? kMaxSplit : split ? std::max(1, std::min(kMaxSplit, fill)) : 1;
         k_scale_v0<T, TV><<<gd, kThreads, 0, st>>>(sys, dc, nd);
         ++k;
         for (int i = 0; i < cfg.kmax - 1; ++i) {
@@ -1222,7 +1233,7 @@ static size_t items_room(const std::vector<BatchMember> &mem, const SolveConfig 
     size_t sum = 0;
     for (const BatchMember &m : mem) {
         const int g = member_gang(m.s, cfg, true);
-        sum += g ? g : room;
+        sum += g ? std::max(g, member_gang(m.s, cfg, false)) : room;
     }
     return chip_config(cfg) ? std::max(room, sum) : 0;
 }
@@ -1505,7 +1516,8 @@ int BatchRun::stage(const BatchMember &m)
 }
 
 // Where the batch's restart cycles run, for the live members (all: empty).  On
-// chip when gangs of the CTAs they like (gang_want) are resident together.
+// chip when gangs of the CTAs they like (gang_want) are resident together, or in a
+// batch below kSoloDofs, in as many launches as these gangs take.
 // Else as up to kMaxBins launches one behind the other, in which gangs are as
 // small as their rows allow and a member that fits no chip has all of one with
 // part of its basis outside.  Else streaming through global memory, all at once:
@@ -1527,21 +1539,8 @@ static int choose_engine(const std::vector<BatchMember> &mem, const SolveConfig 
     std::vector<int> todo;
     for (int i = 0; i < n; ++i)
         if (live.empty() || live[i]) todo.push_back(i);
-    bool chip = chip_config(cfg) && room > 0;
-    long long sum = 0;
-    for (int i : todo)
-        if (chip) {
-            sum += g[i] = member_gang(mem[i].s, cfg, false);
-            chip = g[i] > 0 && sum <= room;
-        }
-    if (!chip && chip_config(cfg) && room > 0) {
-        // launches of dense gangs, the largest first
-        chip = true;
-        for (int i : todo) {
-            g[i] = member_gang(mem[i].s, cfg, true);
-            if (!g[i] && (js[i] = gang_spill(mem[i].s, cfg.kmax, !cfg.mixed)) > 0) g[i] = gang_ctas(B, !cfg.mixed, true);
-            chip = chip && g[i] > 0;
-        }
+    // launches of the gangs, the largest first; a member that fits no chip has one of its own
+    auto pack = [&] {
         std::stable_sort(todo.begin(), todo.end(), [&](int a, int b) { return g[a] > g[b]; });
         std::vector<int> left;
         for (int i : todo) {
@@ -1551,7 +1550,25 @@ static int choose_engine(const std::vector<BatchMember> &mem, const SolveConfig 
             bin[i] = (int)b;
             left[b] = js[i] ? 0 : left[b] - g[i];
         }
-        chip = chip && (int)left.size() <= kMaxBins;
+        return (int)left.size();
+    };
+    bool chip = chip_config(cfg) && room > 0;
+    long long sum = 0;
+    const bool solo = batch_dofs(mem) < kSoloDofs;
+    for (int i : todo)
+        if (chip) {
+            sum += g[i] = member_gang(mem[i].s, cfg, false);
+            chip = g[i] > 0 && (solo || sum <= room);
+        }
+    if (chip) pack();
+    else if (chip_config(cfg) && room > 0) {
+        chip = true;
+        for (int i : todo) {
+            g[i] = member_gang(mem[i].s, cfg, true);
+            if (!g[i] && (js[i] = gang_spill(mem[i].s, cfg.kmax, !cfg.mixed)) > 0) g[i] = gang_ctas(B, !cfg.mixed, true);
+            chip = chip && g[i] > 0;
+        }
+        chip = pack() <= kMaxBins && chip;
     }
     // no memory for the gangs: stream
     for (int i : todo) {
