@@ -310,13 +310,14 @@ void *fg_system_stream(const fg_system *s);
 int fg_bench_matvec(fg_system *const *systems, int count, int precision, int reps,
                     double *ms_per_matvec, double *bytes);
 
-/* Autotuner: times candidate launch shapes of a batch on the batch itself
- * (one restart cycle each, CUDA events on the first system's stream) --
+/* Autotuner: times candidate launch shapes of a batch's streaming restart
+ * cycles on the batch itself
+ * (one cycle each, CUDA events on the first system's stream) --
  * the dof-part size of the Krylov kernels (256 ... 16384 dofs) and, for
  * 3x3 blocks in FP32, the rows per thread of the matvec -- and keeps the fastest for the process, keyed by (block size,
  * precision, batch-size class floor(log2(batch dofs))).  Every later batch
  * of that key (fg_solve_batch, fg_solve_resident, the request server) uses
- * it.  The systems need resident right-hand sides (fg_transport_prepare or
+ * it while its cycles stream (on-chip cycles have none of these).  The systems need resident right-hand sides (fg_transport_prepare or
  * a time-loop set-up).  remeasure 0 returns a cached choice when there is
  * one (from_cache = 1).  The cycles run on the systems' workspaces, which
  * the next solve reinitialises.  No counterpart in the reference (its

@@ -854,11 +854,11 @@ int parts_for(int n, int part_dofs = kPartMax)
 }  // namespace
 
 // ---------------------------------------------------------------- autotuner
-// Measured launch shapes of a batch, chosen by fg_autotune and cached per
+// Measured launch shapes of a batch's streaming cycles, chosen by fg_autotune and cached per
 // (block size, precision, batch-size class = floor(log2(batch dofs))) for
 // the process: the dof-part size of the Krylov kernels and, for 3x3
 // blocks in FP32, the matvec's work items (four rows a thread or one).  A batch
-// with no cached choice uses the built-in rule.
+// with no cached choice, or one that runs on chip, uses the built-in rule.
 struct TuneKey {
     int S, mixed, vhalf, cls;
     bool operator<(const TuneKey &o) const
@@ -906,10 +906,10 @@ namespace {
 // (a pass of its threads) takes the smallest multiple of that with which the
 // parts fill whole rounds of CTAs: 4.0 M dofs FP32 on 152 SMs, a step with 8192
 // dofs in 506 parts 173 us, with 9216 in 452 parts 156; 3 M FP64 391 -> 362.
-int part_dofs_for(const std::vector<BatchMember> &mem, const SolveConfig &cfg)
+int part_dofs_for(const std::vector<BatchMember> &mem, const SolveConfig &cfg, bool tuned)
 {
     fg_tune_choice tc;
-    if (tuned_choice(mem, cfg, tc) && tc.part_dofs > 0) return tc.part_dofs & ~7;
+    if (tuned && tuned_choice(mem, cfg, tc) && tc.part_dofs > 0) return tc.part_dofs & ~7;
     const long long dofs = std::max(1LL, batch_dofs(mem)), round = (cfg.mixed ? 3LL : 4LL) * sm_count();
     if (dofs > 1024 * round) {
         for (long long rounds = 1;; ++rounds)
@@ -930,11 +930,11 @@ int part_dofs_for(const std::vector<BatchMember> &mem, const SolveConfig &cfg)
 // while that leaves a wave of CTAs or less, so that small systems spread out,
 // else four rows per thread.  A tuned choice can pin either (mv3_pipeline 0:
 // always one row per thread); the sums are the same.
-int unit_chunk(const std::vector<BatchMember> &mem, const SolveConfig &cfg)
+int unit_chunk(const std::vector<BatchMember> &mem, const SolveConfig &cfg, bool tuned)
 {
     fg_tune_choice tc;
     const int B = mem[0].s->topo.ndof, one = 32 / B * (kThreads / 32);
-    if (tuned_choice(mem, cfg, tc) && tc.mv3_pipeline == 0) return one;
+    if (tuned && tuned_choice(mem, cfg, tc) && tc.mv3_pipeline == 0) return one;
     return batch_dofs(mem) > 8LL * kThreads * sm_count() ? 4 * one : one;
 }
 
@@ -978,11 +978,14 @@ static int build_plan(Plan &P, std::vector<BatchMember> &mem, const SolveConfig 
         if (m.s->topo.S != P.S) { set_error("a batch must hold systems of one block size"); return FG_ERR_ARG; }
     std::vector<DChunk> dch;
     std::vector<NChunk> nch;
-    const int pdofs = part_dofs_for(mem, cfg);
-    const int uchunk = unit_chunk(mem, cfg);
     P.rprec = cfg.precond == FG_PRECOND_SGSE;
     P.solo = batch_dofs(mem) < kSoloDofs;
     if (cycles && (r = choose_engine(mem, cfg, hs, {}, P.B, st))) return r;
+    // (a tuned choice is one for the streaming kernels)
+    bool chip = false;
+    for (const SysDev &D : hs) chip = chip || D.cy_g > 0;
+    const int pdofs = part_dofs_for(mem, cfg, !chip);
+    const int uchunk = unit_chunk(mem, cfg, !chip);
     for (int s = 0; s < P.nsys; ++s) {
         int n = mem[s].s->topo.n;
         hs[s].nparts = parts_for(n, pdofs);
@@ -1552,7 +1555,8 @@ static int choose_engine(const std::vector<BatchMember> &mem, const SolveConfig 
         }
         return (int)left.size();
     };
-    bool chip = chip_config(cfg) && room > 0;
+    const bool can = chip_config(cfg) && room > 0 && !t_tune_force;   // (the autotuner times streaming cycles)
+    bool chip = can;
     long long sum = 0;
     const bool solo = batch_dofs(mem) < kSoloDofs;
     for (int i : todo)
@@ -1561,7 +1565,7 @@ static int choose_engine(const std::vector<BatchMember> &mem, const SolveConfig 
             chip = g[i] > 0 && (solo || sum <= room);
         }
     if (chip) pack();
-    else if (chip_config(cfg) && room > 0) {
+    else if (can) {
         chip = true;
         for (int i : todo) {
             g[i] = member_gang(mem[i].s, cfg, true);

@@ -101,3 +101,42 @@ def test_tune_set_rejects_bad_choices(fg):
         with pytest.raises(fg.FemGpuError) as e:
             fg.tune_set(systems, **bad)
         assert e.value.code == fg.FG_ERR_ARG
+
+
+def test_on_chip_cycles_ignore_the_choice(fg):
+    probs, systems = _batch(fg)
+    got = []
+    try:
+        for pd in (0, 16384):
+            fg.tune_clear()
+            if pd:
+                fg.tune_set(systems, pd, mv3_pipeline=0)
+            for s, p in zip(systems, probs):
+                s.transport_prepare(p)
+            st = fg.solve_resident(systems, tol=1e-10, precision=fg.FG_PREC_MIXED)
+            got.append(([q["iterations"] for q in st], [s.solution() for s in systems]))
+    finally:
+        fg.tune_clear()
+    assert got[0][0] == got[1][0]
+    assert all(np.array_equal(a, b) for a, b in zip(got[0][1], got[1][1]))
+
+
+@pytest.mark.parametrize("part_dofs", [1024, 16384])
+def test_rows_a_thread_give_the_same_bits_streaming(fg, part_dofs):
+    # five systems of a chip's size each stream; more than a wave of rows, so that the two choices differ
+    probs = [G.transport_problem(n, angle_deg=30.0 + 40 * n, k=1e-4) for n in (480, 485, 491, 500, 503)]
+    systems = [fg.transport_system(p) for p in probs]
+    sols, its = [], []
+    try:
+        for mv in (1, 0):
+            fg.tune_clear()
+            fg.tune_set(systems, part_dofs, mv3_pipeline=mv)
+            for s, p in zip(systems, probs):
+                s.transport_prepare(p)
+            st = fg.solve_resident(systems, tol=1e-10, lmax=3, precision=fg.FG_PREC_MIXED)
+            its.append([q["iterations"] for q in st])
+            sols.append([s.solution() for s in systems])
+    finally:
+        fg.tune_clear()
+    assert its[0] == its[1] and max(its[0]) > 29
+    assert all(np.array_equal(a, b) for a, b in zip(*sols))
