@@ -195,3 +195,40 @@ def test_wait_limit_times_out_and_recovers(fg, precision):
     again = fg.solve_resident([s], tol=1e-10, precision=precision)[0]
     assert again["converged"] == 1 and again["iterations"] == good["iterations"]
     assert np.array_equal(s.solution(), x)
+
+
+def _multi_dof(fg, kind, n):
+    if kind == "ns":
+        p = G.cavity_problem(n, reynolds=1000.0, jitter=0.2)
+        s = fg.ns_system(p)
+        m = p.mesh
+        v = np.stack([np.sin(3 * m.x) * m.y, np.cos(2 * m.y) * m.x, 0.1 * m.x * m.y], 1).reshape(-1)
+        return s, s.ns_assemble(p, np.ascontiguousarray(v[m.type != 0]))
+    # a transport operator for each dof, the dofs of a node coupled
+    K, _ = O.build_k_f_supg(G.transport_problem(n, angle_deg=40.0, k=1e-2))
+    m = G.multi_dof_mesh(n, kind, seed=1)
+    A = np.einsum("eab,rq->earbq", K.reshape(m.nel, 3, 3), 0.9 * np.eye(kind) + 0.1)
+    s = fg.System(m, reorder=False)
+    s.set_blocks(np.ascontiguousarray(A.reshape(m.nel, -1)))
+    return s, np.append(np.random.Generator(np.random.PCG64(9)).uniform(-1.0, 1.0, m.neq), 0.0)
+
+
+# Bases beyond shared memory with 2 to 4 dofs a node, BlockDiag, GMRES(60): one
+# system (a spilling gang) against four of them (which stream), one restart cycle
+@pytest.mark.parametrize("kind,n,precision", [("ns", 181, 64), ("ns", 257, 32), (2, 221, 64), (4, 161, 64), (4, 231, 32)])
+def test_spilling_and_streaming_agree(fg, kind, n, precision):
+    systems, Bs, Fs = [], [], []
+    for _ in range(4):
+        s, F = _multi_dof(fg, kind, n)
+        Bs.append(s.precond_setup(fg.FG_PRECOND_BLOCKDIAG, 0, F))
+        Fs.append(F)
+        systems.append(s)
+    one = systems[0].solve(Bs[0], kmax=60, lmax=1, tol=1e-14, F_true=Fs[0], precision=precision)
+    X, st = fg.solve_batch(systems, Bs, Fs, kmax=60, lmax=1, tol=1e-14, precision=precision)
+    assert all(np.array_equal(X[0], x) for x in X[1:])
+    assert one.stats["iterations"] == st[0]["iterations"] == 59
+    # rounding over 59 steps, times 100 for the triangular system
+    eps = 60 * 100 * (2.0 ** -53 if precision == 64 else 2.0 ** -24)
+    assert np.linalg.norm(one.x - X[0]) <= eps * np.linalg.norm(X[0])
+    a, b = one.stats["true_rel_residual"], st[0]["true_rel_residual"]
+    assert abs(a - b) <= eps * max(a, 1e-3)

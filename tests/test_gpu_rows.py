@@ -129,3 +129,21 @@ def test_scaled_systems(fg, kind, ndof, precision, ea, ef):
         its.append(r.stats["iterations"])
     assert its[0] == its[1]
     assert np.linalg.norm(xs[1] - xs[0]) <= 1e-9 * np.linalg.norm(xs[0])
+
+
+# BlockDiag in the streaming matvec (a node's rows by shuffles): the meshes of
+# test_streamed_solves with 2 to 4 dofs a node
+@pytest.mark.parametrize("kind", [(1, 1), (13, 17), "wheel", (32000, 1), (33000, 1)])
+@pytest.mark.parametrize("ndof", [2, 3, 4])
+def test_streamed_block_diagonal(fg, kind, ndof):
+    m = _mesh(kind, ndof, 7)
+    A = G.random_blocks(m.nel, 3 * ndof, seed=2, dominance=6.0 * ndof)
+    F = np.append(np.random.Generator(np.random.PCG64(9)).uniform(-1.0, 1.0, m.neq), 0.0)
+    s = fg.System(m, reorder=False)
+    s.set_blocks(A)
+    B = s.precond_setup(fg.FG_PRECOND_BLOCKDIAG, 0, F)
+    for prec in (fg.FG_PREC_MIXED16, fg.FG_PREC_MIXED, fg.FG_PREC_FP64):
+        r = s.solve(B, tol=1e-11, F_true=F, precision=prec)
+        assert r.stats["converged"] == 1, r.stats
+        res = np.linalg.norm((F - s.matvec(r.x))[:-1]) / np.linalg.norm(F[:-1])
+        assert res <= 1e-9, prec
