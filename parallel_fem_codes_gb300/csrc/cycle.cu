@@ -74,6 +74,7 @@ constexpr int kWorkers = 512;
 constexpr int kCycThreads = kWorkers + 32;
 constexpr int kGroups = kWorkers / 8;         // 8-lane groups
 constexpr int kMaxSlices = 8;
+static_assert(kMaxRestart <= kGroups, "a group for every basis vector");
 // slices of the CTA's rows in the dots: while every lane keeps 8 packs
 __device__ __forceinline__ int dot_slices(int np, int nv) { return max(1, min(min(kMaxSlices, np / 64), kGroups / nv)); }
 constexpr long long kPollCycles = 4000000000LL;   // ~2 s
@@ -382,33 +383,32 @@ k_cycle(const SysDev *__restrict__ sys, const CycItem *__restrict__ items, int s
                 // nsl groups a basis vector; FP32: a lane's four chains, the lanes and the
                 // slices are added in pairs
                 auto dot = [&](const T *y, T *red) {
-                    for (int h = gid; h - (gid & 3) < nv * nsl; h += kGroups) {
-                        const int j = h % nv, sl = h / nv;
-                        T s4[N];
+                    if (gid - (gid & 3) >= nv * nsl) return;      // a warp without a vector
+                    const int j = gid % nv, sl = gid / nv;
+                    T s4[N];
 #pragma unroll
-                        for (int c = 0; c < N; ++c) s4[c] = (T)0;
-                        if (sl < nsl) {
-                            const T *vj = SPILL && j == i ? vi : slot(j);
+                    for (int c = 0; c < N; ++c) s4[c] = (T)0;
+                    if (sl < nsl) {
+                        const T *vj = SPILL && j == i ? vi : slot(j);
 #pragma unroll 4
-                            for (int p = sl * 8 + l8; p < np; p += 8 * nsl) {
-                                const auto x = ldp(vj + p * N), z = ldp(y + p * N);
+                        for (int p = sl * 8 + l8; p < np; p += 8 * nsl) {
+                            const auto x = ldp(vj + p * N), z = ldp(y + p * N);
 #pragma unroll
-                                for (int c = 0; c < N; ++c) s4[c] += x.v[c] * z.v[c];
-                            }
+                            for (int c = 0; c < N; ++c) s4[c] += x.v[c] * z.v[c];
                         }
-                        Sum<T> t;
-                        if constexpr (N == 4) {
-                            t.h = s4[0];
-                            t.add(s4[1]);
-                            t.add(s4[N - 2]);
-                            t.add(s4[N - 1]);
-                        } else t.h = s4[0] + s4[1];
-                        t.fold(4);
-                        t.fold(2);
-                        t.fold(1);
-                        const T a = t.rounded();
-                        if (sl < nsl && l8 == 0) red[sl * nv + j] = a;
                     }
+                    Sum<T> t;
+                    if constexpr (N == 4) {
+                        t.h = s4[0];
+                        t.add(s4[1]);
+                        t.add(s4[N - 2]);
+                        t.add(s4[N - 1]);
+                    } else t.h = s4[0] + s4[1];
+                    t.fold(4);
+                    t.fold(2);
+                    t.fold(1);
+                    const T a = t.rounded();
+                    if (sl < nsl && l8 == 0) red[sl * nv + j] = a;
                 };
                 // ---- g = V^T v_i (v_i not scaled yet) while the halo arrives
                 if (i > 0) {

@@ -50,9 +50,6 @@ struct Topology {
     std::vector<unsigned short> pt_col;  // npatch * kPatchColStride local colour offsets
     std::vector<int> dofs;       // patch-local dof -> internal dof, bit 31 = shared with another patch
     std::vector<unsigned short> lm16;    // nel*S local indices (internal order), 0xFFFF = sink
-    // x segment of each patch: its dofs lie in [xlo, xlo + xlen) (xlo and
-    // xlen multiples of 8); a 3x3 patch closes before xlen passes kPatchXCap
-    std::vector<int> pt_xlo, pt_xlen;
     std::vector<int> pc_ptr, pc_list;    // patches grouped by patch colour
     // per-patch incidence lists: for patch p, at incl[pt_inc[p]] the list
     // starts (pnd + 1 entries) of each local dof, then the staged product
@@ -133,7 +130,7 @@ struct MvSmem {
     }
 };
 inline size_t mv_smem_bytes(int S, int maxdof, int w) { return MvSmem(S, maxdof, w).total; }
-constexpr int kPatchXCap = 1792;       // largest x segment of a 3x3 patch (entries)
+constexpr int kPatchXCap = 1792;       // widest range of internal indices of a 3x3 patch
 constexpr int kPatchMaxLocalColours = 16;
 constexpr int kPatchColStride = kPatchMaxLocalColours + 1;
 
@@ -147,7 +144,6 @@ int matrix_bandwidth(int n, const int *IA, const int *JA);
 
 // ------------------------------------------------------------ device layout
 constexpr int kMaxColours = 64;
-constexpr int kElemChunk = 1024;   // elements per matvec work item
 constexpr int kMaxParts = 1024;    // dof parts (reduction partials) per system
 // Dofs per part of the Krylov dof kernels, chosen per batch (unless the
 // autotuner cached a choice): 2 sqrt(batch dofs) up to 64k dofs, 4 sqrt above,

@@ -53,13 +53,6 @@ __device__ __forceinline__ float warp_sum(float v)
 template <typename T> __device__ __forceinline__ T ldst(const T *p) { return __ldcs(p); }
 
 
-// Gate of a kernel: 0 = system live, 1 = inside an Arnoldi cycle, < 0 = always.
-__device__ __forceinline__ bool gated(const SysDev &D, int gate)
-{
-    if (gate < 0) return true;
-    return gate == 0 ? D.st->live != 0 : D.st->in_cycle != 0;
-}
-
 // Last-part election: returns true in the CTA that completed the final part
 // of system D (`split` CTAs a part) for counter slot `slot` (all threads of the
 // CTA agree).
@@ -108,14 +101,6 @@ __device__ __forceinline__ void reduce_parts(const SysDev &D, int nv, double *ou
     __syncthreads();
 }
 
-// A matvec input entry in the arithmetic type: an FP16 basis vector is
-// stored as sigma v, so it is scaled back (exactly: sigma is a power of two).
-template <typename TA, typename TX> __device__ __forceinline__ TA in_value(TX v, const SysDev &D)
-{
-    if constexpr (std::is_same<TX, __half>::value) return (TA)(__half2float(v) * D.vsci);
-    else return (TA)v;
-}
-
 // ---------------------------------------------------------------- EBE matvec
 // y[lm] += A_e x[lm] by patches.  A patch is up to patch_elems(S)
 // consecutive elements (internal order: sorted by their smallest dof, so a
@@ -123,10 +108,8 @@ template <typename TA, typename TX> __device__ __forceinline__ TA in_value(TX v,
 // their launch (one launch per patch colour); per patch:
 //  1. x of the patch's dofs is gathered into shared memory;
 //  2. the element products A_e x_e are formed and staged in shared memory
-//     with the elements' local indices, one thread per element (S = 3: each
-//     thread loads its four elements' blocks at once, before step 1, so a
-//     whole patch of loads is in flight); A and lm16 are SoA
-//     [entry][element], so lane-consecutive elements read consecutive
+//     with the elements' local indices, one thread per element; A and lm16 are
+//     SoA [entry][element], so lane-consecutive elements read consecutive
 //     addresses;
 //  3. the staged rows are added into a shared-memory y local colour by local
 //     colour (elements of one local colour share no dof: no atomics, a fixed
@@ -135,25 +118,21 @@ template <typename TA, typename TX> __device__ __forceinline__ TA in_value(TX v,
 //     shared with other patches (patches sharing a dof have different patch
 //     colours and run in different launches, so the updates apply in launch
 //     order, as read-modify-writes would).
-// For 3x3 blocks each thread loads its entries of the patch's dof list
-// with the element data, so the x gather costs one dependent round trip and
-// the write-back none.
+// (3x3 blocks: k_ebe_mv3.)
 // The patch sizes (patch_elems) and this kernel shape were chosen by a
 // measured sweep: an L2 prefetch of the next patch, one thread per block
 // row with small patches, and a two-stage copy pipeline through shared
 // memory were all slower.  The sink (index n) is never written.
-// in_sel: 0 = x (FP64), 1 = V[step] (T), 2 = aux (TX); out_sel: 0 = t64,
-// 1 = t, 2 = aux.
-template <int S, typename TA, typename TX, typename TY>
-__global__ void __launch_bounds__(kThreads, S == 3 ? (sizeof(TA) == 4 ? 3 : 2) : (sizeof(TA) == 4 ? 4 : 3))
+// x and y are FP64; fg_matvec and fg_matvec_noalloc use these (the Krylov engine
+// has the assembled operator, rows.cu).
+template <int S, typename TA>
+__global__ void __launch_bounds__(kThreads, sizeof(TA) == 4 ? 4 : 3)
 k_ebe_mv(const SysDev *__restrict__ sys, const EChunk *__restrict__ ch, const int *__restrict__ nch,
-         int gate, int in_sel, int out_sel, int step, const TX *aux_in, TY *aux_out, int maxdof)
+         const double *__restrict__ X, double *Y, int maxdof)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     constexpr unsigned short kSink = 0xFFFF;
     constexpr int PE = patch_elems(S);
-    constexpr int E = S == 3 ? PE / kThreads : 1;        // S = 3: elements per thread
-    constexpr int DMAX = S == 3 ? 1536 / kThreads : 1;  // S = 3: patch dofs per thread (the patch cap)
     const MvSmem L(S, maxdof, (int)sizeof(TA));
     TA *xs = reinterpret_cast<TA *>(smem_raw + L.xs);
     TA *ys = reinterpret_cast<TA *>(smem_raw + L.ys);
@@ -163,89 +142,33 @@ k_ebe_mv(const SysDev *__restrict__ sys, const EChunk *__restrict__ ch, const in
     for (int c = blockIdx.x; c < total; c += gridDim.x) {
         const EChunk k = ch[c];
         const SysDev &D = sys[k.sys];
-        if (!gated(D, gate)) continue;
-        const TX *X = in_sel == 0 ? (const TX *)D.x
-                    : in_sel == 1 ? (const TX *)D.V + (size_t)step * D.n_pad
-                    : in_sel == 3 ? (const TX *)D.r64 : aux_in;
-        TY *Y = out_sel == 0 ? (TY *)D.t64 : out_sel == 1 ? (TY *)D.t : aux_out;
         const TA *A = sizeof(TA) == 8 ? (const TA *)D.A64 : (const TA *)D.A32;
         const size_t ld = (size_t)D.nel_pad;
         const int p = k.e0;
         const int pe0 = D.pt_elem[p], pne = D.pt_elem[p + 1] - pe0;
         const int pd0 = D.pt_dof[p], pnd = D.pt_dof[p + 1] - pd0;
         const unsigned short *pc = D.pt_col + (size_t)p * kPatchColStride;
-
-        TA av[E][S == 3 ? 9 : 1];
-        unsigned short li[E][S == 3 ? 3 : 1];
-        int dv[DMAX];                         // S = 3: this thread's entries of the patch's dof list
-        if constexpr (S == 3) {
-#pragma unroll
-            for (int u = 0; u < DMAX; ++u) {
-                const int j = threadIdx.x + u * kThreads;
-                dv[u] = j < pnd ? __ldg(D.dofs + pd0 + j) : 0;
-            }
-        }
-        if constexpr (S == 3) {
-#pragma unroll
-            for (int u = 0; u < E; ++u) {
-                const int q = min(threadIdx.x + u * kThreads, pne - 1);
-#pragma unroll
-                for (int a = 0; a < 3; ++a) li[u][a] = __ldcs(D.lm16 + a * ld + pe0 + q);
-#pragma unroll
-                for (int m = 0; m < 9; ++m) av[u][m] = ldst(A + m * ld + pe0 + q);
-            }
-        }
         __syncthreads();                      // the previous patch is done with shared memory
-        if constexpr (S == 3) {
-#pragma unroll
-            for (int u = 0; u < DMAX; ++u) {
-                const int j = threadIdx.x + u * kThreads;
-                if (j < pnd) {
-                    xs[j] = in_value<TA>(X[dv[u] & 0x7fffffff], D);
-                    ys[j] = (TA)0;
-                }
-            }
-        } else {
-            for (int j = threadIdx.x; j < pnd; j += kThreads) {
-                xs[j] = in_value<TA>(X[D.dofs[pd0 + j] & 0x7fffffff], D);
-                ys[j] = (TA)0;
-            }
+        for (int j = threadIdx.x; j < pnd; j += kThreads) {
+            xs[j] = (TA)X[D.dofs[pd0 + j] & 0x7fffffff];
+            ys[j] = (TA)0;
         }
         __syncthreads();
-        if constexpr (S == 3) {
+        for (int q = threadIdx.x; q < pne; q += kThreads) {
+            unsigned short l[S];
+            TA xv[S];
 #pragma unroll
-            for (int u = 0; u < E; ++u) {
-                const int q = threadIdx.x + u * kThreads;
-                if (q >= pne) continue;
-                TA xv[3];
-#pragma unroll
-                for (int a = 0; a < 3; ++a) xv[a] = li[u][a] == kSink ? (TA)0 : xs[li[u][a]];
-#pragma unroll
-                for (int r = 0; r < 3; ++r) {
-                    TA acc = av[u][3 * r] * xv[0];
-                    acc += av[u][3 * r + 1] * xv[1];
-                    acc += av[u][3 * r + 2] * xv[2];
-                    ye[r * PE + q] = acc;
-                    ls[r * PE + q] = li[u][r];
-                }
+            for (int a = 0; a < S; ++a) {
+                l[a] = __ldcs(D.lm16 + a * ld + pe0 + q);
+                xv[a] = l[a] == kSink ? (TA)0 : xs[l[a]];
             }
-        } else {
-            for (int q = threadIdx.x; q < pne; q += kThreads) {
-                unsigned short l[S];
-                TA xv[S];
 #pragma unroll
-                for (int a = 0; a < S; ++a) {
-                    l[a] = __ldcs(D.lm16 + a * ld + pe0 + q);
-                    xv[a] = l[a] == kSink ? (TA)0 : xs[l[a]];
-                }
+            for (int r = 0; r < S; ++r) {
+                TA acc = ldst(A + (size_t)(r * S) * ld + pe0 + q) * xv[0];
 #pragma unroll
-                for (int r = 0; r < S; ++r) {
-                    TA acc = ldst(A + (size_t)(r * S) * ld + pe0 + q) * xv[0];
-#pragma unroll
-                    for (int m = 1; m < S; ++m) acc += ldst(A + (size_t)(r * S + m) * ld + pe0 + q) * xv[m];
-                    ye[r * PE + q] = acc;
-                    ls[r * PE + q] = l[r];
-                }
+                for (int m = 1; m < S; ++m) acc += ldst(A + (size_t)(r * S + m) * ld + pe0 + q) * xv[m];
+                ye[r * PE + q] = acc;
+                ls[r * PE + q] = l[r];
             }
         }
         __syncthreads();
@@ -264,20 +187,12 @@ k_ebe_mv(const SysDev *__restrict__ sys, const EChunk *__restrict__ ch, const in
         // a dof shared with other patches takes a reduction store (no round
         // trip); the patches of one launch share no dof, so each update is
         // Y[d] + v in launch order, as a read-modify-write would be
-        auto put = [&](int j, int dd) {
+        for (int j = threadIdx.x; j < pnd; j += kThreads) {
+            const int dd = D.dofs[pd0 + j];
             const int d = dd & 0x7fffffff;
-            if (d == D.n) return;                         // dof-list padding
-            if (dd < 0) atomicAdd(Y + d, (TY)ys[j]);
-            else Y[d] = (TY)ys[j];
-        };
-        if constexpr (S == 3) {
-#pragma unroll
-            for (int u = 0; u < DMAX; ++u) {
-                const int j = threadIdx.x + u * kThreads;
-                if (j < pnd) put(j, dv[u]);
-            }
-        } else {
-            for (int j = threadIdx.x; j < pnd; j += kThreads) put(j, D.dofs[pd0 + j]);
+            if (d == D.n) continue;                       // dof-list padding
+            if (dd < 0) atomicAdd(Y + d, (double)ys[j]);
+            else Y[d] = (double)ys[j];
         }
     }
 }
@@ -312,10 +227,10 @@ template <int S, typename TA> constexpr int mvb_rows()
     constexpr int g = FG_MVB_GROUPS32 > 0 ? FG_MVB_GROUPS32 : 1;
     return sizeof(TA) == 8 ? 1 : (FG_MVB_GROUPS32 > 0 && S > 3 && S % g == 0) ? S / g : 0;
 }
-template <int S, typename TA, typename TX, typename TY>
+template <int S, typename TA>
 __global__ void __launch_bounds__(kMvbThreads, 2)
 k_ebe_mvb(const SysDev *__restrict__ sys, const EChunk *__restrict__ ch, const int *__restrict__ nch,
-          int gate, int in_sel, int out_sel, int step, const TX *aux_in, TY *aux_out, int maxdof)
+          const double *__restrict__ X, double *Y, int maxdof)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     constexpr unsigned short kSink = 0xFFFF;
@@ -329,11 +244,6 @@ k_ebe_mvb(const SysDev *__restrict__ sys, const EChunk *__restrict__ ch, const i
     for (int c = blockIdx.x; c < total; c += gridDim.x) {
         const EChunk k = ch[c];
         const SysDev &D = sys[k.sys];
-        if (!gated(D, gate)) continue;
-        const TX *X = in_sel == 0 ? (const TX *)D.x
-                    : in_sel == 1 ? (const TX *)D.V + (size_t)step * D.n_pad
-                    : in_sel == 3 ? (const TX *)D.r64 : aux_in;
-        TY *Y = out_sel == 0 ? (TY *)D.t64 : out_sel == 1 ? (TY *)D.t : aux_out;
         const TA *A = sizeof(TA) == 8 ? (const TA *)D.A64 : (const TA *)D.A32;
         const size_t ld = (size_t)D.nel_pad;
         const int p = k.e0;
@@ -342,7 +252,7 @@ k_ebe_mvb(const SysDev *__restrict__ sys, const EChunk *__restrict__ ch, const i
         const unsigned short *pc = D.pt_col + (size_t)p * kPatchColStride;
         __syncthreads();                      // the previous patch is done with shared memory
         for (int j = threadIdx.x; j < pnd; j += kMvbThreads) {
-            xs[j] = in_value<TA>(X[D.dofs[pd0 + j] & 0x7fffffff], D);
+            xs[j] = (TA)X[D.dofs[pd0 + j] & 0x7fffffff];
             ys[j] = (TA)0;
         }
         for (int e = threadIdx.x; e < S * pne; e += kMvbThreads) {
@@ -387,8 +297,8 @@ k_ebe_mvb(const SysDev *__restrict__ sys, const EChunk *__restrict__ ch, const i
             const int dd = D.dofs[pd0 + j];
             const int d = dd & 0x7fffffff;
             if (d == D.n) continue;                       // dof-list padding
-            if (dd < 0) atomicAdd(Y + d, (TY)ys[j]);
-            else Y[d] = (TY)ys[j];
+            if (dd < 0) atomicAdd(Y + d, (double)ys[j]);
+            else Y[d] = (double)ys[j];
         }
     }
 }
@@ -415,12 +325,12 @@ __device__ __forceinline__ void cp_async_wait_all()
 // one shared with other patches (those run in other launches, so the updates
 // apply in launch order).  Two barriers per patch; every thread sums whole
 // dofs, so no shared-memory y and no colour passes.
-template <typename TA, typename TX, typename TY>
+template <typename TA>
 // FP32: 64 registers, 4 CTAs per SM (56 bytes of spills; measured 3.78 vs
 // 3.72 TB/s at 80 registers and 3 CTAs)
 __global__ void __launch_bounds__(kThreads, sizeof(TA) == 4 ? 4 : 2)
 k_ebe_mv3(const SysDev *__restrict__ sys, const EChunk *__restrict__ ch, const int *__restrict__ nch,
-          int gate, int in_sel, int out_sel, int step, const TX *aux_in, TY *aux_out, int maxdof)
+          const double *__restrict__ X, double *Y, int maxdof)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     constexpr unsigned short kSink = 0xFFFF;
@@ -435,11 +345,6 @@ k_ebe_mv3(const SysDev *__restrict__ sys, const EChunk *__restrict__ ch, const i
     for (int c = blockIdx.x; c < total; c += gridDim.x) {
         const EChunk k = ch[c];
         const SysDev &D = sys[k.sys];
-        if (!gated(D, gate)) continue;
-        const TX *X = in_sel == 0 ? (const TX *)D.x
-                    : in_sel == 1 ? (const TX *)D.V + (size_t)step * D.n_pad
-                    : in_sel == 3 ? (const TX *)D.r64 : aux_in;
-        TY *Y = out_sel == 0 ? (TY *)D.t64 : out_sel == 1 ? (TY *)D.t : aux_out;
         const TA *A = sizeof(TA) == 8 ? (const TA *)D.A64 : (const TA *)D.A32;
         const size_t ld = (size_t)D.nel_pad;
         const int p = k.e0;
@@ -473,7 +378,7 @@ k_ebe_mv3(const SysDev *__restrict__ sys, const EChunk *__restrict__ ch, const i
 #pragma unroll
         for (int u = 0; u < DMAX; ++u) {
             const int j = threadIdx.x + u * kThreads;
-            if (j < pnd) xs[j] = in_value<TA>(X[dv[u] & 0x7fffffff], D);
+            if (j < pnd) xs[j] = (TA)X[dv[u] & 0x7fffffff];
         }
         __syncthreads();
 #pragma unroll
@@ -502,8 +407,8 @@ k_ebe_mv3(const SysDev *__restrict__ sys, const EChunk *__restrict__ ch, const i
             const int e0 = ic[j], e1 = ic[j + 1];
             TA v = (TA)0;
             for (int e = e0; e < e1; ++e) v += ye[ic[head + e]];
-            if (dd < 0) atomicAdd(Y + d, (TY)v);          // shared dof: reduction store
-            else Y[d] = (TY)v;
+            if (dd < 0) atomicAdd(Y + d, (double)v);          // shared dof: reduction store
+            else Y[d] = (double)v;
         }
     }
 }
@@ -513,32 +418,27 @@ k_ebe_mv3(const SysDev *__restrict__ sys, const EChunk *__restrict__ ch, const i
 // (W = 4, 8 or 32 from the mean row length; rows of P1 transport hold ~7
 // entries, rows of the 4-dof Euler system ~30): lanes stride the row,
 // shuffle-reduce, one lane stores.  Works on dof parts like the Krylov
-// kernels; same in/out selection as k_ebe_mv.
-template <int W, typename TA, typename TX, typename TY>
+// kernels (fg_matvec; solves use the assembled blocks, rows.cu).
+template <int W, typename TA>
 __global__ void __launch_bounds__(kThreads)
 k_csr_mv(const SysDev *__restrict__ sys, const DChunk *__restrict__ ch, const int *__restrict__ nch,
-         int gate, int in_sel, int out_sel, int step, const TX *aux_in, TY *aux_out)
+         const double *__restrict__ X, double *Y)
 {
     const int total = *nch;
     const int sub = threadIdx.x % W, grp = threadIdx.x / W, ngrp = blockDim.x / W;
     for (int c = blockIdx.x; c < total; c += gridDim.x) {
         const DChunk k = ch[c];
         const SysDev &D = sys[k.sys];
-        if (!gated(D, gate)) continue;
-        const TX *X = in_sel == 0 ? (const TX *)D.x
-                    : in_sel == 1 ? (const TX *)D.V + (size_t)step * D.n_pad
-                    : in_sel == 3 ? (const TX *)D.r64 : aux_in;
-        TY *Y = out_sel == 0 ? (TY *)D.t64 : out_sel == 1 ? (TY *)D.t : aux_out;
         const TA *AA = sizeof(TA) == 8 ? (const TA *)D.AA64 : (const TA *)D.AA32;
         for (int base = k.d0; base < k.d1; base += ngrp) {
             const int row = base + grp;
             TA s = 0;
             if (row < k.d1)
                 for (int q = D.csr_ia[row] + sub; q < D.csr_ia[row + 1]; q += W)
-                    s += ldst(AA + q) * in_value<TA>(X[__ldcs(D.csr_ja + q)], D);
+                    s += ldst(AA + q) * (TA)X[__ldcs(D.csr_ja + q)];
 #pragma unroll
             for (int o = W / 2; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o, W);
-            if (row < k.d1 && sub == 0) Y[row] = (TY)s;
+            if (row < k.d1 && sub == 0) Y[row] = (double)s;
         }
     }
 }
@@ -765,31 +665,31 @@ int sm_count()
 namespace {
 
 // the matvec kernel of an S x S launch: 3x3, the pair kernel, or per element
-template <int S, typename TA, typename TX, typename TY, bool PAIRS>
+template <int S, typename TA, bool PAIRS>
 static auto pick_mv()
 {
-    if constexpr (S == 3) return k_ebe_mv3<TA, TX, TY>;
-    else if constexpr (PAIRS && mvb_rows<S, TA>() > 0) return k_ebe_mvb<S, TA, TX, TY>;
-    else return k_ebe_mv<S, TA, TX, TY>;
+    if constexpr (S == 3) return k_ebe_mv3<TA>;
+    else if constexpr (PAIRS && mvb_rows<S, TA>() > 0) return k_ebe_mvb<S, TA>;
+    else return k_ebe_mv<S, TA>;
 }
 
 struct MvLaunch {
     // Persistent CTAs: as many as fit on the GPU (their dynamic shared memory,
     // mv_smem_bytes, decides how many per SM), at most one per patch.
-    template <typename TA, typename TX, typename TY>
+    template <typename TA>
     static void go(int S, int nitems, cudaStream_t st, const SysDev *sys, const EChunk *ch, const int *nch,
-                   int gate, int in_sel, int out_sel, int step, const TX *ai, TY *ao, int maxdof)
+                   const double *x, double *y, int maxdof)
     {
         switch (S) {
-        case 3: run<3, TA, TX, TY>(nitems, st, sys, ch, nch, gate, in_sel, out_sel, step, ai, ao, maxdof); break;
-        case 6: run<6, TA, TX, TY>(nitems, st, sys, ch, nch, gate, in_sel, out_sel, step, ai, ao, maxdof); break;
-        case 9: run<9, TA, TX, TY>(nitems, st, sys, ch, nch, gate, in_sel, out_sel, step, ai, ao, maxdof); break;
-        case 12: run<12, TA, TX, TY>(nitems, st, sys, ch, nch, gate, in_sel, out_sel, step, ai, ao, maxdof); break;
+        case 3: run<3, TA>(nitems, st, sys, ch, nch, x, y, maxdof); break;
+        case 6: run<6, TA>(nitems, st, sys, ch, nch, x, y, maxdof); break;
+        case 9: run<9, TA>(nitems, st, sys, ch, nch, x, y, maxdof); break;
+        case 12: run<12, TA>(nitems, st, sys, ch, nch, x, y, maxdof); break;
         }
     }
-    template <int S, typename TA, typename TX, typename TY>
-    static void run(int nitems, cudaStream_t st, const SysDev *sys, const EChunk *ch, const int *nch, int gate,
-                    int in_sel, int out_sel, int step, const TX *ai, TY *ao, int maxdof)
+    template <int S, typename TA>
+    static void run(int nitems, cudaStream_t st, const SysDev *sys, const EChunk *ch, const int *nch, const double *x,
+                    double *y, int maxdof)
     {
         const size_t smem = mv_smem_bytes(S, maxdof, sizeof(TA));
         // FP64 S x S blocks: a thread per (element, row) (the FP64 pipe wants
@@ -801,7 +701,7 @@ struct MvLaunch {
         // (~1170 a launch) 3.23 -> 2.83 TB/s; both give the same sums
         constexpr bool can_pair = S > 3 && mvb_rows<S, TA>() > 0;
         const bool pairs = can_pair && nitems <= 6 * sm_count();
-        auto kern = pairs ? pick_mv<S, TA, TX, TY, true>() : pick_mv<S, TA, TX, TY, false>();
+        auto kern = pairs ? pick_mv<S, TA, true>() : pick_mv<S, TA, false>();
         const int nt = pairs ? kMvbThreads : kThreads;
         // the attribute and the occupancy are cached per kernel (last
         // shared-memory size seen); they are host-side queries only
@@ -825,7 +725,7 @@ struct MvLaunch {
             occ = occ_cached[w];
         }
         const int g = std::max(1, std::min(nitems, occ * sm_count()));
-        kern<<<g, nt, smem, st>>>(sys, ch, nch, gate, in_sel, out_sel, step, ai, ao, maxdof);
+        kern<<<g, nt, smem, st>>>(sys, ch, nch, x, y, maxdof);
     }
 };
 
@@ -1492,7 +1392,6 @@ int BatchRun::stage(const BatchMember &m)
     int r = validate_member(s, cfg);
     if (r) return r;
     if ((r = ensure_workspace(s, cfg.kmax, cfg.mixed + cfg.vhalf))) return r;
-    if (s->op == FG_OP_CSR && (r = csr_refresh(s, st))) return r;
     if ((r = rows_refresh(s, cfg.mixed != 0, st))) return r;
     Workspace &w = s->ws;
     size_t vb = 8 * (size_t)s->n_pad;
@@ -1862,13 +1761,13 @@ int matvec_device(fg_system *s, const double *x, double *y, int precision, cudaS
         const DChunk *dcp = dc.as<DChunk>();
         const int *dnp = dn.as<int>();
         if (precision == 32) {
-            if (s->csr_w == 4) k_csr_mv<4, float, double, double><<<g, kThreads, 0, st>>>(sdp, dcp, dnp, -1, 2, 2, 0, x, y);
-            else if (s->csr_w == 8) k_csr_mv<8, float, double, double><<<g, kThreads, 0, st>>>(sdp, dcp, dnp, -1, 2, 2, 0, x, y);
-            else k_csr_mv<32, float, double, double><<<g, kThreads, 0, st>>>(sdp, dcp, dnp, -1, 2, 2, 0, x, y);
+            if (s->csr_w == 4) k_csr_mv<4, float><<<g, kThreads, 0, st>>>(sdp, dcp, dnp, x, y);
+            else if (s->csr_w == 8) k_csr_mv<8, float><<<g, kThreads, 0, st>>>(sdp, dcp, dnp, x, y);
+            else k_csr_mv<32, float><<<g, kThreads, 0, st>>>(sdp, dcp, dnp, x, y);
         } else {
-            if (s->csr_w == 4) k_csr_mv<4, double, double, double><<<g, kThreads, 0, st>>>(sdp, dcp, dnp, -1, 2, 2, 0, x, y);
-            else if (s->csr_w == 8) k_csr_mv<8, double, double, double><<<g, kThreads, 0, st>>>(sdp, dcp, dnp, -1, 2, 2, 0, x, y);
-            else k_csr_mv<32, double, double, double><<<g, kThreads, 0, st>>>(sdp, dcp, dnp, -1, 2, 2, 0, x, y);
+            if (s->csr_w == 4) k_csr_mv<4, double><<<g, kThreads, 0, st>>>(sdp, dcp, dnp, x, y);
+            else if (s->csr_w == 8) k_csr_mv<8, double><<<g, kThreads, 0, st>>>(sdp, dcp, dnp, x, y);
+            else k_csr_mv<32, double><<<g, kThreads, 0, st>>>(sdp, dcp, dnp, x, y);
         }
         FG_CUDA(cudaGetLastError());
         count_launches(1);
@@ -1880,9 +1779,9 @@ int matvec_device(fg_system *s, const double *x, double *y, int precision, cudaS
         const EChunk *cp = ch.as<EChunk>() + off[c];
         const int *np = cnt.as<int>() + c;
         if (precision == 32)
-            MvLaunch::go<float, double, double>(t.S, counts[c], st, sd.as<SysDev>(), cp, np, -1, 2, 2, 0, x, y, D.maxdof);
+            MvLaunch::go<float>(t.S, counts[c], st, sd.as<SysDev>(), cp, np, x, y, D.maxdof);
         else
-            MvLaunch::go<double, double, double>(t.S, counts[c], st, sd.as<SysDev>(), cp, np, -1, 2, 2, 0, x, y, D.maxdof);
+            MvLaunch::go<double>(t.S, counts[c], st, sd.as<SysDev>(), cp, np, x, y, D.maxdof);
     }
     FG_CUDA(cudaGetLastError());
     count_launches(t.npcol);
@@ -1952,9 +1851,9 @@ int launch_matvec_colours(int S, int precision, const SysDev *sys_dev, const ECh
         const EChunk *cp = ch_dev + off_host[c];
         const int *np = counts_dev + c;
         if (precision == 32)
-            MvLaunch::go<float, double, double>(S, cnt, st, sys_dev, cp, np, -1, 2, 2, 0, x, y, maxdof);
+            MvLaunch::go<float>(S, cnt, st, sys_dev, cp, np, x, y, maxdof);
         else
-            MvLaunch::go<double, double, double>(S, cnt, st, sys_dev, cp, np, -1, 2, 2, 0, x, y, maxdof);
+            MvLaunch::go<double>(S, cnt, st, sys_dev, cp, np, x, y, maxdof);
         count_launches(1);
     }
     FG_CUDA(cudaGetLastError());

@@ -390,8 +390,6 @@ int build_topology(Topology &t, int nnodes, int nel, int ndof, const int *ien,
     t.eorder.resize(nel);
     t.pt_elem.clear();
     t.pt_dof.clear();
-    t.pt_xlo.clear();
-    t.pt_xlen.clear();
     t.pt_col.clear();
     t.dofs.clear();
     t.maxdof = 0;
@@ -399,9 +397,11 @@ int build_topology(Topology &t, int nnodes, int nel, int ndof, const int *ien,
     std::vector<uint32_t> lmask;   // per local dof: local colours used
     for (int b = 0, p = 0; b < nact; ++p) {
         // local dofs of the patch, ascending internal index; a 3x3 patch also
-        // keeps its dofs inside one x segment of at most kPatchXCap entries
-        // (8-aligned ends): past that it goes back to its last 16-element
-        // boundary
+        // keeps its dofs inside one segment of at most kPatchXCap internal
+        // indices (8-aligned ends): past that it goes back to its last 16-element
+        // boundary.  (No kernel copies the segment any more; the cut stays
+        // because it sets the order of fg_matvec's sums and which numberings
+        // are refused.)
         std::vector<int> pd;
         int e = b, lo = n, hi = -1;
         size_t keep_pd = 0;
@@ -434,8 +434,6 @@ int build_topology(Topology &t, int nnodes, int nel, int ndof, const int *ien,
         t.pt_col.resize((size_t)(p + 1) * kPatchColStride, 0);
         t.pt_dof.push_back(0);
         std::sort(pd.begin(), pd.end());
-        t.pt_xlo.push_back(pd.front() & ~7);
-        t.pt_xlen.push_back(((pd.back() + 1 + 7) & ~7) - (pd.front() & ~7));
         for (size_t j = 0; j < pd.size(); ++j) { local[pd[j]] = (int)j; owner_count[pd[j]]++; }
         // greedy local colouring in patch order
         lmask.assign(pd.size(), 0u);
@@ -598,9 +596,7 @@ int build_topology(Topology &t, int nnodes, int nel, int ndof, const int *ien,
             const int pd0 = t.pt_dof[p], pnd = t.pt_dof[p + 1] - pd0;
             const int i0 = S == 3 ? t.pt_inc[p] : 0, ni = S == 3 ? t.pt_inc[p + 1] - i0 : 0;
             if (pe0 % 16 || pne < 1 || pne > PE || pe0 + (pne + 15) / 16 * 16 > nel_pad || pd0 % 4 || pnd % 4 ||
-                pnd < 1 || pnd > dcap || i0 % 8 || ni % 8 || ni > icap ||
-                (S == 3 && (t.pt_xlo[p] % 8 || t.pt_xlen[p] % 8 || t.pt_xlen[p] < 8 || t.pt_xlen[p] > kPatchXCap ||
-                            t.pt_xlo[p] + t.pt_xlen[p] > (n + 1 + 31) / 32 * 32))) {
+                pnd < 1 || pnd > dcap || i0 % 8 || ni % 8 || ni > icap) {
                 set_error("internal: matvec patch layout out of its bounds");
                 return FG_ERR_UNSUPPORTED;
             }
