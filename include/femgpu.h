@@ -305,8 +305,10 @@ void *fg_system_stream(const fg_system *s);
  * matvecs (the assembled operator) of V[0] into a work vector, in FP64
  * (precision 64) or FP32 (32), timed with CUDA events on the first
  * system's stream.  *ms_per_matvec receives the mean; *bytes the
- * algorithmic bytes of one matvec: slots*(ndof*ndof*w + 4) + 2*n*w summed
- * over the systems (slots: coupled node pairs, one column each).  Requires a previous solve (workspace) on every system. */
+ * algorithmic bytes of one matvec: slots*(ndof*ndof*w + c) + 2*n*w summed
+ * over the systems (slots: coupled node pairs, one column each of c = 2 bytes
+ * where all couplings lie within 2^15 units, else 4).  Requires a previous
+ * solve (workspace) on every system. */
 int fg_bench_matvec(fg_system *const *systems, int count, int precision, int reps,
                     double *ms_per_matvec, double *bytes);
 

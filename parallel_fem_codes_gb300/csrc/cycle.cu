@@ -38,8 +38,9 @@
 // exchange that follows its reading.
 //
 // Measured (GB300), a whole solve with the pass kernels -> on chip, and an
-// Arnoldi step: 961 equations FP64 8.8 -> 1.9 ms (6 us a step), 16k FP64 26.5 ->
-// 5.8 ms (7 us), 16k FP32 21.9 -> 4.2 ms (5 us), 261k FP32 94 -> 24 ms (9 us).
+// Arnoldi step: 961 equations FP64 8.8 -> 2.0 ms (6 us a step), 16k FP64 26.5 ->
+// 6.3 ms (7 us), 16k FP32 21.9 -> 4.5 ms (5 us), 261k FP32 94 -> 27 ms (9.5 us).
+// (The same build differs by up to 8 % between processes and machines.)
 // What is left of a step is mostly the two trips through L2 of the exchange
 // (2 to 5 us with the CTAs' skew); the basis sweeps take 2 to 3 us.
 //
@@ -79,8 +80,8 @@ static_assert(kMaxRestart <= kGroups, "a group for every basis vector");
 __device__ __forceinline__ int dot_slices(int np, int nv) { return max(1, min(min(kMaxSlices, np / 64), kGroups / nv)); }
 constexpr long long kPollCycles = 4000000000LL;   // ~2 s
 __device__ int g_gang_polls = 1 << 24;            // fg_set_wait_limit
-// gangs up to this size sum all partials in every CTA
-// (129 x 129 FP32, 32 CTAs: 5.3 ms a solve in two trips, 6.4 ms in one)
+// gangs up to this size sum all partials in every CTA (16k equations FP32 in the
+// 32 CTAs of an earlier row count, 64 now: 5.3 ms a solve in two trips, 6.4 in one)
 constexpr int kDirect32 = 8, kDirect64 = 8;
 
 template <typename T> struct Pack { static constexpr int N = 16 / sizeof(T); };
@@ -882,6 +883,11 @@ Residency residency(int B, bool f64, bool spill = false)
 // solve; with 128 / 96 / 64 rows FP64: 961 equations 2.02 / 1.99 / 1.89, a
 // four-step process of 9k 19.1 / 17.0 / 18.2, 16k 5.62 / 5.69 / 5.69, Euler with
 // 4k nodes 5.02 / 4.71 / 4.73; with 32 rows 961 equations 1.87, 9k 19.9.
+// The halo needs no bound but its room: multi-dof meshes keep their node order, and
+// with nodes numbered at random, where every CTA polls the whole newest vector, a step
+// on chip / streaming takes FP64 (FP32) at 65 x 65 nodes of 2 dofs 17 / 32 us (13 / 29), of
+// 3 25 / 35 (15 / 30), of 4 26 / 42 (16 / 36), at 129 x 129 of 2 FP32 25 / 35; larger ones
+// have no room and stream.
 static int gang_want(const fg_system *s, bool f64)
 {
     return f64 ? std::max(64, (int)std::sqrt((double)s->topo.nunits)) : 256;

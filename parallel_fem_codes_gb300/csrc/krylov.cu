@@ -797,11 +797,10 @@ static bool tuned_choice(const std::vector<BatchMember> &mem, const SolveConfig 
 
 namespace {
 
-// part size of a batch (multiple of 8 dofs): the tuned one, else
-// 2 sqrt(batch dofs) up to 64k dofs and 4 sqrt above (where a part's sums are
+// part size of a batch (multiple of 8 dofs): the tuned one, else kPartMin below
+// kSoloDofs, 2 sqrt(batch dofs) up to 64k dofs and 4 sqrt above (where a part's sums are
 // split among CTAs), rounded to the nearest power of two, within [kPartMin,
-// kPartMax] (powers of two: a system solved alone and inside a batch of similar
-// size get the same parts, hence bit-identical results).  A batch that gives
+// kPartMax].  A batch that gives
 // every resident CTA (3 an SM; FP64, which splits the sums, 4) a part of 1024 dofs
 // (a pass of its threads) takes the smallest multiple of that with which the
 // parts fill whole rounds of CTAs: 4.0 M dofs FP32 on 152 SMs, a step with 8192
