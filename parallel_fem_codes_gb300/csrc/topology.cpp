@@ -219,17 +219,18 @@ static int build_rows(Topology &t, const std::vector<int> &IB, const std::vector
     const int ns = (nu + kRowSlice - 1) / kRowSlice;
     t.rw_off.assign(ns + 1, 0);
     long long slots = 0;
+    constexpr long long kMaxSlots = 0x7fffffffLL - 64 * kRowSlice;   // the matvec's 32-bit steps run past the last slot
     for (int s = 0; s < ns; ++s) {
         int w = 0;
         for (int u = s * kRowSlice; u < std::min(nu, (s + 1) * kRowSlice); ++u) w = std::max(w, P[u + 1] - P[u]);
         slots += (long long)w * kRowSlice;
-        if (slots > 0x7fffffffLL) { set_error("the operator's pattern has more entries than 32 bits count"); return FG_ERR_UNSUPPORTED; }
+        if (slots > kMaxSlots) { set_error("the operator's pattern has more entries than 32 bits count"); return FG_ERR_UNSUPPORTED; }
         t.rw_off[s + 1] = (int)slots;
         t.rw_w = std::max(t.rw_w, w);
     }
     // one width for all where that pads little: the matvec then needs no offset
     const long long wide = (long long)ns * t.rw_w * kRowSlice;
-    if (wide <= 0x7fffffffLL && 8 * (wide - slots) <= slots) {
+    if (wide <= kMaxSlots && 8 * (wide - slots) <= slots) {
         t.rw_u = t.rw_w;
         for (int s = 0; s < ns; ++s) t.rw_off[s + 1] = (s + 1) * t.rw_w * kRowSlice;
     }
