@@ -1682,7 +1682,7 @@ void fill_stats(const SysState &s, double secs, fg_solve_stats &o)
     o.seconds = secs;
 }
 
-int solve_batch(std::vector<BatchMember> &mem, const SolveConfig &cfg, fg_solve_stats *stats, cudaStream_t st)
+static int run_batch(std::vector<BatchMember> &mem, const SolveConfig &cfg, fg_solve_stats *stats, cudaStream_t st)
 {
     if (mem.empty()) return FG_OK;
     for (auto &m : mem) {
@@ -1715,6 +1715,14 @@ int solve_batch(std::vector<BatchMember> &mem, const SolveConfig &cfg, fg_solve_
     if (stats)
         for (size_t i = 0; i < mem.size(); ++i) fill_stats(sts[i], secs, stats[i]);
     return FG_OK;
+}
+
+int solve_batch(std::vector<BatchMember> &mem, const SolveConfig &cfg, fg_solve_stats *stats, cudaStream_t st)
+{
+    const int r = run_batch(mem, cfg, stats, st);
+    // copies from the caller's vectors and values of members whose own streams know nothing of st
+    if (r) cudaStreamSynchronize(st);
+    return r;
 }
 
 // Single matvec on device vectors (internal numbering, FP64 in/out).
